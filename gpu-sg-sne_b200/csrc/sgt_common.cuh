@@ -50,9 +50,10 @@ struct SgtState {
   float h_eff;       // grid spacing in embedding units
   int N;             // grid points per axis (n1 + 2)
   int M;             // FFT length per axis (2^k or 3 * 2^k, >= 2N-1)
-  int T;             // tile edge in cells
-  int tiles_dim;     // tiles per axis
+  int T;             // 0: scatter mode, 1: cell mode
+  int tiles_dim;     // cell mode: cells per axis and in all
   int ntiles;
+  int copies;        // scatter mode: copies of the grid (a power of two)
   int nchunks;
   int chunk;         // points per chunk
   int grid_clamped;  // 1 if N was clamped to the allocated FFT size
@@ -86,17 +87,11 @@ struct SgtJobParams {
   int mom_switch;     // last iteration (inclusive) using momentum 0.5
   float eta;
   int mmax;           // largest FFT length per axis allocated
-  int tile_cap;       // max tiles held by the tile arrays
+  long vc_nodes;      // nodes held by the grid copies of the scatter mode
   int chunk_cap;      // max chunks held by the chunk array
   int chunk_min;      // fewest points per S2G chunk (0: 1024, 256 in 3-D)
-  int direct_max;     // largest N of a direct-mode grid (0: no direct mode)
+  int cell_blocks;    // blocks that work in cell mode (0: no cell mode)
 };
-
-// Direct mode (d <= 2): S2G and G2S work on the points in their own order
-// with the whole grid in shared memory, without the tile sort, on grids that
-// are not dense enough for cell mode.  2-D grids up to this many points per
-// axis (64^2 float4 nodes = 64 KB); 1-D grids always.
-#define SGT_DIRECT_N2 64
 
 template <int D> struct Vec;
 template <> struct Vec<1> { typedef float T; };

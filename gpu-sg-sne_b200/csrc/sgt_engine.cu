@@ -86,6 +86,7 @@ struct sgt_job {
         *Frep = nullptr, *Fattr = nullptr;
   float4 *sorted = nullptr;
   float *V = nullptr, *Phi = nullptr;
+  float *Vc = nullptr;  // grid copies of the scatter mode; zero between iterations
   float2 *W = nullptr;
   int mmax = 0, nmax = 0;
   int *tile_count = nullptr, *cursor = nullptr;
@@ -94,12 +95,10 @@ struct sgt_job {
   double *part_sum = nullptr, *part_z = nullptr, *part_kl = nullptr;
   SgtState *st = nullptr;
   SgtState *st_host = nullptr;
-  int nb_pts = 0, nb_bin = 0, nb_s2g = 0, nb_s2gc = 0, nb_g2s = 0, nb_fft = 0, nb_fft_rows = 0, nb_row = 0,
+  int nb_pts = 0, nb_scat = 0, nb_gath = 0, nb_fold = 0, nb_s2gc = 0, nb_g2s = 0, nb_fft = 0, nb_fft_rows = 0, nb_row = 0,
       nb_upd = 0, nb_part = 0;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;  // the two branches of an iteration
-  size_t smem_s2g = 0, smem_s2g8 = 0, smem_fft1 = 0, smem_fft2 = 0;
-  size_t smem_s2gd = 0, smem_g2sd = 0;  // direct-mode S2G and G2S (0: the job never takes it)
-  int nb_s2g8 = 0;  // 3-D tiles of 8 cells
+  size_t smem_fft1 = 0, smem_fft2 = 0;
   cudaGraphExec_t gexec = nullptr;        // one iteration
   cudaGraphExec_t gexec_multi = nullptr;  // SGT_GRAPH_ITERS chained iterations
   std::vector<void *> allocs;
@@ -167,6 +166,9 @@ static int grid_blocks(int nsm, int per_sm) { return std::max(1, nsm * std::max(
 
 // iterations per launch of a job's chained graph (sgt_job_run)
 #define SGT_GRAPH_ITERS 16
+// nodes of the grid copies a job holds at least (32 copies of a 90^2 grid; the
+// largest 2-D grid once)
+#define SGT_COPY_NODES (1 << 18)
 // nonzeros of P from which a job's repulsion chain runs one block per SM
 #define SGT_CHAIN_NARROW_NNZ 16000000L
 
@@ -399,36 +401,8 @@ static sgt_status job_shapes(sgt_job *J) {
   const int nsm = ctx->nsm;
   int occ = 0;
   J->nb_pts = grid_blocks(nsm, 4);
-  constexpr int T = D == 1 ? 512 : (D == 2 ? 32 : 16);
-  const int R = T + 3;
-  J->smem_s2g = sizeof(float) * (D + 1) * (size_t)(D == 1 ? R : (D == 2 ? R * R : R * R * R));
-  CK(cudaFuncSetAttribute(k_s2g<D, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)J->smem_s2g));
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_s2g<D, T>, SGT_THREADS, J->smem_s2g));
-  J->nb_s2g = grid_blocks(nsm, occ);
-  if constexpr (D == 3) {
-    J->smem_s2g8 = sizeof(float) * 4 * 11 * 11 * 11;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_s2g<3, 8>, SGT_THREADS, J->smem_s2g8));
-    J->nb_s2g8 = grid_blocks(nsm, occ);
-  }
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_s2g_cell<D>, SGT_THREADS, 0));
   J->nb_s2gc = grid_blocks(nsm, occ);
-  // direct mode (d <= 2, jobs that can take it): the S2G's grid copy (m
-  // planes of N^d floats) and the G2S's potential grid (N^d nodes)
-  if constexpr (D <= 2) {
-    const size_t dn = (size_t)J->jp.direct_max;
-    const size_t dnodes = D == 1 ? dn : dn * dn;
-    J->smem_s2gd = sizeof(float) * (D + 1) * dnodes;
-    J->smem_g2sd = sizeof(typename Node<D>::T) * dnodes;
-    // the attributes allow the largest job of this dimension (jobs of other
-    // sizes set them too, and every job's launches must stay allowed)
-    const size_t dmax = D == 1 ? 512 : (size_t)SGT_DIRECT_N2 * SGT_DIRECT_N2;
-    CK(cudaFuncSetAttribute(k_s2g_direct<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)(sizeof(float) * (D + 1) * dmax)));
-    CK(cudaFuncSetAttribute(k_g2s_direct<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)(sizeof(typename Node<D>::T) * dmax)));
-  }
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_g2s<D>, SGT_THREADS, 0));
-  J->nb_g2s = grid_blocks(nsm, occ);
   const int M = J->mmax;
   J->smem_fft1 = 0;
   J->smem_fft2 = fft_cols_smem(M, D);
@@ -461,23 +435,22 @@ static sgt_status job_shapes(sgt_job *J) {
   // so one block per SM (each with more points) finishes sooner than four.
   // 1.3M points (67M nonzeros): 337 against 351 us per iteration; 400k
   // (20M): 114 against 119.
-  J->nb_bin = J->nb_pts;
-  if (J->nnz >= SGT_CHAIN_NARROW_NNZ) {
-    J->nb_bin = std::min(J->nb_bin, nsm);
-    J->nb_s2g = std::min(J->nb_s2g, nsm);
-    J->nb_s2g8 = std::min(J->nb_s2g8, nsm);
-    J->nb_s2gc = std::min(J->nb_s2gc, nsm);
-    J->nb_g2s = std::min(J->nb_g2s, nsm);
+  if (J->jp.cell_blocks > 0) {
+    J->jp.cell_blocks = J->nnz >= SGT_CHAIN_NARROW_NNZ ? nsm : J->nb_pts;
+    J->nb_s2gc = std::min(J->nb_s2gc, J->jp.cell_blocks);
+    J->nb_g2s = J->jp.cell_blocks;
   }
+  // scatter mode: a group of SGT_LPP lanes per point, up to 2048 threads an SM
+  const long groups = ((long)J->n * SGT_LPP(D) + SGT_THREADS - 1) / SGT_THREADS;
+  J->nb_scat = (int)std::min(groups, 8L * nsm);
+  J->nb_gath = (int)std::min(groups, 6L * nsm);
+  J->nb_fold = 2 * nsm;
   // small embeddings launch no more blocks than there is work for: idle
   // blocks only take scheduling slots from the jobs that share the GPU
   const int cap = (int)std::max(1L, ((long)J->n + 255) / 256);
   J->nb_pts = std::min(J->nb_pts, cap);
-  J->nb_bin = std::min(J->nb_bin, cap);
-  J->nb_s2g = std::min(J->nb_s2g, cap);
-  J->nb_s2g8 = std::min(J->nb_s2g8, cap);
+  J->nb_fold = std::min(J->nb_fold, cap);
   J->nb_s2gc = std::min(J->nb_s2gc, cap);
-  J->nb_g2s = std::min(J->nb_g2s, cap);
   J->nb_row = std::min(J->nb_row, cap);
   J->nb_upd = std::min(J->nb_upd, cap);
   if constexpr (D == 2) {  // lines of the largest grid this job can take
@@ -485,7 +458,7 @@ static sgt_status job_shapes(sgt_job *J) {
     J->nb_fft_rows = std::min(J->nb_fft_rows, (lines_rows + 7) / 8);
     J->nb_fft = std::min(J->nb_fft, std::max(1, lines_cols));
   }
-  J->nb_part = std::max(std::max(J->nb_pts, J->nb_row), std::max(J->nb_g2s, J->nb_s2g));
+  J->nb_part = std::max(std::max(J->nb_pts, J->nb_row), std::max(J->nb_g2s, J->nb_gath));
   J->nb_part = std::max(J->nb_part, J->nb_upd);
   return SGT_OK;
 }
@@ -500,7 +473,6 @@ static sgt_status job_alloc(sgt_job *J) {
   CKS(jalloc(J, &J->uY, np));
   CKS(jalloc(J, &J->gains, np));
   CKS(jalloc(J, &J->Frep, np));
-  CKS(jalloc(J, &J->sorted, (size_t)J->n));
   int max_grid = J->p.max_grid > 0 ? J->p.max_grid : (D <= 2 ? 512 : 128);
   // 3-D: at most 256 points per axis (tile histogram of 16^3 entries,
   // FFT planes of 512^3)
@@ -520,21 +492,18 @@ static sgt_status job_alloc(sgt_job *J) {
   if (D >= 2) plane *= M;
   if (D >= 3) plane *= M;
   if (D >= 2) CKS(jalloc(J, &J->W, 3 * plane));
+  J->jp.vc_nodes = (long)std::max(nodes, (size_t)SGT_COPY_NODES);
+  CKS(jalloc(J, &J->Vc, (size_t)J->jp.vc_nodes * ncomp));
+  CK(cudaMemsetAsync(J->Vc, 0, sizeof(float) * (size_t)J->jp.vc_nodes * ncomp, ctx->stream));
   CKS(jalloc(J, &J->tile_count, SGT_HIST_MAX));
   CKS(jalloc(J, &J->cursor, SGT_HIST_MAX));
   J->jp.chunk_cap = J->n / 256 + SGT_HIST_MAX + 16;  // 3-D chunks may hold 256 points
   CKS(jalloc(J, &J->chunks, (size_t)J->jp.chunk_cap));
   J->jp.mmax = M;
-  J->jp.tile_cap = SGT_HIST_MAX;
-  // direct mode for the grids up to direct_max that are too sparse for cell
-  // mode; a job with enough points that all of them are dense never takes it
-  // (and its kernels keep the small shared-memory footprint the concurrent
-  // SpMV wants: the direct mode's grid copies shrink the SMs' L1)
-  J->jp.direct_max = D == 1 ? J->nmax : (D == 2 ? std::min(SGT_DIRECT_N2, J->nmax) : 0);
-  if (J->jp.direct_max > 0) {
-    const long c = J->jp.direct_max - 3, dense = 64L * (D == 1 ? c : c * c);
-    if ((long)J->n >= dense && (D == 1 ? c : c * c) <= SGT_HIST_MAX) J->jp.direct_max = 0;
-  }
+  // the sort of the cell mode, for the jobs that can take it (a shard decides
+  // by the points of the whole embedding); job_shapes sets its block count
+  J->jp.cell_blocks = std::max(J->n, J->n_gather) >= SGT_CELL_MIN_N ? 1 : 0;
+  if (J->jp.cell_blocks > 0) CKS(jalloc(J, &J->sorted, (size_t)J->n));
   CKS(jalloc(J, &J->st, 1));
   J->st_host = new SgtState();
   CK(cudaEventCreateWithFlags(&J->ev_fork, cudaEventDisableTiming));
@@ -642,20 +611,25 @@ static sgt_status enqueue_g2g(sgt_job *J, cudaStream_t s, bool pdl) {
   return SGT_OK;
 }
 
-// Centre Ynext into Y, count points per tile, zero the charge grid.
+// Centre Ynext into Y; scatter mode: S2G into the grid copies, cell mode:
+// count points per cell and zero the charge grid.
 template <int D>
 static sgt_status enqueue_bin_count(sgt_job *J, cudaStream_t s) {
   sgt_ctx *ctx = J->ctx;
   typedef typename Vec<D>::T VT;
   typedef typename Node<D>::T NT;
-  k_bin_count<D><<<J->nb_bin, SGT_THREADS, 0, s>>>((const VT *)J->Ynext, (VT *)J->Y, J->n,
-                                                   J->st, J->tile_count, (NT *)J->V, 1, J->jp,
-                                                   J->cursor, J->chunks, J->nb_s2g);
+  if (J->jp.cell_blocks > 0)
+    k_bin_count<D><<<J->jp.cell_blocks, SGT_THREADS, 0, s>>>(
+        (const VT *)J->Ynext, (VT *)J->Y, J->n, J->st, J->tile_count, (NT *)J->V, J->jp, J->cursor,
+        J->chunks, J->nb_s2gc);
+  k_scatter<D><<<J->nb_scat, SGT_THREADS, 0, s>>>((const VT *)J->Ynext, (VT *)J->Y, J->n, J->st,
+                                                  (NT *)J->Vc);
   CK(cudaGetLastError());
   return SGT_OK;
 }
 
-// Sort and S2G (or the direct S2G): the charge grid of this job's points.
+// The charge grid of this job's points: the sum of the grid copies, or (jobs
+// that can take the cell mode) the sort and the S2G over cells.
 // ev (optional): events recorded after the binning and S2G stages.
 template <int D>
 static sgt_status enqueue_scatter_part(sgt_job *J, cudaStream_t s, cudaEvent_t *ev = nullptr) {
@@ -664,24 +638,15 @@ static sgt_status enqueue_scatter_part(sgt_job *J, cudaStream_t s, cudaEvent_t *
   typedef typename Node<D>::T NT;
   const int n = J->n;
   const bool pdl = ev == nullptr;
-  // the S2G stage starts with the sort (tile modes) or is the whole direct
-  // S2G (direct mode), both in k_bin_scatter
   if (ev) CK(cudaEventRecord(ev[1], s));
-  CK(launch_chain(pdl, k_bin_scatter<D>, J->nb_bin, SGT_THREADS, 0, s, (const VT *)J->Y, n, J->st,
-                  J->cursor, J->sorted));
-  if constexpr (D <= 2)
-    if (J->jp.direct_max > 0)
-      CK(launch_chain(pdl, k_s2g_direct<D>, J->nb_bin, SGT_THREADS, J->smem_s2gd, s,
-                      (const VT *)J->Y, n, J->st, (NT *)J->V));
-  // tile mode and cell mode: the kernel of the other mode returns at once
-  constexpr int TT = D == 1 ? 512 : (D == 2 ? 32 : 16);
-  CK(launch_chain(pdl, k_s2g<D, TT>, J->nb_s2g, SGT_THREADS, J->smem_s2g, s,
-                  (const float4 *)J->sorted, J->st, (const int4 *)J->chunks, (NT *)J->V));
-  if constexpr (D == 3)
-    CK(launch_chain(pdl, k_s2g<3, 8>, J->nb_s2g8, SGT_THREADS, J->smem_s2g8, s,
-                    (const float4 *)J->sorted, J->st, (const int4 *)J->chunks, (NT *)J->V));
-  CK(launch_chain(pdl, k_s2g_cell<D>, J->nb_s2gc, SGT_THREADS, 0, s, (const float4 *)J->sorted,
-                  J->st, (const int4 *)J->chunks, (NT *)J->V));
+  CK(launch_chain(pdl, k_fold<D>, J->nb_fold, SGT_THREADS, 0, s, (const SgtState *)J->st,
+                  (NT *)J->Vc, (NT *)J->V));
+  if (J->jp.cell_blocks > 0) {
+    CK(launch_chain(pdl, k_bin_scatter<D>, J->jp.cell_blocks, SGT_THREADS, 0, s, (const VT *)J->Y,
+                    n, J->st, J->cursor, J->sorted));
+    CK(launch_chain(pdl, k_s2g_cell<D>, J->nb_s2gc, SGT_THREADS, 0, s, (const float4 *)J->sorted,
+                    J->st, (const int4 *)J->chunks, (NT *)J->V));
+  }
   if (ev) CK(cudaEventRecord(ev[2], s));
   CK(cudaGetLastError());
   return SGT_OK;
@@ -697,12 +662,11 @@ static sgt_status enqueue_gather_part(sgt_job *J, cudaStream_t s, cudaEvent_t *e
   const bool pdl = ev == nullptr;
   CKS(enqueue_g2g<D>(J, s, pdl));
   if (ev) CK(cudaEventRecord(ev[3], s));
-  CK(launch_chain(pdl, k_g2s<D>, J->nb_g2s, SGT_THREADS, 0, s, (const float4 *)J->sorted, J->st,
-                  (const int4 *)J->chunks, (const NT *)J->Phi, (VT *)J->Frep, J->part_z, J->n));
-  if constexpr (D <= 2)
-    if (J->jp.direct_max > 0)
-      CK(launch_chain(pdl, k_g2s_direct<D>, J->nb_g2s, SGT_THREADS, J->smem_g2sd, s, J->st,
-                      (const NT *)J->Phi, (VT *)J->Frep, J->part_z, J->n, (const VT *)J->Y));
+  if (J->jp.cell_blocks > 0)
+    CK(launch_chain(pdl, k_g2s<D>, J->nb_g2s, SGT_THREADS, 0, s, (const float4 *)J->sorted, J->st,
+                    (const int4 *)J->chunks, (const NT *)J->Phi, (VT *)J->Frep, J->part_z, J->n));
+  CK(launch_chain(pdl, k_gather<D>, J->nb_gath, SGT_THREADS, 0, s, J->st, (const NT *)J->Phi,
+                  (VT *)J->Frep, J->part_z, J->n, (const VT *)J->Y));
   CK(cudaGetLastError());
   return SGT_OK;
 }
@@ -1478,15 +1442,15 @@ sgt_status sgt_job_run(sgt_job *J, int iters) {
 // table of block counts per stage, and one view/prefix table per row-group
 // lane count for the SpMV.
 enum {
-  FS_BIN_COUNT, FS_BIN_SCATTER, FS_S2G, FS_S2G8, FS_S2G_CELL, FS_FFT_X,
-  FS_FFT_MID_FWD, FS_FFT_LAST, FS_FFT_MID_INV, FS_FFT_FINAL, FS_G2S, FS_UPDATE, FS_STAGES
+  FS_BIN_COUNT, FS_SCATTER, FS_FOLD, FS_BIN_SCATTER, FS_S2G_CELL, FS_FFT_X,
+  FS_FFT_MID_FWD, FS_FFT_LAST, FS_FFT_MID_INV, FS_FFT_FINAL, FS_G2S, FS_GATHER, FS_UPDATE, FS_STAGES
 };
 struct BatchGroup {
   int D = 2, njobs = 0;
   const SgtJobView *views = nullptr;
   const int *prefix[FS_STAGES] = {};
   int blocks[FS_STAGES] = {};
-  size_t smem_s2g = 0, smem_s2g8 = 0, smem_fft = 0, smem_s2gd = 0, smem_g2sd = 0;
+  size_t smem_fft = 0;
   // SpMV: one launch per lane count G present
   struct Spmv {
     int G = 16, njobs = 0, blocks = 0;
@@ -1535,7 +1499,7 @@ static sgt_status batch_build(sgt_batch *b, const std::vector<cudaGraph_t> &iter
 
 }  // extern "C"
 
-static void stage_blocks(const sgt_job *J, int *b, int *nb_s2g2 = nullptr);
+static void stage_blocks(const sgt_job *J, int *b);
 
 static SgtJobView job_view(const sgt_job *J) {
   SgtJobView v;
@@ -1549,6 +1513,7 @@ static SgtJobView job_view(const sgt_job *J) {
   v.Fattr = J->Fattr;
   v.sorted = J->sorted;
   v.V = J->V;
+  v.Vc = J->Vc;
   v.Phi = J->Phi;
   v.W = J->W;
   v.tile_count = J->tile_count;
@@ -1564,7 +1529,8 @@ static SgtJobView job_view(const sgt_job *J) {
   v.jp = J->jp;
   v.n = J->n;
   int bl[FS_STAGES];
-  stage_blocks(J, bl, &v.nb_s2g);  // the binning sizes chunks for the fused S2G grid
+  stage_blocks(J, bl);
+  v.nb_s2g = std::max(1, bl[FS_S2G_CELL]);  // the binning sizes chunks for the fused S2G grid
   // short chunks: a chunk is one block's serial work in S2G, and in a fused
   // launch the slowest block of the smallest jobs sets the stage's length
   v.jp.chunk_min = 256;
@@ -1576,19 +1542,22 @@ static SgtJobView job_view(const sgt_job *J) {
 // exist for it).  A job launched alone sizes its grids to fill the GPU; in
 // a fused launch its blocks share the GPU with every other job's, so each
 // job gets blocks in proportion to its work instead (the kernels loop over
-// whatever they are given): a block per 2048 points in the point passes and
-// per 2048 points of chunks in S2G and G2S, up to the job's own grid, and the
-// FFT passes a block per 8 lines of a 64-point grid (they loop over larger
-// ones).  nb_s2g2 is the S2G block count the binning sizes its chunks for.
-static void stage_blocks(const sgt_job *J, int *b, int *nb_s2g2) {
+// whatever they are given): a block per 256 points (128 in 3-D) in S2G and
+// G2S, per 2048 points in the other point passes, up to the job's own grid,
+// and the FFT passes a block per 8 lines of a 64-point grid (they loop over
+// larger ones).
+static void stage_blocks(const sgt_job *J, int *b) {
   for (int k = 0; k < FS_STAGES; k++) b[k] = 0;
   const int work = std::max(1, (J->n + 2047) / 2048);
-  const int s2g = std::min(J->nb_s2g, work);
-  b[FS_BIN_COUNT] = std::min(J->nb_bin, work);
-  b[FS_BIN_SCATTER] = std::min(J->nb_bin, work);
-  b[FS_S2G] = s2g;
-  if (J->d == 3) b[FS_S2G8] = std::min(J->nb_s2g8, 2 * work);
-  b[FS_S2G_CELL] = std::min(J->nb_s2gc, 2 * work);
+  const int fine = (J->d == 3 ? 16 : 8) * work;
+  b[FS_SCATTER] = std::min(J->nb_scat, fine);
+  b[FS_FOLD] = std::min(J->nb_fold, 4);
+  if (J->jp.cell_blocks > 0) {
+    b[FS_BIN_COUNT] = std::min(J->jp.cell_blocks, work);
+    b[FS_G2S] = std::min(J->nb_g2s, 2 * work);
+    b[FS_BIN_SCATTER] = std::min(J->jp.cell_blocks, work);
+    b[FS_S2G_CELL] = std::min(J->nb_s2gc, 2 * work);
+  }
   const int rows64 = J->d == 3 ? (2 * 64 * 64 + 128 * 128) / 8 : (2 * 64 + 128) / 8;
   b[FS_FFT_X] = J->d == 1 ? 1 : std::min(J->nb_fft_rows, rows64);
   if (J->d == 3) b[FS_FFT_MID_FWD] = b[FS_FFT_MID_INV] = std::min(J->nb_fft, 128);
@@ -1596,9 +1565,8 @@ static void stage_blocks(const sgt_job *J, int *b, int *nb_s2g2) {
     b[FS_FFT_LAST] = std::min(J->nb_fft, J->d == 3 ? 128 : 16);
     b[FS_FFT_FINAL] = std::min(J->nb_fft_rows, rows64);
   }
-  b[FS_G2S] = std::min(J->nb_g2s, 2 * work);
+  b[FS_GATHER] = std::min(J->nb_gath, fine);
   b[FS_UPDATE] = std::min(J->nb_upd, work);
-  if (nb_s2g2) *nb_s2g2 = s2g;
 }
 
 // Host images of the tables of fused launches over `jobs` (all CSR): the
@@ -1630,11 +1598,7 @@ static void build_fused_image(const std::vector<sgt_job *> &jobs, FusedImage &im
     o.views = im.views.size();
     for (sgt_job *J : js) {
       im.views.push_back(job_view(J));
-      g.smem_s2g = std::max(g.smem_s2g, J->smem_s2g);
-      g.smem_s2g8 = std::max(g.smem_s2g8, J->smem_s2g8);
       g.smem_fft = std::max(g.smem_fft, J->smem_fft2);
-      g.smem_s2gd = std::max(g.smem_s2gd, J->smem_s2gd);
-      g.smem_g2sd = std::max(g.smem_g2sd, J->smem_g2sd);
     }
     for (int k = 0; k < FS_STAGES; k++) {
       o.prefix[k] = im.ints.size();
@@ -1728,15 +1692,14 @@ static sgt_status enqueue_fused_group(sgt_ctx *ctx, BatchGroup &g) {
     }
   }
   CK(cudaEventRecord(g.ev_spmv, sd));
-  km_bin_count<D><<<FL(FS_BIN_COUNT), 0, c>>>(v, g.prefix[FS_BIN_COUNT], nj);
-  km_bin_scatter<D><<<FL(FS_BIN_SCATTER), 0, c>>>(v, g.prefix[FS_BIN_SCATTER], nj);
-  if constexpr (D <= 2)
-    if (g.smem_s2gd > 0)  // some job of the group can take the direct mode
-      km_s2g_direct<D><<<FL(FS_BIN_SCATTER), g.smem_s2gd, c>>>(v, g.prefix[FS_BIN_SCATTER], nj);
-  constexpr int TT = D == 1 ? 512 : (D == 2 ? 32 : 16);
-  km_s2g<D, TT><<<FL(FS_S2G), g.smem_s2g, c>>>(v, g.prefix[FS_S2G], nj);
-  if constexpr (D == 3) km_s2g<3, 8><<<FL(FS_S2G8), g.smem_s2g8, c>>>(v, g.prefix[FS_S2G8], nj);
-  km_s2g_cell<D><<<FL(FS_S2G_CELL), 0, c>>>(v, g.prefix[FS_S2G_CELL], nj);
+  if (g.blocks[FS_BIN_COUNT] > 0)  // some job of the group can take the cell mode
+    km_bin_count<D><<<FL(FS_BIN_COUNT), 0, c>>>(v, g.prefix[FS_BIN_COUNT], nj);
+  km_scatter<D><<<FL(FS_SCATTER), 0, c>>>(v, g.prefix[FS_SCATTER], nj);
+  km_fold<D><<<FL(FS_FOLD), 0, c>>>(v, g.prefix[FS_FOLD], nj);
+  if (g.blocks[FS_BIN_SCATTER] > 0) {
+    km_bin_scatter<D><<<FL(FS_BIN_SCATTER), 0, c>>>(v, g.prefix[FS_BIN_SCATTER], nj);
+    km_s2g_cell<D><<<FL(FS_S2G_CELL), 0, c>>>(v, g.prefix[FS_S2G_CELL], nj);
+  }
   if constexpr (D == 1) {
     km_conv1d<<<g.blocks[FS_FFT_X], 32, 0, c>>>(v, g.prefix[FS_FFT_X], nj);
   } else {
@@ -1748,10 +1711,8 @@ static sgt_status enqueue_fused_group(sgt_ctx *ctx, BatchGroup &g) {
       km_fft_cols<D, MODE_MID_INV><<<FL(FS_FFT_MID_INV), g.smem_fft, c>>>(v, g.prefix[FS_FFT_MID_INV], nj);
     km_fft_final_x<D><<<FL(FS_FFT_FINAL), 0, c>>>(v, g.prefix[FS_FFT_FINAL], nj);
   }
-  km_g2s<D><<<FL(FS_G2S), 0, c>>>(v, g.prefix[FS_G2S], nj);
-  if constexpr (D <= 2)
-    if (g.smem_g2sd > 0)
-      km_g2s_direct<D><<<FL(FS_G2S), g.smem_g2sd, c>>>(v, g.prefix[FS_G2S], nj);
+  if (g.blocks[FS_G2S] > 0) km_g2s<D><<<FL(FS_G2S), 0, c>>>(v, g.prefix[FS_G2S], nj);
+  km_gather<D><<<FL(FS_GATHER), 0, c>>>(v, g.prefix[FS_GATHER], nj);
   CK(cudaStreamWaitEvent(c, g.ev_spmv, 0));
   km_row_update<D><<<FL(FS_UPDATE), 0, c>>>(v, g.prefix[FS_UPDATE], nj);
   CK(cudaGetLastError());
@@ -1801,17 +1762,6 @@ static sgt_status batch_fused_graph(sgt_batch *b, int R, cudaGraphExec_t *exec) 
 
 template <int D>
 static sgt_status fused_attributes(sgt_ctx *ctx, const BatchGroup &g) {
-  constexpr int TT = D == 1 ? 512 : (D == 2 ? 32 : 16);
-  if constexpr (D <= 2) {  // the largest any group of this dimension asks for
-    const size_t dmax = D == 1 ? 512 : (size_t)SGT_DIRECT_N2 * SGT_DIRECT_N2;
-    CK(cudaFuncSetAttribute(km_s2g_direct<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)(sizeof(float) * (D + 1) * dmax)));
-    CK(cudaFuncSetAttribute(km_g2s_direct<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)(sizeof(typename Node<D>::T) * dmax)));
-  }
-  CK(cudaFuncSetAttribute(km_s2g<D, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem_s2g));
-  if constexpr (D == 3)
-    CK(cudaFuncSetAttribute(km_s2g<3, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem_s2g8));
   if constexpr (D >= 2) {
     CK(cudaFuncSetAttribute(km_fft_cols<D, MODE_LAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem_fft));
     if constexpr (D == 3) {
@@ -2211,7 +2161,8 @@ size_t sgt_job_footprint(const sgt_params *p, int n, long nnz) {
   if (!p || n < 1 || nnz < 0 || p->d < 1 || p->d > 3) return 0;
   const int D = p->d, S = D == 3 ? 4 : D;
   const size_t np = (size_t)n * S;
-  size_t b = 5 * np * 4 + (size_t)n * 16;  // Y, Ynext, uY, gains, Frep; sorted
+  size_t b = 5 * np * 4;  // Y, Ynext, uY, gains, Frep
+  if (n >= SGT_CELL_MIN_N) b += (size_t)n * 16;  // sorted
   int max_grid = p->max_grid > 0 ? p->max_grid : (D <= 2 ? 512 : 128);
   max_grid = std::min(D == 3 ? 256 : 512, std::max(16, max_grid));
   size_t M = 1;
@@ -2221,6 +2172,7 @@ size_t sgt_job_footprint(const sgt_params *p, int n, long nnz) {
   if (D >= 2) { nodes *= nmax; plane *= M; }
   if (D >= 3) { nodes *= nmax; plane *= M; }
   b += 2 * nodes * (D == 1 ? 2 : 4) * 4;                       // V, Phi
+  b += std::max<size_t>(nodes, SGT_COPY_NODES) * (D == 1 ? 2 : 4) * 4;  // grid copies
   if (D >= 2) b += 3 * plane * 8;                               // FFT planes
   b += 2 * 4096 * 4 + ((size_t)n / 256 + 4096 + 16) * 16;        // tiles, chunks
   const size_t parts = std::max<size_t>(148 * 16, ((size_t)n * 32 + 255) / 256);
@@ -2914,21 +2866,19 @@ constexpr int SGT_NA_MAX_GRID_2D = 128;   // points per axis -> FFT length 256
 constexpr int SGT_NA_MMAX_2D = 256;
 constexpr int SGT_NA_MMAX_1D = 1024;
 constexpr int SGT_NA_PARTS = 4096;        // per-block partials of the reductions
-constexpr int SGT_NA_CHUNKS = SGT_NA_MAX_N / 1024 + SGT_HIST_MAX + 16;
+constexpr int SGT_NA_COPY_NODES = 1 << 16;  // grid copies of the scatter mode
+static_assert(SGT_NA_MAX_N < SGT_CELL_MIN_N, "the no-alloc scratch has no cell mode");
 constexpr size_t na_al(size_t b) { return (b + 255) & ~(size_t)255; }
 // byte offsets of every buffer inside the array
 constexpr size_t NA_Y = 0;
 constexpr size_t NA_YNEXT = NA_Y + na_al((size_t)SGT_NA_MAX_N * 2 * 4);
 constexpr size_t NA_FREP = NA_YNEXT + na_al((size_t)SGT_NA_MAX_N * 2 * 4);
-constexpr size_t NA_SORTED = NA_FREP + na_al((size_t)SGT_NA_MAX_N * 2 * 4);
+constexpr size_t NA_VC = NA_FREP + na_al((size_t)SGT_NA_MAX_N * 2 * 4);
 constexpr size_t NA_NODES = (size_t)SGT_NA_MAX_GRID_2D * SGT_NA_MAX_GRID_2D;  // >= 512 (1-D)
-constexpr size_t NA_V = NA_SORTED + na_al((size_t)SGT_NA_MAX_N * 16);
+constexpr size_t NA_V = NA_VC + na_al((size_t)SGT_NA_COPY_NODES * 16);
 constexpr size_t NA_PHI = NA_V + na_al(NA_NODES * 16);
 constexpr size_t NA_W = NA_PHI + na_al(NA_NODES * 16);
-constexpr size_t NA_TILES = NA_W + na_al((size_t)3 * SGT_NA_MMAX_2D * SGT_NA_MMAX_2D * 8);
-constexpr size_t NA_CURSOR = NA_TILES + na_al((size_t)SGT_HIST_MAX * 4);
-constexpr size_t NA_CHUNKS = NA_CURSOR + na_al((size_t)SGT_HIST_MAX * 4);
-constexpr size_t NA_PMIN = NA_CHUNKS + na_al((size_t)SGT_NA_CHUNKS * 16);
+constexpr size_t NA_PMIN = NA_W + na_al((size_t)3 * SGT_NA_MMAX_2D * SGT_NA_MMAX_2D * 8);
 constexpr size_t NA_PMAX = NA_PMIN + na_al((size_t)SGT_NA_PARTS * 16);
 constexpr size_t NA_PSUM = NA_PMAX + na_al((size_t)SGT_NA_PARTS * 16);
 constexpr size_t NA_PZ = NA_PSUM + na_al((size_t)SGT_NA_PARTS * 4 * 8);
@@ -3028,19 +2978,14 @@ extern "C" sgt_status sgt_repulsive_noalloc(sgt_ctx *ctx, int n, int d, float h,
   J.mmax = d == 1 ? SGT_NA_MMAX_1D : SGT_NA_MMAX_2D;
   J.nmax = d == 1 ? 512 : SGT_NA_MAX_GRID_2D;
   J.jp.mmax = J.mmax;
-  J.jp.tile_cap = SGT_HIST_MAX;
-  J.jp.direct_max = d == 1 ? J.nmax : std::min(SGT_DIRECT_N2, J.nmax);
-  J.jp.chunk_cap = SGT_NA_CHUNKS;
+  J.jp.vc_nodes = SGT_NA_COPY_NODES;
   J.Y = (float *)(base + NA_Y);
   J.Ynext = (float *)(base + NA_YNEXT);
   J.Frep = (float *)(base + NA_FREP);
-  J.sorted = (float4 *)(base + NA_SORTED);
+  J.Vc = (float *)(base + NA_VC);
   J.V = (float *)(base + NA_V);
   J.Phi = (float *)(base + NA_PHI);
   J.W = (float2 *)(base + NA_W);
-  J.tile_count = (int *)(base + NA_TILES);
-  J.cursor = (int *)(base + NA_CURSOR);
-  J.chunks = (int4 *)(base + NA_CHUNKS);
   J.part_min = (float4 *)(base + NA_PMIN);
   J.part_max = (float4 *)(base + NA_PMAX);
   J.part_sum = (double *)(base + NA_PSUM);
@@ -3048,11 +2993,11 @@ extern "C" sgt_status sgt_repulsive_noalloc(sgt_ctx *ctx, int n, int d, float h,
   J.st = (SgtState *)(base + NA_STATE);
   sgt_status stt = d == 1 ? job_shapes<1>(&J) : job_shapes<2>(&J);
   if (stt != SGT_OK) return stt;
-  if (std::max(std::max(J.nb_pts, J.nb_s2g), J.nb_g2s) > SGT_NA_PARTS)
+  if (std::max(J.nb_pts, J.nb_gath) > SGT_NA_PARTS)
     return fail(ctx, SGT_ERR_UNSUPPORTED, "sgt_repulsive_noalloc: too many blocks for the partials");
   // the array keeps the previous call's contents: clear what starts at zero
   CK(cudaMemsetAsync(J.st, 0, sizeof(SgtState), s));
-  CK(cudaMemsetAsync(J.tile_count, 0, sizeof(int) * SGT_HIST_MAX, s));
+  CK(cudaMemsetAsync(J.Vc, 0, (size_t)SGT_NA_COPY_NODES * 16, s));
   CKS(pack_y(&J, y, layout, J.Ynext, s));
   CKS(init_stats(&J, s, 0));
   if (d == 1) CKS(enqueue_repulsion<1>(&J, s));

@@ -9,15 +9,33 @@
 //   Z = sum((1+2|y|^2)Phi0 - 2 y.Phi) - n,
 //   F = (y Phi0 - Phi)/Z                   CU/Frep.cu:42-80, HYB/qq.cpp:75-106
 //
-// B200 structure: points are counting-sorted into T^d-cell tiles every
-// iteration; S2G accumulates one tile per chunk of sorted points in shared
-// memory and flushes with vector atomics, so global atomics scale with the
-// grid, not with n*4^d.  Every kernel reads the grid decision from SgtState,
-// so the chain is graph-capturable with fixed launch shapes.
+// B200 structure: two modes, picked per iteration by the grid decision.
+//   scatter mode (T = 0): no sort.  A group of lanes per point adds the
+//     point's weighted charges to one of several copies of the grid with
+//     vector reductions in L2 (k_scatter), k_fold sums the copies into V,
+//     and k_gather gathers with the same lane groups.
+//   cell mode (T = 1; large jobs on grids with many points per cell): the
+//     points are counting-sorted by cell, and S2G sums each cell's points in
+//     registers (k_s2g_cell).
+// Every kernel reads the grid decision from SgtState, so the chain is
+// graph-capturable with fixed launch shapes.
 #pragma once
 #include "sgt_common.cuh"
 
-#define SGT_HIST_MAX 4096  // tiles held in shared memory by the binning kernels
+#define SGT_HIST_MAX 4096  // cells held in shared memory by the binning kernels
+// Scatter mode: lanes that share a point.  The 4 nodes of a stencil row are
+// 64 contiguous bytes (32 in 1-D), so 4 lanes per point make one row one
+// request; 3-D spreads its 16 rows over 16 lanes.  100k points on 64^2 nodes:
+// 22.8 us with 4 lanes per point, 37.1 us with one.
+#define SGT_LPP(D) ((D) == 3 ? 16 : 4)
+// Scatter mode: most copies of the grid.  L2 serialises the reductions that
+// meet on one node; with 32 copies 60k points on 16^2 nodes take 10.5 us
+// instead of 76, 100k on 117^2 10.3 instead of 20.7.  k_fold reads the copies
+// back, so a grid takes them only as it has adds per node.
+#define SGT_COPIES 32
+// Points from which a dense grid is sorted by cell.  Below, scatter mode is
+// faster even with every point in a few hundred cells.
+#define SGT_CELL_MIN_N 300000
 // Points a thread loads before it uses the first of them in the point loops
 // of the binning, S2G (cell mode) and G2S kernels: these kernels are bound by
 // load latency, not bandwidth, at a few warps per SM.
@@ -126,29 +144,24 @@ __device__ void sgt_finalize_grid(SgtState *st, const SgtJobParams &jp,
   long ncell = cells;
   if (D >= 2) ncell *= cells;
   if (D >= 3) ncell *= cells;
-  // cell mode (tile = one cell): the cells fit the tile arrays and hold
-  // enough points each that one block reduction per chunk of a cell is
-  // cheaper than shared-memory atomics that all land on a few nodes
-  const bool cell_mode = ncell <= SGT_HIST_MAX && (long)jp.n >= 64L * ncell;
-  // direct mode (no sort, the grid in shared memory) for the other grids that
-  // fit: few points per node, so its shared-memory atomics rarely collide
-  if (!cell_mode && N <= jp.direct_max) {
-    st->T = 0;
-    st->tiles_dim = 0;
-    st->ntiles = 0;
-    return;
-  }
-  // 3-D tiles of 8 cells while the tile count fits the tile arrays: a
-  // (8+3)^3 x 4-channel shared accumulator is 21 KB (a 16-cell tile: 110 KB),
-  // so each chunk zeroes and flushes 5x fewer nodes and more CTAs fit an SM
-  const int T = cell_mode ? 1 : (D == 1 ? 512 : (D == 2 ? 32 : (cells <= 128 ? 8 : 16)));
-  const int td = (cells + T - 1) / T;
-  int nt = td;
-  if (D >= 2) nt *= td;
-  if (D >= 3) nt *= td;
-  st->T = T;
-  st->tiles_dim = td;
-  st->ntiles = nt;
+  // cell mode: a large job whose cells fit the cell arrays and hold enough
+  // points each that one block reduction per chunk of a cell is cheaper than
+  // a reduction in L2 per point and node
+  const bool cell_mode = jp.n >= SGT_CELL_MIN_N && jp.cell_blocks > 0 && ncell <= SGT_HIST_MAX &&
+                         (long)jp.n >= 64L * ncell;
+  st->T = cell_mode ? 1 : 0;
+  st->tiles_dim = cell_mode ? cells : 0;
+  st->ntiles = cell_mode ? (int)ncell : 0;
+  // scatter mode: a copy per 16 adds that an average node receives, a power
+  // of two that fits the buffer
+  long nodes = N;
+  if (D >= 2) nodes *= N;
+  if (D >= 3) nodes *= N;
+  const long adds = ((long)jp.n << (2 * D)) / nodes;
+  int copies = 1;
+  while (copies < SGT_COPIES && 16L * copies < adds && 2L * copies * nodes <= jp.vc_nodes)
+    copies *= 2;
+  st->copies = copies;
 }
 
 // Scaled coordinate exactly as CU/nuconv.cu:9-36: (y - miny)/maxy, clamp to
@@ -162,10 +175,10 @@ __device__ __forceinline__ float sgt_scale(float y, float miny, float maxy,
 }
 
 template <int D>
-__device__ __forceinline__ int sgt_tile_of(const int *f, int T, int td) {
-  int t = f[0] / T;
-  if (D >= 2) t += td * (f[1] / T);
-  if (D >= 3) t += td * td * (f[2] / T);
+__device__ __forceinline__ int sgt_cell_of(const int *f, int td) {
+  int t = f[0];
+  if (D >= 2) t += td * f[1];
+  if (D >= 3) t += td * td * f[2];
   return t;
 }
 
@@ -279,8 +292,7 @@ __device__ __forceinline__ void bin_scan_block(SgtState *st, const SgtJobParams 
                                                int4 *__restrict__ chunks, int nblk) {
   const int ntiles = st->ntiles;
   // chunk length: about two chunks per persistent S2G CTA, at least 1024
-  // points (256 in 3-D, where a point costs 64 nodes and small jobs need more
-  // chunks than they have 1024-point runs)
+  // points (256 in 3-D, where a point costs 64 nodes)
   int chunk = (jp.n + 2 * nblk - 1) / (2 * nblk);
   chunk = ((chunk + 255) / 256) * 256;
   const int cmin = jp.chunk_min > 0 ? jp.chunk_min : (jp.d == 3 ? 256 : 1024);
@@ -322,16 +334,157 @@ __device__ __forceinline__ void bin_scan_block(SgtState *st, const SgtJobParams 
 }
 
 // ---------------------------------------------------------------------------
-// bin_count: centre (Y = Ynext - mean), zero the grid V, count points per tile
+// Scatter mode: centre the points and add their weighted charges [1, y - c]
+// to the grid copy vb_ mod copies.  SGT_LPP(D) lanes share a point; lane q of
+// a group owns the stencil nodes with x offset q & 3 (3-D: and y offset
+// q >> 2), and every lane works out the point's weights for itself.
+// Bound by the reductions L2 takes: 100k points on 64^2 nodes 10.5 us (1.6M
+// 16-byte node updates), on 117^2 10.3 us, 400k on 512^2 31 us.  In the
+// sorted form this replaces, a tile of the grid in shared memory took 200 to
+// 420 us where clustered points met on few nodes: shared-memory float adds
+// are compare-and-swap loops there.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void red_node(float2 *p, float a, float b) {
+  asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(a), "f"(b) : "memory");
+}
+__device__ __forceinline__ void red_node(float4 *p, float a, float b, float c, float d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c),
+               "f"(d)
+               : "memory");
+}
+// w[q] without a dynamically indexed (local memory) array
+__device__ __forceinline__ float pick4(const float *w, int q) {
+  return q == 0 ? w[0] : (q == 1 ? w[1] : (q == 2 ? w[2] : w[3]));
+}
+
+template <int D>
+__device__ __forceinline__ void k_scatter_body(int vb_, int vg_,
+                                               const typename Vec<D>::T *__restrict__ Ynext,
+                                               typename Vec<D>::T *__restrict__ Y, int n,
+                                               SgtState *st, typename Node<D>::T *Vc) {
+  if (st->T != 0) return;  // cell mode
+  constexpr int L = SGT_LPP(D);
+  const int N = st->N, cells = N - 3;
+  const float maxy = st->maxy, scale = st->scale;
+  // charges are taken about the middle of the grid: F and Z are invariant to
+  // the origin of y, and |y - c| <= maxy/2 halves the cancellation in
+  // (1 + 2|y|^2) Phi0 - 2 y.Phi
+  const float hc = 0.5f * maxy;
+  float mean[3], miny[3];
+#pragma unroll
+  for (int k = 0; k < D; k++) { mean[k] = st->mean[k]; miny[k] = st->miny[k]; }
+  long nodes = N;
+  if (D >= 2) nodes *= N;
+  if (D >= 3) nodes *= N;
+  Vc += (long)(vb_ & (st->copies - 1)) * nodes;
+  const int q = threadIdx.x % L, qx = q & 3;
+  const int step = vg_ * (SGT_THREADS / L);
+  for (int i = vb_ * (SGT_THREADS / L) + threadIdx.x / L; i < n; i += step) {
+    typename Vec<D>::T y = Ynext[i];
+    int f[3];
+    float w[3][4], qc[3];
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+      const float yc = __fsub_rn(comp<D>(y, k), mean[k]);
+      setcomp<D>(y, k, yc);
+      float sh;
+      const float s = sgt_scale(yc, miny[k], maxy, scale, sh);
+      sgt_weights(s, f[k], w[k]);
+      qc[k] = sh - hc;
+      ok = ok && (unsigned)f[k] < (unsigned)cells;
+    }
+    if (q == 0) Y[i] = y;
+    if (!ok) {  // outside the grid: skip the point
+      if (q == 0) atomicOr(&st->error, SGT_EFLAG_CHUNK_OVERFLOW);
+      continue;
+    }
+    const float wx = pick4(w[0], qx);
+    if constexpr (D == 1) {
+      red_node(&Vc[f[0] + qx], wx, wx * qc[0]);
+    } else if constexpr (D == 2) {
+#pragma unroll
+      for (int b = 0; b < 4; b++) {
+        const float wt = w[1][b] * wx;
+        red_node(&Vc[f[0] + qx + N * (f[1] + b)], wt, wt * qc[0], wt * qc[1], 0.f);
+      }
+    } else {
+      const int qy = q >> 2;
+      const float wy = pick4(w[1], qy);
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const float wt = (wy * w[2][c]) * wx;
+        red_node(&Vc[f[0] + qx + (long)N * (f[1] + qy + (long)N * (f[2] + c))], wt, wt * qc[0],
+                 wt * qc[1], wt * qc[2]);
+      }
+    }
+  }
+}
+
+template <int D>
+__global__ void __launch_bounds__(SGT_THREADS, 8)
+k_scatter(const typename Vec<D>::T *__restrict__ Ynext, typename Vec<D>::T *__restrict__ Y, int n,
+          SgtState *st, typename Node<D>::T *Vc) {
+  k_scatter_body<D>(blockIdx.x, gridDim.x, Ynext, Y, n, st, Vc);
+}
+
+// ---------------------------------------------------------------------------
+// fold: V = sum of the grid copies, which are left zero for the next
+// iteration's scatter (they start zero at job creation).  Cell mode: V only
+// (k_bin_count cleared it and k_s2g_cell has added to it), nothing to do.
+// ---------------------------------------------------------------------------
+template <int D>
+__device__ __forceinline__ void k_fold_body(int vb_, int vg_, const SgtState *st,
+                                            typename Node<D>::T *__restrict__ Vc,
+                                            typename Node<D>::T *__restrict__ V) {
+  sgt_pdl_wait();
+  if (st->T != 0) return;
+  const int N = st->N, copies = st->copies;
+  long nodes = N;
+  if (D >= 2) nodes *= N;
+  if (D >= 3) nodes *= N;
+  typename Node<D>::T z;
+  if constexpr (D == 1) z = make_float2(0.f, 0.f); else z = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (long g = vb_ * (long)blockDim.x + threadIdx.x; g < nodes; g += (long)vg_ * blockDim.x) {
+    typename Node<D>::T a = z;
+    for (int c0 = 0; c0 < copies; c0 += 4) {
+      typename Node<D>::T t[4];
+#pragma unroll
+      for (int c = 0; c < 4; c++) t[c] = c0 + c < copies ? Vc[(c0 + c) * nodes + g] : z;
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        a.x += t[c].x;
+        a.y += t[c].y;
+        if constexpr (D >= 2) {
+          a.z += t[c].z;
+          if constexpr (D >= 3) a.w += t[c].w;
+        }
+        if (c0 + c < copies) Vc[(c0 + c) * nodes + g] = z;
+      }
+    }
+    V[g] = a;
+  }
+}
+template <int D>
+__global__ void __launch_bounds__(SGT_THREADS)
+k_fold(const SgtState *st, typename Node<D>::T *__restrict__ Vc,
+       typename Node<D>::T *__restrict__ V) {
+  k_fold_body<D>(blockIdx.x, gridDim.x, st, Vc, V);
+}
+
+// ---------------------------------------------------------------------------
+// bin_count (cell mode): centre (Y = Ynext - mean), zero the grid V, count
+// points per cell
 // ---------------------------------------------------------------------------
 template <int D>
 __device__ __forceinline__ void k_bin_count_body(int vb_, int vg_, const typename Vec<D>::T *__restrict__ Ynext,
             typename Vec<D>::T *__restrict__ Y, int n, SgtState *st,
             int *__restrict__ tile_count, typename Node<D>::T *__restrict__ V,
-            int write_centred, const SgtJobParams &jp, int *__restrict__ cursor,
+            const SgtJobParams &jp, int *__restrict__ cursor,
             int4 *__restrict__ chunks, int nblk) {
+  if (st->T == 0) return;  // scatter mode
   __shared__ int hist[SGT_HIST_MAX];
-  const int ntiles = st->ntiles, T = st->T, td = st->tiles_dim, N = st->N;
+  const int ntiles = st->ntiles, td = st->tiles_dim, N = st->N;
   const float maxy = st->maxy, scale = st->scale;
   float mean[3], miny[3];
 #pragma unroll
@@ -346,30 +499,6 @@ __device__ __forceinline__ void k_bin_count_body(int vb_, int vg_, const typenam
   for (long g = vb_ * (long)blockDim.x + threadIdx.x; g < nodes;
        g += (long)vg_ * blockDim.x)
     V[g] = z;
-  if (T == 0) {  // direct mode: centre only; k_bin_scatter does the S2G
-    if (write_centred) {
-      constexpr int U = SGT_PTS_U;
-      const long stride = (long)vg_ * blockDim.x * U;
-      for (long i0 = ((long)vb_ * blockDim.x + (threadIdx.x & ~31)) * U; i0 < n; i0 += stride) {
-        typename Vec<D>::T yv[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          const long i = i0 + 32 * u + (threadIdx.x & 31);
-          if (i < n) yv[u] = Ynext[i];
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          const long i = i0 + 32 * u + (threadIdx.x & 31);
-          if (i < n) {
-#pragma unroll
-            for (int k = 0; k < D; k++) setcomp<D>(yv[u], k, __fsub_rn(comp<D>(yv[u], k), mean[k]));
-            Y[i] = yv[u];
-          }
-        }
-      }
-    }
-    return;
-  }
   __syncthreads();
   // warp-uniform trip count: lanes with the same tile are merged with
   // match_any and add their count in one shared-memory atomic (points of an
@@ -400,8 +529,8 @@ __device__ __forceinline__ void k_bin_count_body(int vb_, int vg_, const typenam
           const float s = sgt_scale(yc, miny[k], maxy, scale, sh);
           f[k] = (int)floorf(s);
         }
-        if (write_centred) Y[i] = y;
-        key = sgt_tile_of<D>(f, T, td);
+        Y[i] = y;
+        key = sgt_cell_of<D>(f, td);
       }
       const unsigned grp = __match_any_sync(0xffffffffu, key);
       if (key >= 0 && lane == __ffs(grp) - 1) atomicAdd(&hist[key], __popc(grp));
@@ -432,151 +561,13 @@ __global__ void __launch_bounds__(SGT_THREADS)
 k_bin_count(const typename Vec<D>::T *__restrict__ Ynext,
             typename Vec<D>::T *__restrict__ Y, int n, SgtState *st,
             int *__restrict__ tile_count, typename Node<D>::T *__restrict__ V,
-            int write_centred, SgtJobParams jp, int *__restrict__ cursor,
-            int4 *__restrict__ chunks, int nblk) {
-  k_bin_count_body<D>(blockIdx.x, gridDim.x, Ynext, Y, n, st, tile_count, V, write_centred,
-                      jp, cursor, chunks, nblk);
+            SgtJobParams jp, int *__restrict__ cursor, int4 *__restrict__ chunks, int nblk) {
+  k_bin_count_body<D>(blockIdx.x, gridDim.x, Ynext, Y, n, st, tile_count, V, jp, cursor, chunks,
+                      nblk);
 }
 
 // ---------------------------------------------------------------------------
-// Direct-mode S2G (T = 0; d <= 2, grids of at most SGT_DIRECT_N2 points per
-// axis in 2-D that hold fewer than 64 points per cell): no sort.  A block takes a contiguous range of the points in
-// their own order, accumulates their weighted charges [1, y - c] in a copy of
-// the whole grid in shared memory (m planes of N^d floats), and adds the
-// touched nodes to V (zeroed by k_bin_count) with one vector atomic each.
-// The lanes of a warp hold 32 consecutive points.  When they fall in at most
-// four cells (points in a spatial order, the common case after the Morton
-// relabelling), the warp sums each cell's 4^d m values by halving shuffles
-// and distinct lanes publish the totals; otherwise (points scattered over
-// the grid, as early in a run) each lane adds its own values with
-// shared-memory atomics, which then rarely meet on one node.
-// ---------------------------------------------------------------------------
-template <int D>
-__device__ __forceinline__ void s2g_direct_warp(float *Vs, int N, int nodes, int key,
-                                                const int *f, const float (*w)[4],
-                                                const float *qc, int lane) {
-  constexpr int NN = D == 1 ? 4 : 16, C = D + 1, K = NN * C;
-  const unsigned full = 0xffffffffu;
-  const unsigned valid = __ballot_sync(full, key >= 0);
-  if (valid == 0u) return;
-  const unsigned grp = __match_any_sync(full, key);
-  const bool leader = key >= 0 && lane == __ffs(grp) - 1;
-  const int ngroups = __popc(__ballot_sync(full, leader));
-  if (ngroups <= 4) {
-    unsigned rem = valid;
-    while (rem) {  // warp-uniform
-      const int l0 = __ffs(rem) - 1;
-      const int gk = __shfl_sync(full, key, l0);
-      const int g0 = __shfl_sync(full, f[0], l0);
-      const int g1 = D == 2 ? __shfl_sync(full, f[1], l0) : 0;
-      const bool in = key == gk;
-      const unsigned gm = __ballot_sync(full, in);
-      float a[K];
-#pragma unroll
-      for (int a1 = 0; a1 < (D == 2 ? 4 : 1); a1++)
-#pragma unroll
-        for (int a0 = 0; a0 < 4; a0++) {
-          const float wt = in ? (D == 2 ? w[1][a1] : 1.f) * w[0][a0] : 0.f;
-          const int nd = a1 * 4 + a0;
-          a[nd * C] = wt;
-#pragma unroll
-          for (int k = 0; k < D; k++) a[nd * C + 1 + k] = wt * qc[k];
-        }
-      int base = 0;
-      warp_multi_sum<K, 16>(a, lane, base);
-      if ((lane & wsum_full_mask(K, 16)) == 0) {
-#pragma unroll
-        for (int q = 0; q < wsum_count(K, 16); q++) {
-          const int idx = base + q, nd = idx / C, ch = idx % C;
-          const int node = g0 + (nd & 3) + (D == 2 ? N * (g1 + (nd >> 2)) : 0);
-          atomicAdd(&Vs[ch * nodes + node], a[q]);
-        }
-      }
-      rem &= ~gm;
-    }
-  } else if (key >= 0) {
-#pragma unroll
-    for (int a1 = 0; a1 < (D == 2 ? 4 : 1); a1++)
-#pragma unroll
-      for (int a0 = 0; a0 < 4; a0++) {
-        const float wt = (D == 2 ? w[1][a1] : 1.f) * w[0][a0];
-        const int node = f[0] + a0 + (D == 2 ? N * (f[1] + a1) : 0);
-        atomicAdd(&Vs[node], wt);
-#pragma unroll
-        for (int k = 0; k < D; k++) atomicAdd(&Vs[(k + 1) * nodes + node], wt * qc[k]);
-      }
-  }
-}
-
-template <int D>
-__device__ __forceinline__ void k_s2g_direct_body(int vb_, int vg_, const typename Vec<D>::T *__restrict__ Y,
-                                                  int n, SgtState *st,
-                                                  typename Node<D>::T *__restrict__ V) {
-  static_assert(D <= 2, "direct mode is for d <= 2");
-  sgt_pdl_wait();
-  if (st->T != 0) return;  // cell and tile modes: the sort and k_s2g* do it
-  extern __shared__ float sgt_direct_grid[];
-  float *Vs = sgt_direct_grid;
-  constexpr int C = D + 1;
-  const int N = st->N, cells = N - 3;
-  const int nodes = D == 1 ? N : N * N;
-  const float maxy = st->maxy, scale = st->scale, hc = 0.5f * maxy;
-  float miny[2];
-#pragma unroll
-  for (int k = 0; k < D; k++) miny[k] = st->miny[k];
-  for (int e = threadIdx.x; e < C * nodes; e += blockDim.x) Vs[e] = 0.f;
-  __syncthreads();
-  const int per = (n + vg_ - 1) / vg_;
-  const int lo = vb_ * per, hi = min(n, lo + per);
-  const int lane = threadIdx.x & 31;
-  constexpr int U = SGT_PTS_U;
-  for (int i0 = lo + (threadIdx.x & ~31) * U; i0 < hi; i0 += blockDim.x * U) {
-    typename Vec<D>::T yv[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int i = i0 + 32 * u + lane;
-      if (i < hi) yv[u] = Y[i];
-    }
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int i = i0 + 32 * u + lane;
-      int key = -1;
-      int f[2] = {0, 0};
-      float w[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, qc[2] = {0.f, 0.f};
-      if (i < hi) {
-#pragma unroll
-        for (int k = 0; k < D; k++) {
-          float sh;
-          const float sv = sgt_scale(comp<D>(yv[u], k), miny[k], maxy, scale, sh);
-          sgt_weights(sv, f[k], w[k]);
-          qc[k] = sh - hc;
-        }
-        key = D == 1 ? f[0] : f[0] + cells * f[1];
-        if ((unsigned)f[0] >= (unsigned)cells || (D == 2 && (unsigned)f[1] >= (unsigned)cells)) {
-          atomicOr(&st->error, SGT_EFLAG_CHUNK_OVERFLOW);  // outside the grid: skip the point
-          key = -1;
-        }
-      }
-      s2g_direct_warp<D>(Vs, N, nodes, key, f, w, qc, lane);
-    }
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < nodes; e += blockDim.x) {
-    const float a0 = Vs[e], a1 = Vs[nodes + e], a2 = D == 2 ? Vs[2 * nodes + e] : 0.f;
-    if (a0 == 0.f && a1 == 0.f && a2 == 0.f) continue;
-    if constexpr (D == 1) atomicAdd(&V[e], make_float2(a0, a1));
-    else atomicAdd(&V[e], make_float4(a0, a1, a2, 0.f));
-  }
-}
-template <int D>
-__global__ void __launch_bounds__(SGT_THREADS)
-k_s2g_direct(const typename Vec<D>::T *__restrict__ Y, int n, SgtState *st,
-             typename Node<D>::T *__restrict__ V) {
-  k_s2g_direct_body<D>(blockIdx.x, gridDim.x, Y, n, st, V);
-}
-
-// ---------------------------------------------------------------------------
-// bin_scatter: counting-sort points into tile order.  Each CTA owns a
+// bin_scatter: counting-sort points into cell order (cell mode).  Each CTA owns a
 // contiguous range; it counts per tile, reserves its slots with one global
 // atomic per touched tile, then places its points.
 // sorted[p] = (y_0, y_1, y_2 | idx) with idx in the .w bits (.z for d <= 2
@@ -587,8 +578,8 @@ __device__ __forceinline__ void k_bin_scatter_body(int vb_, int vg_, const typen
               int *__restrict__ cursor, float4 *__restrict__ sorted) {
   sgt_pdl_wait();
   __shared__ int lc[SGT_HIST_MAX];
-  if (st->T == 0) return;  // direct mode: k_s2g_direct does the S2G
-  const int ntiles = st->ntiles, T = st->T, td = st->tiles_dim;
+  if (st->T == 0) return;  // scatter mode: no sort
+  const int ntiles = st->ntiles, td = st->tiles_dim;
   const float maxy = st->maxy, scale = st->scale;
   float miny[3];
 #pragma unroll
@@ -623,7 +614,7 @@ __device__ __forceinline__ void k_bin_scatter_body(int vb_, int vg_, const typen
           float sh;
           f[k] = (int)floorf(sgt_scale(comp<D>(yv[u], k), miny[k], maxy, scale, sh));
         }
-        key = sgt_tile_of<D>(f, T, td);
+        key = sgt_cell_of<D>(f, td);
       }
       const unsigned grp = __match_any_sync(0xffffffffu, key);
       if (key >= 0 && lane == __ffs(grp) - 1) atomicAdd(&lc[key], __popc(grp));
@@ -654,7 +645,7 @@ __device__ __forceinline__ void k_bin_scatter_body(int vb_, int vg_, const typen
           f[k] = (int)floorf(sgt_scale(v, miny[k], maxy, scale, sh));
           if (k == 0) rec.x = v; else if (k == 1) rec.y = v; else rec.z = v;
         }
-        key = sgt_tile_of<D>(f, T, td);
+        key = sgt_cell_of<D>(f, td);
       }
       const unsigned grp = __match_any_sync(0xffffffffu, key);
       const int leader = __ffs(grp) - 1;
@@ -672,9 +663,7 @@ k_bin_scatter(const typename Vec<D>::T *__restrict__ Y, int n, SgtState *st,
   k_bin_scatter_body<D>(blockIdx.x, gridDim.x, Y, n, st, cursor, sorted);
 }
 
-// ---------------------------------------------------------------------------
-// S2G over chunks of sorted points; one shared-memory tile per chunk.
-// ---------------------------------------------------------------------------
+// cells and weights of a sorted point
 template <int D>
 __device__ __forceinline__ void sgt_point_stencil(const float4 &rec,
                                                   const float *miny, float maxy,
@@ -688,167 +677,6 @@ __device__ __forceinline__ void sgt_point_stencil(const float4 &rec,
   }
 }
 
-// TT: the tile edge this instance handles; the instances of the other tile
-// edges (and k_s2g_cell in cell mode) return at once.
-template <int D, int TT>
-__device__ __forceinline__ void k_s2g_body(int vb_, int vg_, const float4 *__restrict__ sorted, SgtState *st,
-      const int4 *__restrict__ chunks, typename Node<D>::T *__restrict__ V) {
-  sgt_pdl_wait();
-  extern __shared__ float acc[];  // [D+1][R^D]
-  const int T = st->T, td = st->tiles_dim, N = st->N, nch = st->nchunks;
-  if (T != TT) return;
-  const float maxy = st->maxy, scale = st->scale;
-  // charges are taken about the middle of the grid: F and Z are invariant to
-  // the origin of y, and |y - c| <= maxy/2 halves the cancellation in
-  // (1 + 2|y|^2) Phi0 - 2 y.Phi
-  const float hc = 0.5f * maxy;
-  float miny[3];
-#pragma unroll
-  for (int k = 0; k < D; k++) miny[k] = st->miny[k];
-  const int R = T + 3;
-  int RD = R;
-  if (D >= 2) RD *= R;
-  if (D >= 3) RD *= R;
-  constexpr int m = D + 1;
-  for (int c = vb_; c < nch; c += vg_) {
-    const int4 ch = chunks[c];
-    int o[3] = {0, 0, 0};
-    o[0] = (ch.x % td) * T;
-    if (D >= 2) o[1] = ((ch.x / td) % td) * T;
-    if (D >= 3) o[2] = (ch.x / (td * td)) * T;
-    for (int e = threadIdx.x; e < m * RD; e += blockDim.x) acc[e] = 0.f;
-    __syncthreads();
-    if constexpr (D == 3) {
-      // The lanes of a warp share one point at a time, each owning 2 of its
-      // 64 stencil nodes, so the 32 atomics of an instruction go to 32
-      // distinct nodes.  (With a point per thread, the points of a cluster
-      // sit in few cells and all lanes of a warp collide on the same nodes.)
-      // Points come 32 per warp in one coalesced load; each lane computes
-      // the stencil of its own point and the warp hands the stencils round
-      // by shuffles.
-      const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-      const int a0 = lane & 3, a1 = (lane >> 2) & 3, a2b = lane >> 4;
-      for (int j0 = ch.y + 32 * wid; j0 < ch.y + ch.z; j0 += 32 * nw) {
-        const int jm = min(32, ch.y + ch.z - j0);
-        int f[3] = {0, 0, 0};
-        float w[3][4], ys[3];
-        int node0 = -1;  // this lane's point: base node in the tile, -1 if none
-        if (lane < jm) {
-          const float4 rec = sorted[j0 + lane];
-          sgt_point_stencil<D>(rec, miny, maxy, scale, f, w, ys);
-          const int l0 = f[0] - o[0], l1 = f[1] - o[1], l2 = f[2] - o[2];
-          if ((unsigned)l0 < (unsigned)T && (unsigned)l1 < (unsigned)T &&
-              (unsigned)l2 < (unsigned)T) {
-            node0 = l0 + R * (l1 + R * l2);
-          } else {  // the sort and the binning disagree: skip the point
-            atomicOr(&st->error, SGT_EFLAG_CHUNK_OVERFLOW);
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < 3; k++) {
-            ys[k] = 0.f;
-#pragma unroll
-            for (int a = 0; a < 4; a++) w[k][a] = 0.f;
-          }
-        }
-        for (int t = 0; t < jm; t++) {
-          const int nb = __shfl_sync(0xffffffffu, node0, t);
-          float wx[4], wy4[4], wz4[4], qc[3];
-#pragma unroll
-          for (int a = 0; a < 4; a++) {
-            wx[a] = __shfl_sync(0xffffffffu, w[0][a], t);
-            wy4[a] = __shfl_sync(0xffffffffu, w[1][a], t);
-            wz4[a] = __shfl_sync(0xffffffffu, w[2][a], t);
-          }
-#pragma unroll
-          for (int k = 0; k < 3; k++) qc[k] = __shfl_sync(0xffffffffu, ys[k], t) - hc;
-          if (nb < 0) continue;  // uniform over the warp
-          const float w0 = a0 == 0 ? wx[0] : (a0 == 1 ? wx[1] : (a0 == 2 ? wx[2] : wx[3]));
-          const float w1 = a1 == 0 ? wy4[0] : (a1 == 1 ? wy4[1] : (a1 == 2 ? wy4[2] : wy4[3]));
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            const int a2 = a2b + 2 * h;
-            const float w2 = a2 == 0 ? wz4[0] : (a2 == 1 ? wz4[1] : (a2 == 2 ? wz4[2] : wz4[3]));
-            const float wt = (w1 * w2) * w0;  // the product order of the loop below
-            const int node = nb + a0 + R * (a1 + R * a2);
-            atomicAdd(&acc[node], wt);
-#pragma unroll
-            for (int k = 0; k < 3; k++) atomicAdd(&acc[(k + 1) * RD + node], wt * qc[k]);
-          }
-        }
-      }
-    } else {
-    // each thread walks its own contiguous stretch of the chunk, so the lanes
-    // of a warp sit far apart in the (spatially ordered) chunk and their
-    // shared-memory atomics rarely meet on one node
-    const int per = (ch.z + blockDim.x - 1) / blockDim.x;
-    const int jb = ch.y + threadIdx.x * per, je = min(jb + per, ch.y + ch.z);
-    for (int j = jb; j < je; j++) {
-      const float4 rec = sorted[j];
-      int f[3];
-      float w[3][4], ys[3];
-      sgt_point_stencil<D>(rec, miny, maxy, scale, f, w, ys);
-      const int l0 = f[0] - o[0];
-      const int l1 = D >= 2 ? f[1] - o[1] : 0;
-      const int l2 = D >= 3 ? f[2] - o[2] : 0;
-      // a point outside its tile would mean the sort and the binning
-      // disagree; skip it rather than touch memory outside the tile
-      if ((unsigned)l0 >= (unsigned)T || (unsigned)l1 >= (unsigned)T ||
-          (unsigned)l2 >= (unsigned)T) {
-        atomicOr(&st->error, SGT_EFLAG_CHUNK_OVERFLOW);
-        continue;
-      }
-#pragma unroll
-      for (int a2 = 0; a2 < (D >= 3 ? 4 : 1); a2++)
-#pragma unroll
-        for (int a1 = 0; a1 < (D >= 2 ? 4 : 1); a1++) {
-          float wy = 1.f;
-          if (D >= 2) wy *= w[1][a1];
-          if (D >= 3) wy *= w[2][a2];
-          const int rowbase = (l0) + R * ((l1 + a1) + R * (l2 + a2));
-#pragma unroll
-          for (int a0 = 0; a0 < 4; a0++) {
-            const float wt = wy * w[0][a0];
-            const int node = rowbase + a0;
-            atomicAdd(&acc[node], wt);
-#pragma unroll
-            for (int k = 0; k < D; k++) atomicAdd(&acc[(k + 1) * RD + node], wt * (ys[k] - hc));
-          }
-        }
-    }
-    }
-    __syncthreads();
-    // flush the touched region of this tile into V
-    for (int e = threadIdx.x; e < RD; e += blockDim.x) {
-      const int lx = e % R;
-      const int ly = D >= 2 ? (e / R) % R : 0;
-      const int lz = D >= 3 ? e / (R * R) : 0;
-      const int gx = o[0] + lx, gy = o[1] + ly, gz = o[2] + lz;
-      if (gx >= N || (D >= 2 && gy >= N) || (D >= 3 && gz >= N)) continue;
-      const float a0 = acc[e];
-      const float a1 = acc[RD + e];
-      const float a2 = D >= 2 ? acc[2 * RD + e] : 0.f;
-      const float a3 = D >= 3 ? acc[3 * RD + e] : 0.f;
-      if (a0 == 0.f && a1 == 0.f && a2 == 0.f && a3 == 0.f) continue;
-      long g = gx;
-      if (D >= 2) g += (long)N * gy;
-      if (D >= 3) g += (long)N * N * gz;
-      if constexpr (D == 1) {
-        atomicAdd(&V[g], make_float2(a0, a1));
-      } else {
-        atomicAdd(&V[g], make_float4(a0, a1, a2, a3));
-      }
-    }
-    __syncthreads();
-  }
-}
-template <int D, int TT>
-__global__ void __launch_bounds__(SGT_THREADS)
-k_s2g(const float4 *__restrict__ sorted, SgtState *st,
-      const int4 *__restrict__ chunks, typename Node<D>::T *__restrict__ V) {
-  k_s2g_body<D, TT>(blockIdx.x, gridDim.x, sorted, st, chunks, V);
-}
-
 // ---------------------------------------------------------------------------
 // S2G in cell mode (T = 1): every point of a chunk lies in the chunk's cell,
 // so all of them touch the same 4^d nodes.  Each thread sums its points'
@@ -860,7 +688,7 @@ template <int D>
 __device__ __forceinline__ void k_s2g_cell_body(int vb_, int vg_, const float4 *__restrict__ sorted, SgtState *st,
            const int4 *__restrict__ chunks, typename Node<D>::T *__restrict__ V) {
   sgt_pdl_wait();
-  if (st->T != 1) return;  // tile mode: k_s2g does the work
+  if (st->T != 1) return;  // scatter mode: k_scatter did the S2G
   constexpr int NN = D == 1 ? 4 : 16;  // stencil nodes per pass
   constexpr int C = D + 1;             // charge channels
   constexpr int K = NN * C;
@@ -869,7 +697,7 @@ __device__ __forceinline__ void k_s2g_cell_body(int vb_, int vg_, const float4 *
   __shared__ float red[SGT_THREADS / 32][K];
   const int td = st->tiles_dim, N = st->N, nch = st->nchunks;
   const float maxy = st->maxy, scale = st->scale;
-  const float hc = 0.5f * maxy;  // charge origin, as in k_s2g
+  const float hc = 0.5f * maxy;  // charge origin, as in k_scatter
   float miny[3];
 #pragma unroll
   for (int k = 0; k < D; k++) miny[k] = st->miny[k];
@@ -958,9 +786,9 @@ k_s2g_cell(const float4 *__restrict__ sorted, SgtState *st,
 }
 
 // Interpolated potentials p[0..d] at a point with stencil weights w and base
-// cell f: from a grid Phi (in global or shared memory), or (SM) from the
-// block's copy cn of the 4^d nodes of the point's cell, node a0 + 4 a1 +
-// 16 a2.  Same products in the same order either way.
+// cell f: from the grid Phi, or (SM) from the block's copy cn of the 4^d
+// nodes of the point's cell, node a0 + 4 a1 + 16 a2.  Same products in the
+// same order either way.
 template <int D, bool SM>
 __device__ __forceinline__ void g2s_potentials(const float (*w)[4], const int *f, int N,
                                                const typename Node<D>::T *Phi,
@@ -1024,15 +852,121 @@ __device__ __forceinline__ void g2s_finish(int vb_, int vg_, SgtState *st, doubl
 }
 
 // ---------------------------------------------------------------------------
-// G2S over chunks + repulsive force numerator + Z (FP64, fixed-order finish).
+// G2S + repulsive force numerator + Z (FP64, fixed-order finish).
 // Frep_un[i] = y_i*Phi0 - Phi_{1..d}; Z = sum_i z_i - n.
+// Scatter mode: the points in their own order, SGT_LPP(D) lanes per point.
+// Lane q reads the nodes it would scatter to (a stencil row is one 64-byte
+// request) and the group sums the potentials by shuffles; its first lane
+// forms F and the point's Z.
 // ---------------------------------------------------------------------------
+template <int D>
+__device__ __forceinline__ void k_gather_body(int vb_, int vg_, SgtState *st,
+                                              const typename Node<D>::T *__restrict__ Phi,
+                                              typename Vec<D>::T *__restrict__ Frep_un,
+                                              double *part_z, int n,
+                                              const typename Vec<D>::T *__restrict__ Y) {
+  sgt_pdl_wait();
+  if (st->T != 0) return;  // cell mode: k_g2s
+  __shared__ double wz[SGT_THREADS / 32];
+  __shared__ bool last;
+  constexpr int L = SGT_LPP(D);
+  const int N = st->N, cells = N - 3;
+  const float maxy = st->maxy, scale = st->scale, hc = 0.5f * maxy;
+  float miny[3];
+#pragma unroll
+  for (int k = 0; k < D; k++) miny[k] = st->miny[k];
+  double zacc = 0.0;
+  const int q = threadIdx.x % L, qx = q & 3;
+  const int step = vg_ * (SGT_THREADS / L);
+  const int rounds = (n + step - 1) / step;  // uniform, so that the shuffles converge
+  int i = vb_ * (SGT_THREADS / L) + threadIdx.x / L;
+  for (int r = 0; r < rounds; r++, i += step) {
+    float p[4] = {0.f, 0.f, 0.f, 0.f}, ys[3] = {0.f, 0.f, 0.f};
+    if (i < n) {
+      const typename Vec<D>::T y = Y[i];
+      int f[3];
+      float w[3][4];
+      bool ok = true;
+#pragma unroll
+      for (int k = 0; k < D; k++) {
+        const float sv = sgt_scale(comp<D>(y, k), miny[k], maxy, scale, ys[k]);
+        sgt_weights(sv, f[k], w[k]);
+        ok = ok && (unsigned)f[k] < (unsigned)cells;
+      }
+      if (!ok) {  // outside the grid (S2G skipped it too): no force, no Z
+        if (q == 0) atomicOr(&st->error, SGT_EFLAG_CHUNK_OVERFLOW);
+      } else {
+        const float wx = pick4(w[0], qx);
+        if constexpr (D == 1) {
+          const float2 v = Phi[f[0] + qx];
+          p[0] = wx * v.x;
+          p[1] = wx * v.y;
+        } else if constexpr (D == 2) {
+          float4 v[4];
+#pragma unroll
+          for (int b = 0; b < 4; b++) v[b] = Phi[f[0] + qx + N * (f[1] + b)];
+#pragma unroll
+          for (int b = 0; b < 4; b++) {
+            const float wt = w[1][b] * wx;
+            p[0] += wt * v[b].x;
+            p[1] += wt * v[b].y;
+            p[2] += wt * v[b].z;
+          }
+        } else {
+          const int qy = q >> 2;
+          const float wy = pick4(w[1], qy);
+          float4 v[4];
+#pragma unroll
+          for (int c = 0; c < 4; c++)
+            v[c] = Phi[f[0] + qx + (long)N * (f[1] + qy + (long)N * (f[2] + c))];
+#pragma unroll
+          for (int c = 0; c < 4; c++) {
+            const float wt = (wy * w[2][c]) * wx;
+            p[0] += wt * v[c].x;
+            p[1] += wt * v[c].y;
+            p[2] += wt * v[c].z;
+            p[3] += wt * v[c].w;
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < L; o *= 2)
+#pragma unroll
+      for (int k = 0; k <= D; k++) p[k] += __shfl_xor_sync(0xffffffffu, p[k], o);
+    if (i < n && q == 0) {
+      double ysq = 0.0, dot = 0.0;
+      typename Vec<D>::T fr;
+      if constexpr (D == 3) fr.w = 0.f;
+#pragma unroll
+      for (int k = 0; k < D; k++) {
+        const float yk = ys[k] - hc;
+        ysq += (double)yk * yk;
+        dot += (double)yk * p[k + 1];
+        setcomp<D>(fr, k, yk * p[0] - p[k + 1]);
+      }
+      zacc += (1.0 + 2.0 * ysq) * (double)p[0] - 2.0 * dot;
+      Frep_un[i] = fr;
+    }
+  }
+  g2s_finish(vb_, vg_, st, part_z, n, zacc, wz, last);
+}
+template <int D>
+__global__ void __launch_bounds__(SGT_THREADS, 6)
+k_gather(SgtState *st, const typename Node<D>::T *__restrict__ Phi,
+         typename Vec<D>::T *__restrict__ Frep_un, double *part_z, int n,
+         const typename Vec<D>::T *__restrict__ Y) {
+  k_gather_body<D>(blockIdx.x, gridDim.x, st, Phi, Frep_un, part_z, n, Y);
+}
+
+// Cell mode: the same over the chunks of sorted points.
 template <int D>
 __device__ __forceinline__ void k_g2s_body(int vb_, int vg_, const float4 *__restrict__ sorted, SgtState *st,
       const int4 *__restrict__ chunks,
       const typename Node<D>::T *__restrict__ Phi,
       typename Vec<D>::T *__restrict__ Frep_un, double *part_z, int n) {
   sgt_pdl_wait();
+  if (st->T == 0) return;  // scatter mode: k_gather
   __shared__ double wz[SGT_THREADS / 32];
   __shared__ bool last;
   const int N = st->N, nch = st->nchunks;
@@ -1041,30 +975,26 @@ __device__ __forceinline__ void k_g2s_body(int vb_, int vg_, const float4 *__res
   float miny[3];
 #pragma unroll
   for (int k = 0; k < D; k++) miny[k] = st->miny[k];
-  if (st->T == 0) return;  // direct mode: k_g2s_direct does the G2S
   double zacc = 0.0;
-  // cell mode (T = 1): every point of a chunk reads the same 4^d nodes,
-  // which the block stages once per chunk in shared memory
+  // every point of a chunk reads the same 4^d nodes, which the
+  // block stages once per chunk in shared memory
   constexpr int NNODES = D == 1 ? 4 : (D == 2 ? 16 : 64);
   __shared__ typename Node<D>::T cn[NNODES];
-  const bool cell = st->T == 1;
   const int td = st->tiles_dim;
   for (int c = vb_; c < nch; c += vg_) {
     const int4 ch = chunks[c];
-    int cf[3] = {-1, -1, -1};
-    if (cell) {  // block-uniform
-      cf[0] = ch.x % td;
-      if (D >= 2) cf[1] = (ch.x / td) % td;
-      if (D >= 3) cf[2] = ch.x / (td * td);
-      __syncthreads();  // the previous chunk's points are done with cn
-      for (int e = threadIdx.x; e < NNODES; e += blockDim.x) {
-        long g = cf[0] + (e & 3);
-        if (D >= 2) g += (long)N * (cf[1] + ((e >> 2) & 3));
-        if (D >= 3) g += (long)N * N * (cf[2] + (e >> 4));
-        cn[e] = Phi[g];
-      }
-      __syncthreads();
+    int cf[3] = {0, 0, 0};
+    cf[0] = ch.x % td;
+    if (D >= 2) cf[1] = (ch.x / td) % td;
+    if (D >= 3) cf[2] = ch.x / (td * td);
+    __syncthreads();  // the previous chunk's points are done with cn
+    for (int e = threadIdx.x; e < NNODES; e += blockDim.x) {
+      long g = cf[0] + (e & 3);
+      if (D >= 2) g += (long)N * (cf[1] + ((e >> 2) & 3));
+      if (D >= 3) g += (long)N * N * (cf[2] + (e >> 4));
+      cn[e] = Phi[g];
     }
+    __syncthreads();
     constexpr int U = SGT_PTS_U;
     const int end = ch.y + ch.z;
     for (int j0 = ch.y + threadIdx.x; j0 < end; j0 += U * blockDim.x) {
@@ -1081,7 +1011,7 @@ __device__ __forceinline__ void k_g2s_body(int vb_, int vg_, const float4 *__res
         int f[3];
         float w[3][4], ys[3];
         sgt_point_stencil<D>(rec, miny, maxy, scale, f, w, ys);
-        bool here = cell && f[0] == cf[0];
+        bool here = f[0] == cf[0];
         if (D >= 2) here = here && f[1] == cf[1];
         if (D >= 3) here = here && f[2] == cf[2];
         float p[4] = {0.f, 0.f, 0.f, 0.f};
@@ -1110,82 +1040,6 @@ k_g2s(const float4 *__restrict__ sorted, SgtState *st,
       const typename Node<D>::T *__restrict__ Phi,
       typename Vec<D>::T *__restrict__ Frep_un, double *part_z, int n) {
   k_g2s_body<D>(blockIdx.x, gridDim.x, sorted, st, chunks, Phi, Frep_un, part_z, n);
-}
-
-// ---------------------------------------------------------------------------
-// Direct-mode G2S (T = 0): the points in their own order, the whole potential
-// grid staged in shared memory, F written in place (coalesced), Z as in
-// k_g2s.
-// ---------------------------------------------------------------------------
-template <int D>
-__device__ __forceinline__ void k_g2s_direct_body(int vb_, int vg_, SgtState *st,
-      const typename Node<D>::T *__restrict__ Phi,
-      typename Vec<D>::T *__restrict__ Frep_un, double *part_z, int n,
-      const typename Vec<D>::T *__restrict__ Y) {
-  static_assert(D <= 2, "direct mode is for d <= 2");
-  sgt_pdl_wait();
-  __shared__ double wz[SGT_THREADS / 32];
-  __shared__ bool last;
-  if (st->T != 0) return;  // cell and tile modes: k_g2s does it
-  const int N = st->N;
-  const float maxy = st->maxy, scale = st->scale;
-  const float hc = 0.5f * maxy;
-  float miny[3];
-#pragma unroll
-  for (int k = 0; k < D; k++) miny[k] = st->miny[k];
-  double zacc = 0.0;
-  extern __shared__ float4 sgt_g2s_smem[];
-  typename Node<D>::T *Ps = reinterpret_cast<typename Node<D>::T *>(sgt_g2s_smem);
-  const int nodes = D == 1 ? N : N * N;
-  for (int e = threadIdx.x; e < nodes; e += blockDim.x) Ps[e] = Phi[e];
-  __syncthreads();
-  constexpr int U = SGT_PTS_U;
-  const int lane = threadIdx.x & 31;
-  const long stride = (long)vg_ * blockDim.x * U;
-  for (long i0 = ((long)vb_ * blockDim.x + (threadIdx.x & ~31)) * U; i0 < n; i0 += stride) {
-    typename Vec<D>::T yv[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const long i = i0 + 32 * u + lane;
-      if (i < n) yv[u] = Y[i];
-    }
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const long i = i0 + 32 * u + lane;
-      if (i >= n) break;
-      int f[3];
-      float w[3][4], ys[3];
-#pragma unroll
-      for (int k = 0; k < D; k++) {
-        const float sv = sgt_scale(comp<D>(yv[u], k), miny[k], maxy, scale, ys[k]);
-        sgt_weights(sv, f[k], w[k]);
-      }
-      float p[4] = {0.f, 0.f, 0.f, 0.f};
-      if ((unsigned)f[0] < (unsigned)(N - 3) && (D == 1 || (unsigned)f[1] < (unsigned)(N - 3)))
-        g2s_potentials<D, false>(w, f, N, Ps, Ps, p);
-      else  // outside the grid (S2G skipped it too): no force, no Z
-        atomicOr(&st->error, SGT_EFLAG_CHUNK_OVERFLOW);
-      double ysq = 0.0, dot = 0.0;
-      typename Vec<D>::T fr;
-#pragma unroll
-      for (int k = 0; k < D; k++) {
-        const float yk = ys[k] - hc;
-        ysq += (double)yk * yk;
-        dot += (double)yk * p[k + 1];
-        setcomp<D>(fr, k, yk * p[0] - p[k + 1]);
-      }
-      zacc += (1.0 + 2.0 * ysq) * (double)p[0] - 2.0 * dot;
-      Frep_un[i] = fr;
-    }
-  }
-  g2s_finish(vb_, vg_, st, part_z, n, zacc, wz, last);
-}
-template <int D>
-__global__ void __launch_bounds__(SGT_THREADS)
-k_g2s_direct(SgtState *st, const typename Node<D>::T *__restrict__ Phi,
-             typename Vec<D>::T *__restrict__ Frep_un, double *part_z, int n,
-             const typename Vec<D>::T *__restrict__ Y) {
-  k_g2s_direct_body<D>(blockIdx.x, gridDim.x, st, Phi, Frep_un, part_z, n, Y);
 }
 
 // ---------------------------------------------------------------------------

@@ -19,7 +19,7 @@ struct SgtJobView {
   const void *Ynext_c;
   void *Ynext, *Y, *uY, *gains, *Frep, *Fattr;
   float4 *sorted;
-  void *V, *Phi;
+  void *V, *Vc, *Phi;
   float2 *W;
   int *tile_count, *cursor;
   int4 *chunks;
@@ -56,7 +56,16 @@ km_bin_count(const SgtJobView *__restrict__ views, const int *__restrict__ prefi
   SGT_MULTI_JOB
   typedef typename Vec<D>::T VT;
   k_bin_count_body<D>(vb, vg, (const VT *)v.Ynext_c, (VT *)v.Y, v.n, v.st, v.tile_count,
-                      (typename Node<D>::T *)v.V, 1, v.jp, v.cursor, v.chunks, v.nb_s2g);
+                      (typename Node<D>::T *)v.V, v.jp, v.cursor, v.chunks, v.nb_s2g);
+}
+
+template <int D>
+__global__ void __launch_bounds__(SGT_THREADS, 8)
+km_scatter(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
+  SGT_MULTI_JOB
+  typedef typename Vec<D>::T VT;
+  k_scatter_body<D>(vb, vg, (const VT *)v.Ynext_c, (VT *)v.Y, v.n, v.st,
+                    (typename Node<D>::T *)v.Vc);
 }
 
 template <int D>
@@ -68,17 +77,9 @@ km_bin_scatter(const SgtJobView *__restrict__ views, const int *__restrict__ pre
 
 template <int D>
 __global__ void __launch_bounds__(SGT_THREADS)
-km_s2g_direct(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
+km_fold(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
   SGT_MULTI_JOB
-  k_s2g_direct_body<D>(vb, vg, (const typename Vec<D>::T *)v.Y, v.n, v.st,
-                       (typename Node<D>::T *)v.V);
-}
-
-template <int D, int TT>
-__global__ void __launch_bounds__(SGT_THREADS)
-km_s2g(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
-  SGT_MULTI_JOB
-  k_s2g_body<D, TT>(vb, vg, v.sorted, v.st, v.chunks, (typename Node<D>::T *)v.V);
+  k_fold_body<D>(vb, vg, v.st, (typename Node<D>::T *)v.Vc, (typename Node<D>::T *)v.V);
 }
 
 template <int D>
@@ -126,12 +127,12 @@ km_g2s(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int
 }
 
 template <int D>
-__global__ void __launch_bounds__(SGT_THREADS)
-km_g2s_direct(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
+__global__ void __launch_bounds__(SGT_THREADS, 6)
+km_gather(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
   SGT_MULTI_JOB
   typedef typename Vec<D>::T VT;
-  k_g2s_direct_body<D>(vb, vg, v.st, (const typename Node<D>::T *)v.Phi, (VT *)v.Frep, v.part_z,
-                       v.n, (const VT *)v.Y);
+  k_gather_body<D>(vb, vg, v.st, (const typename Node<D>::T *)v.Phi, (VT *)v.Frep, v.part_z, v.n,
+                   (const VT *)v.Y);
 }
 
 template <int D, int G>
