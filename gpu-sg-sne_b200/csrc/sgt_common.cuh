@@ -20,8 +20,8 @@
 #define SGT_THREADS 256
 
 // Lagrange cubic weights on 4 nodes (CU/gridding.cuh:13-22,
-// HYB/gridding.cpp:29-39).  Node f+a gets w[a]; the point lies between
-// nodes f+1 and f+2.
+// HYB/gridding.cpp:29-39).  The point at place dd of cell f lies between
+// nodes f+1 and f+2; node f+a gets w[a].
 __device__ __forceinline__ float sgt_l1(float x) {
   return 0.5f * x * x * x - 1.0f * x * x - 0.5f * x + 1.0f;
 }
@@ -29,10 +29,7 @@ __device__ __forceinline__ float sgt_l2(float x) {
   const float cc = 1.0f / 6.0f;
   return -cc * x * x * x + 1.0f * x * x - 11.0f * cc * x + 1.0f;
 }
-__device__ __forceinline__ void sgt_weights(float s, int &f, float w[4]) {
-  const float fl = floorf(s);
-  f = (int)fl;
-  const float dd = s - fl;
+__device__ __forceinline__ void sgt_weights(float dd, float w[4]) {
   w[0] = sgt_l2(1.0f + dd);
   w[1] = sgt_l1(dd);
   w[2] = sgt_l1(1.0f - dd);
@@ -47,6 +44,8 @@ struct SgtState {
   float mean[4];     // mean subtracted from Ynext when forming Y
   float maxy;        // max shifted coordinate over all dims
   float scale;       // float(N - 3): scaled coords lie in [0, N-3)
+  float inv_hi, inv_lo;  // scale / maxy in two terms
+  int direct;        // 1: k_spec_* convolve this grid, 0: the FFT passes do
   float h_eff;       // grid spacing in embedding units
   int N;             // grid points per axis (n1 + 2)
   int M;             // FFT length per axis (2^k or 3 * 2^k, >= 2N-1)
@@ -90,6 +89,7 @@ struct SgtJobParams {
   long vc_nodes;      // nodes held by the grid copies of the scatter mode
   int chunk_cap;      // max chunks held by the chunk array
   int chunk_min;      // fewest points per S2G chunk (0: 1024, 256 in 3-D)
+  int conv_max;       // largest N that k_spec_* convolve
   int cell_blocks;    // blocks that work in cell mode (0: no cell mode)
 };
 
@@ -150,6 +150,42 @@ __device__ __forceinline__ float warp_max_f(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
+}
+
+// Sums K per-lane values over the lanes of a warp that differ in the bits up
+// to O (16: the whole warp) in K/2 + K/4 + ... shuffles instead of K per bit: at each step with offset O a lane keeps one half of
+// its values, sends the other half to lane ^ O and adds what it receives; once
+// the count no longer halves, the remaining offsets add whole vectors.  On
+// return acc[q], q < wsum_count(K, O), of lane L holds the warp total of the
+// entry values acc[base + q], with base (zero on entry) advanced by the call;
+// lanes that share a base hold the same totals, and the lanes with
+// (L & wsum_full_mask(K, O)) == 0 are one of each.
+__host__ __device__ constexpr int wsum_count(int k, int o) {
+  return o == 0 ? k : ((k % 2 == 0) ? wsum_count(k / 2, o / 2) : wsum_count(k, o / 2));
+}
+__host__ __device__ constexpr int wsum_full_mask(int k, int o) {
+  return o == 0 ? 0 : ((k % 2 == 0) ? wsum_full_mask(k / 2, o / 2) : (o | wsum_full_mask(k, o / 2)));
+}
+template <int K, int O>
+__device__ __forceinline__ void warp_multi_sum(float *acc, int lane, int &base) {
+  if constexpr (O > 0) {
+    if constexpr (K % 2 == 0) {
+      constexpr int H = K / 2;
+      const bool up = (lane & O) != 0;
+#pragma unroll
+      for (int q = 0; q < H; q++) {
+        const float send = up ? acc[q] : acc[q + H];
+        const float keep = up ? acc[q + H] : acc[q];
+        acc[q] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+      }
+      if (up) base += H;
+      warp_multi_sum<H, O / 2>(acc, lane, base);
+    } else {
+#pragma unroll
+      for (int q = 0; q < K; q++) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], O);
+      warp_multi_sum<K, O / 2>(acc, lane, base);
+    }
+  }
 }
 
 // The 137-entry size table shared with the reference (CU/utils.cu:197-207).

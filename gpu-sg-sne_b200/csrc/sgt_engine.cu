@@ -95,7 +95,7 @@ struct sgt_job {
   double *part_sum = nullptr, *part_z = nullptr, *part_kl = nullptr;
   SgtState *st = nullptr;
   SgtState *st_host = nullptr;
-  int nb_pts = 0, nb_scat = 0, nb_gath = 0, nb_fold = 0, nb_s2gc = 0, nb_g2s = 0, nb_fft = 0, nb_fft_rows = 0, nb_row = 0,
+  int nb_pts = 0, nb_scat = 0, nb_gath = 0, nb_spec = 0, nb_conv = 0, nb_s2gc = 0, nb_g2s = 0, nb_fft = 0, nb_fft_rows = 0, nb_row = 0,
       nb_upd = 0, nb_part = 0;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;  // the two branches of an iteration
   size_t smem_fft1 = 0, smem_fft2 = 0;
@@ -131,6 +131,7 @@ static sgt_status flag_status(sgt_ctx *ctx, int flags, int grid_points, const ch
 }
 cudaStream_t sgti_stream(sgt_ctx *ctx) { return ctx->stream; }
 int sgti_device(sgt_ctx *ctx) { return ctx->device; }
+int sgti_sm_count(sgt_ctx *ctx) { return ctx->nsm; }
 sgt_status sgti_fail(sgt_ctx *ctx, sgt_status s, const std::string &msg) { return fail(ctx, s, msg); }
 #define CK(call)                                                              \
   do {                                                                        \
@@ -405,11 +406,19 @@ static sgt_status job_shapes(sgt_job *J) {
   J->nb_s2gc = grid_blocks(nsm, occ);
   const int M = J->mmax;
   J->smem_fft1 = 0;
-  J->smem_fft2 = fft_cols_smem(M, D);
+  J->smem_fft2 = fft_cols_smem(M);
+  // spectra of the rows, and sums over the rows: a block per row (tile) of
+  // the largest grid they take
+  const int cm = J->jp.conv_max, ct = (cm + SGT_SPEC_TY(D) - 1) / SGT_SPEC_TY(D);
+  // (few blocks beside a long SpMV: even a block with nothing to do waits for
+  // a slot there)
+  const bool beside = J->nnz >= 3000000L;
+  J->nb_spec = D == 1 ? 2 : (D == 3 ? std::min(4 * nsm, cm * cm) : (beside ? 64 : cm));
+  J->nb_conv = D == 1 ? (cm + 7) / 8 : (D == 3 ? std::min(3 * nsm, cm * ct) : std::min(ct, beside ? 64 : cm));
   if constexpr (D == 1) {
     J->nb_fft = 1;
   } else {
-    const int fmax = (int)fft_cols_smem(SGT_FFT_MAXM, D);  // the largest job's
+    const int fmax = (int)fft_cols_smem(SGT_FFT_MAXM);  // the largest job's
     CK(cudaFuncSetAttribute(k_fft_cols<D, MODE_LAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, fmax));
     if constexpr (D == 3) {
       CK(cudaFuncSetAttribute(k_fft_cols<D, MODE_MID_FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, fmax));
@@ -444,12 +453,10 @@ static sgt_status job_shapes(sgt_job *J) {
   const long groups = ((long)J->n * SGT_LPP(D) + SGT_THREADS - 1) / SGT_THREADS;
   J->nb_scat = (int)std::min(groups, 8L * nsm);
   J->nb_gath = (int)std::min(groups, 6L * nsm);
-  J->nb_fold = 2 * nsm;
   // small embeddings launch no more blocks than there is work for: idle
   // blocks only take scheduling slots from the jobs that share the GPU
   const int cap = (int)std::max(1L, ((long)J->n + 255) / 256);
   J->nb_pts = std::min(J->nb_pts, cap);
-  J->nb_fold = std::min(J->nb_fold, cap);
   J->nb_s2gc = std::min(J->nb_s2gc, cap);
   J->nb_row = std::min(J->nb_row, cap);
   J->nb_upd = std::min(J->nb_upd, cap);
@@ -500,6 +507,7 @@ static sgt_status job_alloc(sgt_job *J) {
   J->jp.chunk_cap = J->n / 256 + SGT_HIST_MAX + 16;  // 3-D chunks may hold 256 points
   CKS(jalloc(J, &J->chunks, (size_t)J->jp.chunk_cap));
   J->jp.mmax = M;
+  J->jp.conv_max = std::min(J->nmax, SGT_SPEC_MAX(D));
   // the sort of the cell mode, for the jobs that can take it (a shard decides
   // by the points of the whole embedding); job_shapes sets its block count
   J->jp.cell_blocks = std::max(J->n, J->n_gather) >= SGT_CELL_MIN_N ? 1 : 0;
@@ -591,10 +599,9 @@ template <int D>
 static sgt_status enqueue_g2g(sgt_job *J, cudaStream_t s, bool pdl) {
   sgt_ctx *ctx = J->ctx;
   typedef typename Node<D>::T NT;
-  if constexpr (D == 1) {
-    CK(launch_chain(pdl, k_conv1d, 1, 32, 0, s, (const SgtState *)J->st, (const float2 *)J->V,
-                    (float2 *)J->Phi));
-  } else {
+  CK(launch_chain(pdl, k_spec_cols<D>, J->nb_conv, SGT_THREADS, 0, s, (const SgtState *)J->st,
+                  (const NT *)J->V, (const float2 *)J->W, (NT *)J->Phi));
+  if constexpr (D >= 2) {
     CK(launch_chain(pdl, k_fft_build_x<D>, J->nb_fft_rows, SGT_THREADS, 0, s,
                     (const SgtState *)J->st, (const NT *)J->V, J->W));
     if constexpr (D == 3)
@@ -639,14 +646,14 @@ static sgt_status enqueue_scatter_part(sgt_job *J, cudaStream_t s, cudaEvent_t *
   const int n = J->n;
   const bool pdl = ev == nullptr;
   if (ev) CK(cudaEventRecord(ev[1], s));
-  CK(launch_chain(pdl, k_fold<D>, J->nb_fold, SGT_THREADS, 0, s, (const SgtState *)J->st,
-                  (NT *)J->Vc, (NT *)J->V));
   if (J->jp.cell_blocks > 0) {
     CK(launch_chain(pdl, k_bin_scatter<D>, J->jp.cell_blocks, SGT_THREADS, 0, s, (const VT *)J->Y,
                     n, J->st, J->cursor, J->sorted));
     CK(launch_chain(pdl, k_s2g_cell<D>, J->nb_s2gc, SGT_THREADS, 0, s, (const float4 *)J->sorted,
                     J->st, (const int4 *)J->chunks, (NT *)J->V));
   }
+  CK(launch_chain(pdl, k_spec_rows<D>, J->nb_spec, SGT_THREADS, 0, s, (const SgtState *)J->st,
+                  (NT *)J->Vc, (NT *)J->V, J->W, J->Ygather ? SGT_SPEC_FOLD : SGT_SPEC_BOTH));
   if (ev) CK(cudaEventRecord(ev[2], s));
   CK(cudaGetLastError());
   return SGT_OK;
@@ -660,6 +667,9 @@ static sgt_status enqueue_gather_part(sgt_job *J, cudaStream_t s, cudaEvent_t *e
   typedef typename Vec<D>::T VT;
   typedef typename Node<D>::T NT;
   const bool pdl = ev == nullptr;
+  if (J->Ygather)  // a shard: the grid has been summed over the ranks meanwhile
+    CK(launch_chain(false, k_spec_rows<D>, J->nb_spec, SGT_THREADS, 0, s, (const SgtState *)J->st,
+                    (NT *)J->Vc, (NT *)J->V, J->W, SGT_SPEC_TRANSFORM));
   CKS(enqueue_g2g<D>(J, s, pdl));
   if (ev) CK(cudaEventRecord(ev[3], s));
   if (J->jp.cell_blocks > 0)
@@ -821,8 +831,7 @@ __global__ void k_write_bins(const typename Vec<D>::T *__restrict__ Y, int n,
     const typename Vec<D>::T y = Y[i];
 #pragma unroll
     for (int k = 0; k < D; k++) {
-      float sh;
-      bins[(long)i * D + k] = (uint32_t)floorf(sgt_scale(comp<D>(y, k), st->miny[k], maxy, scale, sh));
+      bins[(long)i * D + k] = (uint32_t)floorf(sgt_scale(comp<D>(y, k), st->miny[k], maxy, scale));
     }
   }
 }
@@ -1442,7 +1451,7 @@ sgt_status sgt_job_run(sgt_job *J, int iters) {
 // table of block counts per stage, and one view/prefix table per row-group
 // lane count for the SpMV.
 enum {
-  FS_BIN_COUNT, FS_SCATTER, FS_FOLD, FS_BIN_SCATTER, FS_S2G_CELL, FS_FFT_X,
+  FS_BIN_COUNT, FS_SCATTER, FS_SPEC, FS_BIN_SCATTER, FS_S2G_CELL, FS_CONV, FS_FFT_X,
   FS_FFT_MID_FWD, FS_FFT_LAST, FS_FFT_MID_INV, FS_FFT_FINAL, FS_G2S, FS_GATHER, FS_UPDATE, FS_STAGES
 };
 struct BatchGroup {
@@ -1551,7 +1560,7 @@ static void stage_blocks(const sgt_job *J, int *b) {
   const int work = std::max(1, (J->n + 2047) / 2048);
   const int fine = (J->d == 3 ? 16 : 8) * work;
   b[FS_SCATTER] = std::min(J->nb_scat, fine);
-  b[FS_FOLD] = std::min(J->nb_fold, 4);
+  b[FS_SPEC] = std::min(J->nb_spec, J->d == 3 ? 128 : (J->d == 2 ? 48 : 1));
   if (J->jp.cell_blocks > 0) {
     b[FS_BIN_COUNT] = std::min(J->jp.cell_blocks, work);
     b[FS_G2S] = std::min(J->nb_g2s, 2 * work);
@@ -1559,7 +1568,8 @@ static void stage_blocks(const sgt_job *J, int *b) {
     b[FS_S2G_CELL] = std::min(J->nb_s2gc, 2 * work);
   }
   const int rows64 = J->d == 3 ? (2 * 64 * 64 + 128 * 128) / 8 : (2 * 64 + 128) / 8;
-  b[FS_FFT_X] = J->d == 1 ? 1 : std::min(J->nb_fft_rows, rows64);
+  b[FS_CONV] = std::min(J->nb_conv, J->d == 3 ? 100 : 48);
+  if (J->d >= 2) b[FS_FFT_X] = std::min(J->nb_fft_rows, rows64);
   if (J->d == 3) b[FS_FFT_MID_FWD] = b[FS_FFT_MID_INV] = std::min(J->nb_fft, 128);
   if (J->d >= 2) {
     b[FS_FFT_LAST] = std::min(J->nb_fft, J->d == 3 ? 128 : 16);
@@ -1695,14 +1705,13 @@ static sgt_status enqueue_fused_group(sgt_ctx *ctx, BatchGroup &g) {
   if (g.blocks[FS_BIN_COUNT] > 0)  // some job of the group can take the cell mode
     km_bin_count<D><<<FL(FS_BIN_COUNT), 0, c>>>(v, g.prefix[FS_BIN_COUNT], nj);
   km_scatter<D><<<FL(FS_SCATTER), 0, c>>>(v, g.prefix[FS_SCATTER], nj);
-  km_fold<D><<<FL(FS_FOLD), 0, c>>>(v, g.prefix[FS_FOLD], nj);
   if (g.blocks[FS_BIN_SCATTER] > 0) {
     km_bin_scatter<D><<<FL(FS_BIN_SCATTER), 0, c>>>(v, g.prefix[FS_BIN_SCATTER], nj);
     km_s2g_cell<D><<<FL(FS_S2G_CELL), 0, c>>>(v, g.prefix[FS_S2G_CELL], nj);
   }
-  if constexpr (D == 1) {
-    km_conv1d<<<g.blocks[FS_FFT_X], 32, 0, c>>>(v, g.prefix[FS_FFT_X], nj);
-  } else {
+  km_spec_rows<D><<<FL(FS_SPEC), 0, c>>>(v, g.prefix[FS_SPEC], nj);
+  km_spec_cols<D><<<FL(FS_CONV), 0, c>>>(v, g.prefix[FS_CONV], nj);
+  if constexpr (D >= 2) {
     km_fft_build_x<D><<<FL(FS_FFT_X), 0, c>>>(v, g.prefix[FS_FFT_X], nj);
     if constexpr (D == 3)
       km_fft_cols<D, MODE_MID_FWD><<<FL(FS_FFT_MID_FWD), g.smem_fft, c>>>(v, g.prefix[FS_FFT_MID_FWD], nj);
@@ -2457,14 +2466,26 @@ sgt_status sgt_last_grids(sgt_ctx *ctx, float *v_grid, float *phi_grid) {
   if (d >= 2) nodes *= N;
   if (d >= 3) nodes *= N;
   std::vector<float> tmp(nodes * nc);
+  // reported as charges [1, y - c] and their potentials, c the grid's middle;
+  // held about the nodes (the potentials only after a direct convolution),
+  // in cells
+  const SgtState &hs = *J->st_host;
+  const double mid = 0.5 * (N - 1), hd = hs.h_eff;
   float *outs[2] = {v_grid, phi_grid};
   const float *srcs[2] = {J->V, J->Phi};
   for (int q = 0; q < 2; q++) {
     if (!outs[q]) continue;
     CK(cudaMemcpyAsync(tmp.data(), srcs[q], sizeof(float) * tmp.size(), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    for (size_t g = 0; g < nodes; g++)
-      for (int c = 0; c < m; c++) outs[q][c * nodes + g] = tmp[g * nc + c];
+    const bool about_node = q == 0 || hs.direct;
+    for (size_t g = 0; g < nodes; g++) {
+      outs[q][g] = tmp[g * nc];
+      size_t place = g;
+      for (int c = 1; c < m; c++, place /= N) {
+        const double x = about_node ? (double)(place % N) - mid : 0.0;
+        outs[q][c * nodes + g] = (float)(hd * (tmp[g * nc + c] + x * tmp[g * nc]));
+      }
+    }
   }
   return SGT_OK;
 }
@@ -2978,6 +2999,7 @@ extern "C" sgt_status sgt_repulsive_noalloc(sgt_ctx *ctx, int n, int d, float h,
   J.mmax = d == 1 ? SGT_NA_MMAX_1D : SGT_NA_MMAX_2D;
   J.nmax = d == 1 ? 512 : SGT_NA_MAX_GRID_2D;
   J.jp.mmax = J.mmax;
+  J.jp.conv_max = std::min(J.nmax, SGT_SPEC_MAX(d));
   J.jp.vc_nodes = SGT_NA_COPY_NODES;
   J.Y = (float *)(base + NA_Y);
   J.Ynext = (float *)(base + NA_YNEXT);

@@ -28,9 +28,6 @@
 #define SGT_FFT_COLS 8  // columns per CTA in column passes (one per warp)
 #define SGT_FFT_PAD 1   // float2 padding per staged column
 #define SGT_FFT_MAXM 1024  // longest FFT: twiddle tables hold M entries
-// d = 2 grids with M <= SGT_FFT_SMALL_M: the whole convolution runs in one CTA
-// in shared memory (conv2d_small_body), and the row passes return at once
-#define SGT_FFT_SMALL_M 64
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -170,10 +167,13 @@ __device__ __forceinline__ float kern_val(float hsq, int M, int x, int y, int z)
   return 1.0f / (b * b);
 }
 
+// Plane p of a node's charges for the FFT: the charges [1, y - y_node] with
+// the origin moved to the grid's middle (x, y, z: the node's place from it).
 template <int D>
-__device__ __forceinline__ float2 node_plane(const typename Node<D>::T &v, int p) {
-  if constexpr (D == 1) return v;
-  else return p == 0 ? make_float2(v.x, v.y) : make_float2(v.z, D == 3 ? v.w : 0.f);
+__device__ __forceinline__ float2 node_plane(const typename Node<D>::T &v, int p, float x, float y,
+                                             float z) {
+  if (p == 0) return make_float2(v.x, v.y + x * v.x);
+  return make_float2(v.z + y * v.x, D == 3 ? v.w + z * v.x : 0.f);
 }
 
 // the FFT lengths the grid decision picks (sgt_fft_length)
@@ -192,47 +192,409 @@ __device__ __forceinline__ float2 node_plane(const typename Node<D>::T &v, int p
   }
 
 // ---------------------------------------------------------------------------
-// d = 1: the whole convolution in one warp
+// Convolution of small and middle grids in two kernels: a discrete Fourier
+// transform along x and a direct sum over the rows.
+//
+//   k_spec_rows  per row of charges: fold the grid copies and transform along
+//                x (M = 2N, frequencies 0..N of the real rows); per row offset
+//                the transforms of K and of x K.
+//   k_spec_cols  per output row: sum over all input rows, frequency by
+//                frequency, transform back along x.
+//
+// The result is Phi0 = sum K V0 and, per axis, Psi_k(g) = sum_s K(g - s)
+// (U_k(s) + (s_k - g_k) V0(s)): the potential of the charges about the output
+// node itself, in cells, so that the force sum_g w_g ((y - y_g) Phi0 - Psi)
+// cancels nothing.  Along x that is K^ Ux^ + i S V0^ with S the sine
+// transform of x K; along the other axes the distance is a number per pair of
+// rows.
+//
+// Why: FFT passes of these grids (16 to 128 points per axis in 2-D, 16 to 40
+// in 3-D, where nearly all iterations run) are three to five kernels bound by
+// latency, pad N to a power of two, and their column pass needs 100 KB of
+// shared memory, for which a block waits until a whole SM has drained of the
+// concurrent SpMV.  The row sums here cost N times more operations than a
+// column FFT and still only a few microseconds, with 256 threads, 64
+// registers and 15 KB a block.  3-D, 20^3: 27 us in five FFT passes.
 // ---------------------------------------------------------------------------
-template <int M>
-__device__ void conv1d_body(const SgtState *st, const float2 *__restrict__ V, float2 *__restrict__ Phi,
-                            const float2 *tw) {
-  constexpr int E = M / 32;
-  const int N = st->N, lane = threadIdx.x & 31;
-  const float hsq = st->h_eff * st->h_eff;
-  float2 k[E], v[E];
-#pragma unroll
-  for (int e = 0; e < E; e++) {
-    const int x = lane + 32 * e;
-    k[e] = make_float2(kern_val(hsq, M, x, 0, 0), 0.f);
-    v[e] = x < N ? V[x] : make_float2(0.f, 0.f);
+#define SGT_SPEC_MAX(D) ((D) == 1 ? 512 : ((D) == 2 ? 128 : 40))
+// k_spec_rows in one go, or its halves (the charge grid of a row-split
+// embedding is summed over the ranks between them)
+#define SGT_SPEC_BOTH 0
+#define SGT_SPEC_FOLD 1
+#define SGT_SPEC_TRANSFORM 2
+#define SGT_SPEC_TY(D) ((D) == 3 ? 4 : 1)  // output rows a block sums together
+
+// floor(a / b) for 0 <= a < 2^16, inv = 1 / b: half a unit away from every
+// integer quotient
+__device__ __forceinline__ int small_div(int a, float inv) { return (int)(((float)a + 0.5f) * inv); }
+
+// second half of a row's spectrum: Uy (and Uz)
+template <int D> struct SpecB { typedef float4 T; };
+template <> struct SpecB<2> { typedef float2 T; };
+
+// The spectra live in the FFT workspace: (V0, Ux) of every row and frequency,
+// then (Uy, Uz), then (K^, S) per row offset.
+template <int D>
+struct SpecBuf {
+  float4 *h0;
+  typename SpecB<D>::T *h1;
+  float2 *k;
+  __device__ __forceinline__ SpecBuf(float2 *W, int rows, int F) {
+    h0 = reinterpret_cast<float4 *>(W);
+    h1 = reinterpret_cast<typename SpecB<D>::T *>(h0 + rows * F);
+    k = reinterpret_cast<float2 *>(h1 + rows * F);
   }
-  wfft_dif<M>(k, tw);
-  wfft_dif<M>(v, tw);
-#pragma unroll
-  for (int e = 0; e < E; e++) v[e] = make_float2(v[e].x * k[e].x, v[e].y * k[e].x);
-  wfft_dit_inv<M>(v, tw);
-  const float inv = 1.0f / (float)M;
-#pragma unroll
-  for (int e = 0; e < E; e++) {
-    const int x = lane + 32 * e;
-    if (x < N) Phi[x] = make_float2(v[e].x * inv, v[e].y * inv);
+};
+
+// tw[j] = exp(-2 pi i j / M)
+__device__ __forceinline__ void spec_twiddles(float2 *tw, int M) {
+  for (int j = threadIdx.x; j < M; j += SGT_THREADS) {
+    float sn, cs;
+    sincospif(__fdiv_rn(2.0f * (float)j, (float)M), &sn, &cs);
+    tw[j] = make_float2(cs, -sn);
   }
 }
 
-__device__ __forceinline__ void k_conv1d_body(int vb_, int vg_, const SgtState *st, const float2 *__restrict__ V, float2 *__restrict__ Phi) {
-  sgt_pdl_wait();
-  __shared__ float2 tw[SGT_FFT_MAXM];
-  fft_twiddles(tw, st->M);
-  __syncthreads();
-  if (threadIdx.x >= 32) return;
-#define C1(L) conv1d_body<L>(st, V, Phi, tw)
-  SGT_FFT_DISPATCH(st->M, C1)
-#undef C1
+// ---------------------------------------------------------------------------
+// fold: V = sum of the grid copies, which are left zero for the next
+// iteration's scatter (they start zero at job creation).  Cell mode: V only
+// (k_bin_count cleared it and k_s2g_cell has added to it), nothing to do.
+// ---------------------------------------------------------------------------
+template <int D>
+__device__ __forceinline__ void k_fold_body(int vb_, int vg_, const SgtState *st,
+                                            typename Node<D>::T *__restrict__ Vc,
+                                            typename Node<D>::T *__restrict__ V) {
+  if (st->T != 0) return;
+  const int N = st->N, copies = st->copies;
+  long nodes = N;
+  if (D >= 2) nodes *= N;
+  if (D >= 3) nodes *= N;
+  typename Node<D>::T z;
+  if constexpr (D == 1) z = make_float2(0.f, 0.f); else z = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (long g = vb_ * (long)blockDim.x + threadIdx.x; g < nodes; g += (long)vg_ * blockDim.x) {
+    typename Node<D>::T a = z;
+    for (int c0 = 0; c0 < copies; c0 += 4) {
+      typename Node<D>::T t[4];
+#pragma unroll
+      for (int c = 0; c < 4; c++) t[c] = c0 + c < copies ? Vc[(c0 + c) * nodes + g] : z;
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        a.x += t[c].x;
+        a.y += t[c].y;
+        if constexpr (D >= 2) {
+          a.z += t[c].z;
+          if constexpr (D >= 3) a.w += t[c].w;
+        }
+        if (c0 + c < copies) Vc[(c0 + c) * nodes + g] = z;
+      }
+    }
+    V[g] = a;
+  }
 }
-__global__ void __launch_bounds__(SGT_THREADS)
-k_conv1d(const SgtState *st, const float2 *__restrict__ V, float2 *__restrict__ Phi) {
-  k_conv1d_body(blockIdx.x, gridDim.x, st, V, Phi);
+template <int D>
+__device__ __forceinline__ void k_spec_rows_body(int vb_, int vg_, const SgtState *st,
+                                                 typename Node<D>::T *__restrict__ Vc,
+                                                 typename Node<D>::T *__restrict__ V,
+                                                 float2 *__restrict__ W, int phase) {
+  const int N = st->N;
+  if (D == 1 || !st->direct || phase == SGT_SPEC_FOLD) {
+    // the fold alone: 1-D, grids of the FFT passes, the shards' scatter phase
+    sgt_pdl_wait();
+    if (phase != SGT_SPEC_TRANSFORM) k_fold_body<D>(vb_, vg_, st, Vc, V);
+    return;
+  }
+  if constexpr (D >= 2) {
+    __shared__ float2 tw[2 * 128];
+    __shared__ float4 row[128];
+    __shared__ float red[SGT_THREADS * 9];
+    const int M = 2 * N, F = N + 1, rows = D == 2 ? N : N * N;
+    if (vb_ >= rows) {
+      sgt_pdl_wait();
+      return;
+    }
+    const float inv_f = 1.0f / (float)F, inv_m = 1.0f / (float)M;
+    const SpecBuf<D> B(W, rows, F);
+    spec_twiddles(tw, M);
+    // thread: frequency f and segment sg of the row
+    const int S = SGT_THREADS / F, t = threadIdx.x;  // F <= 129: S >= 1
+    const int sg = small_div(t, inv_f), f = t - sg * F;
+    const int len = (N + S - 1) / S, x0 = min(sg * len, N), x1 = min(N, x0 + len);
+    const int w0 = f * x0 - M * small_div(f * x0, inv_m);
+    float *K = reinterpret_cast<float *>(row);
+    const float hsq = st->h_eff * st->h_eff;
+    // kernel rows: fixed before the chain began, done while the previous
+    // kernel drains
+    for (int r = vb_; r < rows; r += vg_) {
+      const int dz = D == 2 ? 0 : small_div(r, 1.0f / (float)N), dy = r - dz * N;
+      __syncthreads();
+      for (int x = t; x < N; x += SGT_THREADS) {
+        const float b = 1.0f + hsq * (float)(x * x + dy * dy + dz * dz);
+        K[x] = (x == 0 ? 1.0f : 2.0f) / (b * b);
+      }
+      __syncthreads();
+      if (sg < S) {
+        float kc = 0.f, ks = 0.f;
+        int w = w0;
+        for (int x = x0; x < x1; x++) {
+          const float2 e = tw[w];
+          const float k = K[x];
+          kc += k * e.x;
+          ks -= (float)x * k * e.y;
+          w += f;
+          if (w >= M) w -= M;
+        }
+        red[2 * t] = kc;
+        red[2 * t + 1] = ks;
+      }
+      __syncthreads();
+      if (t < F) {
+        float kc = 0.f, ks = 0.f;
+        for (int g = 0; g < S; g++) {
+          kc += red[2 * (g * F + t)];
+          ks += red[2 * (g * F + t) + 1];
+        }
+        B.k[r * F + t] = make_float2(kc, ks);
+      }
+    }
+    sgt_pdl_wait();
+    const int copies = st->copies;
+    const bool cell = st->T != 0 || phase == SGT_SPEC_TRANSFORM;  // V is complete
+    const long nodes = (long)rows * N;
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r = vb_; r < rows; r += vg_) {
+      __syncthreads();
+      // the row's charges: 4 lanes a node, the copies dealt over them
+      for (int e = t; e < ((4 * N + 31) & ~31); e += SGT_THREADS) {
+        const int x = e >> 2, p = e & 3;
+        float4 a = z4;
+        if (x < N) {
+          const long g = (long)r * N + x;
+          if (cell) {
+            if (p == 0) a = V[g];
+          } else {
+            for (int c0 = p; c0 < copies; c0 += 16) {
+              float4 q[4];
+#pragma unroll
+              for (int u = 0; u < 4; u++)
+                q[u] = c0 + 4 * u < copies ? Vc[(c0 + 4 * u) * nodes + g] : z4;
+#pragma unroll
+              for (int u = 0; u < 4; u++) {
+                a.x += q[u].x; a.y += q[u].y; a.z += q[u].z; a.w += q[u].w;
+                if (c0 + 4 * u < copies) Vc[(c0 + 4 * u) * nodes + g] = z4;
+              }
+            }
+          }
+        }
+#pragma unroll
+        for (int o = 1; o < 4; o *= 2) {
+          a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
+          a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+          a.z += __shfl_xor_sync(0xffffffffu, a.z, o);
+          if (D == 3) a.w += __shfl_xor_sync(0xffffffffu, a.w, o);
+        }
+        if (p == 0 && x < N) {
+          row[x] = a;
+          if (!cell) V[(long)r * N + x] = a;
+        }
+      }
+      __syncthreads();
+      if (sg < S) {
+        float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        int w = w0;
+        for (int x = x0; x < x1; x++) {
+          const float2 e = tw[w];
+          const float4 v = row[x];
+          a[0] += v.x * e.x; a[1] += v.x * e.y;
+          a[2] += v.y * e.x; a[3] += v.y * e.y;
+          a[4] += v.z * e.x; a[5] += v.z * e.y;
+          if constexpr (D == 3) { a[6] += v.w * e.x; a[7] += v.w * e.y; }
+          w += f;
+          if (w >= M) w -= M;
+        }
+#pragma unroll
+        for (int c = 0; c < (D == 3 ? 8 : 6); c++) red[t * 9 + c] = a[c];
+      }
+      __syncthreads();
+      if (t < F) {
+        float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int g = 0; g < S; g++)
+#pragma unroll
+          for (int c = 0; c < (D == 3 ? 8 : 6); c++) a[c] += red[(g * F + t) * 9 + c];
+        B.h0[r * F + t] = make_float4(a[0], a[1], a[2], a[3]);
+        if constexpr (D == 3) B.h1[r * F + t] = make_float4(a[4], a[5], a[6], a[7]);
+        else B.h1[r * F + t] = make_float2(a[4], a[5]);
+      }
+    }
+  }
+}
+template <int D>
+__global__ void __launch_bounds__(SGT_THREADS, 4)
+k_spec_rows(const SgtState *st, typename Node<D>::T *__restrict__ Vc,
+            typename Node<D>::T *__restrict__ V, float2 *__restrict__ W, int phase) {
+  k_spec_rows_body<D>(blockIdx.x, gridDim.x, st, Vc, V, W, phase);
+}
+
+template <int D>
+__device__ __forceinline__ void k_spec_cols_body(int vb_, int vg_, const SgtState *st,
+                                                 const typename Node<D>::T *__restrict__ V,
+                                                 const float2 *__restrict__ W,
+                                                 typename Node<D>::T *__restrict__ Phi) {
+  if constexpr (D == 1) {
+    // 1-D: a warp per output sums over the grid
+    sgt_pdl_wait();
+    const int N = st->N, lane = threadIdx.x & 31;
+    const float hsq = st->h_eff * st->h_eff;
+    constexpr int WPB = SGT_THREADS / 32;
+    for (int x = vb_ * WPB + (threadIdx.x >> 5); x < N; x += vg_ * WPB) {
+      float p0 = 0.f, p1 = 0.f;
+      for (int s = lane; s < N; s += 32) {
+        const float2 v = V[s];
+        const float r = (float)(s - x), b = 1.0f + hsq * (r * r), k = 1.0f / (b * b);
+        p0 += k * v.x;
+        p1 += k * (v.y + r * v.x);
+      }
+      p0 = warp_sum_f(p0);
+      p1 = warp_sum_f(p1);
+      if (lane == 0) Phi[x] = make_float2(p0, p1);
+    }
+  } else {
+    constexpr int TY = SGT_SPEC_TY(D), C = 2 * (D + 1);  // reals per output and frequency
+    if (!st->direct) {
+      sgt_pdl_wait();
+      return;
+    }
+    const int N = st->N, M = 2 * N, F = N + 1, rows = D == 2 ? N : N * N;
+    const int ty = (N + TY - 1) / TY, items = (D == 2 ? 1 : N) * ty;
+    if (vb_ >= items) {
+      sgt_pdl_wait();
+      return;
+    }
+    __shared__ float2 tw[2 * 128];
+    __shared__ float red[SGT_THREADS * 9];
+    __shared__ float What[(D == 2 ? 129 : 41) * TY * (C + 1)];  // [output][frequency][C + 1]
+    spec_twiddles(tw, M);
+    const float inv_f = 1.0f / (float)F, inv_m = 1.0f / (float)M;
+    const SpecBuf<D> B(const_cast<float2 *>(W), rows, F);
+    const int t = threadIdx.x, S = SGT_THREADS / F;
+    const int sg = small_div(t, inv_f), f = t - sg * F;
+    // pieces of the input: H parts of each plane's rows, dealt to the segments
+    const int H = D == 2 ? S : 2, len = (N + H - 1) / H, pieces = (D == 2 ? 1 : N) * H;
+    sgt_pdl_wait();
+    for (int it = vb_; it < items; it += vg_) {
+      const int oz = D == 2 ? 0 : small_div(it, 1.0f / (float)ty), y0 = (it - oz * ty) * TY;
+      const float yc = (float)y0 + 0.5f * (float)(TY - 1);
+      float a[TY][C];
+#pragma unroll
+      for (int j = 0; j < TY; j++)
+#pragma unroll
+        for (int c = 0; c < C; c++) a[j][c] = 0.f;
+      if (sg < S) {
+        for (int pc = sg; pc < pieces; pc += S) {
+          const int z = D == 2 ? 0 : pc >> 1, hpart = D == 2 ? pc : pc & 1;
+          const int r0 = min(hpart * len, N), r1 = min(N, r0 + len);
+          const float dz = (float)(z - oz);
+          const float2 *kp = B.k + (D == 2 ? 0 : abs(z - oz) * N) * F + f;
+          const float4 *h0 = B.h0 + z * N * F + f;
+          const typename SpecB<D>::T *h1 = B.h1 + z * N * F + f;
+          float2 k[TY];  // k[j]: offset y0 + j - r; slides by one per input row
+#pragma unroll
+          for (int j = 1; j < TY; j++) k[j] = kp[abs(min(y0 + j - r0, N - 1)) * F];
+#pragma unroll 4
+          for (int r = r0; r < r1; r++) {
+            k[0] = kp[abs(y0 - r) * F];
+            const float4 v = h0[r * F];
+            const typename SpecB<D>::T u = h1[r * F];
+            const float dy = (float)r - yc;
+            const float uyr = u.x + dy * v.x, uyi = u.y + dy * v.y;
+            float uzr = 0.f, uzi = 0.f;
+            if constexpr (D == 3) {
+              uzr = u.z + dz * v.x;
+              uzi = u.w + dz * v.y;
+            }
+#pragma unroll
+            for (int j = 0; j < TY; j++) {
+              a[j][0] += k[j].x * v.x;
+              a[j][1] += k[j].x * v.y;
+              a[j][2] += k[j].x * v.z - k[j].y * v.y;
+              a[j][3] += k[j].x * v.w + k[j].y * v.x;
+              a[j][4] += k[j].x * uyr;
+              a[j][5] += k[j].x * uyi;
+              if constexpr (D == 3) {
+                a[j][6] += k[j].x * uzr;
+                a[j][7] += k[j].x * uzi;
+              }
+            }
+#pragma unroll
+            for (int j = TY - 1; j > 0; j--) k[j] = k[j - 1];
+          }
+        }
+      }
+      // over the segments, in order
+#pragma unroll
+      for (int j = 0; j < TY; j++) {
+        __syncthreads();
+        if (sg < S) {
+#pragma unroll
+          for (int c = 0; c < C; c++) red[t * 9 + c] = a[j][c];
+        }
+        __syncthreads();
+        for (int e = t; e < F * (C / 2); e += SGT_THREADS) {
+          const int c2 = small_div(e, inv_f), ff = e - c2 * F;
+          float re = 0.f, im = 0.f;
+          for (int g = 0; g < S; g++) {
+            re += red[(g * F + ff) * 9 + 2 * c2];
+            im += red[(g * F + ff) * 9 + 2 * c2 + 1];
+          }
+          const float wt = (ff == 0 || ff == N) ? 1.0f : 2.0f;
+          What[(j * F + ff) * (C + 1) + 2 * c2] = wt * re;
+          What[(j * F + ff) * (C + 1) + 2 * c2 + 1] = wt * im;
+        }
+      }
+      __syncthreads();
+      // back along x: P lanes (a power of two) per output
+      int lp = 0;
+      while ((TY * N << (lp + 1)) <= SGT_THREADS && lp < 3) lp++;
+      const int P = 1 << lp, p = t & (P - 1);
+      const float inv_n = 1.0f / (float)N;
+      for (int o0 = 0; o0 < TY * N; o0 += SGT_THREADS >> lp) {  // uniform
+        const int o = o0 + (t >> lp);
+        const int j = min(small_div(o, inv_n), TY - 1), x = min(o - j * N, N - 1);
+        float q[D + 1];
+#pragma unroll
+        for (int c = 0; c <= D; c++) q[c] = 0.f;
+        const int step = x * P - M * small_div(x * P, inv_m);
+        int w = x * p - M * small_div(x * p, inv_m);
+        for (int ff = p; ff < F; ff += P) {
+          const float2 e = tw[w];  // (cos, -sin): Re(W exp(+i)) = re cos + im (-sin)
+          const float *wh = &What[(j * F + ff) * (C + 1)];
+#pragma unroll
+          for (int c = 0; c <= D; c++) q[c] += wh[2 * c] * e.x + wh[2 * c + 1] * e.y;
+          w += step;
+          if (w >= M) w -= M;
+        }
+#pragma unroll
+        for (int e = 1; e < 8; e *= 2)
+          if (e < P) {
+#pragma unroll
+            for (int c = 0; c <= D; c++) q[c] += __shfl_xor_sync(0xffffffffu, q[c], e);
+          }
+        const int y = y0 + j;
+        if (p == 0 && o < TY * N && y < N) {
+#pragma unroll
+          for (int c = 0; c <= D; c++) q[c] = q[c] / (float)M;
+          q[2] += (yc - (float)y) * q[0];
+          Phi[((long)(D == 2 ? 0 : oz) * N + y) * N + x] =
+              make_float4(q[0], q[1], q[2], D == 3 ? q[D] : 0.f);
+        }
+      }
+    }
+  }
+}
+template <int D>
+__global__ void __launch_bounds__(SGT_THREADS, 3)
+k_spec_cols(const SgtState *st, const typename Node<D>::T *__restrict__ V,
+            const float2 *__restrict__ W, typename Node<D>::T *__restrict__ Phi) {
+  k_spec_cols_body<D>(blockIdx.x, gridDim.x, st, V, W, Phi);
 }
 
 // ---------------------------------------------------------------------------
@@ -250,6 +612,7 @@ __device__ void build_rows_body(int vb_, int vg_, const SgtState *st, const type
   const int nz_d = D == 3 ? N : 1, nz_k = D == 3 ? M : 1;
   const long lines_d = 2L * N * nz_d, lines = lines_d + (long)M * nz_k;
   const int wpb = blockDim.x >> 5;
+  const float mid = 0.5f * (float)(N - 1);  // place of the grid's middle, in nodes
   for (long ln = (long)vb_ * wpb + warp; ln < lines; ln += (long)vg_ * wpb) {
     float2 v[E];
     int p, y, z;
@@ -261,7 +624,8 @@ __device__ void build_rows_body(int vb_, int vg_, const SgtState *st, const type
 #pragma unroll
       for (int e = 0; e < E; e++) {
         const int x = lane + 32 * e;
-        v[e] = x < N ? node_plane<D>(V[x + (long)N * y + (D == 3 ? (long)N * N * z : 0)], p)
+        v[e] = x < N ? node_plane<D>(V[x + (long)N * y + (D == 3 ? (long)N * N * z : 0)], p,
+                                     (float)x - mid, (float)y - mid, (float)z - mid)
                      : make_float2(0.f, 0.f);
       }
     } else {
@@ -283,7 +647,7 @@ template <int D>
 __device__ __forceinline__ void k_fft_build_x_body(int vb_, int vg_, const SgtState *st, const typename Node<D>::T *__restrict__ V, float2 *__restrict__ W) {
   sgt_pdl_wait();
   __shared__ float2 tw[SGT_FFT_MAXM];
-  if (D == 2 && st->M <= SGT_FFT_SMALL_M) return;  // the column pass does it all
+  if (st->direct) return;  // k_spec_cols did it
   fft_twiddles(tw, st->M);
   __syncthreads();
 #define CB(L) build_rows_body<D, L>(vb_, vg_, st, V, W, tw)
@@ -294,95 +658,6 @@ template <int D>
 __global__ void __launch_bounds__(SGT_THREADS)
 k_fft_build_x(const SgtState *st, const typename Node<D>::T *__restrict__ V, float2 *__restrict__ W) {
   k_fft_build_x_body<D>(blockIdx.x, gridDim.x, st, V, W);
-}
-
-// ---------------------------------------------------------------------------
-// d = 2, M <= SGT_FFT_SMALL_M: the three passes below in one CTA, with the
-// planes in shared memory (rows padded to M + 1 points so that the column
-// reads of the lanes fall in distinct banks).  The same transforms, products
-// and scaling in the same order as the multi-CTA passes, so the potentials
-// are the same; small grids (the h-driven grids of most runs) save two
-// passes through global memory and the launch latency between them.
-// Shared memory: twiddles (M), the kernel plane (M rows), the data planes
-// (2 x N rows, N <= M / 2).
-// ---------------------------------------------------------------------------
-template <int M>
-__device__ void conv2d_small_body(const SgtState *st, const float4 *__restrict__ V,
-                                  float2 *__restrict__ Phi2, float2 *sm) {
-  constexpr int E = M / 32, LS = M + 1;
-  const int N = st->N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const float hsq = st->h_eff * st->h_eff;
-  float2 *tw = sm;
-  float2 *kp = sm + M;
-  float2 *dp = kp + M * LS;  // plane p, row y at dp + (p N + y) LS
-  fft_twiddles(tw, M);
-  __syncthreads();
-  // rows along x: the kernel plane (all M rows), the data planes (y < N)
-  for (int ln = warp; ln < M + 2 * N; ln += nw) {
-    float2 v[E];
-    float2 *row;
-    if (ln < M) {
-#pragma unroll
-      for (int e = 0; e < E; e++) v[e] = make_float2(kern_val(hsq, M, lane + 32 * e, ln, 0), 0.f);
-      row = kp + ln * LS;
-    } else {
-      const int r = ln - M, p = r / N, y = r % N;
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        const int x = lane + 32 * e;
-        v[e] = x < N ? node_plane<2>(V[x + (long)N * y], p) : make_float2(0.f, 0.f);
-      }
-      row = dp + (p * N + y) * LS;
-    }
-    wfft_dif<M>(v, tw);
-#pragma unroll
-    for (int e = 0; e < E; e++) row[lane + 32 * e] = v[e];
-  }
-  __syncthreads();
-  // columns along y: the kernel spectrum (real part), then per data plane
-  // forward, product, inverse; rows y >= N of the data are zero and dropped
-  for (int c = warp; c < M; c += nw) {
-    float2 v[E];
-    float kr[E];
-#pragma unroll
-    for (int e = 0; e < E; e++) v[e] = kp[(lane + 32 * e) * LS + c];
-    wfft_dif<M>(v, tw);
-#pragma unroll
-    for (int e = 0; e < E; e++) kr[e] = v[e].x;
-    for (int p = 0; p < 2; p++) {
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        const int y = lane + 32 * e;
-        v[e] = y < N ? dp[(p * N + y) * LS + c] : make_float2(0.f, 0.f);
-      }
-      wfft_dif<M>(v, tw);
-#pragma unroll
-      for (int e = 0; e < E; e++) v[e] = make_float2(v[e].x * kr[e], v[e].y * kr[e]);
-      wfft_dit_inv<M>(v, tw);
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        const int y = lane + 32 * e;
-        if (y < N) dp[(p * N + y) * LS + c] = v[e];
-      }
-    }
-  }
-  __syncthreads();
-  // rows inverse along x, scaled by 1/M^2, into the potential grid
-  float inv = 1.0f / (float)M;
-  inv = inv / (float)M;
-  for (int ln = warp; ln < 2 * N; ln += nw) {
-    const int p = ln % 2, y = ln / 2;
-    float2 v[E];
-#pragma unroll
-    for (int e = 0; e < E; e++) v[e] = dp[(p * N + y) * LS + lane + 32 * e];
-    wfft_dit_inv<M>(v, tw);
-    const long g0 = (long)N * y;
-#pragma unroll
-    for (int e = 0; e < E; e++) {
-      const int x = lane + 32 * e;
-      if (x < N) Phi2[2 * (g0 + x) + p] = make_float2(v[e].x * inv, v[e].y * inv);
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -503,15 +778,7 @@ __device__ __forceinline__ void k_fft_cols_body(int vb_, int vg_, const SgtState
                                                 typename Node<D>::T *__restrict__ Phi) {
   sgt_pdl_wait();
   extern __shared__ float2 sm[];
-  if constexpr (D == 2 && MODE == MODE_LAST) {
-    if (st->M <= SGT_FFT_SMALL_M) {  // block-uniform
-      if (vb_ == 0) {
-        if (st->M == 32) conv2d_small_body<32>(st, V, reinterpret_cast<float2 *>(Phi), sm);
-        else conv2d_small_body<64>(st, V, reinterpret_cast<float2 *>(Phi), sm);
-      }
-      return;
-    }
-  }
+  if (st->direct) return;
   float2 *tw = sm;
   float2 *stg = sm + SGT_FFT_MAXM;
   float *kre = reinterpret_cast<float *>(stg + SGT_FFT_COLS * (st->M + SGT_FFT_PAD));
@@ -565,7 +832,7 @@ template <int D>
 __device__ __forceinline__ void k_fft_final_x_body(int vb_, int vg_, const SgtState *st, const float2 *__restrict__ W, typename Node<D>::T *__restrict__ Phi) {
   sgt_pdl_wait();
   __shared__ float2 tw[SGT_FFT_MAXM];
-  if (D == 2 && st->M <= SGT_FFT_SMALL_M) return;  // the column pass did it all
+  if (st->direct) return;
   fft_twiddles(tw, st->M);
   __syncthreads();
 #define CF(L) final_rows_body<D, L>(vb_, vg_, st, W, reinterpret_cast<float2 *>(Phi), tw)
@@ -578,15 +845,8 @@ k_fft_final_x(const SgtState *st, const float2 *__restrict__ W, typename Node<D>
   k_fft_final_x_body<D>(blockIdx.x, gridDim.x, st, W, Phi);
 }
 
-// shared memory of a column pass for FFT length Mmax; in d = 2 also enough
-// for the one-CTA convolution of the small lengths that Mmax admits
-__host__ __device__ inline size_t fft_cols_smem(int Mmax, int d = 3) {
-  size_t b = sizeof(float2) * (SGT_FFT_MAXM + (size_t)SGT_FFT_COLS * (Mmax + SGT_FFT_PAD)) +
-             sizeof(float) * (size_t)SGT_FFT_COLS * Mmax;
-  if (d == 2) {
-    const size_t m = Mmax < SGT_FFT_SMALL_M ? (size_t)Mmax : (size_t)SGT_FFT_SMALL_M;
-    const size_t small = sizeof(float2) * (m + m * (m + 1) + m * (m + 1));  // twiddles, kernel, 2 x m/2 data rows
-    if (small > b) b = small;
-  }
-  return b;
+// shared memory of a column pass for FFT length Mmax
+__host__ __device__ inline size_t fft_cols_smem(int Mmax) {
+  return sizeof(float2) * (SGT_FFT_MAXM + (size_t)SGT_FFT_COLS * (Mmax + SGT_FFT_PAD)) +
+         sizeof(float) * (size_t)SGT_FFT_COLS * Mmax;
 }

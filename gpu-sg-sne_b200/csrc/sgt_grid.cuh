@@ -12,7 +12,7 @@
 // B200 structure: two modes, picked per iteration by the grid decision.
 //   scatter mode (T = 0): no sort.  A group of lanes per point adds the
 //     point's weighted charges to one of several copies of the grid with
-//     vector reductions in L2 (k_scatter), k_fold sums the copies into V,
+//     vector reductions in L2 (k_scatter), k_spec_rows sums the copies into V,
 //     and k_gather gathers with the same lane groups.
 //   cell mode (T = 1; large jobs on grids with many points per cell): the
 //     points are counting-sorted by cell, and S2G sums each cell's points in
@@ -30,7 +30,7 @@
 #define SGT_LPP(D) ((D) == 3 ? 16 : 4)
 // Scatter mode: most copies of the grid.  L2 serialises the reductions that
 // meet on one node; with 32 copies 60k points on 16^2 nodes take 10.5 us
-// instead of 76, 100k on 117^2 10.3 instead of 20.7.  k_fold reads the copies
+// instead of 76, 100k on 117^2 10.3 instead of 20.7.  k_spec_rows reads the copies
 // back, so a grid takes them only as it has adds per node.
 #define SGT_COPIES 32
 // Points from which a dense grid is sorted by cell.  Below, scatter mode is
@@ -40,42 +40,6 @@
 // of the binning, S2G (cell mode) and G2S kernels: these kernels are bound by
 // load latency, not bandwidth, at a few warps per SM.
 #define SGT_PTS_U 4
-
-// Sums K per-lane values over the 32 lanes of a warp in K/2 + K/4 + ...
-// shuffles instead of 5K: at each step with offset O a lane keeps one half of
-// its values, sends the other half to lane ^ O and adds what it receives; once
-// the count no longer halves, the remaining offsets add whole vectors.  On
-// return acc[q], q < wsum_count(K, 16), of lane L holds the warp total of the
-// entry values acc[base + q], with base (zero on entry) advanced by the call;
-// lanes that share a base hold the same totals, and the lanes with
-// (L & wsum_full_mask(K, 16)) == 0 are one of each.
-__host__ __device__ constexpr int wsum_count(int k, int o) {
-  return o == 0 ? k : ((k % 2 == 0) ? wsum_count(k / 2, o / 2) : wsum_count(k, o / 2));
-}
-__host__ __device__ constexpr int wsum_full_mask(int k, int o) {
-  return o == 0 ? 0 : ((k % 2 == 0) ? wsum_full_mask(k / 2, o / 2) : (o | wsum_full_mask(k, o / 2)));
-}
-template <int K, int O>
-__device__ __forceinline__ void warp_multi_sum(float *acc, int lane, int &base) {
-  if constexpr (O > 0) {
-    if constexpr (K % 2 == 0) {
-      constexpr int H = K / 2;
-      const bool up = (lane & O) != 0;
-#pragma unroll
-      for (int q = 0; q < H; q++) {
-        const float send = up ? acc[q] : acc[q + H];
-        const float keep = up ? acc[q + H] : acc[q];
-        acc[q] = keep + __shfl_xor_sync(0xffffffffu, send, O);
-      }
-      if (up) base += H;
-      warp_multi_sum<H, O / 2>(acc, lane, base);
-    } else {
-#pragma unroll
-      for (int q = 0; q < K; q++) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], O);
-      warp_multi_sum<K, O / 2>(acc, lane, base);
-    }
-  }
-}
 
 // Smallest FFT length >= need among 32, 64, 96, 128, 192, ..., 768, 1024
 // (2^k and 3 * 2^k): the 3 * 2^k lengths cut the padding of grids just above
@@ -139,6 +103,10 @@ __device__ void sgt_finalize_grid(SgtState *st, const SgtJobParams &jp,
   st->N = N;
   st->M = M;
   st->scale = (float)(unsigned)(N - 3);
+  const double inv = (double)(N - 3) / (double)maxy;
+  st->inv_hi = (float)inv;
+  st->inv_lo = (float)(inv - (double)st->inv_hi);
+  st->direct = N <= jp.conv_max ? 1 : 0;
   st->h_eff = __fdiv_rn(maxy, (float)(n1 - 1) - 1.1920928955078125e-7f);
   const int cells = n1 - 1;  // floor bins lie in [0, n1-2]
   long ncell = cells;
@@ -165,14 +133,43 @@ __device__ void sgt_finalize_grid(SgtState *st, const SgtJobParams &jp,
 }
 
 // Scaled coordinate exactly as CU/nuconv.cu:9-36: (y - miny)/maxy, clamp to
-// 1-FLT_EPSILON, times (N-3).  Returns the shifted coordinate too.
-__device__ __forceinline__ float sgt_scale(float y, float miny, float maxy,
-                                           float scale, float &shifted) {
-  shifted = __fsub_rn(y, miny);
-  float v = __fdiv_rn(shifted, maxy);
+// 1-FLT_EPSILON, times (N-3).  The cells are the floors of these values.
+__device__ __forceinline__ float sgt_scale(float y, float miny, float maxy, float scale) {
+  float v = __fdiv_rn(__fsub_rn(y, miny), maxy);
   if (v >= 1.0f) v = 1.0f - 1.1920928955078125e-7f;
   return __fmul_rn(v, scale);
 }
+
+// Grid geometry of the current iteration, read once per thread.
+template <int D>
+struct GridGeom {
+  float miny[D], maxy, scale, inv_hi, inv_lo;
+  int N, cells;
+  __device__ __forceinline__ explicit GridGeom(const SgtState *st) {
+#pragma unroll
+    for (int k = 0; k < D; k++) miny[k] = st->miny[k];
+    maxy = st->maxy;
+    scale = st->scale;
+    inv_hi = st->inv_hi;
+    inv_lo = st->inv_lo;
+    N = st->N;
+    cells = N - 3;
+  }
+  // Cell f of coordinate y along axis k, and the point's place dd in it, in
+  // cells.  The cell is the floor of the reference's rounded coordinate; the
+  // place is taken from y itself with a two-term (N-3)/maxy and the rounding
+  // error of the shift, so it is good to a few 2^-24 of a cell however far
+  // the cell is from the origin (the rounded coordinate's error grows with
+  // the cell number, 3e-6 of a cell at cell 25).
+  __device__ __forceinline__ float place(float y, int k, int &f) const {
+    const float fl = floorf(sgt_scale(y, miny[k], maxy, scale));
+    f = (int)fl;
+    const float sh = __fsub_rn(y, miny[k]);
+    const float bb = __fsub_rn(sh, y);
+    const float err = __fsub_rn(__fsub_rn(y, __fsub_rn(sh, bb)), __fadd_rn(miny[k], bb));
+    return __fmaf_rn(sh, inv_hi, -fl) + __fmaf_rn(sh, inv_lo, __fmul_rn(err, inv_hi));
+  }
+};
 
 template <int D>
 __device__ __forceinline__ int sgt_cell_of(const int *f, int td) {
@@ -334,8 +331,11 @@ __device__ __forceinline__ void bin_scan_block(SgtState *st, const SgtJobParams 
 }
 
 // ---------------------------------------------------------------------------
-// Scatter mode: centre the points and add their weighted charges [1, y - c]
-// to the grid copy vb_ mod copies.  SGT_LPP(D) lanes share a point; lane q of
+// Scatter mode: centre the points and add their weighted charges to the grid
+// copy vb_ mod copies.  The charges at a node are [1, y - y_node], the
+// distance in cells: F and Z do not depend on the origin that y is measured
+// from, and with the node's own place as origin no sum cancels (k_gather,
+// k_spec_cols; the FFT passes move the origin to the grid's middle).  SGT_LPP(D) lanes share a point; lane q of
 // a group owns the stencil nodes with x offset q & 3 (3-D: and y offset
 // q >> 2), and every lane works out the point's weights for itself.
 // Bound by the reductions L2 takes: 100k points on 64^2 nodes 10.5 us (1.6M
@@ -364,15 +364,11 @@ __device__ __forceinline__ void k_scatter_body(int vb_, int vg_,
                                                SgtState *st, typename Node<D>::T *Vc) {
   if (st->T != 0) return;  // cell mode
   constexpr int L = SGT_LPP(D);
-  const int N = st->N, cells = N - 3;
-  const float maxy = st->maxy, scale = st->scale;
-  // charges are taken about the middle of the grid: F and Z are invariant to
-  // the origin of y, and |y - c| <= maxy/2 halves the cancellation in
-  // (1 + 2|y|^2) Phi0 - 2 y.Phi
-  const float hc = 0.5f * maxy;
-  float mean[3], miny[3];
+  const GridGeom<D> g(st);
+  const int N = g.N;
+  float mean[D];
 #pragma unroll
-  for (int k = 0; k < D; k++) { mean[k] = st->mean[k]; miny[k] = st->miny[k]; }
+  for (int k = 0; k < D; k++) mean[k] = st->mean[k];
   long nodes = N;
   if (D >= 2) nodes *= N;
   if (D >= 3) nodes *= N;
@@ -382,40 +378,39 @@ __device__ __forceinline__ void k_scatter_body(int vb_, int vg_,
   for (int i = vb_ * (SGT_THREADS / L) + threadIdx.x / L; i < n; i += step) {
     typename Vec<D>::T y = Ynext[i];
     int f[3];
-    float w[3][4], qc[3];
+    float w[3][4], u[3];  // u: distance from node 0 of the stencil, in cells
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < D; k++) {
       const float yc = __fsub_rn(comp<D>(y, k), mean[k]);
       setcomp<D>(y, k, yc);
-      float sh;
-      const float s = sgt_scale(yc, miny[k], maxy, scale, sh);
-      sgt_weights(s, f[k], w[k]);
-      qc[k] = sh - hc;
-      ok = ok && (unsigned)f[k] < (unsigned)cells;
+      const float dd = g.place(yc, k, f[k]);
+      sgt_weights(dd, w[k]);
+      u[k] = dd + 1.0f;
+      ok = ok && (unsigned)f[k] < (unsigned)g.cells;
     }
     if (q == 0) Y[i] = y;
     if (!ok) {  // outside the grid: skip the point
       if (q == 0) atomicOr(&st->error, SGT_EFLAG_CHUNK_OVERFLOW);
       continue;
     }
-    const float wx = pick4(w[0], qx);
+    const float wx = pick4(w[0], qx), ux = u[0] - (float)qx;
     if constexpr (D == 1) {
-      red_node(&Vc[f[0] + qx], wx, wx * qc[0]);
+      red_node(&Vc[f[0] + qx], wx, wx * ux);
     } else if constexpr (D == 2) {
 #pragma unroll
       for (int b = 0; b < 4; b++) {
         const float wt = w[1][b] * wx;
-        red_node(&Vc[f[0] + qx + N * (f[1] + b)], wt, wt * qc[0], wt * qc[1], 0.f);
+        red_node(&Vc[f[0] + qx + N * (f[1] + b)], wt, wt * ux, wt * (u[1] - (float)b), 0.f);
       }
     } else {
       const int qy = q >> 2;
-      const float wy = pick4(w[1], qy);
+      const float wy = pick4(w[1], qy) * wx, uy = u[1] - (float)qy;
 #pragma unroll
       for (int c = 0; c < 4; c++) {
-        const float wt = (wy * w[2][c]) * wx;
-        red_node(&Vc[f[0] + qx + (long)N * (f[1] + qy + (long)N * (f[2] + c))], wt, wt * qc[0],
-                 wt * qc[1], wt * qc[2]);
+        const float wt = wy * w[2][c];
+        red_node(&Vc[f[0] + qx + (long)N * (f[1] + qy + (long)N * (f[2] + c))], wt, wt * ux,
+                 wt * uy, wt * (u[2] - (float)c));
       }
     }
   }
@@ -426,50 +421,6 @@ __global__ void __launch_bounds__(SGT_THREADS, 8)
 k_scatter(const typename Vec<D>::T *__restrict__ Ynext, typename Vec<D>::T *__restrict__ Y, int n,
           SgtState *st, typename Node<D>::T *Vc) {
   k_scatter_body<D>(blockIdx.x, gridDim.x, Ynext, Y, n, st, Vc);
-}
-
-// ---------------------------------------------------------------------------
-// fold: V = sum of the grid copies, which are left zero for the next
-// iteration's scatter (they start zero at job creation).  Cell mode: V only
-// (k_bin_count cleared it and k_s2g_cell has added to it), nothing to do.
-// ---------------------------------------------------------------------------
-template <int D>
-__device__ __forceinline__ void k_fold_body(int vb_, int vg_, const SgtState *st,
-                                            typename Node<D>::T *__restrict__ Vc,
-                                            typename Node<D>::T *__restrict__ V) {
-  sgt_pdl_wait();
-  if (st->T != 0) return;
-  const int N = st->N, copies = st->copies;
-  long nodes = N;
-  if (D >= 2) nodes *= N;
-  if (D >= 3) nodes *= N;
-  typename Node<D>::T z;
-  if constexpr (D == 1) z = make_float2(0.f, 0.f); else z = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (long g = vb_ * (long)blockDim.x + threadIdx.x; g < nodes; g += (long)vg_ * blockDim.x) {
-    typename Node<D>::T a = z;
-    for (int c0 = 0; c0 < copies; c0 += 4) {
-      typename Node<D>::T t[4];
-#pragma unroll
-      for (int c = 0; c < 4; c++) t[c] = c0 + c < copies ? Vc[(c0 + c) * nodes + g] : z;
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        a.x += t[c].x;
-        a.y += t[c].y;
-        if constexpr (D >= 2) {
-          a.z += t[c].z;
-          if constexpr (D >= 3) a.w += t[c].w;
-        }
-        if (c0 + c < copies) Vc[(c0 + c) * nodes + g] = z;
-      }
-    }
-    V[g] = a;
-  }
-}
-template <int D>
-__global__ void __launch_bounds__(SGT_THREADS)
-k_fold(const SgtState *st, typename Node<D>::T *__restrict__ Vc,
-       typename Node<D>::T *__restrict__ V) {
-  k_fold_body<D>(blockIdx.x, gridDim.x, st, Vc, V);
 }
 
 // ---------------------------------------------------------------------------
@@ -525,9 +476,7 @@ __device__ __forceinline__ void k_bin_count_body(int vb_, int vg_, const typenam
         for (int k = 0; k < D; k++) {
           const float yc = __fsub_rn(comp<D>(y, k), mean[k]);
           setcomp<D>(y, k, yc);
-          float sh;
-          const float s = sgt_scale(yc, miny[k], maxy, scale, sh);
-          f[k] = (int)floorf(s);
+          f[k] = (int)floorf(sgt_scale(yc, miny[k], maxy, scale));
         }
         Y[i] = y;
         key = sgt_cell_of<D>(f, td);
@@ -611,8 +560,7 @@ __device__ __forceinline__ void k_bin_scatter_body(int vb_, int vg_, const typen
         int f[3] = {0, 0, 0};
 #pragma unroll
         for (int k = 0; k < D; k++) {
-          float sh;
-          f[k] = (int)floorf(sgt_scale(comp<D>(yv[u], k), miny[k], maxy, scale, sh));
+          f[k] = (int)floorf(sgt_scale(comp<D>(yv[u], k), miny[k], maxy, scale));
         }
         key = sgt_cell_of<D>(f, td);
       }
@@ -640,9 +588,8 @@ __device__ __forceinline__ void k_bin_scatter_body(int vb_, int vg_, const typen
         int f[3] = {0, 0, 0};
 #pragma unroll
         for (int k = 0; k < D; k++) {
-          float sh;
           const float v = comp<D>(yv[u], k);
-          f[k] = (int)floorf(sgt_scale(v, miny[k], maxy, scale, sh));
+          f[k] = (int)floorf(sgt_scale(v, miny[k], maxy, scale));
           if (k == 0) rec.x = v; else if (k == 1) rec.y = v; else rec.z = v;
         }
         key = sgt_cell_of<D>(f, td);
@@ -663,17 +610,15 @@ k_bin_scatter(const typename Vec<D>::T *__restrict__ Y, int n, SgtState *st,
   k_bin_scatter_body<D>(blockIdx.x, gridDim.x, Y, n, st, cursor, sorted);
 }
 
-// cells and weights of a sorted point
+// cell, weights and distances from stencil node 0 (in cells) of a sorted point
 template <int D>
-__device__ __forceinline__ void sgt_point_stencil(const float4 &rec,
-                                                  const float *miny, float maxy,
-                                                  float scale, int *f,
-                                                  float (*w)[4], float *ys) {
+__device__ __forceinline__ void sgt_point_stencil(const float4 &rec, const GridGeom<D> &g, int *f,
+                                                  float (*w)[4], float *u) {
 #pragma unroll
   for (int k = 0; k < D; k++) {
-    const float v = k == 0 ? rec.x : (k == 1 ? rec.y : rec.z);
-    const float s = sgt_scale(v, miny[k], maxy, scale, ys[k]);
-    sgt_weights(s, f[k], w[k]);
+    const float dd = g.place(k == 0 ? rec.x : (k == 1 ? rec.y : rec.z), k, f[k]);
+    sgt_weights(dd, w[k]);
+    u[k] = dd + 1.0f;
   }
 }
 
@@ -696,11 +641,7 @@ __device__ __forceinline__ void k_s2g_cell_body(int vb_, int vg_, const float4 *
   constexpr int PASSES = D == 3 ? 4 : 1;
   __shared__ float red[SGT_THREADS / 32][K];
   const int td = st->tiles_dim, N = st->N, nch = st->nchunks;
-  const float maxy = st->maxy, scale = st->scale;
-  const float hc = 0.5f * maxy;  // charge origin, as in k_scatter
-  float miny[3];
-#pragma unroll
-  for (int k = 0; k < D; k++) miny[k] = st->miny[k];
+  const GridGeom<D> gg(st);
   float *Vf = reinterpret_cast<float *>(V);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int c = vb_; c < nch; c += vg_) {
@@ -727,8 +668,8 @@ __device__ __forceinline__ void k_s2g_cell_body(int vb_, int vg_, const float4 *
         for (int u = 0; u < U; u++) {
           if (j0 + u * blockDim.x >= end) break;
           int f[3];
-          float w[3][4], ys[3];
-          sgt_point_stencil<D>(rv[u], miny, maxy, scale, f, w, ys);
+          float w[3][4], du[3];
+          sgt_point_stencil<D>(rv[u], gg, f, w, du);
           bool ok = f[0] == cf[0];
           if (D >= 2) ok = ok && f[1] == cf[1];
           if (D >= 3) ok = ok && f[2] == cf[2];
@@ -736,9 +677,6 @@ __device__ __forceinline__ void k_s2g_cell_body(int vb_, int vg_, const float4 *
             atomicOr(&st->error, SGT_EFLAG_CHUNK_OVERFLOW);
             continue;
           }
-          float qc[3];
-#pragma unroll
-          for (int k = 0; k < D; k++) qc[k] = ys[k] - hc;
           const float wz = D == 3 ? w[2][pass] : 1.f;
 #pragma unroll
           for (int a1 = 0; a1 < (D >= 2 ? 4 : 1); a1++) {
@@ -748,8 +686,9 @@ __device__ __forceinline__ void k_s2g_cell_body(int vb_, int vg_, const float4 *
               const float wt = wy * w[0][a0];
               const int nd = a1 * 4 + a0;
               acc[nd * C] += wt;
-#pragma unroll
-              for (int k = 0; k < D; k++) acc[nd * C + 1 + k] += wt * qc[k];
+              acc[nd * C + 1] += wt * (du[0] - (float)a0);
+              if constexpr (D >= 2) acc[nd * C + 2] += wt * (du[1] - (float)a1);
+              if constexpr (D >= 3) acc[nd * C + 3] += wt * (du[2] - (float)pass);
             }
           }
         }
@@ -785,13 +724,16 @@ k_s2g_cell(const float4 *__restrict__ sorted, SgtState *st,
   k_s2g_cell_body<D>(blockIdx.x, gridDim.x, sorted, st, chunks, V);
 }
 
-// Interpolated potentials p[0..d] at a point with stencil weights w and base
-// cell f: from the grid Phi, or (SM) from the block's copy cn of the 4^d
-// nodes of the point's cell, node a0 + 4 a1 + 16 a2.  Same products in the
-// same order either way.
+// Interpolated p[0] = Phi0 and p[1 + k] = y_k Phi0 - Phi_k (the repulsive
+// force numerator in cells) at a point with stencil weights w and base cell
+// f: from the grid Phi, or (SM) from the block's copy cn of the 4^d nodes of
+// the point's cell, node a0 + 4 a1 + 16 a2.  o: the point's distance from the
+// origin that Phi_k is taken about, per axis, less `loc` per node: the node
+// itself after the direct convolution (o = distance from stencil node 0,
+// loc = 1), the grid's middle after the FFT (loc = 0).
 template <int D, bool SM>
-__device__ __forceinline__ void g2s_potentials(const float (*w)[4], const int *f, int N,
-                                               const typename Node<D>::T *Phi,
+__device__ __forceinline__ void g2s_potentials(const float (*w)[4], const float *o, float loc,
+                                               const int *f, int N, const typename Node<D>::T *Phi,
                                                const typename Node<D>::T *cn, float *p) {
 #pragma unroll
   for (int a2 = 0; a2 < (D >= 3 ? 4 : 1); a2++)
@@ -810,13 +752,29 @@ __device__ __forceinline__ void g2s_potentials(const float (*w)[4], const int *f
         if constexpr (SM) v = cn[a0 + 4 * (a1 + 4 * a2)];
         else v = Phi[base + a0];
         p[0] += wt * v.x;
-        p[1] += wt * v.y;
+        p[1] += wt * ((o[0] - loc * (float)a0) * v.x - v.y);
         if constexpr (D >= 2) {
-          p[2] += wt * v.z;
-          if constexpr (D >= 3) p[3] += wt * v.w;
+          p[2] += wt * ((o[1] - loc * (float)a1) * v.x - v.z);
+          if constexpr (D >= 3) p[3] += wt * ((o[2] - loc * (float)a2) * v.x - v.w);
         }
       }
     }
+}
+
+// Force numerator and z of a point from its p (g2s_potentials) and its
+// distance m from the grid's middle in cells: z_i = Phi0 + 2 (y_i - c).F_i,
+// which is (1 + 2|y|^2) Phi0 - 2 y.Phi without its cancellation.
+template <int D>
+__device__ __forceinline__ double point_force(const float *p, const float *m, float h,
+                                              typename Vec<D>::T &fr) {
+  double dot = 0.0;
+  if constexpr (D == 3) fr.w = 0.f;
+#pragma unroll
+  for (int k = 0; k < D; k++) {
+    setcomp<D>(fr, k, h * p[k + 1]);
+    dot += (double)m[k] * (double)p[k + 1];
+  }
+  return (double)p[0] + 2.0 * (double)h * (double)h * dot;
 }
 
 // Z of a G2S launch: the block's FP64 partial, then the last block to finish
@@ -870,37 +828,39 @@ __device__ __forceinline__ void k_gather_body(int vb_, int vg_, SgtState *st,
   __shared__ double wz[SGT_THREADS / 32];
   __shared__ bool last;
   constexpr int L = SGT_LPP(D);
-  const int N = st->N, cells = N - 3;
-  const float maxy = st->maxy, scale = st->scale, hc = 0.5f * maxy;
-  float miny[3];
-#pragma unroll
-  for (int k = 0; k < D; k++) miny[k] = st->miny[k];
+  const GridGeom<D> g(st);
+  const int N = g.N;
+  const float h = st->h_eff, half = 0.5f * g.scale;
+  const bool direct = st->direct != 0;
   double zacc = 0.0;
   const int q = threadIdx.x % L, qx = q & 3;
   const int step = vg_ * (SGT_THREADS / L);
   const int rounds = (n + step - 1) / step;  // uniform, so that the shuffles converge
   int i = vb_ * (SGT_THREADS / L) + threadIdx.x / L;
   for (int r = 0; r < rounds; r++, i += step) {
-    float p[4] = {0.f, 0.f, 0.f, 0.f}, ys[3] = {0.f, 0.f, 0.f};
+    float p[4] = {0.f, 0.f, 0.f, 0.f}, m[3] = {0.f, 0.f, 0.f};
     if (i < n) {
       const typename Vec<D>::T y = Y[i];
       int f[3];
-      float w[3][4];
+      float w[3][4], o[3];
       bool ok = true;
 #pragma unroll
       for (int k = 0; k < D; k++) {
-        const float sv = sgt_scale(comp<D>(y, k), miny[k], maxy, scale, ys[k]);
-        sgt_weights(sv, f[k], w[k]);
-        ok = ok && (unsigned)f[k] < (unsigned)cells;
+        const float dd = g.place(comp<D>(y, k), k, f[k]);
+        sgt_weights(dd, w[k]);
+        m[k] = ((float)f[k] - half) + dd;
+        o[k] = direct ? dd + 1.0f : m[k];
+        ok = ok && (unsigned)f[k] < (unsigned)g.cells;
       }
       if (!ok) {  // outside the grid (S2G skipped it too): no force, no Z
         if (q == 0) atomicOr(&st->error, SGT_EFLAG_CHUNK_OVERFLOW);
       } else {
-        const float wx = pick4(w[0], qx);
+        const float loc = direct ? 1.0f : 0.0f;
+        const float wx = pick4(w[0], qx), ox = o[0] - loc * (float)qx;
         if constexpr (D == 1) {
           const float2 v = Phi[f[0] + qx];
           p[0] = wx * v.x;
-          p[1] = wx * v.y;
+          p[1] = wx * (ox * v.x - v.y);
         } else if constexpr (D == 2) {
           float4 v[4];
 #pragma unroll
@@ -909,43 +869,34 @@ __device__ __forceinline__ void k_gather_body(int vb_, int vg_, SgtState *st,
           for (int b = 0; b < 4; b++) {
             const float wt = w[1][b] * wx;
             p[0] += wt * v[b].x;
-            p[1] += wt * v[b].y;
-            p[2] += wt * v[b].z;
+            p[1] += wt * (ox * v[b].x - v[b].y);
+            p[2] += wt * ((o[1] - loc * (float)b) * v[b].x - v[b].z);
           }
         } else {
           const int qy = q >> 2;
-          const float wy = pick4(w[1], qy);
+          const float wy = pick4(w[1], qy) * wx, oy = o[1] - loc * (float)qy;
           float4 v[4];
 #pragma unroll
           for (int c = 0; c < 4; c++)
             v[c] = Phi[f[0] + qx + (long)N * (f[1] + qy + (long)N * (f[2] + c))];
 #pragma unroll
           for (int c = 0; c < 4; c++) {
-            const float wt = (wy * w[2][c]) * wx;
+            const float wt = wy * w[2][c];
             p[0] += wt * v[c].x;
-            p[1] += wt * v[c].y;
-            p[2] += wt * v[c].z;
-            p[3] += wt * v[c].w;
+            p[1] += wt * (ox * v[c].x - v[c].y);
+            p[2] += wt * (oy * v[c].x - v[c].z);
+            p[3] += wt * ((o[2] - loc * (float)c) * v[c].x - v[c].w);
           }
         }
       }
     }
 #pragma unroll
-    for (int o = 1; o < L; o *= 2)
+    for (int e = 1; e < L; e *= 2)
 #pragma unroll
-      for (int k = 0; k <= D; k++) p[k] += __shfl_xor_sync(0xffffffffu, p[k], o);
+      for (int k = 0; k <= D; k++) p[k] += __shfl_xor_sync(0xffffffffu, p[k], e);
     if (i < n && q == 0) {
-      double ysq = 0.0, dot = 0.0;
       typename Vec<D>::T fr;
-      if constexpr (D == 3) fr.w = 0.f;
-#pragma unroll
-      for (int k = 0; k < D; k++) {
-        const float yk = ys[k] - hc;
-        ysq += (double)yk * yk;
-        dot += (double)yk * p[k + 1];
-        setcomp<D>(fr, k, yk * p[0] - p[k + 1]);
-      }
-      zacc += (1.0 + 2.0 * ysq) * (double)p[0] - 2.0 * dot;
+      zacc += point_force<D>(p, m, h, fr);
       Frep_un[i] = fr;
     }
   }
@@ -970,11 +921,10 @@ __device__ __forceinline__ void k_g2s_body(int vb_, int vg_, const float4 *__res
   __shared__ double wz[SGT_THREADS / 32];
   __shared__ bool last;
   const int N = st->N, nch = st->nchunks;
-  const float maxy = st->maxy, scale = st->scale;
-  const float hc = 0.5f * maxy;  // charge origin used by S2G
-  float miny[3];
-#pragma unroll
-  for (int k = 0; k < D; k++) miny[k] = st->miny[k];
+  const GridGeom<D> gg(st);
+  const float h = st->h_eff, half = 0.5f * gg.scale;
+  const bool direct = st->direct != 0;
+  const float loc = direct ? 1.0f : 0.0f;
   double zacc = 0.0;
   // every point of a chunk reads the same 4^d nodes, which the
   // block stages once per chunk in shared memory
@@ -1009,24 +959,21 @@ __device__ __forceinline__ void k_g2s_body(int vb_, int vg_, const float4 *__res
         if (j0 + u * blockDim.x >= end) break;
         const float4 rec = rv[u];
         int f[3];
-        float w[3][4], ys[3];
-        sgt_point_stencil<D>(rec, miny, maxy, scale, f, w, ys);
+        float w[3][4], o[3], m[3];
+        sgt_point_stencil<D>(rec, gg, f, w, o);
         bool here = f[0] == cf[0];
         if (D >= 2) here = here && f[1] == cf[1];
         if (D >= 3) here = here && f[2] == cf[2];
-        float p[4] = {0.f, 0.f, 0.f, 0.f};
-        if (here) g2s_potentials<D, true>(w, f, N, Phi, cn, p);
-        else g2s_potentials<D, false>(w, f, N, Phi, cn, p);
-        double ysq = 0.0, dot = 0.0;
-        typename Vec<D>::T fr;
 #pragma unroll
         for (int k = 0; k < D; k++) {
-          const float yk = ys[k] - hc;
-          ysq += (double)yk * yk;
-          dot += (double)yk * p[k + 1];
-          setcomp<D>(fr, k, yk * p[0] - p[k + 1]);
+          m[k] = ((float)f[k] - half) + (o[k] - 1.0f);
+          if (!direct) o[k] = m[k];
         }
-        zacc += (1.0 + 2.0 * ysq) * (double)p[0] - 2.0 * dot;
+        float p[4] = {0.f, 0.f, 0.f, 0.f};
+        if (here) g2s_potentials<D, true>(w, o, loc, f, N, Phi, cn, p);
+        else g2s_potentials<D, false>(w, o, loc, f, N, Phi, cn, p);
+        typename Vec<D>::T fr;
+        zacc += point_force<D>(p, m, h, fr);
         Frep_un[__float_as_int(rec.w)] = fr;
       }
     }

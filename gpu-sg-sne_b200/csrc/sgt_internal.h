@@ -9,6 +9,7 @@
 
 cudaStream_t sgti_stream(sgt_ctx *ctx);
 int sgti_device(sgt_ctx *ctx);
+int sgti_sm_count(sgt_ctx *ctx);
 // records msg as the context's last error and returns s
 sgt_status sgti_fail(sgt_ctx *ctx, sgt_status s, const std::string &msg);
 // Stream-ordered device allocation (free with cudaFreeAsync) from the

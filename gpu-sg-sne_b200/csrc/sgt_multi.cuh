@@ -77,22 +77,25 @@ km_bin_scatter(const SgtJobView *__restrict__ views, const int *__restrict__ pre
 
 template <int D>
 __global__ void __launch_bounds__(SGT_THREADS)
-km_fold(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
-  SGT_MULTI_JOB
-  k_fold_body<D>(vb, vg, v.st, (typename Node<D>::T *)v.Vc, (typename Node<D>::T *)v.V);
-}
-
-template <int D>
-__global__ void __launch_bounds__(SGT_THREADS)
 km_s2g_cell(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
   SGT_MULTI_JOB
   k_s2g_cell_body<D>(vb, vg, v.sorted, v.st, v.chunks, (typename Node<D>::T *)v.V);
 }
 
-__global__ void __launch_bounds__(SGT_THREADS)
-km_conv1d(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
+template <int D>
+__global__ void __launch_bounds__(SGT_THREADS, 4)
+km_spec_rows(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
   SGT_MULTI_JOB
-  k_conv1d_body(vb, vg, v.st, (const float2 *)v.V, (float2 *)v.Phi);
+  k_spec_rows_body<D>(vb, vg, v.st, (typename Node<D>::T *)v.Vc, (typename Node<D>::T *)v.V, v.W,
+                      SGT_SPEC_BOTH);
+}
+
+template <int D>
+__global__ void __launch_bounds__(SGT_THREADS, 3)
+km_spec_cols(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
+  SGT_MULTI_JOB
+  k_spec_cols_body<D>(vb, vg, v.st, (const typename Node<D>::T *)v.V, v.W,
+                      (typename Node<D>::T *)v.Phi);
 }
 
 template <int D>

@@ -47,9 +47,8 @@ __global__ void k_cell_keys(const typename Vec<D>::T *__restrict__ Ynext, int n,
     unsigned f[3] = {0, 0, 0};
 #pragma unroll
     for (int k = 0; k < D; k++) {
-      float sh;
       const float yc = __fsub_rn(comp<D>(y, k), st->mean[k]);
-      const float v = fmaxf(floorf(sgt_scale(yc, st->miny[k], maxy, res, sh)), 0.f);
+      const float v = fmaxf(floorf(sgt_scale(yc, st->miny[k], maxy, res)), 0.f);
       f[k] = min((unsigned)v, (unsigned)res - 1u);
     }
     unsigned key;
