@@ -2,9 +2,9 @@
 // front of the perplexity equalisation (the reference's command line tool
 // calls FLANN, an approximate search, at
 // CU/testing_modules/demo_perplexity.cu:131; this search is exact).
-// Two methods return the same bits: the SIMT search (k_knn) and, for up to
-// 64 dimensions and 32 neighbours, a tensor-core filter (k_knn_tc, further
-// down) whose candidates are re-ranked with the SIMT search's arithmetic.
+// Two methods return the same bits: the SIMT search (k_knn) and a tensor-core
+// filter (k_knn_tc, further down) whose candidates are re-ranked with the SIMT
+// search's arithmetic.
 //
 // SIMT search: one query per thread, 128 queries per CTA.  Candidates stream through
 // shared memory in tiles of 64 points x 64 dimensions, queries in tiles of
@@ -20,6 +20,8 @@
 #include "../../include/sgtsne_b200.h"
 #include "sgt_internal.h"
 #include "sgt_async.cuh"
+
+#include <cuda_bf16.h>
 
 #include <algorithm>
 #include <string>
@@ -124,47 +126,67 @@ k_knn(const float *__restrict__ X, int n, int dim, int k, const int *__restrict_
 
 
 // ---------------------------------------------------------------------------
-// Tensor-core filter (points of up to 64 dimensions, k up to 32).
+// Tensor-core filter.
 //
-// Every squared distance is evaluated on the tensor cores as one dot product
-// of augmented rows: a query (q, 1, -|q|^2/2) and a candidate
-// (c, -|c|^2/2, 1) give q.c - (|q|^2 + |c|^2)/2 = -d^2/2.  The MMAs are of
-// kind::tf32 in three terms (hi.hi + hi.lo + lo.hi, where x = hi + lo with
-// hi = tf32(x), lo = tf32(x - hi): about 22 bits of each product), FP32
-// accumulation in tensor memory.  Each query keeps the KNN_TC_CAP nearest
-// candidates under that approximation; the list is then re-ranked with the
-// exact arithmetic of k_knn (sums of squared differences in dimension
+// q.c - |c|^2/2 = (|q|^2 - d^2)/2 ranks the candidates c of a query q.  The
+// products run on the tensor cores as BF16 MMAs (kind::f16) in three terms,
+// hi.hi + hi.lo + lo.hi with x = hi + lo + e, hi = bf16(x), lo = bf16(x - hi),
+// |e| <= 2^-18 |x|, FP32 accumulation in tensor memory; points that are BF16
+// numbers themselves (8-bit images) have zero low parts and take the first
+// term alone.  The list of nearest candidates under these keys is re-ranked
+// with the exact arithmetic of k_knn (sums of squared differences in dimension
 // order), so returned distances are bit-identical to it.  A query whose list
-// could miss a true neighbour -- the list's largest approximate distance
-// minus the error bound EPS * (|q|^2 + max |c|^2) not above the k-th exact
-// distance -- is redone by k_knn.
+// could miss a true neighbour is redone by k_knn: the nearest candidate ever
+// dropped, less the bound EPS (|q|^2 + max |c|^2) on a key's error, has to lie
+// beyond the k-th exact distance.
 //
-// Operands: each block of 128 points is stored once, before the search, as
-// the image of its shared-memory tile in each role: K-major, no swizzle,
-// core matrices of 8 rows x 16 bytes; unit u (4 dimensions) of all 128 rows
-// is 2 KB, so the leading-dimension offset (next 4 dimensions) is 2048 B and
-// the stride offset (next 8 rows) 128 B.  hi and lo images follow each
-// other.  A CTA holds the images of one or two blocks of 128 queries and
-// streams candidate images through two or three stages by bulk copies; one
-// thread issues the MMAs of each 128 x 128 tile into one of two
-// tensor-memory accumulators per query block while that block's four warps
-// scan the other (tcgen05.ld, one query row per thread).
+// Lists: a query's candidates are scanned by two threads (one per half of
+// each tile's columns), each with an unordered buffer of CAP entries in L2.
+// A key above the thread's threshold is appended; when a buffer is nearly
+// full its warp selects the L best by a bitwise search for the L-th key
+// (E = CAP / 32 entries a lane, one warp-wide count per bit) and that key
+// becomes the threshold.  CAP / L = 3 to 4 times as many candidates are seen
+// between selections each time, so a query needs a handful of them, and the
+// scan of a tile is a load, an add and a compare per candidate.  (Lists kept
+// sorted or with their maximum at hand in registers cost a serial pass per
+// candidate admitted, with the whole block waiting: 12 ms per wave of query
+// blocks, 62 ms of 62 at 100,000 points.)
+//
+// Operands: blocks of 128 query rows and 256 candidate rows are stored once
+// as images of their shared-memory tiles: K-major, no swizzle, core matrices
+// of 8 rows x 16 bytes (8 dimensions), unit u of all rows contiguous, hi and
+// lo parts one after the other.  Points of up to 64 dimensions keep the query
+// image resident and stream candidate tiles; wider points stream both in
+// chunks of 64 dimensions.  One thread issues the copies and MMAs; each
+// 128 x 256 tile accumulates into one of two halves of tensor memory while
+// eight warps scan the other.
 //
 // Descriptor fields follow the PTX ISA's tcgen05 shared-memory and
 // instruction descriptors (the same bit layout as CUTLASS's
 // cute::UMMA::SmemDescriptor and UMMA::InstrDescriptor): start address,
 // leading and stride byte offsets in 16-byte units, version 1 at bit 46,
-// no swizzle; D format F32 at bit 4, A and B formats TF32 (2) at bits 7 and
+// no swizzle; D format F32 at bit 4, A and B formats BF16 (1) at bits 7 and
 // 10, both K-major, N/8 at bit 17 and M/16 at bit 24.
-constexpr int KNN_TC_M = 128;
-constexpr int KNN_TC_MAXK = 32;
-constexpr float KNN_TC_EPS = 1e-4f;
+constexpr int KNN_TC_M = 128;      // queries per block
+constexpr int KNN_TC_N = 256;      // candidates per tile
+constexpr int KNN_TC_KU = 8;       // units (of 8 dimensions) per chunk
+constexpr int KNN_TC_MAXK = 32;    // limits of SGT_KNN_TENSOR
+constexpr int KNN_TC_MAXDIM = 64;
+constexpr int KNN_TC_SCAN = 256;   // scanning threads; one more warp issues
+constexpr int KNN_TC_THREADS = KNN_TC_SCAN + 32;
+constexpr unsigned KNN_TC_APART = KNN_TC_KU * KNN_TC_M * 16;  // bytes of a chunk's part
+constexpr unsigned KNN_TC_BPART = KNN_TC_KU * KNN_TC_N * 16;
+constexpr unsigned KNN_TC_SMEM = 4 * (KNN_TC_APART + KNN_TC_BPART);  // 192 KB
 
-__device__ __forceinline__ float tf32_rna(float x) {
-  unsigned r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return __uint_as_float(r);
+// Bound on the error of 2 key = |q|^2 - d^2, relative to |q|^2 + max |c|^2:
+// 2^-21 of the products' sum per accumulated MMA of 16 dimensions and, in
+// three terms, twice 3 * 2^-18 for the neglected parts.
+__host__ __device__ inline float knn_tc_eps(int dim, bool exact) {
+  const float steps = (float)((dim + 15) / 16);
+  return exact ? (steps + 1.f) * 4.8e-7f
+               : (dim <= KNN_TC_MAXDIM ? 1e-4f : 2.4e-5f + 3.f * steps * 4.8e-7f);
 }
+
 // shared-memory matrix descriptor: K-major, no swizzle
 __device__ __forceinline__ unsigned long long umma_desc(unsigned addr, unsigned lbo,
                                                         unsigned sbo) {
@@ -172,12 +194,12 @@ __device__ __forceinline__ unsigned long long umma_desc(unsigned addr, unsigned 
          ((unsigned long long)((lbo >> 4) & 0x3FFFu) << 16) |
          ((unsigned long long)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
-__device__ __forceinline__ void umma_tf32(unsigned dtmem, unsigned long long a,
+__device__ __forceinline__ void umma_bf16(unsigned dtmem, unsigned long long a,
                                           unsigned long long b, unsigned idesc, unsigned acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(dtmem), "l"(a), "l"(b), "r"(idesc), "r"(acc));
 }
 __device__ __forceinline__ void umma_commit(unsigned bar) {
@@ -185,11 +207,34 @@ __device__ __forceinline__ void umma_commit(unsigned bar) {
       "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
       : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+// bounded wait that also ends when another thread of the block gave up
+__device__ __forceinline__ bool mbar_wait_or(unsigned bar, unsigned parity, volatile int *gave_up) {
+  const long long t0 = clock64();
+  while (true) {
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if (*gave_up) return false;
+    if (clock64() - t0 > SGT_SPIN_CYCLES) {
+      *gave_up = 1;
+      return false;
+    }
+  }
 }
 __device__ __forceinline__ void tmem_ld32(unsigned taddr, float *v) {
   unsigned r[32];
@@ -209,358 +254,426 @@ __device__ __forceinline__ void tmem_ld32(unsigned taddr, float *v) {
   for (int j = 0; j < 32; j++) v[j] = __uint_as_float(r[j]);
 }
 
-// hi/lo images of every 128-point block in its two roles ([block][part]
-// [unit][row] float4; unused dimensions are zero), and the squared norms
-// (FP32, dimension order) with their maximum.  A query row is
-// (x, 1, -|x|^2/2) and a candidate row (x, -|x|^2/2, 1) in dimensions
-// dim and dim + 1, so one product is q.c - (|q|^2 + |c|^2)/2 = -d^2/2.
-// Query rows past n are zero; candidate rows past n are (0, -1e30, 0), at
-// distance 2e30 from every query, so they are admitted only while a list is
-// not yet full and sort after every real candidate.
-__global__ void k_knn_norms(const float *__restrict__ X, int n, int dim, float *__restrict__ nrm,
-                            unsigned *__restrict__ nmax) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+// BF16 (round to nearest even) of a float, as its upper 16 bits; inf and NaN
+// keep their meaning
+__device__ __forceinline__ unsigned bf16_bits(float x) {
+  return (unsigned)__bfloat16_as_ushort(__float2bfloat16_rn(x));
+}
+__device__ __forceinline__ float bf16_value(unsigned b) { return __uint_as_float(b << 16); }
+
+// squared norms (FP32, dimension order), their maximum, the candidates' key
+// offsets -|c|^2/2 (-inf behind the last point: never admitted), and whether
+// some coordinate is no BF16 number; a warp per point
+__global__ void k_knn_norms(const float *__restrict__ X, int n, int npad, int dim,
+                            float *__restrict__ nrm, float *__restrict__ off,
+                            unsigned *__restrict__ nmax, int *__restrict__ inexact) {
+  __shared__ float tile[8][32][33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // a warp takes 32 points; 32 x 32 tiles turn coalesced loads into a
+  // point per lane
+  for (int i0 = (blockIdx.x * 8 + w) * 32; i0 < npad; i0 += gridDim.x * 256) {
     float s = 0.f;
-    for (int kk = 0; kk < dim; kk++) s = fmaf(X[(long)i * dim + kk], X[(long)i * dim + kk], s);
-    nrm[i] = s;
-    atomicMax(nmax, __float_as_uint(s));  // non-negative floats order as integers
+    bool low = false;
+    for (int k0 = 0; k0 < dim; k0 += 32) {
+      __syncwarp();
+      for (int r = 0; r < 32; r++)
+        tile[w][r][lane] = i0 + r < n && k0 + lane < dim ? X[(long)(i0 + r) * dim + k0 + lane] : 0.f;
+      __syncwarp();
+      for (int kk = 0; kk < min(32, dim - k0); kk++) {
+        const float x = tile[w][lane][kk];
+        s = fmaf(x, x, s);
+        low |= bf16_value(bf16_bits(x)) != x;
+      }
+    }
+    const int i = i0 + lane;
+    if (i < n) nrm[i] = s;
+    if (i < npad) off[i] = i < n ? -0.5f * s : -INFINITY;
+    // non-negative floats order as integers (a NaN norm as the largest)
+    const unsigned m = __reduce_max_sync(0xffffffffu, i < n ? __float_as_uint(s) : 0u);
+    if (lane == 0) atomicMax(nmax, m);
+    if (__any_sync(0xffffffffu, low) && lane == 0) *inexact = 1;
   }
 }
 
-__global__ void k_knn_split(const float *__restrict__ X, const float *__restrict__ nrm, int n,
-                            int dim, int U, int nblk, float4 *__restrict__ imgA,
-                            float4 *__restrict__ imgB) {
-  const long total = (long)nblk * U * KNN_TC_M;
+// hi/lo images of the points in blocks of `rows` ([block][part][unit][row],
+// 8 dimensions of 2 bytes); rows past n and unused dimensions are zero.
+__global__ void k_knn_split(const float *__restrict__ X, int n, int dim, int U, int rows, int nblk,
+                            uint4 *__restrict__ img) {
+  const long total = (long)nblk * rows * U;
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total;
        e += (long)gridDim.x * blockDim.x) {
-    const int row = (int)(e % KNN_TC_M);
-    const int u = (int)((e / KNN_TC_M) % U);
-    const int b = (int)(e / ((long)KNN_TC_M * U));
-    const int i = b * KNN_TC_M + row;
-    float xa[4], xb[4];
+    const int row = (int)(e % rows);
+    const int u = (int)((e / rows) % U);
+    const int b = (int)(e / ((long)rows * U));
+    const int i = b * rows + row;
+    unsigned h[8], l[8];
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const int kk = 4 * u + c;
-      float x = 0.f, ya = 0.f, yb = (i >= n && kk == dim) ? -1e30f : 0.f;
-      if (i < n) {
-        if (kk < dim) {
-          x = X[(long)i * dim + kk];
-          ya = yb = x;
-        } else if (kk == dim) {
-          ya = 1.f;
-          yb = -0.5f * nrm[i];
-        } else if (kk == dim + 1) {
-          ya = -0.5f * nrm[i];
-          yb = 1.f;
-        }
-      }
-      xa[c] = ya;
-      xb[c] = yb;
+    for (int c = 0; c < 8; c++) {
+      const int kk = 8 * u + c;
+      const float x = i < n && kk < dim ? X[(long)i * dim + kk] : 0.f;
+      h[c] = bf16_bits(x);
+      l[c] = bf16_bits(x - bf16_value(h[c]));
     }
-    float ha[4], la[4], hb[4], lb[4];
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      ha[c] = tf32_rna(xa[c]);
-      la[c] = tf32_rna(xa[c] - ha[c]);
-      hb[c] = tf32_rna(xb[c]);
-      lb[c] = tf32_rna(xb[c] - hb[c]);
-    }
-    const long base = (long)b * 2 * U * KNN_TC_M;
-    const long oh = base + (long)u * KNN_TC_M + row, ol = base + (long)(U + u) * KNN_TC_M + row;
-    imgA[oh] = make_float4(ha[0], ha[1], ha[2], ha[3]);
-    imgA[ol] = make_float4(la[0], la[1], la[2], la[3]);
-    imgB[oh] = make_float4(hb[0], hb[1], hb[2], hb[3]);
-    imgB[ol] = make_float4(lb[0], lb[1], lb[2], lb[3]);
+    uint4 vh, vl;
+    vh = make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4] | h[5] << 16, h[6] | h[7] << 16);
+    vl = make_uint4(l[0] | l[1] << 16, l[2] | l[3] << 16, l[4] | l[5] << 16, l[6] | l[7] << 16);
+    const long base = (long)b * 2 * U * rows + (long)u * rows + row;
+    img[base] = vh;
+    img[base + (long)U * rows] = vl;
   }
 }
 
-// Candidate list of the filter, in registers (every index below is a
-// compile-time constant after unrolling): KNN_TC_CAP entries, unordered,
-// with the position and value of its largest entry (the admission
-// threshold).  Candidates that beat the threshold wait in a per-thread queue;
-// when one thread's queue could overflow, the whole warp merges its queues
-// at once, so the lists of a warp's 32 queries are updated together rather
-// than one query at a time.
-constexpr int KNN_TC_CAP = 64;
-constexpr int KNN_TC_QMAX = 64;
+// floats as unsigned integers in the same order
+__device__ __forceinline__ unsigned knn_ordered(float x) {
+  const unsigned b = __float_as_uint(x);
+  return b ^ ((b >> 31) ? 0xffffffffu : 0x80000000u);
+}
+__device__ __forceinline__ float knn_unordered(unsigned u) {
+  return __uint_as_float((u >> 31) ? u ^ 0x80000000u : ~u);
+}
 
-struct TcList {
-  float d[KNN_TC_CAP];
-  int j[KNN_TC_CAP];
-  float thr;  // largest entry (distance, index) and its slot
-  int thi, mp;
-  float mthr;  // -thr/2: a tile value v (= -d^2/2) admits its candidate when v > mthr
-  __device__ __forceinline__ void init() {
+// The largest T with at least `want` of the warp's entries u >= T (entries of
+// value 0 are empty; more than `want` are not), stopping early when exactly
+// `want` reach it.
+template <int E>
+__device__ __forceinline__ unsigned knn_kth(const unsigned *u, int want) {
+  unsigned T = 0;
+  for (int bit = 31; bit >= 0; bit--) {
+    const unsigned trial = T | (1u << bit);
+    unsigned c = 0;
 #pragma unroll
-    for (int e = 0; e < KNN_TC_CAP; e++) {
-      d[e] = INFINITY;
-      j[e] = 0x7fffffff;
+    for (int i = 0; i < E; i++) c += u[i] >= trial;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((int)c >= want) T = trial;
+    if ((int)c == want) break;
+  }
+  return T;
+}
+
+// One warp keeps the L best of a buffer's cnt > L entries, in place; returns
+// the threshold: no dropped key is above it.
+template <int L, int CAP>
+__device__ __forceinline__ float knn_select(float2 *buf, int cnt) {
+  constexpr int E = CAP / 32;
+  const int lane = threadIdx.x & 31;
+  float2 v[E];
+  unsigned u[E];
+#pragma unroll
+  for (int i = 0; i < E; i++) {
+    const int e = lane + 32 * i;
+    v[i] = e < cnt ? buf[e] : make_float2(-INFINITY, 0.f);
+    u[i] = e < cnt ? knn_ordered(v[i].x) : 0u;
+  }
+  const unsigned T = knn_kth<E>(u, L);
+  __syncwarp();
+  // all above T, then as many of those equal to it as fit
+  int at = 0;
+#pragma unroll
+  for (int pass = 0; pass < 2; pass++)
+#pragma unroll
+    for (int i = 0; i < E; i++) {
+      const bool keep = pass == 0 ? u[i] > T : u[i] == T;
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      const int slot = at + __popc(m & ((1u << lane) - 1u));
+      if (keep && slot < L) buf[slot] = v[i];
+      at += __popc(m);
     }
-    thr = INFINITY;
-    thi = 0x7fffffff;
-    mp = 0;
-    mthr = -INFINITY;
-  }
-  __device__ __forceinline__ void offer(float dd, int jj) {
-    if (!knn_less(dd, jj, thr, thi)) return;
-#pragma unroll
-    for (int e = 0; e < KNN_TC_CAP; e++)
-      if (e == mp) {
-        d[e] = dd;
-        j[e] = jj;
-      }
-    thr = d[0];
-    thi = j[0];
-    mp = 0;
-#pragma unroll
-    for (int e = 1; e < KNN_TC_CAP; e++)
-      if (knn_less(thr, thi, d[e], j[e])) {
-        thr = d[e];
-        thi = j[e];
-        mp = e;
-      }
-    mthr = -0.5f * thr;
-  }
-};
+  __syncwarp();
+  return knn_unordered(T);
+}
 
-// One CTA holds QB (1 or 2) blocks of 128 queries: warps 4a..4a+3 own query
-// block a, whose two accumulators sit at tensor-memory columns 256a and
-// 256a + 128; every candidate tile streamed in serves all of them.
-__global__ void __launch_bounds__(2 * KNN_TC_M, 1)
-k_knn_tc(const float4 *__restrict__ imgA, const float4 *__restrict__ imgB,
-         const float *__restrict__ nrm, const unsigned *__restrict__ nmax,
-         const float *__restrict__ X, int n, int dim, int U, int QB, int nstage, int k,
-         int *__restrict__ idx, float *__restrict__ d2,
-         int *__restrict__ redo, int *__restrict__ nredo, int *__restrict__ err) {
+// A block walks over query blocks; warps 0-7 scan (warp w: rows 32 (w & 3)..,
+// columns 128 (w >> 2)..), lane 0 of warp 8 issues copies and MMAs.
+template <int L, int CAP>
+__global__ void __launch_bounds__(KNN_TC_THREADS, 1)
+k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict__ imgB,
+         const float *__restrict__ nrm, const float *__restrict__ off,
+         const unsigned *__restrict__ nmax, const int *__restrict__ inexact,
+         const float *__restrict__ X, int n, int dim, int U, int k, float2 *__restrict__ bufs,
+         int *__restrict__ idx, float *__restrict__ d2, int *__restrict__ redo,
+         int *__restrict__ nredo, int *__restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) unsigned long long bars[7];  // A full, B full x3, MMA done x2
+  // full x4, empty x4, accumulator full x2, empty x2, resident A
+  __shared__ __align__(8) unsigned long long bars[13];
   __shared__ unsigned tslot;
-  __shared__ volatile int abort_flag;
-  const int t = threadIdx.x, warp = t >> 5;
-  const int nt = (n + KNN_TC_M - 1) / KNN_TC_M;
-  const int qb0 = blockIdx.x * QB;           // first query block of the CTA
-  const int na = min(QB, nt - qb0);          // query blocks that exist
-  const int qa = warp >> 2;                  // this warp's query block
-  const int q = (qb0 + qa) * KNN_TC_M + (t & (KNN_TC_M - 1));
-  const unsigned tcols = 256u * (unsigned)QB;
-  const unsigned ubytes = (unsigned)U * 2048u, pbytes = 2u * ubytes;
-  const unsigned sA = smem_u32(smem);
-  const unsigned barA = smem_u32(&bars[0]);
-  const unsigned barM[2] = {smem_u32(&bars[4]), smem_u32(&bars[5])};
-  const char *gA = reinterpret_cast<const char *>(imgA);
-  const char *gB = reinterpret_cast<const char *>(imgB);
+  __shared__ volatile int gave_up;
+  __shared__ int s_cnt[KNN_TC_SCAN];
+  __shared__ float s_thr[KNN_TC_SCAN];
+  __shared__ int s_idx[8][L];
+  __shared__ float s_d[8][L];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int nq = (n + KNN_TC_M - 1) / KNN_TC_M, ntile = (n + KNN_TC_N - 1) / KNN_TC_N;
+  const int nch = (U + KNN_TC_KU - 1) / KNN_TC_KU;
+  const bool three = *inexact != 0, resident = nch == 1;
+  const int parts = three ? 2 : 1, nst = three ? 2 : 4;
+  const unsigned sm0 = smem_u32(smem);
+  const unsigned a_bytes = resident ? 0u : parts * KNN_TC_APART;
+  const unsigned st_bytes = a_bytes + parts * KNN_TC_BPART;
+  const unsigned st0 = sm0 + (resident ? parts * KNN_TC_APART : 0u);
+  auto bar_full = [&](int st) { return smem_u32(&bars[st]); };
+  auto bar_free = [&](int st) { return smem_u32(&bars[4 + st]); };
+  auto bar_acc = [&](int b) { return smem_u32(&bars[8 + b]); };
+  auto bar_scan = [&](int b) { return smem_u32(&bars[10 + b]); };
+  const unsigned bar_a = smem_u32(&bars[12]);
   if (t == 0) {
-    abort_flag = 0;
-    for (int b = 0; b < 6; b++) mbar_init(smem_u32(&bars[b]), 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    gave_up = 0;
+    for (int b = 0; b < 13; b++) mbar_init(smem_u32(&bars[b]), b == 10 || b == 11 ? 8 : 1);
+    mbar_fence_init();
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 ::"r"(smem_u32(&tslot)), "r"(tcols));
+                 ::"r"(smem_u32(&tslot)), "r"(512u));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const unsigned tmem = tslot;
-  // thread 0: copies and MMAs issued and not yet waited for, with the parity
-  // of the phase each completes.  Tile ti sits in stage ti % nstage.
-  bool cpend[3] = {false, false, false}, mpend[2] = {false, false};
-  unsigned cpar[3] = {0, 0, 0}, mpar[2] = {0, 0};
-  auto stage_addr = [&](int st) { return sA + (unsigned)(QB + st) * pbytes; };
-  auto bar_full = [&](int st) { return smem_u32(&bars[1 + st]); };
-  auto load_tile = [&](int ti) {
-    const int st = ti % nstage;
-    mbar_expect_tx(bar_full(st), pbytes);
-    bulk_g2s(stage_addr(st), gB + (size_t)ti * pbytes, pbytes, bar_full(st));
-    cpend[st] = true;
-    cpar[st] = (unsigned)((ti / nstage) & 1);
-  };
-  if (t == 0) {
-    mbar_expect_tx(barA, (unsigned)na * pbytes);
-    for (int a = 0; a < na; a++)
-      bulk_g2s(sA + (unsigned)a * pbytes, gA + (size_t)(qb0 + a) * pbytes, pbytes, barA);
-    for (int ti = 0; ti < nstage && ti < nt; ti++) load_tile(ti);
-  }
-  // D = A B^T: M = 128, N = 128, FP32 accumulate, TF32 A and B, both K-major
-  const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((128u >> 3) << 17) |
-                         ((128u >> 4) << 24);
-  const float qn = q < n ? nrm[q] : 0.f;
-  TcList L;
-  L.init();
-  if (q >= n) {  // admits nothing
-    L.thr = -INFINITY;
-    L.mthr = INFINITY;
-  }
-  // queue of candidates that beat the threshold (local memory, written
-  // rarely): drained, by the whole warp at once, once a thread could
-  // overflow it during the next 32 columns
-  float qd[KNN_TC_QMAX];
-  int qi[KNN_TC_QMAX];
-  int qc = 0;
-  bool ok = true;
-  for (int it = 0; it <= nt; it++) {
-    if (it < nt && t == 0 && ok) {  // MMAs of tile it into accumulator it & 1
-      const int st = it % nstage, s = it & 1;
-      if (it == 0) ok = mbar_wait(barA, 0);
-      if (ok) ok = mbar_wait(bar_full(st), (unsigned)((it / nstage) & 1));
-      if (ok) {
-        cpend[st] = false;
-        tc_fence_after();
-        const unsigned sb = stage_addr(st);
-        // the start address is the descriptor's low field: a K step of
-        // 4096 B adds 256
-        const unsigned long long bh = umma_desc(sb, 2048, 128);
-        const unsigned long long bl = umma_desc(sb + ubytes, 2048, 128);
-        for (int a = 0; a < na; a++) {
-          const unsigned dt = tmem + 256u * (unsigned)a + (unsigned)s * 128u;
-          const unsigned long long ah = umma_desc(sA + (unsigned)a * pbytes, 2048, 128);
-          const unsigned long long al = umma_desc(sA + (unsigned)a * pbytes + ubytes, 2048, 128);
-          for (int ks = 0; ks < U / 2; ks++) {
-            const unsigned long long o = (unsigned long long)ks * 256u;
-            umma_tf32(dt, ah + o, bh + o, idesc, ks > 0 ? 1u : 0u);
-            umma_tf32(dt, ah + o, bl + o, idesc, 1u);
-            umma_tf32(dt, al + o, bh + o, idesc, 1u);
+  const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((KNN_TC_N >> 3) << 17) |
+                         ((KNN_TC_M >> 4) << 24);
+  const float eps = knn_tc_eps(dim, !three), cmax = __uint_as_float(*nmax);
+  // running counts of tiles and of pipeline steps over all query blocks
+  unsigned tiles = 0, steps = 0, loads = 0, blocks = 0;
+  for (int qb = blockIdx.x; qb < nq; qb += gridDim.x, blocks++) {
+    if (warp == 8) {
+      if (lane == 0) {
+        const unsigned total = (unsigned)ntile * (unsigned)nch;
+        bool ok = true;
+        // copies of step g of this block: chunk g % nch of tile g / nch
+        auto load = [&](unsigned g) {
+          const int st = (int)(loads % (unsigned)nst);
+          const unsigned turn = loads / (unsigned)nst;
+          if (turn > 0) ok = ok && mbar_wait_or(bar_free(st), (turn - 1) & 1, &gave_up);
+          if (!ok) return;
+          const int tile = (int)(g / (unsigned)nch), ch = (int)(g % (unsigned)nch);
+          const int uc = min(KNN_TC_KU, U - ch * KNN_TC_KU);
+          const unsigned sb = st0 + st * st_bytes;
+          mbar_expect_tx(bar_full(st), parts * uc * 16u * (KNN_TC_N + (resident ? 0 : KNN_TC_M)));
+          for (int p = 0; p < parts; p++) {
+            if (!resident)
+              bulk_g2s(sb + p * KNN_TC_APART,
+                       imgA + (((size_t)qb * 2 + p) * U + ch * KNN_TC_KU) * KNN_TC_M * 16,
+                       uc * KNN_TC_M * 16u, bar_full(st));
+            bulk_g2s(sb + a_bytes + p * KNN_TC_BPART,
+                     imgB + (((size_t)tile * 2 + p) * U + ch * KNN_TC_KU) * KNN_TC_N * 16,
+                     uc * KNN_TC_N * 16u, bar_full(st));
           }
+          loads++;
+        };
+        if (resident) {
+          // every MMA of the last query block has been waited for (its tiles
+          // were scanned), so its image can be replaced
+          mbar_expect_tx(bar_a, parts * (unsigned)U * KNN_TC_M * 16u);
+          for (int p = 0; p < parts; p++)
+            bulk_g2s(sm0 + p * KNN_TC_APART, imgA + ((size_t)qb * 2 + p) * U * KNN_TC_M * 16,
+                     (unsigned)U * KNN_TC_M * 16u, bar_a);
+          ok = mbar_wait_or(bar_a, blocks & 1, &gave_up);
         }
-        umma_commit(barM[s]);
-        mpend[s] = true;
-        mpar[s] = (unsigned)((it >> 1) & 1);
-      }
-      if (!ok) abort_flag = 1;
-    }
-    if (it >= 1) {  // scan tile it - 1
-      const int pt = it - 1, s = pt & 1;
-      // warp-uniform decisions: tcgen05.ld is executed by whole warps
-      bool go = __all_sync(0xffffffffu, ok && !abort_flag);
-      if (go) {
-        go = __all_sync(0xffffffffu, mbar_wait(barM[s], (unsigned)((pt >> 1) & 1)));
-        if (!go) {
-          ok = false;
-          abort_flag = 1;
+        for (unsigned g = 0; g < (unsigned)(nst - 1) && g < total && ok; g++) load(g);
+        for (unsigned g = 0; g < total && ok; g++, steps++) {
+          const int st = (int)(steps % (unsigned)nst), ch = (int)(g % (unsigned)nch);
+          const int ab = (int)(tiles & 1u);
+          if (ch == 0 && tiles >= 2)  // the accumulator has been scanned
+            ok = ok && mbar_wait_or(bar_scan(ab), ((tiles >> 1) - 1) & 1, &gave_up);
+          ok = ok && mbar_wait_or(bar_full(st), (steps / (unsigned)nst) & 1, &gave_up);
+          if (!ok) break;
+          tc_fence_after();
+          const unsigned sb = st0 + st * st_bytes;
+          const unsigned aa = resident ? sm0 : sb, bb = sb + a_bytes;
+          const int ks = min(KNN_TC_KU, U - ch * KNN_TC_KU) / 2;
+          const unsigned dt = tmem + (unsigned)ab * KNN_TC_N;
+          for (int term = 0; term < (three ? 3 : 1); term++) {
+            // hi.hi, hi.lo, lo.hi; a K step of 16 dimensions is two units
+            unsigned long long da = umma_desc(aa + (term == 2 ? KNN_TC_APART : 0u), KNN_TC_M * 16, 128);
+            unsigned long long db = umma_desc(bb + (term == 1 ? KNN_TC_BPART : 0u), KNN_TC_N * 16, 128);
+            for (int s = 0; s < ks; s++) {
+              umma_bf16(dt, da, db, idesc, ch > 0 || term > 0 || s > 0 ? 1u : 0u);
+              da += 2 * KNN_TC_M;
+              db += 2 * KNN_TC_N;
+            }
+          }
+          umma_commit(bar_free(st));
+          if (ch == nch - 1) {
+            umma_commit(bar_acc(ab));
+            tiles++;
+          }
+          // its stage is free once the MMAs of step g - 1 are done; those of
+          // step g keep the tensor cores busy meanwhile
+          if (g + nst - 1 < total) load(g + nst - 1);
         }
+        if (!ok) gave_up = 1;
       }
-      __syncwarp();
-      if (go) {
+    } else {
+      const int row = (warp & 3) * 32 + lane, half = warp >> 2;
+      const int q = qb * KNN_TC_M + row;
+      float2 *buf = bufs + ((size_t)blockIdx.x * KNN_TC_SCAN + t) * CAP;
+      float2 *wbuf = bufs + ((size_t)blockIdx.x * KNN_TC_SCAN + warp * 32) * CAP;
+      float thr = q < n ? -INFINITY : INFINITY;
+      int cnt = 0;
+      bool ok = true;
+      for (int tile = 0; tile < ntile; tile++, tiles++) {
+        const int ab = (int)(tiles & 1u);
+        ok = __all_sync(0xffffffffu, mbar_wait_or(bar_acc(ab), (tiles >> 1) & 1, &gave_up));
+        if (!ok) break;
         tc_fence_after();
-        if (t == 0) {
-          mpend[s] = false;
-          // the MMAs of tile pt are done with their stage: refill it
-          if (pt + nstage < nt) load_tile(pt + nstage);
-        }
-      }
-      if (go && qa < na) {
 #pragma unroll 1
         for (int c0 = 0; c0 < 128; c0 += 32) {
           float v[32];
-          __syncwarp();  // converged for the warp-wide tcgen05.ld
-          tmem_ld32(tmem + ((unsigned)((warp & 3) * 32) << 16) + 256u * (unsigned)qa +
-                        (unsigned)s * 128u + (unsigned)c0,
-                    v);
-          const int j0 = pt * KNN_TC_M + c0;
-          // admission: -2 v < thr, i.e. v > -thr/2 (exact in FP32); the
-          // query itself is admitted too and dropped at the re-rank
-          const float m = L.mthr;
+          __syncwarp();
+          tmem_ld32(tmem + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)ab * KNN_TC_N +
+                        (unsigned)(half * 128 + c0), v);
+          const int j0 = tile * KNN_TC_N + half * 128 + c0;
+          const float4 *o4 = reinterpret_cast<const float4 *>(off + j0);
           bool any = false;
 #pragma unroll
-          for (int h = 0; h < 32; h++) any |= v[h] > m;
+          for (int h = 0; h < 8; h++) {
+            const float4 o = __ldg(&o4[h]);
+            v[4 * h] += o.x;
+            v[4 * h + 1] += o.y;
+            v[4 * h + 2] += o.z;
+            v[4 * h + 3] += o.w;
+            any |= v[4 * h] > thr || v[4 * h + 1] > thr || v[4 * h + 2] > thr || v[4 * h + 3] > thr;
+          }
           if (any) {
 #pragma unroll
             for (int h = 0; h < 32; h++)
-              if (v[h] > m) {
-                qd[qc] = -2.f * v[h];
-                qi[qc] = j0 + h;
-                qc++;
-              }
+              if (v[h] > thr) buf[cnt++] = make_float2(v[h], __int_as_float(j0 + h));
           }
-          if (__any_sync(0xffffffffu, qc > KNN_TC_QMAX - 32)) {
-#pragma unroll 1
-            for (int e = 0; e < qc; e++) L.offer(qd[e], qi[e]);
-            qc = 0;
-          }
-        }
-      }
-      tc_fence_before();
-      if (__syncthreads_or(!ok || abort_flag)) {  // block-uniform
-        ok = false;
-        break;
-      }
-    }
-  }
-#pragma unroll 1
-  for (int e = 0; e < qc; e++) L.offer(qd[e], qi[e]);
-  if (!ok) {
-    if (t == 0) {
-      atomicExch(err, 1);
-      // let the copies and MMAs in flight finish before the memory is released
-      for (int st = 0; st < 3; st++)
-        if (cpend[st]) mbar_wait(bar_full(st), cpar[st]);
-      for (int s = 0; s < 2; s++)
-        if (mpend[s]) mbar_wait(barM[s], mpar[s]);
-    }
-  } else if (q < n) {
-    // exact re-rank with the arithmetic of k_knn, then a sort by (distance,
-    // index); unused slots keep (inf, INT_MAX) and sort last
-    // a list that never filled holds every candidate
-    const float tail = L.thr;
-    const bool full = L.thr != INFINITY;
-    const float *xq = X + (long)q * dim;
-#pragma unroll
-    for (int e = 0; e < KNN_TC_CAP; e++) {
-      if (L.j[e] >= n || L.j[e] == q) {  // empty slot, padding row or the query itself
-        L.d[e] = INFINITY;
-        L.j[e] = 0x7fffffff;
-        continue;
-      }
-      const float *xc = X + (long)L.j[e] * dim;
-      float a = 0.f;
-      for (int kk = 0; kk < dim; kk++) {
-        const float df = __ldg(&xq[kk]) - __ldg(&xc[kk]);
-        a = fmaf(df, df, a);
-      }
-      L.d[e] = a;
-    }
-#pragma unroll
-    for (int size = 2; size <= KNN_TC_CAP; size <<= 1)
-#pragma unroll
-      for (int stride = size >> 1; stride > 0; stride >>= 1)
-#pragma unroll
-        for (int e = 0; e < KNN_TC_CAP; e++) {
-          const int l = e ^ stride;
-          if (l > e) {
-            const bool up = (e & size) == 0;
-            if (up == knn_less(L.d[l], L.j[l], L.d[e], L.j[e])) {
-              const float td = L.d[e];
-              const int tj = L.j[e];
-              L.d[e] = L.d[l];
-              L.j[e] = L.j[l];
-              L.d[l] = td;
-              L.j[l] = tj;
+          // room for the next 32 columns
+          unsigned full = __ballot_sync(0xffffffffu, cnt > CAP - 32);
+          while (full) {
+            const int s = __ffs(full) - 1;
+            full &= full - 1;
+            const int c = __shfl_sync(0xffffffffu, cnt, s);
+            __syncwarp();
+            const float nt = knn_select<L, CAP>(wbuf + (size_t)s * CAP, c);
+            if (lane == s) {
+              cnt = L;
+              thr = nt;
             }
           }
         }
-    float dk = L.d[0];
-#pragma unroll
-    for (int e = 0; e < KNN_TC_CAP; e++)
-      if (e == k - 1) dk = L.d[e];
-    const float bound = KNN_TC_EPS * (qn + __uint_as_float(*nmax));
-    if (!full || tail - bound > dk) {
-#pragma unroll
-      for (int e = 0; e < KNN_TC_CAP; e++)
-        if (e < k) {
-          idx[(long)q * k + e] = L.j[e];
-          d2[(long)q * k + e] = L.d[e];
-        }
-    } else {
-      redo[atomicAdd(nredo, 1)] = q;
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_scan(ab));
+      }
+      s_cnt[t] = cnt;
+      s_thr[t] = thr;
+      if (!ok) gave_up = 1;
     }
+    __syncthreads();
+    if (gave_up) break;  // block-uniform: written before the barrier
+    if (warp < 8) {
+      // re-rank: a warp per query
+      for (int r = warp; r < KNN_TC_M; r += 8) {
+        const int q = qb * KNN_TC_M + r;
+        if (q >= n) break;
+        constexpr int E = CAP / 32;
+        const float2 *b0 = bufs + ((size_t)blockIdx.x * KNN_TC_SCAN + r) * CAP;
+        const float2 *b1 = b0 + (size_t)128 * CAP;
+        const int c0 = s_cnt[r], c1 = s_cnt[128 + r];
+        float tail = fmaxf(s_thr[r], s_thr[128 + r]);  // no dropped key is above it
+        unsigned u[2 * E];
+        int j[2 * E];
+#pragma unroll
+        for (int i = 0; i < 2 * E; i++) {
+          const int e = lane + 32 * (i % E);
+          const bool in = e < (i < E ? c0 : c1);
+          const float2 v = in ? (i < E ? b0 : b1)[e] : make_float2(0.f, 0.f);
+          j[i] = __float_as_int(v.y);
+          u[i] = in && j[i] != q ? knn_ordered(v.x) : 0u;  // without the query itself
+        }
+        unsigned T = 1;  // everything
+        const int have = c0 + c1;
+        if (have > L) {
+          T = knn_kth<2 * E>(u, L);
+          if (T == 0) T = 1;  // fewer than L entries besides the query
+          else tail = fmaxf(tail, knn_unordered(T));
+        }
+        int m = 0;
+        __syncwarp();
+#pragma unroll
+        for (int pass = 0; pass < 2; pass++)
+#pragma unroll
+          for (int i = 0; i < 2 * E; i++) {
+            const bool keep = pass == 0 ? u[i] > T : u[i] == T;
+            const unsigned mk = __ballot_sync(0xffffffffu, keep);
+            const int slot = m + __popc(mk & ((1u << lane) - 1u));
+            if (keep && slot < L) s_idx[warp][slot] = j[i];
+            m += __popc(mk);
+          }
+        m = min(m, L);
+        __syncwarp();
+        const float *xq = X + (long)q * dim;
+        for (int e = lane; e < m; e += 32) {
+          const float *xc = X + (long)s_idx[warp][e] * dim;
+          float acc = 0.f;
+          int kk = 0;
+          if ((dim & 3) == 0 && (reinterpret_cast<size_t>(X) & 15) == 0) {
+#pragma unroll 4
+            for (; kk < dim; kk += 4) {
+              const float4 a = __ldg(reinterpret_cast<const float4 *>(xq + kk));
+              const float4 c = __ldg(reinterpret_cast<const float4 *>(xc + kk));
+              float df = a.x - c.x;
+              acc = fmaf(df, df, acc);
+              df = a.y - c.y;
+              acc = fmaf(df, df, acc);
+              df = a.z - c.z;
+              acc = fmaf(df, df, acc);
+              df = a.w - c.w;
+              acc = fmaf(df, df, acc);
+            }
+          } else {
+#pragma unroll 8
+            for (; kk < dim; kk++) {
+              const float df = __ldg(&xq[kk]) - __ldg(&xc[kk]);
+              acc = fmaf(df, df, acc);
+            }
+          }
+          s_d[warp][e] = acc;
+        }
+        __syncwarp();
+        // the k nearest by (distance, index): each entry's rank is the number
+        // of entries before it
+        float dk = INFINITY;
+        for (int e = lane; e < m; e += 32) {
+          const float d = s_d[warp][e];
+          const int ji = s_idx[warp][e];
+          int rank = 0;
+          for (int o = 0; o < m; o++) rank += knn_less(s_d[warp][o], s_idx[warp][o], d, ji);
+          if (rank < k) {
+            idx[(long)q * k + rank] = ji;
+            d2[(long)q * k + rank] = d;
+          }
+          if (rank == k - 1) dk = d;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dk = fminf(dk, __shfl_xor_sync(0xffffffffu, dk, o));
+        // settled: nothing was dropped, or all that was is farther than the
+        // k-th exact distance (false for NaN: such queries are redone too)
+        const float qn = nrm[q];
+        const bool settled =
+            m >= k && (tail == -INFINITY || qn - 2.f * tail - eps * (qn + cmax) > dk);
+        if (!settled && lane == 0) redo[atomicAdd(nredo, 1)] = q;
+        __syncwarp();
+      }
+    }
+    __syncthreads();  // the lists are free for the next query block
+  }
+  if (gave_up && t == KNN_TC_SCAN) {
+    atomicExch(err, 1);
+    // let the copies and MMAs in flight finish before the memory is released:
+    // every load is waited for in order, and a commit covers all MMAs
+    for (unsigned l = steps; l < loads; l++)
+      mbar_wait(bar_full((int)(l % (unsigned)nst)), (l / (unsigned)nst) & 1);
+    if (steps > 0)
+      mbar_wait(bar_free((int)((steps - 1) % (unsigned)nst)), ((steps - 1) / (unsigned)nst) & 1);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tcols));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
 }
 
 }  // namespace
@@ -580,23 +693,35 @@ static sgt_status knn_simt(sgt_ctx *ctx, int n, int dim, const float *X, int k,
   return SGT_OK;
 }
 
+template <int L, int CAP>
+static cudaError_t knn_tc_launch(int nb, cudaStream_t s, const unsigned char *imgA,
+                                 const unsigned char *imgB, const float *nrm, const float *off,
+                                 const unsigned *nmax, const int *inexact, const float *X, int n,
+                                 int dim, int U, int k, float2 *bufs, int *idx, float *d2,
+                                 int *redo, int *cnt) {
+  cudaError_t e = cudaFuncSetAttribute(
+      k_knn_tc<L, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KNN_TC_SMEM);
+  if (e != cudaSuccess) return e;
+  k_knn_tc<L, CAP><<<nb, KNN_TC_THREADS, KNN_TC_SMEM, s>>>(
+      imgA, imgB, nrm, off, nmax, inexact, X, n, dim, U, k, bufs, idx, d2, redo, cnt, cnt + 1);
+  return cudaGetLastError();
+}
+
 static sgt_status knn_tc(sgt_ctx *ctx, int n, int dim, const float *X, int k, int *idx,
                          float *d2, int *n_redo) {
   cudaStream_t s = sgti_stream(ctx);
-  const int U = ((dim + 2 + 7) / 8) * 2;  // the dimensions and two norm columns
-  const int nblk = (n + KNN_TC_M - 1) / KNN_TC_M;
-  const size_t img_bytes = (size_t)nblk * 2 * U * 2048;
-  const size_t pbytes = (size_t)2 * U * 2048;
-  // QB query tiles (two when they fit beside two candidate stages, so each
-  // candidate tile streamed in serves 256 queries) and two or three candidate
-  // stages; at least 120 KB so that one CTA runs per SM (its tensor-memory
-  // columns are then never contended)
-  const size_t smem_max = 227 * 1024 - 1024;
-  const int QB = 4 * pbytes <= smem_max ? 2 : 1;
-  const int nstage = (QB + 3) * pbytes <= smem_max ? 3 : 2;
-  const size_t smem = std::max<size_t>((QB + nstage) * pbytes, 120 * 1024);
+  const int U = ((dim + 15) / 16) * 2;  // units of 8 dimensions, in pairs (one MMA)
+  const int nq = (n + KNN_TC_M - 1) / KNN_TC_M, ntile = (n + KNN_TC_N - 1) / KNN_TC_N;
+  const size_t a_bytes = (size_t)nq * 2 * U * KNN_TC_M * 16;
+  const size_t b_bytes = (size_t)ntile * 2 * U * KNN_TC_N * 16;
+  const int nb = std::min(nq, sgti_sm_count(ctx));
+  // list length (neighbours and a margin) and buffer capacity
+  const int cap = k <= 32 ? 256 : (k <= 96 ? 384 : 448);
   char *buf = nullptr;
-  const size_t o_nrm = 2 * img_bytes, o_max = o_nrm + sizeof(float) * (size_t)nblk * KNN_TC_M;
+  const int npad = ntile * KNN_TC_N;
+  const size_t o_nrm = a_bytes + b_bytes, o_off = o_nrm + sizeof(float) * (size_t)npad;
+  const size_t o_buf = o_off + sizeof(float) * (size_t)npad;
+  const size_t o_max = o_buf + sizeof(float2) * (size_t)nb * KNN_TC_SCAN * cap;
   const size_t o_cnt = o_max + 16, o_redo = o_cnt + 16;
   const size_t total = o_redo + sizeof(int) * (size_t)n;
   cudaError_t e = sgti_alloc(ctx, (void **)&buf, total, s);
@@ -604,25 +729,33 @@ static sgt_status knn_tc(sgt_ctx *ctx, int n, int dim, const float *X, int k, in
     (void)cudaGetLastError();  // not sticky: clear it for the caller's next check
     return sgti_fail(ctx, SGT_ERR_NO_MEMORY, "sgt_knn: tensor-core operand images");
   }
-  float4 *imgA = reinterpret_cast<float4 *>(buf);
-  float4 *imgB = reinterpret_cast<float4 *>(buf + img_bytes);
-  float *nrm = reinterpret_cast<float *>(buf + o_nrm);
+  unsigned char *imgA = reinterpret_cast<unsigned char *>(buf);
+  unsigned char *imgB = imgA + a_bytes;
+  float *nrm = reinterpret_cast<float *>(buf + o_nrm), *off = reinterpret_cast<float *>(buf + o_off);
+  float2 *bufs = reinterpret_cast<float2 *>(buf + o_buf);
   unsigned *nmax = reinterpret_cast<unsigned *>(buf + o_max);
+  int *inexact = reinterpret_cast<int *>(buf + o_max + 4);
   int *cnt = reinterpret_cast<int *>(buf + o_cnt);  // [0] queries to redo, [1] error
   int *redo = reinterpret_cast<int *>(buf + o_redo);
   int hc[2] = {0, 0};
   e = cudaMemsetAsync(buf + o_max, 0, 32, s);
   if (e == cudaSuccess) {
-    const long items = (long)nblk * U * KNN_TC_M;
-    const int nb = (int)std::min<long>((items + 255) / 256, 148L * 16);
-    k_knn_norms<<<(n + 255) / 256, 256, 0, s>>>(X, n, dim, nrm, nmax);
-    k_knn_split<<<nb, 256, 0, s>>>(X, nrm, n, dim, U, nblk, imgA, imgB);
-    e = cudaFuncSetAttribute(k_knn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_knn_norms<<<std::min((npad + 255) / 256, 148 * 4), 256, 0, s>>>(X, n, npad, dim, nrm, off,
+                                                                      nmax, inexact);
+    k_knn_split<<<148 * 8, 256, 0, s>>>(X, n, dim, U, KNN_TC_M, nq, (uint4 *)imgA);
+    k_knn_split<<<148 * 8, 256, 0, s>>>(X, n, dim, U, KNN_TC_N, ntile, (uint4 *)imgB);
+    e = cudaGetLastError();
   }
   if (e == cudaSuccess) {
-    k_knn_tc<<<(nblk + QB - 1) / QB, KNN_TC_M * QB, smem, s>>>(
-        imgA, imgB, nrm, nmax, X, n, dim, U, QB, nstage, k, idx, d2, redo, cnt, cnt + 1);
-    e = cudaGetLastError();
+    if (k <= 32)
+      e = knn_tc_launch<64, 256>(nb, s, imgA, imgB, nrm, off, nmax, inexact, X, n, dim, U, k, bufs,
+                                 idx, d2, redo, cnt);
+    else if (k <= 96)
+      e = knn_tc_launch<128, 384>(nb, s, imgA, imgB, nrm, off, nmax, inexact, X, n, dim, U, k,
+                                  bufs, idx, d2, redo, cnt);
+    else
+      e = knn_tc_launch<192, 448>(nb, s, imgA, imgB, nrm, off, nmax, inexact, X, n, dim, U, k,
+                                  bufs, idx, d2, redo, cnt);
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -647,7 +780,7 @@ extern "C" sgt_status sgt_knn_ex(sgt_ctx *ctx, int n, int dim, const float *X, i
   if (k > KNN_MAXK || k >= n)
     return sgti_fail(ctx, SGT_ERR_UNSUPPORTED,
                      "sgt_knn: k must be below n and at most " + std::to_string(KNN_MAXK));
-  const bool tc_ok = dim <= 64 && k <= KNN_TC_MAXK && n <= (1 << 28);
+  const bool tc_ok = dim <= KNN_TC_MAXDIM && k <= KNN_TC_MAXK && n <= (1 << 28);
   if (method == SGT_KNN_TENSOR && !tc_ok)
     return sgti_fail(ctx, SGT_ERR_UNSUPPORTED,
                      "sgt_knn: the tensor-core filter takes dim <= 64 and k <= 32");
@@ -655,9 +788,11 @@ extern "C" sgt_status sgt_knn_ex(sgt_ctx *ctx, int n, int dim, const float *X, i
     return sgti_fail(ctx, SGT_ERR_CUDA, "sgt_knn: set device");
   if (n_redo) *n_redo = 0;
   sgt_status st;
-  if (method == SGT_KNN_TENSOR || (method == SGT_KNN_AUTO && tc_ok && n >= 4096)) {
+  // the automatic choice takes the filter for any width and k; below 4096
+  // points the SIMT search has no images to make
+  if (method == SGT_KNN_TENSOR || (method == SGT_KNN_AUTO && n >= 4096 && n <= (1 << 28))) {
     st = knn_tc(ctx, n, dim, X, k, idx, d2, n_redo);
-    // the filter's operand images (about 16 bytes per point and dimension)
+    // the filter's operand images (about 8 bytes per point and dimension)
     // did not fit: the automatic choice falls back to the SIMT search
     if (st == SGT_ERR_NO_MEMORY && method == SGT_KNN_AUTO)
       st = knn_simt(ctx, n, dim, X, k, nullptr, n, idx, d2);

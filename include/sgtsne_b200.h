@@ -455,14 +455,14 @@ sgt_status sgt_knn(sgt_ctx *ctx, int n, int dim, const float *X, int k, int *idx
 
 /* Search methods of sgt_knn_ex; all return the same bits.
    SGT_KNN_SIMT: sums of squared differences, one query per thread.
-   SGT_KNN_TENSOR: dim <= 64 and k <= 32 only.  Distances
-     |q|^2 + |c|^2 - 2 q.c of all pairs on the tensor cores (TF32 in three
-     terms, FP32 accumulation) keep a list of 64 candidates per query,
-     re-ranked with the SIMT arithmetic; queries whose list could miss a
-     neighbour under the filter's error bound are redone by the SIMT search.
-   SGT_KNN_AUTO: the tensor-core filter where it applies and n >= 4096,
-     the SIMT search otherwise or when the filter's operand images (about
-     16 bytes per point and dimension) do not fit in device memory. */
+   SGT_KNN_TENSOR: dim <= 64 and k <= 32 only.  Keys q.c - |c|^2/2 of all
+     pairs on the tensor cores (BF16 in three terms, or one for points that
+     are BF16 numbers, FP32 accumulation) keep a list of candidates per
+     query, re-ranked with the SIMT arithmetic; queries whose list could miss
+     a neighbour under the filter's error bound are redone by the SIMT search.
+   SGT_KNN_AUTO: the tensor-core filter, for any dim and k, from n = 4096;
+     the SIMT search below, or when the filter's operand images (about
+     8 bytes per point and dimension) do not fit in device memory. */
 enum { SGT_KNN_AUTO = 0, SGT_KNN_SIMT = 1, SGT_KNN_TENSOR = 2 };
 
 /* sgt_knn with a method; *n_redo (may be NULL) receives the number of
