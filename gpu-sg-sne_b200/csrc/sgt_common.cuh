@@ -202,9 +202,13 @@ __device__ __constant__ int c_grid_sizes[137] = {
     504, 512};
 
 __device__ __forceinline__ int sgt_best_grid_size_dev(int ng) {
-  for (int i = 0; i < 137; i++)
-    if (ng + 2 <= c_grid_sizes[i]) return c_grid_sizes[i] - 2;
-  return c_grid_sizes[136] - 2;
+  int lo = 0, hi = 136;  // the first entry >= ng + 2, or the last
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (ng + 2 <= c_grid_sizes[mid]) hi = mid;
+    else lo = mid + 1;
+  }
+  return c_grid_sizes[lo] - 2;
 }
 
 // Error bits in SgtState::error

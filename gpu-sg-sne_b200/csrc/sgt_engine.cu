@@ -451,8 +451,9 @@ static sgt_status job_shapes(sgt_job *J) {
   }
   // scatter mode: a group of SGT_LPP lanes per point, up to 2048 threads an SM
   const long groups = ((long)J->n * SGT_LPP(D) + SGT_THREADS - 1) / SGT_THREADS;
+  const long ggroups = ((long)J->n * SGT_GLPP + SGT_THREADS - 1) / SGT_THREADS;
   J->nb_scat = (int)std::min(groups, 8L * nsm);
-  J->nb_gath = (int)std::min(groups, 6L * nsm);
+  J->nb_gath = (int)std::min(ggroups, (D == 3 ? 3L : 6L) * nsm);
   // small embeddings launch no more blocks than there is work for: idle
   // blocks only take scheduling slots from the jobs that share the GPU
   const int cap = (int)std::max(1L, ((long)J->n + 255) / 256);

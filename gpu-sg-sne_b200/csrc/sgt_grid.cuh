@@ -28,6 +28,9 @@
 // request; 3-D spreads its 16 rows over 16 lanes.  100k points on 64^2 nodes:
 // 22.8 us with 4 lanes per point, 37.1 us with one.
 #define SGT_LPP(D) ((D) == 3 ? 16 : 4)
+// Lanes per point of the gather: 4 in 3-D too.  Loads of 16 rows fly in one
+// lane as well as in 16, and the stencil is worked out 4 times instead of 16.
+#define SGT_GLPP 4
 // Scatter mode: most copies of the grid.  L2 serialises the reductions that
 // meet on one node; with 32 copies 60k points on 16^2 nodes take 10.5 us
 // instead of 76, 100k on 117^2 10.3 instead of 20.7.  k_spec_rows reads the copies
@@ -179,6 +182,82 @@ __device__ __forceinline__ int sgt_cell_of(const int *f, int td) {
   return t;
 }
 
+// Per-block min/max/sum of the coordinates -> partials; the last block to
+// finish reduces all partials and turns them into the grid decision.  Returns
+// true in thread 0 of that block.  Both reductions are trees of shuffles, in
+// a fixed order: walked by one thread, 592 partials took 80 of the 84 us that
+// the statistics of 100,000 points cost.
+template <int D>
+__device__ __forceinline__ bool block_finish_stats(int vb_, int vg_, SgtState *st,
+                                                   const SgtJobParams &jp, unsigned *done,
+                                                   bool centre, float *mn, float *mx, double *sm,
+                                                   float4 *part_min, float4 *part_max,
+                                                   double *part_sum) {
+  constexpr int W = SGT_THREADS / 32;
+  __shared__ float smin[W][4], smax[W][4];
+  __shared__ double ssum[W][4];
+  __shared__ bool last;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  // the block's values in warp 0's lanes, lane l holding warp l's
+  auto reduce = [&](float *lo, float *hi, double *s) {
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+      lo[k] = warp_min_f(lo[k]);
+      hi[k] = warp_max_f(hi[k]);
+      s[k] = warp_sum_d(s[k]);
+      if (l == 0) { smin[w][k] = lo[k]; smax[w][k] = hi[k]; ssum[w][k] = s[k]; }
+    }
+    __syncthreads();
+    if (w == 0) {
+#pragma unroll
+      for (int k = 0; k < D; k++) {
+        lo[k] = l < W ? smin[l][k] : INFINITY;
+        hi[k] = l < W ? smax[l][k] : -INFINITY;
+        s[k] = l < W ? ssum[l][k] : 0.0;
+#pragma unroll
+        for (int o = W / 2; o > 0; o >>= 1) {
+          lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
+          hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
+          s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+        }
+      }
+    }
+  };
+  reduce(mn, mx, sm);
+  if (threadIdx.x == 0) {
+    part_min[vb_] = make_float4(mn[0], D > 1 ? mn[1] : 0.f, D > 2 ? mn[2] : 0.f, 0.f);
+    part_max[vb_] = make_float4(mx[0], D > 1 ? mx[1] : 0.f, D > 2 ? mx[2] : 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < D; k++) part_sum[vb_ * 4 + k] = sm[k];
+    __threadfence();
+    last = (atomicAdd(done, 1u) == (unsigned)vg_ - 1u);
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+  double s[3] = {0, 0, 0};
+  for (int b = threadIdx.x; b < vg_; b += blockDim.x) {
+    const float4 a = __ldcg(&part_min[b]), c = __ldcg(&part_max[b]);
+    lo[0] = fminf(lo[0], a.x); hi[0] = fmaxf(hi[0], c.x);
+    if (D > 1) { lo[1] = fminf(lo[1], a.y); hi[1] = fmaxf(hi[1], c.y); }
+    if (D > 2) { lo[2] = fminf(lo[2], a.z); hi[2] = fmaxf(hi[2], c.z); }
+#pragma unroll
+    for (int k = 0; k < D; k++) s[k] += __ldcg(&part_sum[b * 4 + k]);
+  }
+  reduce(lo, hi, s);
+  if (threadIdx.x != 0) return false;
+#pragma unroll
+  for (int k = 0; k < D; k++) {
+    st->minv[k] = lo[k];
+    st->maxv[k] = hi[k];
+    st->sum[k] = s[k];
+  }
+  sgt_finalize_grid<D>(st, jp, lo, hi, s, centre);
+  *done = 0;
+  return true;
+}
+
 // ---------------------------------------------------------------------------
 // init: stats of a given coordinate array (first iteration / operator mode)
 // ---------------------------------------------------------------------------
@@ -187,12 +266,9 @@ __global__ void __launch_bounds__(SGT_THREADS)
 k_init_stats(const typename Vec<D>::T *__restrict__ Y, int n, SgtState *st,
              SgtJobParams jp, float4 *part_min, float4 *part_max,
              double *part_sum, int centre) {
-  __shared__ float smin[SGT_THREADS / 32][4], smax[SGT_THREADS / 32][4];
-  __shared__ double ssum[SGT_THREADS / 32][4];
-  __shared__ bool last;
-  float mn[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
-  float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-  double sm[4] = {0, 0, 0, 0};
+  float mn[3] = {INFINITY, INFINITY, INFINITY};
+  float mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+  double sm[3] = {0, 0, 0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += gridDim.x * blockDim.x) {
     const typename Vec<D>::T y = Y[i];
@@ -204,50 +280,9 @@ k_init_stats(const typename Vec<D>::T *__restrict__ Y, int n, SgtState *st,
       sm[k] += (double)v;
     }
   }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-#pragma unroll
-  for (int k = 0; k < D; k++) {
-    mn[k] = warp_min_f(mn[k]);
-    mx[k] = warp_max_f(mx[k]);
-    sm[k] = warp_sum_d(sm[k]);
-    if (l == 0) { smin[w][k] = mn[k]; smax[w][k] = mx[k]; ssum[w][k] = sm[k]; }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float4 a = make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
-    float4 b = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
-    double s[4] = {0, 0, 0, 0};
-    for (int j = 0; j < SGT_THREADS / 32; j++) {
-      a.x = fminf(a.x, smin[j][0]); b.x = fmaxf(b.x, smax[j][0]); s[0] += ssum[j][0];
-      if (D > 1) { a.y = fminf(a.y, smin[j][1]); b.y = fmaxf(b.y, smax[j][1]); s[1] += ssum[j][1]; }
-      if (D > 2) { a.z = fminf(a.z, smin[j][2]); b.z = fmaxf(b.z, smax[j][2]); s[2] += ssum[j][2]; }
-    }
-    part_min[blockIdx.x] = a;
-    part_max[blockIdx.x] = b;
-    for (int k = 0; k < 4; k++) part_sum[blockIdx.x * 4 + k] = s[k];
-    __threadfence();
-    const unsigned prev = atomicAdd(&st->done_init, 1u);
-    last = (prev == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (last && threadIdx.x == 0) {
-    __threadfence();
-    float lo[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
-    float hi[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    double s[4] = {0, 0, 0, 0};
-    for (int b = 0; b < (int)gridDim.x; b++) {
-      lo[0] = fminf(lo[0], __ldcg(&part_min[b].x));
-      hi[0] = fmaxf(hi[0], __ldcg(&part_max[b].x));
-      if (D > 1) { lo[1] = fminf(lo[1], __ldcg(&part_min[b].y)); hi[1] = fmaxf(hi[1], __ldcg(&part_max[b].y)); }
-      if (D > 2) { lo[2] = fminf(lo[2], __ldcg(&part_min[b].z)); hi[2] = fmaxf(hi[2], __ldcg(&part_max[b].z)); }
-      for (int k = 0; k < D; k++) s[k] += __ldcg(&part_sum[b * 4 + k]);
-    }
-    for (int k = 0; k < D; k++) { st->minv[k] = lo[k]; st->maxv[k] = hi[k]; st->sum[k] = s[k]; }
-    sgt_finalize_grid<D>(st, jp, lo, hi, s, centre != 0);
-    st->done_init = 0;
-  }
+  block_finish_stats<D>(blockIdx.x, gridDim.x, st, jp, &st->done_init, centre != 0, mn, mx, sm,
+                        part_min, part_max, part_sum);
 }
-
 
 // ---------------------------------------------------------------------------
 // bin scan (run by the last block of bin_count): tile offsets and the chunk
@@ -677,18 +712,24 @@ __device__ __forceinline__ void k_s2g_cell_body(int vb_, int vg_, const float4 *
             atomicOr(&st->error, SGT_EFLAG_CHUNK_OVERFLOW);
             continue;
           }
+          // weights times distances, per axis: every sum below is one
+          // multiply-add of two of them
+          float wu[4];
+#pragma unroll
+          for (int a0 = 0; a0 < 4; a0++) wu[a0] = w[0][a0] * (du[0] - (float)a0);
           const float wz = D == 3 ? w[2][pass] : 1.f;
 #pragma unroll
           for (int a1 = 0; a1 < (D >= 2 ? 4 : 1); a1++) {
             const float wy = (D >= 2 ? w[1][a1] : 1.f) * wz;
+            const float wv = D >= 2 ? wy * (du[1] - (float)a1) : 0.f;
+            const float ww = D >= 3 ? wy * (du[2] - (float)pass) : 0.f;
 #pragma unroll
             for (int a0 = 0; a0 < 4; a0++) {
-              const float wt = wy * w[0][a0];
               const int nd = a1 * 4 + a0;
-              acc[nd * C] += wt;
-              acc[nd * C + 1] += wt * (du[0] - (float)a0);
-              if constexpr (D >= 2) acc[nd * C + 2] += wt * (du[1] - (float)a1);
-              if constexpr (D >= 3) acc[nd * C + 3] += wt * (du[2] - (float)pass);
+              acc[nd * C] += wy * w[0][a0];
+              acc[nd * C + 1] += wy * wu[a0];
+              if constexpr (D >= 2) acc[nd * C + 2] += wv * w[0][a0];
+              if constexpr (D >= 3) acc[nd * C + 3] += ww * w[0][a0];
             }
           }
         }
@@ -726,11 +767,11 @@ k_s2g_cell(const float4 *__restrict__ sorted, SgtState *st,
 
 // Interpolated p[0] = Phi0 and p[1 + k] = y_k Phi0 - Phi_k (the repulsive
 // force numerator in cells) at a point with stencil weights w and base cell
-// f: from the grid Phi, or (SM) from the block's copy cn of the 4^d nodes of
-// the point's cell, node a0 + 4 a1 + 16 a2.  o: the point's distance from the
-// origin that Phi_k is taken about, per axis, less `loc` per node: the node
-// itself after the direct convolution (o = distance from stencil node 0,
-// loc = 1), the grid's middle after the FFT (loc = 0).
+// f.  o: the point's distance per axis from the origin that Phi_k is taken
+// about.  SM: the nodes come from the block's copy cn of the 4^d nodes of the
+// point's cell, node a0 + 4 a1 + 16 a2, already about one origin.  Otherwise
+// from the grid Phi, whose origin moves by loc per node (1: the node itself
+// after k_spec_cols, o counts from stencil node 0; 0: the grid's middle).
 template <int D, bool SM>
 __device__ __forceinline__ void g2s_potentials(const float (*w)[4], const float *o, float loc,
                                                const int *f, int N, const typename Node<D>::T *Phi,
@@ -749,16 +790,22 @@ __device__ __forceinline__ void g2s_potentials(const float (*w)[4], const float 
       for (int a0 = 0; a0 < 4; a0++) {
         const float wt = wy * w[0][a0];
         typename Node<D>::T v;
-        if constexpr (SM) v = cn[a0 + 4 * (a1 + 4 * a2)];
-        else v = Phi[base + a0];
-        p[0] += wt * v.x;
-        p[1] += wt * ((o[0] - loc * (float)a0) * v.x - v.y);
-        if constexpr (D >= 2) {
-          p[2] += wt * ((o[1] - loc * (float)a1) * v.x - v.z);
-          if constexpr (D >= 3) p[3] += wt * ((o[2] - loc * (float)a2) * v.x - v.w);
+        if constexpr (SM) {
+          v = cn[a0 + 4 * (a1 + 4 * a2)];
+        } else {
+          v = Phi[base + a0];
+          v.y += loc * (float)a0 * v.x;
+          if constexpr (D >= 2) v.z += loc * (float)a1 * v.x;
+          if constexpr (D >= 3) v.w += loc * (float)a2 * v.x;
         }
+        p[0] += wt * v.x;
+        p[1] += wt * v.y;
+        if constexpr (D >= 2) p[2] += wt * v.z;
+        if constexpr (D >= 3) p[3] += wt * v.w;
       }
     }
+#pragma unroll
+  for (int k = 0; k < D; k++) p[k + 1] = o[k] * p[0] - p[k + 1];
 }
 
 // Force numerator and z of a point from its p (g2s_potentials) and its
@@ -812,8 +859,8 @@ __device__ __forceinline__ void g2s_finish(int vb_, int vg_, SgtState *st, doubl
 // ---------------------------------------------------------------------------
 // G2S + repulsive force numerator + Z (FP64, fixed-order finish).
 // Frep_un[i] = y_i*Phi0 - Phi_{1..d}; Z = sum_i z_i - n.
-// Scatter mode: the points in their own order, SGT_LPP(D) lanes per point.
-// Lane q reads the nodes it would scatter to (a stencil row is one 64-byte
+// Scatter mode: the points in their own order, SGT_GLPP lanes per point.
+// Lane q reads the nodes with x offset q (a stencil row is one 64-byte
 // request) and the group sums the potentials by shuffles; its first lane
 // forms F and the point's Z.
 // ---------------------------------------------------------------------------
@@ -827,13 +874,14 @@ __device__ __forceinline__ void k_gather_body(int vb_, int vg_, SgtState *st,
   if (st->T != 0) return;  // cell mode: k_g2s
   __shared__ double wz[SGT_THREADS / 32];
   __shared__ bool last;
-  constexpr int L = SGT_LPP(D);
+  constexpr int L = SGT_GLPP, R = D == 1 ? 1 : (D == 2 ? 4 : 16);  // stencil rows
   const GridGeom<D> g(st);
   const int N = g.N;
   const float h = st->h_eff, half = 0.5f * g.scale;
   const bool direct = st->direct != 0;
+  const float loc = direct ? 1.0f : 0.0f;
   double zacc = 0.0;
-  const int q = threadIdx.x % L, qx = q & 3;
+  const int qx = threadIdx.x % L;
   const int step = vg_ * (SGT_THREADS / L);
   const int rounds = (n + step - 1) / step;  // uniform, so that the shuffles converge
   int i = vb_ * (SGT_THREADS / L) + threadIdx.x / L;
@@ -841,7 +889,7 @@ __device__ __forceinline__ void k_gather_body(int vb_, int vg_, SgtState *st,
     float p[4] = {0.f, 0.f, 0.f, 0.f}, m[3] = {0.f, 0.f, 0.f};
     if (i < n) {
       const typename Vec<D>::T y = Y[i];
-      int f[3];
+      int f[3] = {0, 0, 0};
       float w[3][4], o[3];
       bool ok = true;
 #pragma unroll
@@ -853,40 +901,24 @@ __device__ __forceinline__ void k_gather_body(int vb_, int vg_, SgtState *st,
         ok = ok && (unsigned)f[k] < (unsigned)g.cells;
       }
       if (!ok) {  // outside the grid (S2G skipped it too): no force, no Z
-        if (q == 0) atomicOr(&st->error, SGT_EFLAG_CHUNK_OVERFLOW);
+        if (qx == 0) atomicOr(&st->error, SGT_EFLAG_CHUNK_OVERFLOW);
       } else {
-        const float loc = direct ? 1.0f : 0.0f;
+        typename Node<D>::T v[R];
+        const typename Node<D>::T *ph = Phi + f[0] + qx + (D >= 2 ? N * f[1] : 0) +
+                                        (D >= 3 ? (long)N * N * f[2] : 0);
+#pragma unroll
+        for (int b = 0; b < R; b++)
+          v[b] = ph[(D >= 2 ? N * (b & 3) : 0) + (D >= 3 ? N * N * (b >> 2) : 0)];
         const float wx = pick4(w[0], qx), ox = o[0] - loc * (float)qx;
-        if constexpr (D == 1) {
-          const float2 v = Phi[f[0] + qx];
-          p[0] = wx * v.x;
-          p[1] = wx * (ox * v.x - v.y);
-        } else if constexpr (D == 2) {
-          float4 v[4];
 #pragma unroll
-          for (int b = 0; b < 4; b++) v[b] = Phi[f[0] + qx + N * (f[1] + b)];
-#pragma unroll
-          for (int b = 0; b < 4; b++) {
-            const float wt = w[1][b] * wx;
-            p[0] += wt * v[b].x;
-            p[1] += wt * (ox * v[b].x - v[b].y);
-            p[2] += wt * ((o[1] - loc * (float)b) * v[b].x - v[b].z);
-          }
-        } else {
-          const int qy = q >> 2;
-          const float wy = pick4(w[1], qy) * wx, oy = o[1] - loc * (float)qy;
-          float4 v[4];
-#pragma unroll
-          for (int c = 0; c < 4; c++)
-            v[c] = Phi[f[0] + qx + (long)N * (f[1] + qy + (long)N * (f[2] + c))];
-#pragma unroll
-          for (int c = 0; c < 4; c++) {
-            const float wt = wy * w[2][c];
-            p[0] += wt * v[c].x;
-            p[1] += wt * (ox * v[c].x - v[c].y);
-            p[2] += wt * (oy * v[c].x - v[c].z);
-            p[3] += wt * ((o[2] - loc * (float)c) * v[c].x - v[c].w);
-          }
+        for (int b = 0; b < R; b++) {
+          float wt = wx;
+          if (D >= 2) wt *= w[1][b & 3];
+          if (D >= 3) wt *= w[2][b >> 2];
+          p[0] += wt * v[b].x;
+          p[1] += wt * (ox * v[b].x - v[b].y);
+          if constexpr (D >= 2) p[2] += wt * ((o[1] - loc * (float)(b & 3)) * v[b].x - v[b].z);
+          if constexpr (D >= 3) p[3] += wt * ((o[2] - loc * (float)(b >> 2)) * v[b].x - v[b].w);
         }
       }
     }
@@ -894,7 +926,7 @@ __device__ __forceinline__ void k_gather_body(int vb_, int vg_, SgtState *st,
     for (int e = 1; e < L; e *= 2)
 #pragma unroll
       for (int k = 0; k <= D; k++) p[k] += __shfl_xor_sync(0xffffffffu, p[k], e);
-    if (i < n && q == 0) {
+    if (i < n && qx == 0) {
       typename Vec<D>::T fr;
       zacc += point_force<D>(p, m, h, fr);
       Frep_un[i] = fr;
@@ -903,7 +935,7 @@ __device__ __forceinline__ void k_gather_body(int vb_, int vg_, SgtState *st,
   g2s_finish(vb_, vg_, st, part_z, n, zacc, wz, last);
 }
 template <int D>
-__global__ void __launch_bounds__(SGT_THREADS, 6)
+__global__ void __launch_bounds__(SGT_THREADS, D == 3 ? 3 : 6)
 k_gather(SgtState *st, const typename Node<D>::T *__restrict__ Phi,
          typename Vec<D>::T *__restrict__ Frep_un, double *part_z, int n,
          const typename Vec<D>::T *__restrict__ Y) {
@@ -942,7 +974,13 @@ __device__ __forceinline__ void k_g2s_body(int vb_, int vg_, const float4 *__res
       long g = cf[0] + (e & 3);
       if (D >= 2) g += (long)N * (cf[1] + ((e >> 2) & 3));
       if (D >= 3) g += (long)N * N * (cf[2] + (e >> 4));
-      cn[e] = Phi[g];
+      // the potentials about the cell's stencil node 0 (k_spec_cols leaves
+      // them about each node)
+      typename Node<D>::T v = Phi[g];
+      v.y += loc * (float)(e & 3) * v.x;
+      if constexpr (D >= 2) v.z += loc * (float)((e >> 2) & 3) * v.x;
+      if constexpr (D >= 3) v.w += loc * (float)(e >> 4) * v.x;
+      cn[e] = v;
     }
     __syncthreads();
     constexpr int U = SGT_PTS_U;

@@ -130,7 +130,7 @@ km_g2s(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int
 }
 
 template <int D>
-__global__ void __launch_bounds__(SGT_THREADS, 6)
+__global__ void __launch_bounds__(SGT_THREADS, D == 3 ? 3 : 6)
 km_gather(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
   SGT_MULTI_JOB
   typedef typename Vec<D>::T VT;

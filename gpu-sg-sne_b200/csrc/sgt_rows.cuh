@@ -80,85 +80,6 @@ __device__ __forceinline__ float sgn_f(float x) {
   return x == 0.f ? 0.f : (x < 0.f ? -1.f : 1.f);
 }
 
-// Per-block min/max/sum of Ynext -> partials; the last block reduces all
-// partials with every thread and turns them into the next grid decision.
-template <int D>
-__device__ __forceinline__ void block_finish_stats(int vb_, int vg_, SgtState *st, const SgtJobParams &jp,
-                                                   float *mn, float *mx, double *sm,
-                                                   float4 *part_min, float4 *part_max,
-                                                   double *part_sum, int iter, float alpha,
-                                                   float mom) {
-  __shared__ float smin[SGT_THREADS / 32][3], smax[SGT_THREADS / 32][3];
-  __shared__ double ssum[SGT_THREADS / 32][3];
-  __shared__ bool last;
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-#pragma unroll
-  for (int k = 0; k < D; k++) {
-    const float a = warp_min_f(mn[k]), b = warp_max_f(mx[k]);
-    const double s = warp_sum_d(sm[k]);
-    if (l == 0) { smin[w][k] = a; smax[w][k] = b; ssum[w][k] = s; }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float4 a = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
-    float4 b = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
-    double s[3] = {0, 0, 0};
-    for (int j = 0; j < SGT_THREADS / 32; j++) {
-      a.x = fminf(a.x, smin[j][0]); b.x = fmaxf(b.x, smax[j][0]); s[0] += ssum[j][0];
-      if (D > 1) { a.y = fminf(a.y, smin[j][1]); b.y = fmaxf(b.y, smax[j][1]); s[1] += ssum[j][1]; }
-      if (D > 2) { a.z = fminf(a.z, smin[j][2]); b.z = fmaxf(b.z, smax[j][2]); s[2] += ssum[j][2]; }
-    }
-    part_min[vb_] = a;
-    part_max[vb_] = b;
-    for (int k = 0; k < 3; k++) part_sum[vb_ * 4 + k] = s[k];
-    __threadfence();
-    last = (atomicAdd(&st->done_row, 1u) == vg_ - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  double s[3] = {0, 0, 0};
-  for (int b = threadIdx.x; b < (int)vg_; b += blockDim.x) {
-    const float4 a = __ldcg(&part_min[b]), c = __ldcg(&part_max[b]);
-    lo[0] = fminf(lo[0], a.x); hi[0] = fmaxf(hi[0], c.x);
-    lo[1] = fminf(lo[1], a.y); hi[1] = fmaxf(hi[1], c.y);
-    lo[2] = fminf(lo[2], a.z); hi[2] = fmaxf(hi[2], c.z);
-    for (int k = 0; k < D; k++) s[k] += __ldcg(&part_sum[b * 4 + k]);
-  }
-  // fixed-order tree: warp shuffles then warp 0 over the warp results
-#pragma unroll
-  for (int k = 0; k < D; k++) {
-    lo[k] = warp_min_f(lo[k]);
-    hi[k] = warp_max_f(hi[k]);
-    s[k] = warp_sum_d(s[k]);
-  }
-  __syncthreads();
-  if (l == 0)
-    for (int k = 0; k < D; k++) { smin[w][k] = lo[k]; smax[w][k] = hi[k]; ssum[w][k] = s[k]; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < D; k++) {
-      lo[k] = INFINITY; hi[k] = -INFINITY; s[k] = 0;
-      for (int j = 0; j < SGT_THREADS / 32; j++) {
-        lo[k] = fminf(lo[k], smin[j][k]);
-        hi[k] = fmaxf(hi[k], smax[j][k]);
-        s[k] += ssum[j][k];
-      }
-      st->minv[k] = lo[k];
-      st->maxv[k] = hi[k];
-      st->sum[k] = s[k];
-      if (!isfinite(lo[k]) || !isfinite(hi[k])) st->error |= SGT_EFLAG_NONFINITE;
-    }
-    sgt_finalize_grid<D>(st, jp, lo, hi, s, true);
-    st->alpha = alpha;
-    st->momentum = mom;
-    st->iter = iter + 1;
-    st->done_row = 0;
-  }
-}
-
-
 // ---------------------------------------------------------------------------
 // Fused iteration row kernel.  FUSED: compute F_attr from CSR; otherwise read
 // it from Fattr (COO / ELL formats).  Writes Ynext, uY, gains; the last CTA
@@ -258,7 +179,15 @@ __device__ __forceinline__ void k_row_update_body(int vb_, int vg_, const int *_
       Ynext[i] = yn;
     }
   }
-  block_finish_stats<D>(vb_, vg_, st, jp, mn, mx, sm, part_min, part_max, part_sum, iter, alpha, mom);
+  if (block_finish_stats<D>(vb_, vg_, st, jp, &st->done_row, true, mn, mx, sm, part_min, part_max,
+                            part_sum)) {
+#pragma unroll
+    for (int k = 0; k < D; k++)
+      if (!isfinite(st->minv[k]) || !isfinite(st->maxv[k])) st->error |= SGT_EFLAG_NONFINITE;
+    st->alpha = alpha;
+    st->momentum = mom;
+    st->iter = iter + 1;
+  }
 }
 template <int D, int G, bool FUSED>
 __global__ void __launch_bounds__(SGT_THREADS)
@@ -355,10 +284,25 @@ k_attr_ell(int n, int W, const unsigned *__restrict__ cols,
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const typename Vec<D>::T yi = Y[i];
     float acc[3] = {0.f, 0.f, 0.f};
-    for (int k = 0; k < W; k++) {
+    // 4 slots of the row in flight at a time
+    int k = 0;
+    for (; k + 4 <= W; k += 4) {
+      unsigned c[4];
+      float v[4];
+      typename Vec<D>::T yj[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        c[q] = __ldcs(&cols[(long)(k + q) * n + i]);
+        v[q] = __ldcs(&vals[(long)(k + q) * n + i]);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++) yj[q] = __ldg(&Y[c[q]]);
+#pragma unroll
+      for (int q = 0; q < 4; q++) attr_term<D>(yi, yj[q], v[q], acc);
+    }
+    for (; k < W; k++) {
       const long s = (long)k * n + i;
-      const unsigned c = __ldg(&cols[s]);
-      attr_term<D>(yi, __ldg(&Y[c]), __ldg(&vals[s]), acc);
+      attr_term<D>(yi, __ldg(&Y[__ldg(&cols[s])]), __ldg(&vals[s]), acc);
     }
     typename Vec<D>::T f;
     if constexpr (D == 3) f.w = 0.f;
@@ -369,7 +313,11 @@ k_attr_ell(int n, int W, const unsigned *__restrict__ cols,
 }
 
 // COO (rows sorted, CU/pq.cuh:77-118 and the hybrid tail CU/hybridpq.cu:71-113):
-// one element per lane, warp segmented sum by row, one atomic per segment.
+// 4 consecutive elements per lane (16-byte loads where the arrays allow them),
+// summed while their row lasts; runs that end inside a lane go to F at once,
+// the lanes' last runs through a warp segmented sum by row, one atomic per
+// segment.  Bound by the gathers of Y: an element per lane spent 25 shuffles
+// on each, 45 us for the 5M elements of 100,000 rows.
 // F must hold the ELL result or zero.
 template <int D>
 __global__ void __launch_bounds__(SGT_THREADS)
@@ -379,28 +327,65 @@ k_attr_coo(long nnz, const unsigned *__restrict__ rows, const unsigned *__restri
   constexpr int S = D == 3 ? 4 : D;
   const int lane = threadIdx.x & 31;
   const long warps = (long)gridDim.x * blockDim.x / 32;
-  for (long base = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32 * 32; base < nnz;
-       base += warps * 32) {
-    const long e = base + lane;
-    const bool ok = e < nnz;
-    unsigned r = ok ? __ldg(&rows[e]) : 0xffffffffu;
-    float acc[3] = {0.f, 0.f, 0.f};
-    if (ok) attr_term<D>(__ldg(&Y[r]), __ldg(&Y[__ldg(&cols[e])]), __ldg(&vals[e]), acc);
-    // segmented inclusive scan (rows are non-decreasing along the warp)
+  const bool wide = ((reinterpret_cast<size_t>(rows) | reinterpret_cast<size_t>(cols) |
+                      reinterpret_cast<size_t>(vals)) & 15) == 0;
+  for (long base = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32 * 128; base < nnz;
+       base += warps * 128) {
+    const long e = base + 4 * lane;
+    unsigned r[4], c[4];
+    float v[4];
+    if (wide && e + 4 <= nnz) {
+      const uint4 r4 = __ldcs(reinterpret_cast<const uint4 *>(rows + e));
+      const uint4 c4 = __ldcs(reinterpret_cast<const uint4 *>(cols + e));
+      const float4 v4 = __ldcs(reinterpret_cast<const float4 *>(vals + e));
+      r[0] = r4.x; r[1] = r4.y; r[2] = r4.z; r[3] = r4.w;
+      c[0] = c4.x; c[1] = c4.y; c[2] = c4.z; c[3] = c4.w;
+      v[0] = v4.x; v[1] = v4.y; v[2] = v4.z; v[3] = v4.w;
+    } else {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned ro = __shfl_up_sync(0xffffffffu, r, o);
-#pragma unroll
-      for (int k = 0; k < D; k++) {
-        const float v = __shfl_up_sync(0xffffffffu, acc[k], o);
-        if (lane >= o && ro == r) acc[k] += v;
+      for (int q = 0; q < 4; q++) {
+        const bool ok = e + q < nnz;
+        r[q] = ok ? __ldg(&rows[e + q]) : 0xffffffffu;
+        c[q] = ok ? __ldg(&cols[e + q]) : 0u;
+        v[q] = ok ? __ldg(&vals[e + q]) : 0.f;
       }
     }
-    const unsigned rn = __shfl_down_sync(0xffffffffu, r, 1);
-    const bool tail = ok && (lane == 31 || rn != r);
-    if (tail) {
+    typename Vec<D>::T yj[4];
 #pragma unroll
-      for (int k = 0; k < D; k++) atomicAdd(&F[(long)r * S + k], acc[k]);
+    for (int q = 0; q < 4; q++) yj[q] = __ldg(&Y[c[q]]);
+    unsigned cur = r[0];
+    float acc[3] = {0.f, 0.f, 0.f};
+    typename Vec<D>::T yi = __ldg(&Y[cur == 0xffffffffu ? 0u : cur]);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if (r[q] != cur) {
+#pragma unroll
+        for (int k = 0; k < D; k++) atomicAdd(&F[(long)cur * S + k], acc[k]);
+#pragma unroll
+        for (int k = 0; k < 3; k++) acc[k] = 0.f;
+        cur = r[q];
+        if (cur != 0xffffffffu) yi = __ldg(&Y[cur]);
+      }
+      if (cur != 0xffffffffu) attr_term<D>(yi, yj[q], v[q], acc);
+    }
+    // segmented inclusive scan of the last runs (rows do not decrease along
+    // the warp, so a lane whose last run continues its predecessor's holds
+    // nothing else)
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned ro = __shfl_up_sync(0xffffffffu, cur, o);
+#pragma unroll
+      for (int k = 0; k < D; k++) {
+        const float a = __shfl_up_sync(0xffffffffu, acc[k], o);
+        if (lane >= o && ro == cur) acc[k] += a;
+      }
+    }
+    const unsigned rn = __shfl_down_sync(0xffffffffu, cur, 1);
+    // the next lane may begin with this row and end with another: its first
+    // run has gone to F by itself
+    if (cur != 0xffffffffu && (lane == 31 || rn != cur)) {
+#pragma unroll
+      for (int k = 0; k < D; k++) atomicAdd(&F[(long)cur * S + k], acc[k]);
     }
   }
 }
