@@ -95,7 +95,7 @@ struct sgt_job {
   double *part_sum = nullptr, *part_z = nullptr, *part_kl = nullptr;
   SgtState *st = nullptr;
   SgtState *st_host = nullptr;
-  int nb_pts = 0, nb_scat = 0, nb_gath = 0, nb_spec = 0, nb_conv = 0, nb_s2gc = 0, nb_g2s = 0, nb_fft = 0, nb_fft_rows = 0, nb_row = 0,
+  int nb_pts = 0, nb_scat = 0, nb_gath = 0, nb_spec = 0, nb_spec_y = 0, nb_conv = 0, nb_s2gc = 0, nb_g2s = 0, nb_fft = 0, nb_fft_rows = 0, nb_row = 0,
       nb_upd = 0, nb_part = 0;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;  // the two branches of an iteration
   size_t smem_fft1 = 0, smem_fft2 = 0;
@@ -414,6 +414,7 @@ static sgt_status job_shapes(sgt_job *J) {
   // a slot there)
   const bool beside = J->nnz >= 3000000L;
   J->nb_spec = D == 1 ? 2 : (D == 3 ? std::min(4 * nsm, cm * cm) : (beside ? 64 : cm));
+  J->nb_spec_y = 2 * nsm;
   J->nb_conv = D == 1 ? (cm + 7) / 8 : (D == 3 ? std::min(3 * nsm, cm * ct) : std::min(ct, beside ? 64 : cm));
   if constexpr (D == 1) {
     J->nb_fft = 1;
@@ -600,8 +601,13 @@ template <int D>
 static sgt_status enqueue_g2g(sgt_job *J, cudaStream_t s, bool pdl) {
   sgt_ctx *ctx = J->ctx;
   typedef typename Node<D>::T NT;
+  if constexpr (D == 3) {
+    CK(launch_chain(pdl, k_spec_y, J->nb_spec_y, SGT_THREADS, 0, s, (const SgtState *)J->st, J->W));
+    CK(launch_chain(pdl, k_spec_z, J->nb_spec_y, SGT_THREADS, 0, s, (const SgtState *)J->st, J->W));
+  }
   CK(launch_chain(pdl, k_spec_cols<D>, J->nb_conv, SGT_THREADS, 0, s, (const SgtState *)J->st,
                   (const NT *)J->V, (const float2 *)J->W, (NT *)J->Phi));
+  if (J->nmax <= J->jp.conv_max) return SGT_OK;  // no grid of this job takes the FFT passes
   if constexpr (D >= 2) {
     CK(launch_chain(pdl, k_fft_build_x<D>, J->nb_fft_rows, SGT_THREADS, 0, s,
                     (const SgtState *)J->st, (const NT *)J->V, J->W));
@@ -1452,7 +1458,7 @@ sgt_status sgt_job_run(sgt_job *J, int iters) {
 // table of block counts per stage, and one view/prefix table per row-group
 // lane count for the SpMV.
 enum {
-  FS_BIN_COUNT, FS_SCATTER, FS_SPEC, FS_BIN_SCATTER, FS_S2G_CELL, FS_CONV, FS_FFT_X,
+  FS_BIN_COUNT, FS_SCATTER, FS_SPEC, FS_BIN_SCATTER, FS_S2G_CELL, FS_SPEC_Y, FS_CONV, FS_FFT_X,
   FS_FFT_MID_FWD, FS_FFT_LAST, FS_FFT_MID_INV, FS_FFT_FINAL, FS_G2S, FS_GATHER, FS_UPDATE, FS_STAGES
 };
 struct BatchGroup {
@@ -1570,9 +1576,11 @@ static void stage_blocks(const sgt_job *J, int *b) {
   }
   const int rows64 = J->d == 3 ? (2 * 64 * 64 + 128 * 128) / 8 : (2 * 64 + 128) / 8;
   b[FS_CONV] = std::min(J->nb_conv, J->d == 3 ? 100 : 48);
-  if (J->d >= 2) b[FS_FFT_X] = std::min(J->nb_fft_rows, rows64);
-  if (J->d == 3) b[FS_FFT_MID_FWD] = b[FS_FFT_MID_INV] = std::min(J->nb_fft, 128);
-  if (J->d >= 2) {
+  if (J->d == 3) b[FS_SPEC_Y] = std::min(J->nb_spec_y, 64);
+  const bool fft = J->d >= 2 && J->nmax > J->jp.conv_max;
+  if (fft) b[FS_FFT_X] = std::min(J->nb_fft_rows, rows64);
+  if (fft && J->d == 3) b[FS_FFT_MID_FWD] = b[FS_FFT_MID_INV] = std::min(J->nb_fft, 128);
+  if (fft) {
     b[FS_FFT_LAST] = std::min(J->nb_fft, J->d == 3 ? 128 : 16);
     b[FS_FFT_FINAL] = std::min(J->nb_fft_rows, rows64);
   }
@@ -1711,15 +1719,21 @@ static sgt_status enqueue_fused_group(sgt_ctx *ctx, BatchGroup &g) {
     km_s2g_cell<D><<<FL(FS_S2G_CELL), 0, c>>>(v, g.prefix[FS_S2G_CELL], nj);
   }
   km_spec_rows<D><<<FL(FS_SPEC), 0, c>>>(v, g.prefix[FS_SPEC], nj);
+  if constexpr (D == 3) {
+    km_spec_y<<<FL(FS_SPEC_Y), 0, c>>>(v, g.prefix[FS_SPEC_Y], nj);
+    km_spec_z<<<FL(FS_SPEC_Y), 0, c>>>(v, g.prefix[FS_SPEC_Y], nj);
+  }
   km_spec_cols<D><<<FL(FS_CONV), 0, c>>>(v, g.prefix[FS_CONV], nj);
   if constexpr (D >= 2) {
-    km_fft_build_x<D><<<FL(FS_FFT_X), 0, c>>>(v, g.prefix[FS_FFT_X], nj);
-    if constexpr (D == 3)
-      km_fft_cols<D, MODE_MID_FWD><<<FL(FS_FFT_MID_FWD), g.smem_fft, c>>>(v, g.prefix[FS_FFT_MID_FWD], nj);
-    km_fft_cols<D, MODE_LAST><<<FL(FS_FFT_LAST), g.smem_fft, c>>>(v, g.prefix[FS_FFT_LAST], nj);
-    if constexpr (D == 3)
-      km_fft_cols<D, MODE_MID_INV><<<FL(FS_FFT_MID_INV), g.smem_fft, c>>>(v, g.prefix[FS_FFT_MID_INV], nj);
-    km_fft_final_x<D><<<FL(FS_FFT_FINAL), 0, c>>>(v, g.prefix[FS_FFT_FINAL], nj);
+    if (g.blocks[FS_FFT_X] > 0) {  // some job's grids can outgrow k_spec_*
+      km_fft_build_x<D><<<FL(FS_FFT_X), 0, c>>>(v, g.prefix[FS_FFT_X], nj);
+      if constexpr (D == 3)
+        km_fft_cols<D, MODE_MID_FWD><<<FL(FS_FFT_MID_FWD), g.smem_fft, c>>>(v, g.prefix[FS_FFT_MID_FWD], nj);
+      km_fft_cols<D, MODE_LAST><<<FL(FS_FFT_LAST), g.smem_fft, c>>>(v, g.prefix[FS_FFT_LAST], nj);
+      if constexpr (D == 3)
+        km_fft_cols<D, MODE_MID_INV><<<FL(FS_FFT_MID_INV), g.smem_fft, c>>>(v, g.prefix[FS_FFT_MID_INV], nj);
+      km_fft_final_x<D><<<FL(FS_FFT_FINAL), 0, c>>>(v, g.prefix[FS_FFT_FINAL], nj);
+    }
   }
   if (g.blocks[FS_G2S] > 0) km_g2s<D><<<FL(FS_G2S), 0, c>>>(v, g.prefix[FS_G2S], nj);
   km_gather<D><<<FL(FS_GATHER), 0, c>>>(v, g.prefix[FS_GATHER], nj);

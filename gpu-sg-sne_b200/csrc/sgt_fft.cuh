@@ -192,37 +192,40 @@ __device__ __forceinline__ float2 node_plane(const typename Node<D>::T &v, int p
   }
 
 // ---------------------------------------------------------------------------
-// Convolution of small and middle grids in two kernels: a discrete Fourier
-// transform along x and a direct sum over the rows.
+// Convolution of small and middle grids: plain discrete Fourier transforms
+// (M = 2N, any N) along all axes but the last, a direct sum along that one.
 //
-//   k_spec_rows  per row of charges: fold the grid copies and transform along
-//                x (M = 2N, frequencies 0..N of the real rows); per row offset
-//                the transforms of K and of x K.
-//   k_spec_cols  per output row: sum over all input rows, frequency by
-//                frequency, transform back along x.
+//   k_spec_rows  per row of charges: fold the grid copies, transform along x
+//                (frequencies 0..N of the real rows); per row offset the
+//                transforms of K and of x K.
+//   k_spec_y     3-D, per plane and frequency: transform along y; likewise the
+//                kernel's planes, with the transform of y K.
+//   k_spec_z     3-D, per pair of frequencies: sum over the input planes.
+//   k_spec_cols  per output row: 2-D, sum over the input rows; 3-D, transform
+//                back along y; then back along x.
 //
 // The result is Phi0 = sum K V0 and, per axis, Psi_k(g) = sum_s K(g - s)
 // (U_k(s) + (s_k - g_k) V0(s)): the potential of the charges about the output
 // node itself, in cells, so that the force sum_g w_g ((y - y_g) Phi0 - Psi)
-// cancels nothing.  Along x that is K^ Ux^ + i S V0^ with S the sine
-// transform of x K; along the other axes the distance is a number per pair of
-// rows.
+// cancels nothing.  Along a transformed axis that is K^ U^ + i S V0^ with S
+// the sine transform of x K; along the summed one the distance is a number.
 //
-// Why: FFT passes of these grids (16 to 128 points per axis in 2-D, 16 to 40
-// in 3-D, where nearly all iterations run) are three to five kernels bound by
-// latency, pad N to a power of two, and their column pass needs 100 KB of
-// shared memory, for which a block waits until a whole SM has drained of the
-// concurrent SpMV.  The row sums here cost N times more operations than a
-// column FFT and still only a few microseconds, with 256 threads, 64
-// registers and 15 KB a block.  3-D, 20^3: 27 us in five FFT passes.
+// Why: FFT passes of these grids (16 to 128 points per axis, where nearly all
+// iterations run) are three to five kernels bound by latency, pad N to a
+// power of two or three times one, and their column pass needs 100 KB of
+// shared memory in 2-D, for which a block waits until a whole SM has drained
+// of the concurrent SpMV.  The plain transforms cost more operations than FFTs
+// and still only a few microseconds, with 256 threads and 15 KB a block.
 // ---------------------------------------------------------------------------
-#define SGT_SPEC_MAX(D) ((D) == 1 ? 512 : ((D) == 2 ? 128 : 40))
+#define SGT_SPEC_MAX(D) ((D) == 1 ? 512 : 128)
 // k_spec_rows in one go, or its halves (the charge grid of a row-split
 // embedding is summed over the ranks between them)
 #define SGT_SPEC_BOTH 0
 #define SGT_SPEC_FOLD 1
 #define SGT_SPEC_TRANSFORM 2
-#define SGT_SPEC_TY(D) ((D) == 3 ? 4 : 1)  // output rows a block sums together
+#define SGT_SPEC_TY(D) ((D) == 3 ? 4 : 1)  // output rows a block takes together
+#define SGT_SPEC_FS 8  // 3-D: x frequencies a block of k_spec_y takes together
+#define SGT_SPEC_TZ 4  // 3-D: output planes a warp of k_spec_z sums together
 
 // floor(a / b) for 0 <= a < 2^16, inv = 1 / b: half a unit away from every
 // integer quotient
@@ -232,15 +235,24 @@ __device__ __forceinline__ int small_div(int a, float inv) { return (int)(((floa
 template <int D> struct SpecB { typedef float4 T; };
 template <> struct SpecB<2> { typedef float2 T; };
 
-// The spectra live in the FFT workspace: (V0, Ux) of every row and frequency,
-// then (Uy, Uz), then (K^, S) per row offset.
+// The spectra live in the FFT workspace.  Rows: (V0, Ux) of every row and
+// frequency, then (Uy, Uz), then (K^, S) per row offset.  3-D: before them the
+// plane spectra g (plane, y frequency, x frequency; 8 floats) and the kernel's
+// k2 ((K^, Sx, Sy) per plane offset and pair of frequencies up to N); the
+// summed spectra h take the rows' place once k_spec_y has read those.
 template <int D>
 struct SpecBuf {
+  float4 *g, *k2, *h;
   float4 *h0;
   typename SpecB<D>::T *h1;
   float2 *k;
-  __device__ __forceinline__ SpecBuf(float2 *W, int rows, int F) {
-    h0 = reinterpret_cast<float4 *>(W);
+  __device__ __forceinline__ SpecBuf(float2 *W, int N) {
+    const long F = N + 1, rows = D == 2 ? N : (long)N * N;
+    float4 *p = reinterpret_cast<float4 *>(W);
+    g = p;
+    k2 = p + (D == 3 ? 4 * rows * F : 0);
+    h = k2 + (D == 3 ? (long)N * F * F : 0);
+    h0 = h;
     h1 = reinterpret_cast<typename SpecB<D>::T *>(h0 + rows * F);
     k = reinterpret_cast<float2 *>(h1 + rows * F);
   }
@@ -313,7 +325,7 @@ __device__ __forceinline__ void k_spec_rows_body(int vb_, int vg_, const SgtStat
       return;
     }
     const float inv_f = 1.0f / (float)F, inv_m = 1.0f / (float)M;
-    const SpecBuf<D> B(W, rows, F);
+    const SpecBuf<D> B(W, N);
     spec_twiddles(tw, M);
     // thread: frequency f and segment sg of the row
     const int S = SGT_THREADS / F, t = threadIdx.x;  // F <= 129: S >= 1
@@ -353,7 +365,7 @@ __device__ __forceinline__ void k_spec_rows_body(int vb_, int vg_, const SgtStat
           kc += red[2 * (g * F + t)];
           ks += red[2 * (g * F + t) + 1];
         }
-        B.k[r * F + t] = make_float2(kc, ks);
+        B.k[(long)r * F + t] = make_float2(kc, ks);
       }
     }
     sgt_pdl_wait();
@@ -420,9 +432,10 @@ __device__ __forceinline__ void k_spec_rows_body(int vb_, int vg_, const SgtStat
         for (int g = 0; g < S; g++)
 #pragma unroll
           for (int c = 0; c < (D == 3 ? 8 : 6); c++) a[c] += red[(g * F + t) * 9 + c];
-        B.h0[r * F + t] = make_float4(a[0], a[1], a[2], a[3]);
-        if constexpr (D == 3) B.h1[r * F + t] = make_float4(a[4], a[5], a[6], a[7]);
-        else B.h1[r * F + t] = make_float2(a[4], a[5]);
+        const long at = (long)r * F + t;
+        B.h0[at] = make_float4(a[0], a[1], a[2], a[3]);
+        if constexpr (D == 3) B.h1[at] = make_float4(a[4], a[5], a[6], a[7]);
+        else B.h1[at] = make_float2(a[4], a[5]);
       }
     }
   }
@@ -432,6 +445,156 @@ __global__ void __launch_bounds__(SGT_THREADS, 4)
 k_spec_rows(const SgtState *st, typename Node<D>::T *__restrict__ Vc,
             typename Node<D>::T *__restrict__ V, float2 *__restrict__ W, int phase) {
   k_spec_rows_body<D>(blockIdx.x, gridDim.x, st, Vc, V, W, phase);
+}
+
+// 3-D: transform along y.  A block takes a plane (or a plane offset of the
+// kernel) and SGT_SPEC_FS x frequencies, the inputs in shared memory; a thread
+// sums an output frequency pair over the N rows, 16 multiply-adds per row.
+__device__ __forceinline__ void k_spec_y_body(int vb_, int vg_, const SgtState *st,
+                                              float2 *__restrict__ W) {
+  if (!st->direct) {
+    sgt_pdl_wait();
+    return;
+  }
+  constexpr int FS = SGT_SPEC_FS;
+  const int N = st->N, M = 2 * N, F = N + 1, fb = (F + FS - 1) / FS, items = N * fb;
+  if (vb_ >= 2 * items) {
+    sgt_pdl_wait();
+    return;
+  }
+  __shared__ float2 tw[2 * 128];
+  __shared__ float4 in[128 * FS * 2];
+  const SpecBuf<3> B(W, N);
+  spec_twiddles(tw, M);
+  const int t = threadIdx.x;
+  const float inv_fb = 1.0f / (float)fb;
+  sgt_pdl_wait();
+  for (int it = vb_; it < 2 * items; it += vg_) {
+    const bool kernel = it >= items;
+    const int e = kernel ? it - items : it;
+    const int z = small_div(e, inv_fb), f0 = (e - z * fb) * FS, nf = min(FS, F - f0);
+    __syncthreads();
+    if (!kernel) {
+      for (int q = t; q < N * FS; q += SGT_THREADS) {
+        const int y = q / FS, f = min(q % FS, nf - 1);
+        const long at = ((long)z * N + y) * F + f0 + f;
+        in[2 * q] = B.h0[at];
+        in[2 * q + 1] = B.h1[at];
+      }
+      __syncthreads();
+      for (int q = t; q < M * FS; q += SGT_THREADS) {
+        const int ky = q / FS, f = q % FS;
+        float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        int w = 0;
+        for (int y = 0; y < N; y++) {
+          const float2 c = tw[w];
+          const float4 u = in[2 * (y * FS + f)], v = in[2 * (y * FS + f) + 1];
+          a[0] += u.x * c.x - u.y * c.y; a[1] += u.x * c.y + u.y * c.x;
+          a[2] += u.z * c.x - u.w * c.y; a[3] += u.z * c.y + u.w * c.x;
+          a[4] += v.x * c.x - v.y * c.y; a[5] += v.x * c.y + v.y * c.x;
+          a[6] += v.z * c.x - v.w * c.y; a[7] += v.z * c.y + v.w * c.x;
+          w += ky;
+          if (w >= M) w -= M;
+        }
+        if (f < nf) {
+          float4 *g = B.g + 2 * (((long)z * M + ky) * F + f0 + f);
+          g[0] = make_float4(a[0], a[1], a[2], a[3]);
+          g[1] = make_float4(a[4], a[5], a[6], a[7]);
+        }
+      }
+    } else {
+      float2 *kin = reinterpret_cast<float2 *>(in);
+      for (int q = t; q < N * FS; q += SGT_THREADS) {
+        const int y = q / FS, f = min(q % FS, nf - 1);
+        float2 k = B.k[((long)z * N + y) * F + f0 + f];
+        if (y > 0) { k.x *= 2.0f; k.y *= 2.0f; }
+        kin[q] = k;
+      }
+      __syncthreads();
+      for (int q = t; q < F * FS; q += SGT_THREADS) {
+        const int ky = q / FS, f = q % FS;
+        float kk = 0.f, sx = 0.f, sy = 0.f;
+        int w = 0;
+        for (int y = 0; y < N; y++) {
+          const float2 c = tw[w], k = kin[y * FS + f];
+          kk += k.x * c.x;
+          sx += k.y * c.x;
+          sy -= (float)y * k.x * c.y;
+          w += ky;
+          if (w >= M) w -= M;
+        }
+        if (f < nf) B.k2[((long)z * F + ky) * F + f0 + f] = make_float4(kk, sx, sy, 0.f);
+      }
+    }
+  }
+}
+__global__ void __launch_bounds__(SGT_THREADS, 4)
+k_spec_y(const SgtState *st, float2 *__restrict__ W) {
+  k_spec_y_body(blockIdx.x, gridDim.x, st, W);
+}
+
+// 3-D: sum over the input planes, frequency by frequency.  A lane holds a
+// frequency pair, a warp SGT_SPEC_TZ output planes (52 multiply-adds per input
+// plane; the kernel's values slide through registers), a block 32 pairs and
+// 8 warps of planes.
+__device__ __forceinline__ void k_spec_z_body(int vb_, int vg_, const SgtState *st,
+                                              float2 *__restrict__ W) {
+  sgt_pdl_wait();
+  if (!st->direct) return;
+  constexpr int TZ = SGT_SPEC_TZ, WPB = SGT_THREADS / 32;
+  const int N = st->N, M = 2 * N, F = N + 1, pairs = M * F;
+  const int pb = (pairs + 31) / 32, zb = (N + TZ * WPB - 1) / (TZ * WPB), items = pb * zb;
+  const SpecBuf<3> B(W, N);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int it = vb_; it < items; it += vg_) {
+    const int zt = it / pb, pr = (it - zt * pb) * 32 + lane;
+    const int z0 = (zt * WPB + warp) * TZ;
+    if (z0 >= N || pr >= pairs) continue;
+    const int ky = pr / F, f = pr - ky * F;
+    const bool up = ky > N;  // K^ and Sx are even in ky, Sy odd
+    const float4 *k2 = B.k2 + (long)(up ? M - ky : ky) * F + f;
+    const float sgn = up ? -1.0f : 1.0f;
+    const long ks = (long)F * F, gs = (long)M * F;
+    const float4 *g = B.g + 2 * (long)pr;
+    float a[TZ][8];
+#pragma unroll
+    for (int j = 0; j < TZ; j++)
+#pragma unroll
+      for (int c = 0; c < 8; c++) a[j][c] = 0.f;
+    float4 k[TZ];  // k[j]: offset z0 + j - z
+#pragma unroll
+    for (int j = 1; j < TZ; j++) k[j] = k2[min(z0 + j, N - 1) * ks];
+#pragma unroll 2
+    for (int z = 0; z < N; z++) {
+      k[0] = k2[abs(z0 - z) * ks];
+      const float4 u = g[2 * z * gs], v = g[2 * z * gs + 1];
+#pragma unroll
+      for (int j = 0; j < TZ; j++) {
+        const float dz = (float)(z - z0 - j), sy = sgn * k[j].z;
+        a[j][0] += k[j].x * u.x;
+        a[j][1] += k[j].x * u.y;
+        a[j][2] += k[j].x * u.z - k[j].y * u.y;
+        a[j][3] += k[j].x * u.w + k[j].y * u.x;
+        a[j][4] += k[j].x * v.x - sy * u.y;
+        a[j][5] += k[j].x * v.y + sy * u.x;
+        a[j][6] += k[j].x * (v.z + dz * u.x);
+        a[j][7] += k[j].x * (v.w + dz * u.y);
+      }
+#pragma unroll
+      for (int j = TZ - 1; j > 0; j--) k[j] = k[j - 1];
+    }
+#pragma unroll
+    for (int j = 0; j < TZ; j++)
+      if (z0 + j < N) {
+        float4 *h = B.h + 2 * ((z0 + j) * gs + pr);
+        h[0] = make_float4(a[j][0], a[j][1], a[j][2], a[j][3]);
+        h[1] = make_float4(a[j][4], a[j][5], a[j][6], a[j][7]);
+      }
+  }
+}
+__global__ void __launch_bounds__(SGT_THREADS, 2)
+k_spec_z(const SgtState *st, float2 *__restrict__ W) {
+  k_spec_z_body(blockIdx.x, gridDim.x, st, W);
 }
 
 template <int D>
@@ -463,7 +626,7 @@ __device__ __forceinline__ void k_spec_cols_body(int vb_, int vg_, const SgtStat
       sgt_pdl_wait();
       return;
     }
-    const int N = st->N, M = 2 * N, F = N + 1, rows = D == 2 ? N : N * N;
+    const int N = st->N, M = 2 * N, F = N + 1;
     const int ty = (N + TY - 1) / TY, items = (D == 2 ? 1 : N) * ty;
     if (vb_ >= items) {
       sgt_pdl_wait();
@@ -471,67 +634,71 @@ __device__ __forceinline__ void k_spec_cols_body(int vb_, int vg_, const SgtStat
     }
     __shared__ float2 tw[2 * 128];
     __shared__ float red[SGT_THREADS * 9];
-    __shared__ float What[(D == 2 ? 129 : 41) * TY * (C + 1)];  // [output][frequency][C + 1]
+    __shared__ float What[129 * (C + 1)];  // [frequency][C + 1]
     spec_twiddles(tw, M);
     const float inv_f = 1.0f / (float)F, inv_m = 1.0f / (float)M;
-    const SpecBuf<D> B(const_cast<float2 *>(W), rows, F);
+    const SpecBuf<D> B(const_cast<float2 *>(W), N);
     const int t = threadIdx.x, S = SGT_THREADS / F;
     const int sg = small_div(t, inv_f), f = t - sg * F;
-    // pieces of the input: H parts of each plane's rows, dealt to the segments
-    const int H = D == 2 ? S : 2, len = (N + H - 1) / H, pieces = (D == 2 ? 1 : N) * H;
+    // the segments share the input rows (2-D) or y frequencies (3-D)
+    const int nin = D == 2 ? N : M, len = (nin + S - 1) / S;
+    const int r0 = min(sg * len, nin), r1 = min(nin, r0 + len);
     sgt_pdl_wait();
+    __syncthreads();  // the twiddles
     for (int it = vb_; it < items; it += vg_) {
       const int oz = D == 2 ? 0 : small_div(it, 1.0f / (float)ty), y0 = (it - oz * ty) * TY;
-      const float yc = (float)y0 + 0.5f * (float)(TY - 1);
       float a[TY][C];
 #pragma unroll
       for (int j = 0; j < TY; j++)
 #pragma unroll
         for (int c = 0; c < C; c++) a[j][c] = 0.f;
       if (sg < S) {
-        for (int pc = sg; pc < pieces; pc += S) {
-          const int z = D == 2 ? 0 : pc >> 1, hpart = D == 2 ? pc : pc & 1;
-          const int r0 = min(hpart * len, N), r1 = min(N, r0 + len);
-          const float dz = (float)(z - oz);
-          const float2 *kp = B.k + (D == 2 ? 0 : abs(z - oz) * N) * F + f;
-          const float4 *h0 = B.h0 + z * N * F + f;
-          const typename SpecB<D>::T *h1 = B.h1 + z * N * F + f;
-          float2 k[TY];  // k[j]: offset y0 + j - r; slides by one per input row
-#pragma unroll
-          for (int j = 1; j < TY; j++) k[j] = kp[abs(min(y0 + j - r0, N - 1)) * F];
+        if constexpr (D == 2) {
+          const float2 *kp = B.k + f;
+          const float4 *h0 = B.h0 + f;
+          const typename SpecB<D>::T *h1 = B.h1 + f;
 #pragma unroll 4
           for (int r = r0; r < r1; r++) {
-            k[0] = kp[abs(y0 - r) * F];
+            const float2 k = kp[abs(y0 - r) * F];
             const float4 v = h0[r * F];
             const typename SpecB<D>::T u = h1[r * F];
-            const float dy = (float)r - yc;
-            const float uyr = u.x + dy * v.x, uyi = u.y + dy * v.y;
-            float uzr = 0.f, uzi = 0.f;
-            if constexpr (D == 3) {
-              uzr = u.z + dz * v.x;
-              uzi = u.w + dz * v.y;
-            }
+            const float dy = (float)(r - y0);
+            a[0][0] += k.x * v.x;
+            a[0][1] += k.x * v.y;
+            a[0][2] += k.x * v.z - k.y * v.y;
+            a[0][3] += k.x * v.w + k.y * v.x;
+            a[0][4] += k.x * (u.x + dy * v.x);
+            a[0][5] += k.x * (u.y + dy * v.y);
+          }
+        } else {
+          const float4 *h = B.h + 2 * ((long)oz * M * F + f);
+          int w[TY];
+#pragma unroll
+          for (int j = 0; j < TY; j++) w[j] = (y0 + j) * r0 - M * small_div((y0 + j) * r0, inv_m);
+#pragma unroll 2
+          for (int r = r0; r < r1; r++) {
+            const float4 u = h[2 * (long)r * F], v = h[2 * (long)r * F + 1];
 #pragma unroll
             for (int j = 0; j < TY; j++) {
-              a[j][0] += k[j].x * v.x;
-              a[j][1] += k[j].x * v.y;
-              a[j][2] += k[j].x * v.z - k[j].y * v.y;
-              a[j][3] += k[j].x * v.w + k[j].y * v.x;
-              a[j][4] += k[j].x * uyr;
-              a[j][5] += k[j].x * uyi;
-              if constexpr (D == 3) {
-                a[j][6] += k[j].x * uzr;
-                a[j][7] += k[j].x * uzi;
-              }
+              const float2 c = tw[w[j]];  // (cos, -sin): times (cos + i sin)
+              a[j][0] += u.x * c.x + u.y * c.y; a[j][1] += u.y * c.x - u.x * c.y;
+              a[j][2] += u.z * c.x + u.w * c.y; a[j][3] += u.w * c.x - u.z * c.y;
+              a[j][4] += v.x * c.x + v.y * c.y; a[j][5] += v.y * c.x - v.x * c.y;
+              a[j][6] += v.z * c.x + v.w * c.y; a[j][7] += v.w * c.x - v.z * c.y;
+              w[j] += y0 + j;
+              if (w[j] >= M) w[j] -= M;
             }
-#pragma unroll
-            for (int j = TY - 1; j > 0; j--) k[j] = k[j - 1];
           }
         }
       }
-      // over the segments, in order
+      // back along x: P lanes (a power of two) per output
+      int lp = 0;
+      while ((N << (lp + 1)) <= SGT_THREADS && lp < 3) lp++;
+      const int P = 1 << lp, p = t & (P - 1);
+      const float scale = D == 2 ? 1.0f / (float)M : 1.0f / ((float)M * (float)M);
 #pragma unroll
       for (int j = 0; j < TY; j++) {
+        // the segments' sums, in order
         __syncthreads();
         if (sg < S) {
 #pragma unroll
@@ -546,45 +713,35 @@ __device__ __forceinline__ void k_spec_cols_body(int vb_, int vg_, const SgtStat
             im += red[(g * F + ff) * 9 + 2 * c2 + 1];
           }
           const float wt = (ff == 0 || ff == N) ? 1.0f : 2.0f;
-          What[(j * F + ff) * (C + 1) + 2 * c2] = wt * re;
-          What[(j * F + ff) * (C + 1) + 2 * c2 + 1] = wt * im;
+          What[ff * (C + 1) + 2 * c2] = wt * re;
+          What[ff * (C + 1) + 2 * c2 + 1] = wt * im;
         }
-      }
-      __syncthreads();
-      // back along x: P lanes (a power of two) per output
-      int lp = 0;
-      while ((TY * N << (lp + 1)) <= SGT_THREADS && lp < 3) lp++;
-      const int P = 1 << lp, p = t & (P - 1);
-      const float inv_n = 1.0f / (float)N;
-      for (int o0 = 0; o0 < TY * N; o0 += SGT_THREADS >> lp) {  // uniform
-        const int o = o0 + (t >> lp);
-        const int j = min(small_div(o, inv_n), TY - 1), x = min(o - j * N, N - 1);
-        float q[D + 1];
-#pragma unroll
-        for (int c = 0; c <= D; c++) q[c] = 0.f;
-        const int step = x * P - M * small_div(x * P, inv_m);
-        int w = x * p - M * small_div(x * p, inv_m);
-        for (int ff = p; ff < F; ff += P) {
-          const float2 e = tw[w];  // (cos, -sin): Re(W exp(+i)) = re cos + im (-sin)
-          const float *wh = &What[(j * F + ff) * (C + 1)];
-#pragma unroll
-          for (int c = 0; c <= D; c++) q[c] += wh[2 * c] * e.x + wh[2 * c + 1] * e.y;
-          w += step;
-          if (w >= M) w -= M;
-        }
-#pragma unroll
-        for (int e = 1; e < 8; e *= 2)
-          if (e < P) {
-#pragma unroll
-            for (int c = 0; c <= D; c++) q[c] += __shfl_xor_sync(0xffffffffu, q[c], e);
-          }
+        __syncthreads();
         const int y = y0 + j;
-        if (p == 0 && o < TY * N && y < N) {
+        for (int o0 = 0; o0 < N; o0 += SGT_THREADS >> lp) {  // uniform
+          const int o = o0 + (t >> lp), x = min(o, N - 1);
+          float q[D + 1];
 #pragma unroll
-          for (int c = 0; c <= D; c++) q[c] = q[c] / (float)M;
-          q[2] += (yc - (float)y) * q[0];
-          Phi[((long)(D == 2 ? 0 : oz) * N + y) * N + x] =
-              make_float4(q[0], q[1], q[2], D == 3 ? q[D] : 0.f);
+          for (int c = 0; c <= D; c++) q[c] = 0.f;
+          const int step = x * P - M * small_div(x * P, inv_m);
+          int w = x * p - M * small_div(x * p, inv_m);
+          for (int ff = p; ff < F; ff += P) {
+            const float2 e = tw[w];  // (cos, -sin): Re(W exp(+i)) = re cos + im (-sin)
+            const float *wh = &What[ff * (C + 1)];
+#pragma unroll
+            for (int c = 0; c <= D; c++) q[c] += wh[2 * c] * e.x + wh[2 * c + 1] * e.y;
+            w += step;
+            if (w >= M) w -= M;
+          }
+#pragma unroll
+          for (int e = 1; e < 8; e *= 2)
+            if (e < P) {
+#pragma unroll
+              for (int c = 0; c <= D; c++) q[c] += __shfl_xor_sync(0xffffffffu, q[c], e);
+            }
+          if (p == 0 && o < N && y < N)
+            Phi[((long)(D == 2 ? 0 : oz) * N + y) * N + x] = make_float4(
+                q[0] * scale, q[1] * scale, q[2] * scale, D == 3 ? q[D] * scale : 0.f);
         }
       }
     }

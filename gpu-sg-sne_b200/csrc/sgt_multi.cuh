@@ -90,6 +90,18 @@ km_spec_rows(const SgtJobView *__restrict__ views, const int *__restrict__ prefi
                       SGT_SPEC_BOTH);
 }
 
+__global__ void __launch_bounds__(SGT_THREADS, 4)
+km_spec_y(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
+  SGT_MULTI_JOB
+  k_spec_y_body(vb, vg, v.st, v.W);
+}
+
+__global__ void __launch_bounds__(SGT_THREADS, 2)
+km_spec_z(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
+  SGT_MULTI_JOB
+  k_spec_z_body(vb, vg, v.st, v.W);
+}
+
 template <int D>
 __global__ void __launch_bounds__(SGT_THREADS, 3)
 km_spec_cols(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
