@@ -128,7 +128,8 @@ k_knn(const float *__restrict__ X, int n, int dim, int k, const int *__restrict_
 // ---------------------------------------------------------------------------
 // Tensor-core filter.
 //
-// q.c - |c|^2/2 = (|q|^2 - d^2)/2 ranks the candidates c of a query q.  The
+// q.c - |c|^2/2 = (|q|^2 - d^2)/2 ranks the candidates c of a query q: one dot
+// product of (q, 1, 1, 1) and (c, the three BF16 terms of -|c|^2/2).  The
 // products run on the tensor cores as BF16 MMAs (kind::f16) in three terms,
 // hi.hi + hi.lo + lo.hi with x = hi + lo + e, hi = bf16(x), lo = bf16(x - hi),
 // |e| <= 2^-18 |x|, FP32 accumulation in tensor memory; points that are BF16
@@ -169,22 +170,19 @@ k_knn(const float *__restrict__ X, int n, int dim, int k, const int *__restrict_
 // 10, both K-major, N/8 at bit 17 and M/16 at bit 24.
 constexpr int KNN_TC_M = 128;      // queries per block
 constexpr int KNN_TC_N = 256;      // candidates per tile
-constexpr int KNN_TC_KU = 8;       // units (of 8 dimensions) per chunk
+constexpr int KNN_TC_RES = 8;      // units (of 8 dimensions) up to which a query image is resident
 constexpr int KNN_TC_MAXK = 32;    // limits of SGT_KNN_TENSOR
 constexpr int KNN_TC_MAXDIM = 64;
-constexpr int KNN_TC_SCAN = 256;   // scanning threads; one more warp issues
-constexpr int KNN_TC_THREADS = KNN_TC_SCAN + 32;
-constexpr unsigned KNN_TC_APART = KNN_TC_KU * KNN_TC_M * 16;  // bytes of a chunk's part
-constexpr unsigned KNN_TC_BPART = KNN_TC_KU * KNN_TC_N * 16;
-constexpr unsigned KNN_TC_SMEM = 4 * (KNN_TC_APART + KNN_TC_BPART);  // 192 KB
+constexpr int KNN_TC_SCAN = 256;   // scanning threads; two more warps issue MMAs and copies
+constexpr int KNN_TC_THREADS = KNN_TC_SCAN + 64;
+constexpr unsigned KNN_TC_SMEM = 192 * 1024;
 
 // Bound on the error of 2 key = |q|^2 - d^2, relative to |q|^2 + max |c|^2:
 // 2^-21 of the products' sum per accumulated MMA of 16 dimensions and, in
 // three terms, twice 3 * 2^-18 for the neglected parts.
 __host__ __device__ inline float knn_tc_eps(int dim, bool exact) {
-  const float steps = (float)((dim + 15) / 16);
-  return exact ? (steps + 1.f) * 4.8e-7f
-               : (dim <= KNN_TC_MAXDIM ? 1e-4f : 2.4e-5f + 3.f * steps * 4.8e-7f);
+  const float steps = (float)((dim + 3 + 15) / 16);
+  return exact ? (steps + 1.f) * 4.8e-7f : 2.4e-5f + 3.f * steps * 4.8e-7f;
 }
 
 // shared-memory matrix descriptor: K-major, no swizzle
@@ -236,6 +234,7 @@ __device__ __forceinline__ bool mbar_wait_or(unsigned bar, unsigned parity, vola
     }
   }
 }
+// starts a load of 32 columns; tmem_wait before the values are used
 __device__ __forceinline__ void tmem_ld32(unsigned taddr, float *v) {
   unsigned r[32];
   asm volatile(
@@ -249,9 +248,14 @@ __device__ __forceinline__ void tmem_ld32(unsigned taddr, float *v) {
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
         "=r"(r[31])
       : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int j = 0; j < 32; j++) v[j] = __uint_as_float(r[j]);
+}
+// waits for the loads in flight; v (their destination) is not read before
+__device__ __forceinline__ void tmem_wait(float *v) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < 32; j++) asm volatile("" : "+f"(v[j]));
 }
 
 // BF16 (round to nearest even) of a float, as its upper 16 bits; inf and NaN
@@ -261,17 +265,15 @@ __device__ __forceinline__ unsigned bf16_bits(float x) {
 }
 __device__ __forceinline__ float bf16_value(unsigned b) { return __uint_as_float(b << 16); }
 
-// squared norms (FP32, dimension order), their maximum, the candidates' key
-// offsets -|c|^2/2 (-inf behind the last point: never admitted), and whether
-// some coordinate is no BF16 number; a warp per point
-__global__ void k_knn_norms(const float *__restrict__ X, int n, int npad, int dim,
-                            float *__restrict__ nrm, float *__restrict__ off,
+// squared norms (FP32, dimension order), their maximum, and whether some
+// coordinate is no BF16 number
+__global__ void k_knn_norms(const float *__restrict__ X, int n, int dim, float *__restrict__ nrm,
                             unsigned *__restrict__ nmax, int *__restrict__ inexact) {
   __shared__ float tile[8][32][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   // a warp takes 32 points; 32 x 32 tiles turn coalesced loads into a
   // point per lane
-  for (int i0 = (blockIdx.x * 8 + w) * 32; i0 < npad; i0 += gridDim.x * 256) {
+  for (int i0 = (blockIdx.x * 8 + w) * 32; i0 < n; i0 += gridDim.x * 256) {
     float s = 0.f;
     bool low = false;
     for (int k0 = 0; k0 < dim; k0 += 32) {
@@ -287,7 +289,6 @@ __global__ void k_knn_norms(const float *__restrict__ X, int n, int npad, int di
     }
     const int i = i0 + lane;
     if (i < n) nrm[i] = s;
-    if (i < npad) off[i] = i < n ? -0.5f * s : -INFINITY;
     // non-negative floats order as integers (a NaN norm as the largest)
     const unsigned m = __reduce_max_sync(0xffffffffu, i < n ? __float_as_uint(s) : 0u);
     if (lane == 0) atomicMax(nmax, m);
@@ -296,8 +297,12 @@ __global__ void k_knn_norms(const float *__restrict__ X, int n, int npad, int di
 }
 
 // hi/lo images of the points in blocks of `rows` ([block][part][unit][row],
-// 8 dimensions of 2 bytes); rows past n and unused dimensions are zero.
-__global__ void k_knn_split(const float *__restrict__ X, int n, int dim, int U, int rows, int nblk,
+// 8 dimensions of 2 bytes), as queries (ones in columns dim .. dim + 2 of the
+// hi part) or candidates (-|c|^2/2 in three BF16 terms there).  Unused columns
+// and rows past n are zero, but candidate rows past n have the key -inf, which
+// no threshold admits.
+__global__ void k_knn_split(const float *__restrict__ X, const float *__restrict__ nrm, int n,
+                            int dim, int U, int rows, int nblk, int candidates,
                             uint4 *__restrict__ img) {
   const long total = (long)nblk * rows * U;
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total;
@@ -313,6 +318,19 @@ __global__ void k_knn_split(const float *__restrict__ X, int n, int dim, int U, 
       const float x = i < n && kk < dim ? X[(long)i * dim + kk] : 0.f;
       h[c] = bf16_bits(x);
       l[c] = bf16_bits(x - bf16_value(h[c]));
+      if (kk >= dim && kk < dim + 3) {
+        if (!candidates) {
+          h[c] = i < n ? 0x3f80u : 0u;  // 1
+        } else if (i >= n) {
+          h[c] = kk == dim ? 0xff80u : 0u;  // -inf
+        } else {
+          const float a = -0.5f * nrm[i];
+          const float h1 = bf16_value(bf16_bits(a)), r1 = a - h1;
+          const float h2 = bf16_value(bf16_bits(r1));
+          h[c] = kk == dim ? bf16_bits(a) : (kk == dim + 1 ? bf16_bits(r1) : bf16_bits(r1 - h2));
+        }
+        l[c] = 0u;
+      }
     }
     uint4 vh, vl;
     vh = make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4] | h[5] << 16, h[6] | h[7] << 16);
@@ -337,8 +355,18 @@ __device__ __forceinline__ float knn_unordered(unsigned u) {
 // `want` reach it.
 template <int E>
 __device__ __forceinline__ unsigned knn_kth(const unsigned *u, int want) {
-  unsigned T = 0;
-  for (int bit = 31; bit >= 0; bit--) {
+  // the bits that all entries share need no search
+  unsigned hi = 0, lo = 0xffffffffu;
+#pragma unroll
+  for (int i = 0; i < E; i++) {
+    hi = max(hi, u[i]);
+    lo = min(lo, u[i] - 1u);  // an empty entry becomes the largest number
+  }
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  lo = __reduce_min_sync(0xffffffffu, lo) + 1u;
+  const int top = 31 - __clz((int)(hi ^ lo));  // -1: all equal
+  unsigned T = top < 0 ? hi : hi & ~((2u << top) - 1u);
+  for (int bit = top; bit >= 0; bit--) {
     const unsigned trial = T | (1u << bit);
     unsigned c = 0;
 #pragma unroll
@@ -383,41 +411,46 @@ __device__ __forceinline__ float knn_select(float2 *buf, int cnt) {
 }
 
 // A block walks over query blocks; warps 0-7 scan (warp w: rows 32 (w & 3)..,
-// columns 128 (w >> 2)..), lane 0 of warp 8 issues copies and MMAs.
+// columns 128 (w >> 2)..), lane 0 of warp 8 issues the MMAs, lane 0 of warp 9
+// the copies.
 template <int L, int CAP>
 __global__ void __launch_bounds__(KNN_TC_THREADS, 1)
 k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict__ imgB,
-         const float *__restrict__ nrm, const float *__restrict__ off,
+         const float *__restrict__ nrm,
          const unsigned *__restrict__ nmax, const int *__restrict__ inexact,
          const float *__restrict__ X, int n, int dim, int U, int k, float2 *__restrict__ bufs,
          int *__restrict__ idx, float *__restrict__ d2, int *__restrict__ redo,
          int *__restrict__ nredo, int *__restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  // full x4, empty x4, accumulator full x2, empty x2, resident A
-  __shared__ __align__(8) unsigned long long bars[13];
+  // full x8, empty x8, accumulator full x2, empty x2, resident A
+  __shared__ __align__(8) unsigned long long bars[21];
   __shared__ unsigned tslot;
   __shared__ volatile int gave_up;
   __shared__ int s_cnt[KNN_TC_SCAN];
   __shared__ float s_thr[KNN_TC_SCAN];
+  __shared__ volatile float s_live[KNN_TC_SCAN];
   __shared__ int s_idx[8][L];
   __shared__ float s_d[8][L];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int nq = (n + KNN_TC_M - 1) / KNN_TC_M, ntile = (n + KNN_TC_N - 1) / KNN_TC_N;
-  const int nch = (U + KNN_TC_KU - 1) / KNN_TC_KU;
-  const bool three = *inexact != 0, resident = nch == 1;
-  const int parts = three ? 2 : 1, nst = three ? 2 : 4;
+  const int ku = U <= KNN_TC_RES ? 4 : 8, nch = (U + ku - 1) / ku;  // units and number of chunks
+  const unsigned apart = ku * KNN_TC_M * 16u, bpart = ku * KNN_TC_N * 16u;
+  const bool three = *inexact != 0, resident = U <= KNN_TC_RES;
+  const int parts = three ? 2 : 1;
   const unsigned sm0 = smem_u32(smem);
-  const unsigned a_bytes = resident ? 0u : parts * KNN_TC_APART;
-  const unsigned st_bytes = a_bytes + parts * KNN_TC_BPART;
-  const unsigned st0 = sm0 + (resident ? parts * KNN_TC_APART : 0u);
+  const unsigned a_bytes = resident ? 0u : parts * apart;
+  const unsigned st_bytes = a_bytes + parts * bpart;
+  const unsigned res_part = (unsigned)U * KNN_TC_M * 16u;  // a part of a resident query image
+  const unsigned st0 = sm0 + (resident ? parts * res_part : 0u);
+  const int nst = min(8, (int)((sm0 + KNN_TC_SMEM - st0) / st_bytes));
   auto bar_full = [&](int st) { return smem_u32(&bars[st]); };
-  auto bar_free = [&](int st) { return smem_u32(&bars[4 + st]); };
-  auto bar_acc = [&](int b) { return smem_u32(&bars[8 + b]); };
-  auto bar_scan = [&](int b) { return smem_u32(&bars[10 + b]); };
-  const unsigned bar_a = smem_u32(&bars[12]);
+  auto bar_free = [&](int st) { return smem_u32(&bars[8 + st]); };
+  auto bar_acc = [&](int b) { return smem_u32(&bars[16 + b]); };
+  auto bar_scan = [&](int b) { return smem_u32(&bars[18 + b]); };
+  const unsigned bar_a = smem_u32(&bars[20]);
   if (t == 0) {
     gave_up = 0;
-    for (int b = 0; b < 13; b++) mbar_init(smem_u32(&bars[b]), b == 10 || b == 11 ? 8 : 1);
+    for (int b = 0; b < 21; b++) mbar_init(smem_u32(&bars[b]), b == 18 || b == 19 ? 8 : 1);
     mbar_fence_init();
   }
   if (warp == 0) {
@@ -435,57 +468,57 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
   // running counts of tiles and of pipeline steps over all query blocks
   unsigned tiles = 0, steps = 0, loads = 0, blocks = 0;
   for (int qb = blockIdx.x; qb < nq; qb += gridDim.x, blocks++) {
-    if (warp == 8) {
-      if (lane == 0) {
-        const unsigned total = (unsigned)ntile * (unsigned)nch;
+    const unsigned total = (unsigned)ntile * (unsigned)nch;  // pipeline steps of a query block
+    if (warp == 9) {
+      if (lane == 0) {  // copies: step g is chunk g % nch of tile g / nch
         bool ok = true;
-        // copies of step g of this block: chunk g % nch of tile g / nch
-        auto load = [&](unsigned g) {
+        if (resident) {
+          // every MMA of the last query block has been waited for (its tiles
+          // were scanned), so its image can be replaced
+          mbar_expect_tx(bar_a, parts * res_part);
+          for (int p = 0; p < parts; p++)
+            bulk_g2s(sm0 + p * res_part, imgA + ((size_t)qb * 2 + p) * res_part, res_part, bar_a);
+        }
+        for (unsigned g = 0; g < total; g++, loads++) {
           const int st = (int)(loads % (unsigned)nst);
           const unsigned turn = loads / (unsigned)nst;
-          if (turn > 0) ok = ok && mbar_wait_or(bar_free(st), (turn - 1) & 1, &gave_up);
-          if (!ok) return;
+          if (turn > 0) ok = mbar_wait_or(bar_free(st), (turn - 1) & 1, &gave_up);
+          if (!ok) break;
           const int tile = (int)(g / (unsigned)nch), ch = (int)(g % (unsigned)nch);
-          const int uc = min(KNN_TC_KU, U - ch * KNN_TC_KU);
+          const int uc = min(ku, U - ch * ku);
           const unsigned sb = st0 + st * st_bytes;
           mbar_expect_tx(bar_full(st), parts * uc * 16u * (KNN_TC_N + (resident ? 0 : KNN_TC_M)));
           for (int p = 0; p < parts; p++) {
             if (!resident)
-              bulk_g2s(sb + p * KNN_TC_APART,
-                       imgA + (((size_t)qb * 2 + p) * U + ch * KNN_TC_KU) * KNN_TC_M * 16,
+              bulk_g2s(sb + p * apart, imgA + (((size_t)qb * 2 + p) * U + ch * ku) * KNN_TC_M * 16,
                        uc * KNN_TC_M * 16u, bar_full(st));
-            bulk_g2s(sb + a_bytes + p * KNN_TC_BPART,
-                     imgB + (((size_t)tile * 2 + p) * U + ch * KNN_TC_KU) * KNN_TC_N * 16,
+            bulk_g2s(sb + a_bytes + p * bpart,
+                     imgB + (((size_t)tile * 2 + p) * U + ch * ku) * KNN_TC_N * 16,
                      uc * KNN_TC_N * 16u, bar_full(st));
           }
-          loads++;
-        };
-        if (resident) {
-          // every MMA of the last query block has been waited for (its tiles
-          // were scanned), so its image can be replaced
-          mbar_expect_tx(bar_a, parts * (unsigned)U * KNN_TC_M * 16u);
-          for (int p = 0; p < parts; p++)
-            bulk_g2s(sm0 + p * KNN_TC_APART, imgA + ((size_t)qb * 2 + p) * U * KNN_TC_M * 16,
-                     (unsigned)U * KNN_TC_M * 16u, bar_a);
-          ok = mbar_wait_or(bar_a, blocks & 1, &gave_up);
         }
-        for (unsigned g = 0; g < (unsigned)(nst - 1) && g < total && ok; g++) load(g);
-        for (unsigned g = 0; g < total && ok; g++, steps++) {
+      }
+    } else if (warp == 8) {
+      if (lane == 0) {  // MMAs
+        bool ok = true;
+        if (resident) ok = mbar_wait_or(bar_a, blocks & 1, &gave_up);
+        for (unsigned g = 0; g < total && ok; g++) {
           const int st = (int)(steps % (unsigned)nst), ch = (int)(g % (unsigned)nch);
           const int ab = (int)(tiles & 1u);
           if (ch == 0 && tiles >= 2)  // the accumulator has been scanned
-            ok = ok && mbar_wait_or(bar_scan(ab), ((tiles >> 1) - 1) & 1, &gave_up);
+            ok = mbar_wait_or(bar_scan(ab), ((tiles >> 1) - 1) & 1, &gave_up);
           ok = ok && mbar_wait_or(bar_full(st), (steps / (unsigned)nst) & 1, &gave_up);
           if (!ok) break;
           tc_fence_after();
           const unsigned sb = st0 + st * st_bytes;
-          const unsigned aa = resident ? sm0 : sb, bb = sb + a_bytes;
-          const int ks = min(KNN_TC_KU, U - ch * KNN_TC_KU) / 2;
+          const unsigned aa = resident ? sm0 + ch * apart : sb, bb = sb + a_bytes;
+          const unsigned alo = resident ? res_part : apart;
+          const int ks = min(ku, U - ch * ku) / 2;
           const unsigned dt = tmem + (unsigned)ab * KNN_TC_N;
           for (int term = 0; term < (three ? 3 : 1); term++) {
             // hi.hi, hi.lo, lo.hi; a K step of 16 dimensions is two units
-            unsigned long long da = umma_desc(aa + (term == 2 ? KNN_TC_APART : 0u), KNN_TC_M * 16, 128);
-            unsigned long long db = umma_desc(bb + (term == 1 ? KNN_TC_BPART : 0u), KNN_TC_N * 16, 128);
+            unsigned long long da = umma_desc(aa + (term == 2 ? alo : 0u), KNN_TC_M * 16, 128);
+            unsigned long long db = umma_desc(bb + (term == 1 ? bpart : 0u), KNN_TC_N * 16, 128);
             for (int s = 0; s < ks; s++) {
               umma_bf16(dt, da, db, idesc, ch > 0 || term > 0 || s > 0 ? 1u : 0u);
               da += 2 * KNN_TC_M;
@@ -493,15 +526,12 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
             }
           }
           umma_commit(bar_free(st));
+          steps++;
           if (ch == nch - 1) {
             umma_commit(bar_acc(ab));
             tiles++;
           }
-          // its stage is free once the MMAs of step g - 1 are done; those of
-          // step g keep the tensor cores busy meanwhile
-          if (g + nst - 1 < total) load(g + nst - 1);
         }
-        if (!ok) gave_up = 1;
       }
     } else {
       const int row = (warp & 3) * 32 + lane, half = warp >> 2;
@@ -511,34 +541,45 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
       float thr = q < n ? -INFINITY : INFINITY;
       int cnt = 0;
       bool ok = true;
+      s_live[t] = -INFINITY;
+      asm volatile("bar.sync 1, %0;" ::"n"(KNN_TC_SCAN) : "memory");  // the scanning warps
       for (int tile = 0; tile < ntile; tile++, tiles++) {
         const int ab = (int)(tiles & 1u);
         ok = __all_sync(0xffffffffu, mbar_wait_or(bar_acc(ab), (tiles >> 1) & 1, &gave_up));
         if (!ok) break;
         tc_fence_after();
+        // L keys of the other half of the query's columns lie above its
+        // threshold: what is not above that is no neighbour either
+        thr = fmaxf(thr, s_live[t ^ 128]);
+        const unsigned tcol = tmem + ((unsigned)((warp & 3) * 32) << 16) +
+                              (unsigned)ab * KNN_TC_N + (unsigned)half * 128u;
+        float v[32], nv[32];
+        __syncwarp();
+        tmem_ld32(tcol, nv);
 #pragma unroll 1
         for (int c0 = 0; c0 < 128; c0 += 32) {
-          float v[32];
+          tmem_wait(nv);
+#pragma unroll
+          for (int h = 0; h < 32; h++) v[h] = nv[h];
           __syncwarp();
-          tmem_ld32(tmem + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)ab * KNN_TC_N +
-                        (unsigned)(half * 128 + c0), v);
+          if (c0 < 96) tmem_ld32(tcol + (unsigned)c0 + 32u, nv);  // in flight meanwhile
           const int j0 = tile * KNN_TC_N + half * 128 + c0;
-          const float4 *o4 = reinterpret_cast<const float4 *>(off + j0);
-          bool any = false;
+          // by all 32 columns, then by fours: a warp seldom has a key to append
+          // once the lists have settled
+          float m4[8];
 #pragma unroll
-          for (int h = 0; h < 8; h++) {
-            const float4 o = __ldg(&o4[h]);
-            v[4 * h] += o.x;
-            v[4 * h + 1] += o.y;
-            v[4 * h + 2] += o.z;
-            v[4 * h + 3] += o.w;
-            any |= v[4 * h] > thr || v[4 * h + 1] > thr || v[4 * h + 2] > thr || v[4 * h + 3] > thr;
-          }
-          if (any) {
+          for (int h = 0; h < 8; h++)
+            m4[h] = fmaxf(fmaxf(v[4 * h], v[4 * h + 1]), fmaxf(v[4 * h + 2], v[4 * h + 3]));
+          const float m32 = fmaxf(fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])),
+                                  fmaxf(fmaxf(m4[4], m4[5]), fmaxf(m4[6], m4[7])));
+          if (!__any_sync(0xffffffffu, m32 > thr)) continue;
 #pragma unroll
-            for (int h = 0; h < 32; h++)
-              if (v[h] > thr) buf[cnt++] = make_float2(v[h], __int_as_float(j0 + h));
-          }
+          for (int h = 0; h < 8; h++)
+            if (__any_sync(0xffffffffu, m4[h] > thr)) {
+#pragma unroll
+              for (int g = 4 * h; g < 4 * h + 4; g++)
+                if (v[g] > thr) buf[cnt++] = make_float2(v[g], __int_as_float(j0 + g));
+            }
           // room for the next 32 columns
           unsigned full = __ballot_sync(0xffffffffu, cnt > CAP - 32);
           while (full) {
@@ -549,7 +590,8 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
             const float nt = knn_select<L, CAP>(wbuf + (size_t)s * CAP, c);
             if (lane == s) {
               cnt = L;
-              thr = nt;
+              thr = fmaxf(thr, nt);
+              s_live[t] = thr;
             }
           }
         }
@@ -589,6 +631,14 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
           T = knn_kth<2 * E>(u, L);
           if (T == 0) T = 1;  // fewer than L entries besides the query
           else tail = fmaxf(tail, knn_unordered(T));
+        }
+        // only a candidate whose key is within the bound of the k-th key can
+        // be among the k nearest (a NaN bound keeps all)
+        const float qn = nrm[q], bound = eps * (qn + cmax);
+        if (have > k) {
+          const unsigned K = knn_kth<2 * E>(u, k);
+          const unsigned cut = K == 0 ? 0u : knn_ordered(knn_unordered(K) - bound);
+          if (bound == bound && cut > T && cut <= K) T = cut;
         }
         int m = 0;
         __syncwarp();
@@ -651,22 +701,21 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
         for (int o = 16; o > 0; o >>= 1) dk = fminf(dk, __shfl_xor_sync(0xffffffffu, dk, o));
         // settled: nothing was dropped, or all that was is farther than the
         // k-th exact distance (false for NaN: such queries are redone too)
-        const float qn = nrm[q];
-        const bool settled =
-            m >= k && (tail == -INFINITY || qn - 2.f * tail - eps * (qn + cmax) > dk);
+        const bool settled = m >= k && (tail == -INFINITY || qn - 2.f * tail - bound > dk);
         if (!settled && lane == 0) redo[atomicAdd(nredo, 1)] = q;
         __syncwarp();
       }
     }
     __syncthreads();  // the lists are free for the next query block
   }
-  if (gave_up && t == KNN_TC_SCAN) {
-    atomicExch(err, 1);
-    // let the copies and MMAs in flight finish before the memory is released:
-    // every load is waited for in order, and a commit covers all MMAs
-    for (unsigned l = steps; l < loads; l++)
-      mbar_wait(bar_full((int)(l % (unsigned)nst)), (l / (unsigned)nst) & 1);
-    if (steps > 0)
+  if (gave_up) {
+    // let the copies and MMAs in flight finish before the memory is released
+    if (t == KNN_TC_SCAN + 32) {
+      atomicExch(err, 1);
+      for (unsigned l = loads > (unsigned)nst ? loads - nst : 0; l < loads; l++)
+        mbar_wait(bar_full((int)(l % (unsigned)nst)), (l / (unsigned)nst) & 1);
+    }
+    if (t == KNN_TC_SCAN && steps > 0)
       mbar_wait(bar_free((int)((steps - 1) % (unsigned)nst)), ((steps - 1) / (unsigned)nst) & 1);
   }
   tc_fence_before();
@@ -695,7 +744,7 @@ static sgt_status knn_simt(sgt_ctx *ctx, int n, int dim, const float *X, int k,
 
 template <int L, int CAP>
 static cudaError_t knn_tc_launch(int nb, cudaStream_t s, const unsigned char *imgA,
-                                 const unsigned char *imgB, const float *nrm, const float *off,
+                                 const unsigned char *imgB, const float *nrm,
                                  const unsigned *nmax, const int *inexact, const float *X, int n,
                                  int dim, int U, int k, float2 *bufs, int *idx, float *d2,
                                  int *redo, int *cnt) {
@@ -703,14 +752,15 @@ static cudaError_t knn_tc_launch(int nb, cudaStream_t s, const unsigned char *im
       k_knn_tc<L, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KNN_TC_SMEM);
   if (e != cudaSuccess) return e;
   k_knn_tc<L, CAP><<<nb, KNN_TC_THREADS, KNN_TC_SMEM, s>>>(
-      imgA, imgB, nrm, off, nmax, inexact, X, n, dim, U, k, bufs, idx, d2, redo, cnt, cnt + 1);
+      imgA, imgB, nrm, nmax, inexact, X, n, dim, U, k, bufs, idx, d2, redo, cnt, cnt + 1);
   return cudaGetLastError();
 }
 
 static sgt_status knn_tc(sgt_ctx *ctx, int n, int dim, const float *X, int k, int *idx,
                          float *d2, int *n_redo) {
   cudaStream_t s = sgti_stream(ctx);
-  const int U = ((dim + 15) / 16) * 2;  // units of 8 dimensions, in pairs (one MMA)
+  // units of 8 dimensions, in pairs (one MMA): the dimensions and three columns
+  const int U = ((dim + 3 + 15) / 16) * 2;
   const int nq = (n + KNN_TC_M - 1) / KNN_TC_M, ntile = (n + KNN_TC_N - 1) / KNN_TC_N;
   const size_t a_bytes = (size_t)nq * 2 * U * KNN_TC_M * 16;
   const size_t b_bytes = (size_t)ntile * 2 * U * KNN_TC_N * 16;
@@ -718,9 +768,8 @@ static sgt_status knn_tc(sgt_ctx *ctx, int n, int dim, const float *X, int k, in
   // list length (neighbours and a margin) and buffer capacity
   const int cap = k <= 32 ? 256 : (k <= 96 ? 384 : 448);
   char *buf = nullptr;
-  const int npad = ntile * KNN_TC_N;
-  const size_t o_nrm = a_bytes + b_bytes, o_off = o_nrm + sizeof(float) * (size_t)npad;
-  const size_t o_buf = o_off + sizeof(float) * (size_t)npad;
+  const size_t o_nrm = a_bytes + b_bytes;
+  const size_t o_buf = o_nrm + sizeof(float) * (((size_t)n + 3) / 4 * 4);
   const size_t o_max = o_buf + sizeof(float2) * (size_t)nb * KNN_TC_SCAN * cap;
   const size_t o_cnt = o_max + 16, o_redo = o_cnt + 16;
   const size_t total = o_redo + sizeof(int) * (size_t)n;
@@ -731,7 +780,7 @@ static sgt_status knn_tc(sgt_ctx *ctx, int n, int dim, const float *X, int k, in
   }
   unsigned char *imgA = reinterpret_cast<unsigned char *>(buf);
   unsigned char *imgB = imgA + a_bytes;
-  float *nrm = reinterpret_cast<float *>(buf + o_nrm), *off = reinterpret_cast<float *>(buf + o_off);
+  float *nrm = reinterpret_cast<float *>(buf + o_nrm);
   float2 *bufs = reinterpret_cast<float2 *>(buf + o_buf);
   unsigned *nmax = reinterpret_cast<unsigned *>(buf + o_max);
   int *inexact = reinterpret_cast<int *>(buf + o_max + 4);
@@ -740,21 +789,20 @@ static sgt_status knn_tc(sgt_ctx *ctx, int n, int dim, const float *X, int k, in
   int hc[2] = {0, 0};
   e = cudaMemsetAsync(buf + o_max, 0, 32, s);
   if (e == cudaSuccess) {
-    k_knn_norms<<<std::min((npad + 255) / 256, 148 * 4), 256, 0, s>>>(X, n, npad, dim, nrm, off,
-                                                                      nmax, inexact);
-    k_knn_split<<<148 * 8, 256, 0, s>>>(X, n, dim, U, KNN_TC_M, nq, (uint4 *)imgA);
-    k_knn_split<<<148 * 8, 256, 0, s>>>(X, n, dim, U, KNN_TC_N, ntile, (uint4 *)imgB);
+    k_knn_norms<<<std::min((n + 255) / 256, 148 * 4), 256, 0, s>>>(X, n, dim, nrm, nmax, inexact);
+    k_knn_split<<<148 * 8, 256, 0, s>>>(X, nrm, n, dim, U, KNN_TC_M, nq, 0, (uint4 *)imgA);
+    k_knn_split<<<148 * 8, 256, 0, s>>>(X, nrm, n, dim, U, KNN_TC_N, ntile, 1, (uint4 *)imgB);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) {
     if (k <= 32)
-      e = knn_tc_launch<64, 256>(nb, s, imgA, imgB, nrm, off, nmax, inexact, X, n, dim, U, k, bufs,
+      e = knn_tc_launch<64, 256>(nb, s, imgA, imgB, nrm, nmax, inexact, X, n, dim, U, k, bufs,
                                  idx, d2, redo, cnt);
     else if (k <= 96)
-      e = knn_tc_launch<128, 384>(nb, s, imgA, imgB, nrm, off, nmax, inexact, X, n, dim, U, k,
+      e = knn_tc_launch<128, 384>(nb, s, imgA, imgB, nrm, nmax, inexact, X, n, dim, U, k,
                                   bufs, idx, d2, redo, cnt);
     else
-      e = knn_tc_launch<192, 448>(nb, s, imgA, imgB, nrm, off, nmax, inexact, X, n, dim, U, k,
+      e = knn_tc_launch<192, 448>(nb, s, imgA, imgB, nrm, nmax, inexact, X, n, dim, U, k,
                                   bufs, idx, d2, redo, cnt);
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, s);
