@@ -628,17 +628,16 @@ static sgt_status enqueue_g2g(sgt_job *J, cudaStream_t s, bool pdl) {
 // Centre Ynext into Y; scatter mode: S2G into the grid copies, cell mode:
 // count points per cell and zero the charge grid.
 template <int D>
-static sgt_status enqueue_bin_count(sgt_job *J, cudaStream_t s) {
+static sgt_status enqueue_bin_count(sgt_job *J, cudaStream_t s, bool pdl) {
   sgt_ctx *ctx = J->ctx;
   typedef typename Vec<D>::T VT;
   typedef typename Node<D>::T NT;
   if (J->jp.cell_blocks > 0)
-    k_bin_count<D><<<J->jp.cell_blocks, SGT_THREADS, 0, s>>>(
-        (const VT *)J->Ynext, (VT *)J->Y, J->n, J->st, J->tile_count, (NT *)J->V, J->jp, J->cursor,
-        J->chunks, J->nb_s2gc);
-  k_scatter<D><<<J->nb_scat, SGT_THREADS, 0, s>>>((const VT *)J->Ynext, (VT *)J->Y, J->n, J->st,
-                                                  (NT *)J->Vc);
-  CK(cudaGetLastError());
+    CK(launch_chain(pdl, k_bin_count<D>, J->jp.cell_blocks, SGT_THREADS, 0, s,
+                    (const VT *)J->Ynext, (VT *)J->Y, J->n, J->st, J->tile_count, (NT *)J->V,
+                    J->jp, J->cursor, J->chunks, J->nb_s2gc));
+  CK(launch_chain(pdl, k_scatter<D>, J->nb_scat, SGT_THREADS, 0, s, (const VT *)J->Ynext,
+                  (VT *)J->Y, J->n, J->st, (NT *)J->Vc));
   return SGT_OK;
 }
 
@@ -698,7 +697,7 @@ static sgt_status enqueue_repulsion_rest(sgt_job *J, cudaStream_t s, cudaEvent_t
 
 template <int D>
 static sgt_status enqueue_repulsion(sgt_job *J, cudaStream_t s, cudaEvent_t *ev = nullptr) {
-  CKS(enqueue_bin_count<D>(J, s));
+  CKS(enqueue_bin_count<D>(J, s, ev == nullptr));
   return enqueue_repulsion_rest<D>(J, s, ev);
 }
 
@@ -767,7 +766,7 @@ static sgt_status enqueue_iteration(sgt_job *J, cudaStream_t s) {
   CK(cudaStreamWaitEvent(ctx->side, J->ev_fork, 0));
   CKS(dispatch_attractive<D>(J, ctx->side));
   CK(cudaEventRecord(J->ev_join, ctx->side));
-  CKS(enqueue_bin_count<D>(J, s));
+  CKS(enqueue_bin_count<D>(J, s, true));
   CKS(enqueue_repulsion_rest<D>(J, s));
   CK(cudaStreamWaitEvent(s, J->ev_join, 0));
   return enqueue_combine<D>(J, s);
@@ -1995,7 +1994,7 @@ static sgt_status shard_scatter_d(sgt_shard *sh) {
   CK(cudaEventRecord(J->ev_join, ctx->side));
   // every float of the buffer is reduced: clear what this grid does not use
   CK(cudaMemsetAsync(sh->grid, 0, sizeof(float) * sh->grid_floats, s));
-  CKS(enqueue_bin_count<D>(J, s));
+  CKS(enqueue_bin_count<D>(J, s, false));
   return enqueue_scatter_part<D>(J, s);
 }
 
