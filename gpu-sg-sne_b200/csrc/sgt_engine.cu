@@ -98,7 +98,7 @@ struct sgt_job {
   int nb_pts = 0, nb_scat = 0, nb_gath = 0, nb_spec = 0, nb_spec_y = 0, nb_conv = 0, nb_s2gc = 0, nb_g2s = 0, nb_fft = 0, nb_fft_rows = 0, nb_row = 0,
       nb_upd = 0, nb_part = 0;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;  // the two branches of an iteration
-  size_t smem_fft1 = 0, smem_fft2 = 0;
+  size_t smem_fft2 = 0;
   cudaGraphExec_t gexec = nullptr;        // one iteration
   cudaGraphExec_t gexec_multi = nullptr;  // SGT_GRAPH_ITERS chained iterations
   std::vector<void *> allocs;
@@ -405,7 +405,6 @@ static sgt_status job_shapes(sgt_job *J) {
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_s2g_cell<D>, SGT_THREADS, 0));
   J->nb_s2gc = grid_blocks(nsm, occ);
   const int M = J->mmax;
-  J->smem_fft1 = 0;
   J->smem_fft2 = fft_cols_smem(M);
   // spectra of the rows, and sums over the rows: a block per row (tile) of
   // the largest grid they take
@@ -430,15 +429,8 @@ static sgt_status job_shapes(sgt_job *J) {
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fft_build_x<D>, SGT_THREADS, 0));
     J->nb_fft_rows = grid_blocks(nsm, occ);
   }
-  occ = 0;
-  switch (J->G) {
-    case 4: CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_row_update<D, 4, true>, SGT_THREADS, 0)); break;
-    case 8: CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_row_update<D, 8, true>, SGT_THREADS, 0)); break;
-    case 16: CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_row_update<D, 16, true>, SGT_THREADS, 0)); break;
-    default: CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_row_update<D, 32, true>, SGT_THREADS, 0)); break;
-  }
-  J->nb_row = grid_blocks(nsm, occ);
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_row_update<D, 1, false>, SGT_THREADS, 0));
+  J->nb_row = J->nb_pts;  // the KL sum
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_row_update<D>, SGT_THREADS, 0));
   J->nb_upd = grid_blocks(nsm, occ);
   // A job whose SpMV is large runs its repulsion chain beside an SpMV that
   // holds every SM: a chain kernel's blocks start only as SpMV blocks retire,
@@ -745,8 +737,8 @@ template <int D>
 static sgt_status enqueue_combine(sgt_job *J, cudaStream_t s) {
   sgt_ctx *ctx = J->ctx;
   typedef typename Vec<D>::T VT;
-  k_row_update<D, 1, false><<<J->nb_upd, SGT_THREADS, 0, s>>>(
-      nullptr, nullptr, (const VT *)J->Fattr, (const VT *)J->Y, (const VT *)J->Frep,
+  k_row_update<D><<<J->nb_upd, SGT_THREADS, 0, s>>>(
+      (const VT *)J->Fattr, (const VT *)J->Y, (const VT *)J->Frep,
       (VT *)J->uY, (VT *)J->gains, (VT *)J->Ynext, J->st, J->jp, J->part_min, J->part_max,
       J->part_sum);
   CK(cudaGetLastError());

@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(SGT_THREADS)
 km_row_update(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
   SGT_MULTI_JOB
   typedef typename Vec<D>::T VT;
-  k_row_update_body<D, 1, false>(vb, vg, nullptr, nullptr, (const VT *)v.Fattr, (const VT *)v.Y,
-                                 (const VT *)v.Frep, (VT *)v.uY, (VT *)v.gains, (VT *)v.Ynext,
-                                 v.st, v.jp, v.part_min, v.part_max, v.part_sum);
+  k_row_update_body<D>(vb, vg, (const VT *)v.Fattr, (const VT *)v.Y, (const VT *)v.Frep,
+                       (VT *)v.uY, (VT *)v.gains, (VT *)v.Ynext, v.st, v.jp, v.part_min,
+                       v.part_max, v.part_sum);
 }

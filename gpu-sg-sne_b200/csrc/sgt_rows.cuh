@@ -81,19 +81,20 @@ __device__ __forceinline__ float sgn_f(float x) {
 }
 
 // ---------------------------------------------------------------------------
-// Fused iteration row kernel.  FUSED: compute F_attr from CSR; otherwise read
-// it from Fattr (COO / ELL formats).  Writes Ynext, uY, gains; the last CTA
-// turns the per-block min/max/sum of Ynext into the next grid decision.
+// Forces and update, a point per thread: dY, gains, momentum, Ynext; the last
+// block turns the per-block min/max/sum of Ynext into the next grid decision.
+// Bound by memory at large n (64 n S bytes: 1.3M points in 20 us), by the
+// chain of the finish at small (7 us).
 // ---------------------------------------------------------------------------
-template <int D, int G, bool FUSED>
-__device__ __forceinline__ void k_row_update_body(int vb_, int vg_, const int *__restrict__ rowptr, const int2 *__restrict__ pairs,
+template <int D>
+__device__ __forceinline__ void k_row_update_body(int vb_, int vg_,
              const typename Vec<D>::T *__restrict__ Fattr,
              const typename Vec<D>::T *__restrict__ Y,
              const typename Vec<D>::T *__restrict__ Frep_un,
              typename Vec<D>::T *__restrict__ uY,
              typename Vec<D>::T *__restrict__ gains,
              typename Vec<D>::T *__restrict__ Ynext, SgtState *st,
-             SgtJobParams jp, float4 *part_min, float4 *part_max,
+             const SgtJobParams &jp, float4 *part_min, float4 *part_max,
              double *part_sum) {
   const int n = jp.n;
   const int iter = st->iter;
@@ -103,81 +104,29 @@ __device__ __forceinline__ void k_row_update_body(int vb_, int vg_, const int *_
   const float Zf = (float)st->Z;
   float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
   double sm[3] = {0, 0, 0};
-  const int lane = threadIdx.x % G;
-  const int grp = (vb_ * blockDim.x + threadIdx.x) / G;
-  const int ngrp = vg_ * blockDim.x / G;
-  // uniform trip count per warp so the group shuffles stay converged
-  const int rounds = (n + ngrp - 1) / ngrp;
-  // the next row's extents are loaded one round ahead
-  int nb_s = 0, nb_e = 0;
-  if (FUSED && grp < n) {
-    nb_s = __ldcs(&rowptr[grp]);
-    nb_e = __ldcs(&rowptr[grp + 1]);
-  }
-  for (int r = 0; r < rounds; r++) {
-    const int i = grp + r * ngrp;
-    const bool valid = i < n;
-    const int rs = nb_s, re = nb_e;
-    if (FUSED && i + ngrp < n) {
-      nb_s = __ldcs(&rowptr[i + ngrp]);
-      nb_e = __ldcs(&rowptr[i + ngrp + 1]);
+  for (int i = vb_ * blockDim.x + threadIdx.x; i < n; i += vg_ * blockDim.x) {
+    const typename Vec<D>::T yi = Y[i], fa = Fattr[i], fr = __ldcs(&Frep_un[i]);
+    typename Vec<D>::T u = __ldcs(&uY[i]), g = __ldcs(&gains[i]), yn = yi;
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+      const float frep = comp<D>(fr, k) / Zf;
+      const float dy = alpha * comp<D>(fa, k) - frep;
+      float gk = comp<D>(g, k), uk = comp<D>(u, k);
+      gk = (sgn_f(dy) != sgn_f(uk)) ? (float)((double)gk + 0.2) : (float)((double)gk * 0.8);
+      if ((double)gk < 0.01) gk = (float)0.01;
+      uk = mom * uk - eta * gk * dy;
+      const float y = comp<D>(yi, k) + uk;
+      setcomp<D>(g, k, gk);
+      setcomp<D>(u, k, uk);
+      setcomp<D>(yn, k, y);
+      mn[k] = fminf(mn[k], y);
+      mx[k] = fmaxf(mx[k], y);
+      sm[k] += (double)y;
     }
-    typename Vec<D>::T yi, fr, u, g;
-    if (valid) {
-      yi = Y[i];
-      if (lane == 0) {  // update operands, independent of the row sum
-        fr = __ldcs(&Frep_un[i]);
-        u = __ldcs(&uY[i]);
-        g = __ldcs(&gains[i]);
-      }
-    }
-    float acc[3] = {0.f, 0.f, 0.f};
-    if (FUSED) {
-      if (valid) {
-        constexpr int U = 4;
-        for (int t0 = rs + lane; t0 < re; t0 += U * G) {
-          int2 pr[U];
-#pragma unroll
-          for (int q = 0; q < U; q++) {
-            const int t = t0 + q * G;
-            pr[q] = t < re ? __ldcs(&pairs[t]) : make_int2(i, 0);
-          }
-          typename Vec<D>::T yj[U];
-#pragma unroll
-          for (int q = 0; q < U; q++) yj[q] = __ldg(&Y[pr[q].x]);
-#pragma unroll
-          for (int q = 0; q < U; q++) attr_term<D>(yi, yj[q], __int_as_float(pr[q].y), acc);
-        }
-      }
-      group_reduce<D, G>(acc);
-    } else if (valid) {
-      const typename Vec<D>::T fa = Fattr[i];
-#pragma unroll
-      for (int k = 0; k < D; k++) acc[k] = comp<D>(fa, k);
-    }
-    if (valid && lane == 0) {
-      typename Vec<D>::T yn = yi;
-#pragma unroll
-      for (int k = 0; k < D; k++) {
-        const float frep = comp<D>(fr, k) / Zf;
-        const float dy = alpha * acc[k] - frep;
-        float gk = comp<D>(g, k), uk = comp<D>(u, k);
-        gk = (sgn_f(dy) != sgn_f(uk)) ? (float)((double)gk + 0.2) : (float)((double)gk * 0.8);
-        if ((double)gk < 0.01) gk = (float)0.01;
-        uk = mom * uk - eta * gk * dy;
-        const float y = comp<D>(yi, k) + uk;
-        setcomp<D>(g, k, gk);
-        setcomp<D>(u, k, uk);
-        setcomp<D>(yn, k, y);
-        mn[k] = fminf(mn[k], y);
-        mx[k] = fmaxf(mx[k], y);
-        sm[k] += (double)y;
-      }
-      if constexpr (D == 3) { u.w = 0.f; g.w = 0.f; yn.w = 0.f; }
-      __stcs(&uY[i], u);
-      __stcs(&gains[i], g);
-      Ynext[i] = yn;
-    }
+    if constexpr (D == 3) { u.w = 0.f; g.w = 0.f; yn.w = 0.f; }
+    __stcs(&uY[i], u);
+    __stcs(&gains[i], g);
+    Ynext[i] = yn;
   }
   if (block_finish_stats<D>(vb_, vg_, st, jp, &st->done_row, true, mn, mx, sm, part_min, part_max,
                             part_sum)) {
@@ -189,10 +138,9 @@ __device__ __forceinline__ void k_row_update_body(int vb_, int vg_, const int *_
     st->iter = iter + 1;
   }
 }
-template <int D, int G, bool FUSED>
+template <int D>
 __global__ void __launch_bounds__(SGT_THREADS)
-k_row_update(const int *__restrict__ rowptr, const int2 *__restrict__ pairs,
-             const typename Vec<D>::T *__restrict__ Fattr,
+k_row_update(const typename Vec<D>::T *__restrict__ Fattr,
              const typename Vec<D>::T *__restrict__ Y,
              const typename Vec<D>::T *__restrict__ Frep_un,
              typename Vec<D>::T *__restrict__ uY,
@@ -200,7 +148,8 @@ k_row_update(const int *__restrict__ rowptr, const int2 *__restrict__ pairs,
              typename Vec<D>::T *__restrict__ Ynext, SgtState *st,
              SgtJobParams jp, float4 *part_min, float4 *part_max,
              double *part_sum) {
-  k_row_update_body<D, G, FUSED>(blockIdx.x, gridDim.x, rowptr, pairs, Fattr, Y, Frep_un, uY, gains, Ynext, st, jp, part_min, part_max, part_sum);
+  k_row_update_body<D>(blockIdx.x, gridDim.x, Fattr, Y, Frep_un, uY, gains, Ynext, st, jp,
+                       part_min, part_max, part_sum);
 }
 
 
