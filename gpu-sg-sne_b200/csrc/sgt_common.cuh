@@ -88,7 +88,7 @@ struct SgtJobParams {
   int mmax;           // largest FFT length per axis allocated
   long vc_nodes;      // nodes held by the grid copies of the scatter mode
   int chunk_cap;      // max chunks held by the chunk array
-  int chunk_min;      // fewest points per S2G chunk (0: 1024, 256 in 3-D)
+  int chunk_min;      // cell mode: fewest points per chunk (0: 1024, 256 in 3-D)
   int conv_max;       // largest N that k_spec_* convolve
   int cell_blocks;    // blocks that work in cell mode (0: no cell mode)
 };

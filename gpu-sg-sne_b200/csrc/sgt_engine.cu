@@ -34,6 +34,8 @@ struct sgt_ctx {
   // repulsion chain on `stream` (forked and joined with events, so captured
   // graphs get two parallel branches)
   cudaStream_t side = nullptr;
+  // second branch stream: the FFT passes beside the small-grid convolution
+  cudaStream_t side2 = nullptr;
   int nsm = 148;
   std::string err;
   sgt_job *scratch = nullptr;  // buffers of the operator entry points
@@ -98,6 +100,7 @@ struct sgt_job {
   int nb_pts = 0, nb_scat = 0, nb_gath = 0, nb_spec = 0, nb_spec_y = 0, nb_conv = 0, nb_s2gc = 0, nb_g2s = 0, nb_fft = 0, nb_fft_rows = 0, nb_row = 0,
       nb_upd = 0, nb_part = 0;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;  // the two branches of an iteration
+  cudaEvent_t ev_fft = nullptr, ev_fft_done = nullptr;  // the FFT branch of the repulsion
   size_t smem_fft2 = 0;
   cudaGraphExec_t gexec = nullptr;        // one iteration
   cudaGraphExec_t gexec_multi = nullptr;  // SGT_GRAPH_ITERS chained iterations
@@ -174,6 +177,9 @@ static int grid_blocks(int nsm, int per_sm) { return std::max(1, nsm * std::max(
 // nodes of the grid copies a job holds at least (32 copies of a 90^2 grid; the
 // largest 2-D grid once)
 #define SGT_COPY_NODES (1 << 18)
+// nonzeros of P from which the SpMV outlasts a small job's repulsion chain
+// (15 us) and blocks beside it wait for slots
+#define SGT_LONG_SPMV_NNZ 3000000L
 // nonzeros of P from which a job's repulsion chain runs one block per SM
 #define SGT_CHAIN_NARROW_NNZ 16000000L
 
@@ -253,6 +259,7 @@ sgt_status sgt_create(int device, sgt_ctx **out) {
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->side2, cudaStreamNonBlocking);
   if (e == cudaSuccess) {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
@@ -267,6 +274,7 @@ sgt_status sgt_create(int device, sgt_ctx **out) {
   if (e != cudaSuccess) {
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     if (ctx->side) cudaStreamDestroy(ctx->side);
+    if (ctx->side2) cudaStreamDestroy(ctx->side2);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return SGT_ERR_CUDA;
@@ -296,6 +304,7 @@ void sgt_destroy(sgt_ctx *ctx) {
     cudaMemPoolDestroy(ctx->pool);
   }
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
+  if (ctx->side2) cudaStreamDestroy(ctx->side2);
   if (ctx->side) cudaStreamDestroy(ctx->side);
   delete ctx;
 }
@@ -415,7 +424,7 @@ static sgt_status job_shapes(sgt_job *J) {
   const int cm = J->jp.conv_max, ct = (cm + SGT_SPEC_TY(D) - 1) / SGT_SPEC_TY(D);
   // (few blocks beside a long SpMV: even a block with nothing to do waits for
   // a slot there)
-  const bool beside = J->nnz >= 3000000L;
+  const bool beside = J->nnz >= SGT_LONG_SPMV_NNZ;
   J->nb_spec = D == 1 ? 2 : (D == 3 ? std::min(4 * nsm, cm * cm) : (beside ? 64 : cm));
   J->nb_spec_y = 2 * nsm;
   J->nb_conv = D == 1 ? (cm + 7) / 8 : (D == 3 ? std::min(3 * nsm, cm * ct) : std::min(ct, beside ? 64 : cm));
@@ -479,8 +488,7 @@ static sgt_status job_alloc(sgt_job *J) {
   CKS(jalloc(J, &J->gains, np));
   CKS(jalloc(J, &J->Frep, np));
   int max_grid = J->p.max_grid > 0 ? J->p.max_grid : (D <= 2 ? 512 : 128);
-  // 3-D: at most 256 points per axis (tile histogram of 16^3 entries,
-  // FFT planes of 512^3)
+  // 3-D: at most 256 points per axis (FFT planes of 512^3)
   max_grid = std::min(D == 3 ? 256 : 512, std::max(16, max_grid));
   int M = 1;
   while (M < 2 * max_grid - 1) M <<= 1;
@@ -514,6 +522,8 @@ static sgt_status job_alloc(sgt_job *J) {
   J->st_host = new SgtState();
   CK(cudaEventCreateWithFlags(&J->ev_fork, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&J->ev_join, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&J->ev_fft, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&J->ev_fft_done, cudaEventDisableTiming));
   CK(cudaMemsetAsync(J->tile_count, 0, sizeof(int) * SGT_HIST_MAX, ctx->stream));
   CK(cudaMemsetAsync(J->st, 0, sizeof(SgtState), ctx->stream));
   return SGT_OK;
@@ -593,8 +603,10 @@ static cudaError_t launch_chain(bool pdl, void (*k)(KArgs...), int grid, int blo
   return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
+// The convolution of the grids that k_spec_* take (the kernels return at once
+// on larger ones).
 template <int D>
-static sgt_status enqueue_g2g(sgt_job *J, cudaStream_t s, bool pdl) {
+static sgt_status enqueue_g2g_small(sgt_job *J, cudaStream_t s, bool pdl) {
   sgt_ctx *ctx = J->ctx;
   typedef typename Node<D>::T NT;
   if constexpr (D == 3) {
@@ -603,9 +615,16 @@ static sgt_status enqueue_g2g(sgt_job *J, cudaStream_t s, bool pdl) {
   }
   CK(launch_chain(pdl, k_spec_cols<D>, J->nb_conv, SGT_THREADS, 0, s, (const SgtState *)J->st,
                   (const NT *)J->V, (const float2 *)J->W, (NT *)J->Phi));
-  if (J->nmax <= J->jp.conv_max) return SGT_OK;  // no grid of this job takes the FFT passes
+  return SGT_OK;
+}
+
+// The FFT passes of the larger grids (returning at once on the others).
+template <int D>
+static sgt_status enqueue_g2g_fft(sgt_job *J, cudaStream_t s, bool first_pdl, bool pdl) {
+  sgt_ctx *ctx = J->ctx;
+  typedef typename Node<D>::T NT;
   if constexpr (D >= 2) {
-    CK(launch_chain(pdl, k_fft_build_x<D>, J->nb_fft_rows, SGT_THREADS, 0, s,
+    CK(launch_chain(first_pdl, k_fft_build_x<D>, J->nb_fft_rows, SGT_THREADS, 0, s,
                     (const SgtState *)J->st, (const NT *)J->V, J->W));
     if constexpr (D == 3)
       CK(launch_chain(pdl, k_fft_cols<D, MODE_MID_FWD>, J->nb_fft, SGT_THREADS, J->smem_fft2, s,
@@ -618,6 +637,21 @@ static sgt_status enqueue_g2g(sgt_job *J, cudaStream_t s, bool pdl) {
     CK(launch_chain(pdl, k_fft_final_x<D>, J->nb_fft_rows, SGT_THREADS, 0, s,
                     (const SgtState *)J->st, (const float2 *)J->W, (NT *)J->Phi));
   }
+  return SGT_OK;
+}
+
+// G2S after one of the convolutions, or after both on one stream
+template <int D>
+static sgt_status enqueue_g2s(sgt_job *J, cudaStream_t s, bool pdl, int after) {
+  sgt_ctx *ctx = J->ctx;
+  typedef typename Vec<D>::T VT;
+  typedef typename Node<D>::T NT;
+  if (J->jp.cell_blocks > 0)
+    CK(launch_chain(pdl, k_g2s<D>, J->nb_g2s, SGT_THREADS, 0, s, (const float4 *)J->sorted, J->st,
+                    (const int4 *)J->chunks, (const NT *)J->Phi, (VT *)J->Frep, J->part_z, J->n,
+                    after));
+  CK(launch_chain(pdl, k_gather<D>, J->nb_gath, SGT_THREADS, 0, s, J->st, (const NT *)J->Phi,
+                  (VT *)J->Frep, J->part_z, J->n, (const VT *)J->Y, after));
   return SGT_OK;
 }
 
@@ -666,25 +700,37 @@ static sgt_status enqueue_scatter_part(sgt_job *J, cudaStream_t s, cudaEvent_t *
 template <int D>
 static sgt_status enqueue_gather_part(sgt_job *J, cudaStream_t s, cudaEvent_t *ev = nullptr) {
   sgt_ctx *ctx = J->ctx;
-  typedef typename Vec<D>::T VT;
   typedef typename Node<D>::T NT;
   const bool pdl = ev == nullptr;
   if (J->Ygather)  // a shard: the grid has been summed over the ranks meanwhile
     CK(launch_chain(false, k_spec_rows<D>, J->nb_spec, SGT_THREADS, 0, s, (const SgtState *)J->st,
                     (NT *)J->Vc, (NT *)J->V, J->W, SGT_SPEC_TRANSFORM));
-  CKS(enqueue_g2g<D>(J, s, pdl));
+  const bool fft = J->nmax > J->jp.conv_max;  // some grid of this job takes the FFT passes
+  if (fft && !ev && J->ev_fft && J->nnz < SGT_LONG_SPMV_NNZ) {
+    // The two convolutions, each with its G2S, on branches of their own: the
+    // kernels of the one that this grid does not take return at once, and
+    // launched in turn those empty launches cost 2.5 us of a 28 us iteration
+    // (10k points 28.7 -> 26.0 us).  Beside a long SpMV a third branch costs
+    // more than it hides: 60k points, 9.8M nonzeros 64 -> 67 us.
+    CK(cudaEventRecord(J->ev_fft, s));
+    CK(cudaStreamWaitEvent(ctx->side2, J->ev_fft, 0));
+    CKS(enqueue_g2g_fft<D>(J, ctx->side2, false, pdl));
+    CKS(enqueue_g2s<D>(J, ctx->side2, pdl, SGT_G2S_FFT));
+    CK(cudaEventRecord(J->ev_fft_done, ctx->side2));
+    CKS(enqueue_g2g_small<D>(J, s, pdl));
+    CKS(enqueue_g2s<D>(J, s, pdl, SGT_G2S_SMALL));
+    CK(cudaStreamWaitEvent(s, J->ev_fft_done, 0));
+    return SGT_OK;
+  }
+  CKS(enqueue_g2g_small<D>(J, s, pdl));
+  if (fft) CKS(enqueue_g2g_fft<D>(J, s, pdl, pdl));
   if (ev) CK(cudaEventRecord(ev[3], s));
-  if (J->jp.cell_blocks > 0)
-    CK(launch_chain(pdl, k_g2s<D>, J->nb_g2s, SGT_THREADS, 0, s, (const float4 *)J->sorted, J->st,
-                    (const int4 *)J->chunks, (const NT *)J->Phi, (VT *)J->Frep, J->part_z, J->n));
-  CK(launch_chain(pdl, k_gather<D>, J->nb_gath, SGT_THREADS, 0, s, J->st, (const NT *)J->Phi,
-                  (VT *)J->Frep, J->part_z, J->n, (const VT *)J->Y));
-  CK(cudaGetLastError());
+  CKS(enqueue_g2s<D>(J, s, pdl, SGT_G2S_BOTH));
   return SGT_OK;
 }
 
-// The rest of the repulsion: tile offsets, sort, S2G, G2G, G2S and Z.
-// ev (optional): events recorded after the binning, S2G and G2G stages.
+// The rest of the repulsion: (cell mode) sort and S2G, then G2G, G2S and Z.
+// ev (optional): events recorded after the sort, S2G and G2G stages.
 template <int D>
 static sgt_status enqueue_repulsion_rest(sgt_job *J, cudaStream_t s, cudaEvent_t *ev = nullptr) {
   CKS(enqueue_scatter_part<D>(J, s, ev));
@@ -1269,6 +1315,8 @@ void sgt_job_destroy(sgt_job *J) {
   delete J->st_host;
   if (J->ev_fork) cudaEventDestroy(J->ev_fork);
   if (J->ev_join) cudaEventDestroy(J->ev_join);
+  if (J->ev_fft) cudaEventDestroy(J->ev_fft);
+  if (J->ev_fft_done) cudaEventDestroy(J->ev_fft_done);
   delete J;
 }
 
@@ -2193,7 +2241,7 @@ size_t sgt_job_footprint(const sgt_params *p, int n, long nnz) {
   b += 2 * nodes * (D == 1 ? 2 : 4) * 4;                       // V, Phi
   b += std::max<size_t>(nodes, SGT_COPY_NODES) * (D == 1 ? 2 : 4) * 4;  // grid copies
   if (D >= 2) b += 3 * plane * 8;                               // FFT planes
-  b += 2 * 4096 * 4 + ((size_t)n / 256 + 4096 + 16) * 16;        // tiles, chunks
+  b += 2 * 4096 * 4 + ((size_t)n / 256 + 4096 + 16) * 16;        // cells, chunks
   const size_t parts = std::max<size_t>(148 * 16, ((size_t)n * 32 + 255) / 256);
   b += parts * (16 + 16 + 32 + 8 + 8) + 1024;                   // partials, state
   b += ((size_t)n + 1) * 4;                                     // rowptr
@@ -2477,7 +2525,7 @@ sgt_status sgt_last_grids(sgt_ctx *ctx, float *v_grid, float *phi_grid) {
   if (d >= 3) nodes *= N;
   std::vector<float> tmp(nodes * nc);
   // reported as charges [1, y - c] and their potentials, c the grid's middle;
-  // held about the nodes (the potentials only after a direct convolution),
+  // held about the nodes (the potentials only after the small-grid convolution),
   // in cells
   const SgtState &hs = *J->st_host;
   const double mid = 0.5 * (N - 1), hd = hs.h_eff;

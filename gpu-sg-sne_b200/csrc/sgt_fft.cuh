@@ -6,9 +6,11 @@
 // the sum of those terms is exactly the aperiodic convolution.  Here the
 // same convolution is one cyclic convolution of length M >= 2N-1 per axis
 // (the smallest M = 2^k or 3 * 2^k): output nodes x < N only meet kernel
-// offsets |x - x'| <= N-1 <= M/2, so K_c[r] = K(min(r, M-r)) reproduces it.  Two real charge channels ride in
-// one complex plane (K_c is real and even, so its transform is real and the
-// channels separate after the inverse).
+// offsets |x - x'| <= N-1 <= M/2, so K_c[r] = K(min(r, M-r)) reproduces it.
+// Two real charge channels ride in one complex plane (K_c is real and even,
+// so its transform is real and the channels separate after the inverse).
+// Grids up to SgtJobParams::conv_max points per axis take plain transforms of
+// length 2N instead (the k_spec kernels at the end of this file).
 //
 // FFTs are register-resident: one warp owns one line of M <= 1024 points, a
 // lane holds the E = M/32 points lane + 32 e; butterflies whose span holds

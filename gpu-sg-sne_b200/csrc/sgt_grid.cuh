@@ -285,7 +285,7 @@ k_init_stats(const typename Vec<D>::T *__restrict__ Y, int n, SgtState *st,
 }
 
 // ---------------------------------------------------------------------------
-// bin scan (run by the last block of bin_count): tile offsets and the chunk
+// bin scan (run by the last block of bin_count): cell offsets and the chunk
 // work list
 // ---------------------------------------------------------------------------
 // exclusive scan over the threads of a block (blockDim a multiple of 32)
@@ -316,7 +316,7 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *total) {
   return excl;
 }
 
-// Thread t owns the tiles [t per, t per + per); the counts (written by other
+// Thread t owns the cells [t per, t per + per); the counts (written by other
 // blocks' atomics) are read from L2.
 __device__ __forceinline__ void bin_scan_block(SgtState *st, const SgtJobParams &jp,
                                                int *__restrict__ tile_count,
@@ -375,7 +375,7 @@ __device__ __forceinline__ void bin_scan_block(SgtState *st, const SgtJobParams 
 // q >> 2), and every lane works out the point's weights for itself.
 // Bound by the reductions L2 takes: 100k points on 64^2 nodes 10.5 us (1.6M
 // 16-byte node updates), on 117^2 10.3 us, 400k on 512^2 31 us.  In the
-// sorted form this replaces, a tile of the grid in shared memory took 200 to
+// sorted form it took over from, a tile of the grid in shared memory took 200 to
 // 420 us where clustered points met on few nodes: shared-memory float adds
 // are compare-and-swap loops there.
 // ---------------------------------------------------------------------------
@@ -488,9 +488,9 @@ __device__ __forceinline__ void k_bin_count_body(int vb_, int vg_, const typenam
        g += (long)vg_ * blockDim.x)
     V[g] = z;
   __syncthreads();
-  // warp-uniform trip count: lanes with the same tile are merged with
+  // warp-uniform trip count: lanes with the same cell are merged with
   // match_any and add their count in one shared-memory atomic (points of an
-  // embedding cluster on few tiles).  A warp takes SGT_PTS_U runs of 32
+  // embedding cluster in few cells).  A warp takes SGT_PTS_U runs of 32
   // points per round and issues all their loads before the first use.
   const int lane = threadIdx.x & 31;
   constexpr int U = SGT_PTS_U;
@@ -525,7 +525,7 @@ __device__ __forceinline__ void k_bin_count_body(int vb_, int vg_, const typenam
   __syncthreads();
   for (int t = threadIdx.x; t < ntiles; t += blockDim.x)
     if (hist[t]) atomicAdd(&tile_count[t], hist[t]);
-  // the last block to finish turns the tile counts into tile offsets and
+  // the last block to finish turns the cell counts into cell offsets and
   // the chunk list (no separate launch between the count and the sort)
   // (the barrier orders the block's count atomics before thread 0's
   // device-scope fence, which is cumulative over them)
@@ -554,8 +554,8 @@ k_bin_count(const typename Vec<D>::T *__restrict__ Ynext,
 
 // ---------------------------------------------------------------------------
 // bin_scatter: counting-sort points into cell order (cell mode).  Each CTA owns a
-// contiguous range; it counts per tile, reserves its slots with one global
-// atomic per touched tile, then places its points.
+// contiguous range; it counts per cell, reserves its slots with one global
+// atomic per touched cell, then places its points.
 // sorted[p] = the point's places in its cell per axis, and its index in the .w
 // bits: S2G and G2S know the cell from the chunk and need not work it out again
 // (s2g and g2s of 1.3M points 29.5 + 38 us with coordinates).
@@ -576,7 +576,7 @@ __device__ __forceinline__ void k_bin_scatter_body(int vb_, int vg_, const typen
   const int lo = vb_ * per, hi = min(n, lo + per);
   for (int t = threadIdx.x; t < ntiles; t += blockDim.x) lc[t] = 0;
   __syncthreads();
-  // warp-uniform trip counts; lanes of one tile are merged with match_any,
+  // warp-uniform trip counts; lanes of one cell are merged with match_any,
   // the group leader does the shared-memory atomic and the lanes take
   // consecutive slots in lane order.  A warp takes SGT_PTS_U runs of 32
   // points per round and issues all their loads before the first use.
@@ -803,6 +803,15 @@ __device__ __forceinline__ double point_force(const float *p, const float *m, fl
   return (double)p[0] + 2.0 * (double)h * (double)h * dot;
 }
 
+// Which convolution's potentials a G2S launch gathers; the other launch of the
+// iteration returns at once.
+#define SGT_G2S_BOTH 0
+#define SGT_G2S_SMALL 1
+#define SGT_G2S_FFT 2
+__device__ __forceinline__ bool g2s_skips(const SgtState *st, int after) {
+  return after != SGT_G2S_BOTH && (after == SGT_G2S_SMALL) != (st->direct != 0);
+}
+
 // Z of a G2S launch: the block's FP64 partial, then the last block to finish
 // sums the partials in block order and writes Z = sum - n.
 __device__ __forceinline__ void g2s_finish(int vb_, int vg_, SgtState *st, double *part_z, int n,
@@ -848,9 +857,9 @@ __device__ __forceinline__ void k_gather_body(int vb_, int vg_, SgtState *st,
                                               const typename Node<D>::T *__restrict__ Phi,
                                               typename Vec<D>::T *__restrict__ Frep_un,
                                               double *part_z, int n,
-                                              const typename Vec<D>::T *__restrict__ Y) {
+                                              const typename Vec<D>::T *__restrict__ Y, int after) {
   sgt_pdl_wait();
-  if (st->T != 0) return;  // cell mode: k_g2s
+  if (st->T != 0 || g2s_skips(st, after)) return;  // cell mode: k_g2s
   __shared__ double wz[SGT_THREADS / 32];
   __shared__ bool last;
   constexpr int L = SGT_GLPP, R = D == 1 ? 1 : (D == 2 ? 4 : 16);  // stencil rows
@@ -917,8 +926,8 @@ template <int D>
 __global__ void __launch_bounds__(SGT_THREADS, D == 3 ? 3 : 6)
 k_gather(SgtState *st, const typename Node<D>::T *__restrict__ Phi,
          typename Vec<D>::T *__restrict__ Frep_un, double *part_z, int n,
-         const typename Vec<D>::T *__restrict__ Y) {
-  k_gather_body<D>(blockIdx.x, gridDim.x, st, Phi, Frep_un, part_z, n, Y);
+         const typename Vec<D>::T *__restrict__ Y, int after) {
+  k_gather_body<D>(blockIdx.x, gridDim.x, st, Phi, Frep_un, part_z, n, Y, after);
 }
 
 // Cell mode: the same over the chunks of sorted points.
@@ -926,9 +935,9 @@ template <int D>
 __device__ __forceinline__ void k_g2s_body(int vb_, int vg_, const float4 *__restrict__ sorted, SgtState *st,
       const int4 *__restrict__ chunks,
       const typename Node<D>::T *__restrict__ Phi,
-      typename Vec<D>::T *__restrict__ Frep_un, double *part_z, int n) {
+      typename Vec<D>::T *__restrict__ Frep_un, double *part_z, int n, int after) {
   sgt_pdl_wait();
-  if (st->T == 0) return;  // scatter mode: k_gather
+  if (st->T == 0 || g2s_skips(st, after)) return;  // scatter mode: k_gather
   __shared__ double wz[SGT_THREADS / 32];
   __shared__ bool last;
   const int N = st->N, nch = st->nchunks;
@@ -996,8 +1005,8 @@ __global__ void __launch_bounds__(SGT_THREADS)
 k_g2s(const float4 *__restrict__ sorted, SgtState *st,
       const int4 *__restrict__ chunks,
       const typename Node<D>::T *__restrict__ Phi,
-      typename Vec<D>::T *__restrict__ Frep_un, double *part_z, int n) {
-  k_g2s_body<D>(blockIdx.x, gridDim.x, sorted, st, chunks, Phi, Frep_un, part_z, n);
+      typename Vec<D>::T *__restrict__ Frep_un, double *part_z, int n, int after) {
+  k_g2s_body<D>(blockIdx.x, gridDim.x, sorted, st, chunks, Phi, Frep_un, part_z, n, after);
 }
 
 // ---------------------------------------------------------------------------

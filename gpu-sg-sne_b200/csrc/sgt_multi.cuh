@@ -138,7 +138,7 @@ km_g2s(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int
   SGT_MULTI_JOB
   typedef typename Vec<D>::T VT;
   k_g2s_body<D>(vb, vg, v.sorted, v.st, v.chunks, (const typename Node<D>::T *)v.Phi,
-                (VT *)v.Frep, v.part_z, v.n);
+                (VT *)v.Frep, v.part_z, v.n, SGT_G2S_BOTH);
 }
 
 template <int D>
@@ -147,7 +147,7 @@ km_gather(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, 
   SGT_MULTI_JOB
   typedef typename Vec<D>::T VT;
   k_gather_body<D>(vb, vg, v.st, (const typename Node<D>::T *)v.Phi, (VT *)v.Frep, v.part_z, v.n,
-                   (const VT *)v.Y);
+                   (const VT *)v.Y, SGT_G2S_BOTH);
 }
 
 template <int D, int G>
