@@ -170,9 +170,10 @@ static int grid_blocks(int nsm, int per_sm) { return std::max(1, nsm * std::max(
 
 // iterations per launch of a job's chained graph (sgt_job_run)
 #define SGT_GRAPH_ITERS 16
-// Iterations of one call from which that graph is made on the way (unless
-// sgt_job_prepare has): it takes 1.9 ms to instantiate and saves about 1 us
-// per iteration against launches of the one-iteration graph.
+// Iterations, of one call or as the job's max_iter announces them, from which
+// that graph is made on the way (unless sgt_job_prepare has): it takes 1.9 ms
+// to instantiate and saves about 1 us per iteration against launches of the
+// one-iteration graph.
 #define SGT_GRAPH_REPAYS 512
 // nodes of the grid copies a job holds at least (32 copies of a 90^2 grid; the
 // largest 2-D grid once)
@@ -1450,7 +1451,8 @@ static sgt_status run_one(sgt_job *J) {
 static sgt_status run_chunk(sgt_job *J, int iters) {
   sgt_ctx *ctx = J->ctx;
   int left = iters;
-  if (left >= SGT_GRAPH_REPAYS && !J->gexec_multi)
+  if (left >= SGT_GRAPH_ITERS && !J->gexec_multi &&
+      std::max(left, J->p.max_iter) >= SGT_GRAPH_REPAYS)
     CKS(instantiate(J, SGT_GRAPH_ITERS, &J->gexec_multi));
   for (; J->gexec_multi && left >= SGT_GRAPH_ITERS; left -= SGT_GRAPH_ITERS)
     CK(cudaGraphLaunch(J->gexec_multi, ctx->stream));
