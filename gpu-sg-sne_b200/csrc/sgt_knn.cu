@@ -158,7 +158,7 @@ k_knn(const float *__restrict__ X, int n, int dim, int k, const int *__restrict_
 // of 8 rows x 16 bytes (8 dimensions), unit u of all rows contiguous, hi and
 // lo parts one after the other.  Points of up to 64 dimensions keep the query
 // image resident and stream candidate tiles; wider points stream both in
-// chunks of 64 dimensions.  One thread issues the copies and MMAs; each
+// chunks of 64 dimensions.  One thread issues the copies, one the MMAs; each
 // 128 x 256 tile accumulates into one of two halves of tensor memory while
 // eight warps scan the other.
 //
@@ -410,6 +410,102 @@ __device__ __forceinline__ float knn_select(float2 *buf, int cnt) {
   return knn_unordered(T);
 }
 
+// Exact distances of m candidates to query q by one warp: d[e] is candidate
+// e's sum of squared differences in dimension order, as k_knn forms it.  A
+// lane's sum is a serial chain over its candidate's row; read by the lanes
+// themselves, 32 rows make 32 cache lines per request, and the L1 tag rate
+// bound the filter's tail (1.3 ms per wave of query blocks of 784 dimensions
+// and k = 90, 0.65 now: 60,000 points 20.4 -> 12.6 ms; 100,000 points of 50
+// dimensions 12.9 -> 11.4 ms).  So runs of KNN_RR_W dimensions of 32 candidates and the query are
+// copied to shared memory by lanes side by side, KNN_RR_ST - 1 runs ahead.
+constexpr int KNN_RR_W = 32;              // dimensions per run
+constexpr int KNN_RR_LD = KNN_RR_W + 4;   // row pitch in floats: float4 reads without conflicts
+constexpr int KNN_RR_ST = 5;              // runs in flight
+constexpr unsigned KNN_RR_BYTES = 24 * 1024;  // a warp's share of the operand memory
+static_assert(KNN_RR_ST * 33 * KNN_RR_LD * 4 <= KNN_RR_BYTES && 8 * KNN_RR_BYTES <= KNN_TC_SMEM,
+              "re-rank staging");
+
+// global -> shared copy of B bytes; zeros when !in
+template <int B>
+__device__ __forceinline__ void cp_async(unsigned dst, const float *src, bool in) {
+  if constexpr (B == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
+                 "r"(in ? 16 : 0) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(B),
+                 "r"(in ? B : 0) : "memory");
+}
+// rows 0..31: candidates list[0..31], row 32: the query; dimensions k0 ..
+// k0 + KNN_RR_W - 1, zeros from dim
+template <int F>
+__device__ __forceinline__ void knn_stage(const float *__restrict__ X, int dim, int q,
+                                          const int *list, int k0, unsigned dst) {
+  constexpr int PER = KNN_RR_W / F, ROWS = 32 / PER;  // lanes per row, rows per request
+  const int lane = threadIdx.x & 31, r0 = lane / PER, kk = k0 + (lane % PER) * F;
+  const bool in = kk < dim;
+  const float *src = X + (in ? kk : 0);
+  dst += (r0 * KNN_RR_LD + (lane % PER) * F) * 4u;
+#pragma unroll 8
+  for (int r = 0; r < 32; r += ROWS)
+    cp_async<4 * F>(dst + r * (KNN_RR_LD * 4u), src + (long)list[r + r0] * dim, in);
+  if (r0 == 0) cp_async<4 * F>(dst + 32 * (KNN_RR_LD * 4u), src + (long)q * dim, in);
+}
+// (list has entries to the next multiple of 32 from m)
+__device__ __forceinline__ void knn_rerank(const float *__restrict__ X, int dim, int q, int m,
+                                           const int *list, float *d, float *stage) {
+  const int lane = threadIdx.x & 31;
+  const int nrun = (dim + KNN_RR_W - 1) / KNN_RR_W, total = nrun * ((m + 31) / 32);
+  const size_t xa = reinterpret_cast<size_t>(X);
+  // floats per copy: rows start on multiples of it
+  const int f = (dim & 3) == 0 && (xa & 15) == 0 ? 4 : ((dim & 1) == 0 && (xa & 7) == 0 ? 2 : 1);
+  int ic = 0, ik = 0, is = 0;  // next run to issue: first candidate, first dimension, stage
+  auto issue = [&](int s) {
+    if (s < total) {
+      const unsigned dst = smem_u32(stage + is * 33 * KNN_RR_LD);
+      if (f == 4) knn_stage<4>(X, dim, q, list + ic, ik, dst);
+      else if (f == 2) knn_stage<2>(X, dim, q, list + ic, ik, dst);
+      else knn_stage<1>(X, dim, q, list + ic, ik, dst);
+      ik += KNN_RR_W;
+      if (ik >= dim) { ik = 0; ic += 32; }
+      if (++is == KNN_RR_ST) is = 0;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int s = 0; s < KNN_RR_ST - 1; s++) issue(s);
+  int cc = 0, ck = 0, cs = 0;
+  float acc = 0.f;
+  for (int s = 0; s < total; s++) {
+    issue(s + KNN_RR_ST - 1);  // into the stage read last
+    asm volatile("cp.async.wait_group %0;" ::"n"(KNN_RR_ST - 1) : "memory");
+    __syncwarp();
+    const float *b = stage + cs * 33 * KNN_RR_LD, *mine = b + lane * KNN_RR_LD,
+                *qr = b + 32 * KNN_RR_LD;
+    const int w = min(KNN_RR_W, dim - ck);  // zero padding adds nothing
+#pragma unroll 8
+    for (int kk = 0; kk < w; kk += 4) {
+      const float4 a = *reinterpret_cast<const float4 *>(qr + kk);
+      const float4 c = *reinterpret_cast<const float4 *>(mine + kk);
+      float df = a.x - c.x;
+      acc = fmaf(df, df, acc);
+      df = a.y - c.y;
+      acc = fmaf(df, df, acc);
+      df = a.z - c.z;
+      acc = fmaf(df, df, acc);
+      df = a.w - c.w;
+      acc = fmaf(df, df, acc);
+    }
+    ck += KNN_RR_W;
+    if (++cs == KNN_RR_ST) cs = 0;
+    if (ck >= dim) {
+      if (cc + lane < m) d[cc + lane] = acc;
+      acc = 0.f;
+      ck = 0;
+      cc += 32;
+    }
+    __syncwarp();
+  }
+}
+
 // A block walks over query blocks; warps 0-7 scan (warp w: rows 32 (w & 3)..,
 // columns 128 (w >> 2)..), lane 0 of warp 8 issues the MMAs, lane 0 of warp 9
 // the copies.
@@ -606,7 +702,9 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
     __syncthreads();
     if (gave_up) break;  // block-uniform: written before the barrier
     if (warp < 8) {
-      // re-rank: a warp per query
+      // re-rank: a warp per query.  All copies into the operand memory and all
+      // MMAs that read it have been waited for; the warps share it.
+      float *stage = reinterpret_cast<float *>(smem + warp * KNN_RR_BYTES);
       for (int r = warp; r < KNN_TC_M; r += 8) {
         const int q = qb * KNN_TC_M + r;
         if (q >= n) break;
@@ -634,7 +732,9 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
         }
         // only a candidate whose key is within the bound of the k-th key can
         // be among the k nearest (a NaN bound keeps all)
-        const float qn = nrm[q], bound = eps * (qn + cmax);
+        // (products may lose terms below the smallest normal number: 1e-37 a
+        // dimension covers them)
+        const float qn = nrm[q], bound = eps * (qn + cmax) + 1e-37f * (float)dim;
         if (have > k) {
           const unsigned K = knn_kth<2 * E>(u, k);
           const unsigned cut = K == 0 ? 0u : knn_ordered(knn_unordered(K) - bound);
@@ -653,35 +753,9 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
             m += __popc(mk);
           }
         m = min(m, L);
+        if (m + lane < (m + 31) / 32 * 32) s_idx[warp][m + lane] = q;
         __syncwarp();
-        const float *xq = X + (long)q * dim;
-        for (int e = lane; e < m; e += 32) {
-          const float *xc = X + (long)s_idx[warp][e] * dim;
-          float acc = 0.f;
-          int kk = 0;
-          if ((dim & 3) == 0 && (reinterpret_cast<size_t>(X) & 15) == 0) {
-#pragma unroll 4
-            for (; kk < dim; kk += 4) {
-              const float4 a = __ldg(reinterpret_cast<const float4 *>(xq + kk));
-              const float4 c = __ldg(reinterpret_cast<const float4 *>(xc + kk));
-              float df = a.x - c.x;
-              acc = fmaf(df, df, acc);
-              df = a.y - c.y;
-              acc = fmaf(df, df, acc);
-              df = a.z - c.z;
-              acc = fmaf(df, df, acc);
-              df = a.w - c.w;
-              acc = fmaf(df, df, acc);
-            }
-          } else {
-#pragma unroll 8
-            for (; kk < dim; kk++) {
-              const float df = __ldg(&xq[kk]) - __ldg(&xc[kk]);
-              acc = fmaf(df, df, acc);
-            }
-          }
-          s_d[warp][e] = acc;
-        }
+        knn_rerank(X, dim, q, m, s_idx[warp], s_d[warp], stage);
         __syncwarp();
         // the k nearest by (distance, index): each entry's rank is the number
         // of entries before it
@@ -701,11 +775,14 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
         for (int o = 16; o > 0; o >>= 1) dk = fminf(dk, __shfl_xor_sync(0xffffffffu, dk, o));
         // settled: nothing was dropped, or all that was is farther than the
         // k-th exact distance (false for NaN: such queries are redone too)
-        const bool settled = m >= k && (tail == -INFINITY || qn - 2.f * tail - bound > dk);
+        const bool settled = m >= k && ((tail == -INFINITY && bound < INFINITY) ||
+                                        qn - 2.f * tail - bound > dk);
         if (!settled && lane == 0) redo[atomicAdd(nredo, 1)] = q;
         __syncwarp();
       }
     }
+    // order this memory's plain accesses before the next block's bulk copies
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();  // the lists are free for the next query block
   }
   if (gave_up) {
@@ -836,9 +913,14 @@ extern "C" sgt_status sgt_knn_ex(sgt_ctx *ctx, int n, int dim, const float *X, i
     return sgti_fail(ctx, SGT_ERR_CUDA, "sgt_knn: set device");
   if (n_redo) *n_redo = 0;
   sgt_status st;
-  // the automatic choice takes the filter for any width and k; below 4096
-  // points the SIMT search has no images to make
-  if (method == SGT_KNN_TENSOR || (method == SGT_KNN_AUTO && n >= 4096 && n <= (1 << 28))) {
+  // The automatic choice takes the filter for any width and k where its
+  // set-up of 50 us and the re-ranking of whole blocks of 128 queries are less
+  // than the SIMT search's serial list updates (filter against SIMT search,
+  // us): 256 points 10-D k = 15 175 / 267, 50-D k = 30 204 / 1912, 784-D
+  // k = 90 952 / 6537; 1024 points 3-D k = 4 274 / 256, 50-D k = 30
+  // 301 / 5745; 128 points 10-D k = 15 158 / 154.
+  const int n_min = k >= 10 ? 256 : 1024;
+  if (method == SGT_KNN_TENSOR || (method == SGT_KNN_AUTO && n >= n_min && n <= (1 << 28))) {
     st = knn_tc(ctx, n, dim, X, k, idx, d2, n_redo);
     // the filter's operand images (about 8 bytes per point and dimension)
     // did not fit: the automatic choice falls back to the SIMT search
