@@ -218,8 +218,11 @@ __device__ __forceinline__ float2 node_plane(const typename Node<D>::T &v, int p
 // shared memory in 2-D, for which a block waits until a whole SM has drained
 // of the concurrent SpMV.  The plain transforms cost more operations than FFTs
 // and still only a few microseconds, with 256 threads and 15 KB a block.
+// 3-D grids above 80 points per axis take the FFT passes: the plain transforms
+// grow with N^4 (whole iterations of 8,000 points, plain transforms against
+// FFTs: 52 points per axis 170 / 250 us, 75 560 / 744, 98 1589 / 1369).
 // ---------------------------------------------------------------------------
-#define SGT_SPEC_MAX(D) ((D) == 1 ? 512 : 128)
+#define SGT_SPEC_MAX(D) ((D) == 1 ? 512 : ((D) == 2 ? 128 : 80))
 // k_spec_rows in one go, or its halves (the charge grid of a row-split
 // embedding is summed over the ranks between them)
 #define SGT_SPEC_BOTH 0
