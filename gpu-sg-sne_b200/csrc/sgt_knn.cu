@@ -20,6 +20,7 @@
 #include "../../include/sgtsne_b200.h"
 #include "sgt_internal.h"
 #include "sgt_async.cuh"
+#include "sgt_knn_rules.h"
 
 #include <cuda_bf16.h>
 
@@ -138,8 +139,9 @@ k_knn(const float *__restrict__ X, int n, int dim, int k, const int *__restrict_
 // with the exact arithmetic of k_knn (sums of squared differences in dimension
 // order), so returned distances are bit-identical to it.  A query whose list
 // could miss a true neighbour is redone by k_knn: the nearest candidate ever
-// dropped, less the bound EPS (|q|^2 + max |c|^2) on a key's error, has to lie
-// beyond the k-th exact distance.
+// dropped, less the bound EPS (|q|^2 + max |c|^2) on a key's error and the
+// rounding of a returned distance (both in sgt_knn_rules.h), has to lie beyond
+// the k-th distance.
 //
 // Lists: a query's candidates are scanned by two threads (one per half of
 // each tile's columns), each with an unordered buffer of CAP entries in L2.
@@ -176,14 +178,6 @@ constexpr int KNN_TC_MAXDIM = 64;
 constexpr int KNN_TC_SCAN = 256;   // scanning threads; two more warps issue MMAs and copies
 constexpr int KNN_TC_THREADS = KNN_TC_SCAN + 64;
 constexpr unsigned KNN_TC_SMEM = 192 * 1024;
-
-// Bound on the error of 2 key = |q|^2 - d^2, relative to |q|^2 + max |c|^2:
-// 2^-21 of the products' sum per accumulated MMA of 16 dimensions and, in
-// three terms, twice 3 * 2^-18 for the neglected parts.
-__host__ __device__ inline float knn_tc_eps(int dim, bool exact) {
-  const float steps = (float)((dim + 3 + 15) / 16);
-  return exact ? (steps + 1.f) * 4.8e-7f : 2.4e-5f + 3.f * steps * 4.8e-7f;
-}
 
 // shared-memory matrix descriptor: K-major, no swizzle
 __device__ __forceinline__ unsigned long long umma_desc(unsigned addr, unsigned lbo,
@@ -265,8 +259,9 @@ __device__ __forceinline__ unsigned bf16_bits(float x) {
 }
 __device__ __forceinline__ float bf16_value(unsigned b) { return __uint_as_float(b << 16); }
 
-// squared norms (FP32, dimension order), their maximum, and whether some
-// coordinate is no BF16 number
+// squared norms (FP64 sums, rounded to FP32: an FP32 sum's error grows with the
+// width, past a distance that is small against the norms), their maximum, and
+// whether some coordinate is no BF16 number
 __global__ void k_knn_norms(const float *__restrict__ X, int n, int dim, float *__restrict__ nrm,
                             unsigned *__restrict__ nmax, int *__restrict__ inexact) {
   __shared__ float tile[8][32][33];
@@ -274,7 +269,7 @@ __global__ void k_knn_norms(const float *__restrict__ X, int n, int dim, float *
   // a warp takes 32 points; 32 x 32 tiles turn coalesced loads into a
   // point per lane
   for (int i0 = (blockIdx.x * 8 + w) * 32; i0 < n; i0 += gridDim.x * 256) {
-    float s = 0.f;
+    double sum = 0.0;
     bool low = false;
     for (int k0 = 0; k0 < dim; k0 += 32) {
       __syncwarp();
@@ -283,11 +278,12 @@ __global__ void k_knn_norms(const float *__restrict__ X, int n, int dim, float *
       __syncwarp();
       for (int kk = 0; kk < min(32, dim - k0); kk++) {
         const float x = tile[w][lane][kk];
-        s = fmaf(x, x, s);
+        sum = fma((double)x, (double)x, sum);
         low |= bf16_value(bf16_bits(x)) != x;
       }
     }
     const int i = i0 + lane;
+    const float s = (float)sum;
     if (i < n) nrm[i] = s;
     // non-negative floats order as integers (a NaN norm as the largest)
     const unsigned m = __reduce_max_sync(0xffffffffu, i < n ? __float_as_uint(s) : 0u);
@@ -560,7 +556,8 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
   const unsigned tmem = tslot;
   const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((KNN_TC_N >> 3) << 17) |
                          ((KNN_TC_M >> 4) << 24);
-  const float eps = knn_tc_eps(dim, !three), cmax = __uint_as_float(*nmax);
+  const float eps = sgt_knn_eps(dim, !three), gamma = sgt_knn_gamma(dim),
+              cmax = __uint_as_float(*nmax);
   // running counts of tiles and of pipeline steps over all query blocks
   unsigned tiles = 0, steps = 0, loads = 0, blocks = 0;
   for (int qb = blockIdx.x; qb < nq; qb += gridDim.x, blocks++) {
@@ -731,13 +728,16 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
           else tail = fmaxf(tail, knn_unordered(T));
         }
         // only a candidate whose key is within the bound of the k-th key can
-        // be among the k nearest (a NaN bound keeps all)
+        // be among the k nearest: those of the k best keys have distances of
+        // at most far, times 1 + gamma as they are formed (a NaN bound keeps
+        // all)
         // (products may lose terms below the smallest normal number: 1e-37 a
         // dimension covers them)
         const float qn = nrm[q], bound = eps * (qn + cmax) + 1e-37f * (float)dim;
         if (have > k) {
           const unsigned K = knn_kth<2 * E>(u, k);
-          const unsigned cut = K == 0 ? 0u : knn_ordered(knn_unordered(K) - bound);
+          const float kth = knn_unordered(K), far = fmaxf(qn - 2.f * kth + bound, 0.f);
+          const unsigned cut = K == 0 ? 0u : knn_ordered(kth - (bound + 1.1f * gamma * far));
           if (bound == bound && cut > T && cut <= K) T = cut;
         }
         int m = 0;
@@ -773,10 +773,12 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) dk = fminf(dk, __shfl_xor_sync(0xffffffffu, dk, o));
-        // settled: nothing was dropped, or all that was is farther than the
-        // k-th exact distance (false for NaN: such queries are redone too)
+        // settled: nothing was dropped, or the distance of all that was, as it
+        // would be formed, is larger than the k-th (false for NaN: such queries
+        // are redone too)
+        const float near = qn - 2.f * tail - bound;
         const bool settled = m >= k && ((tail == -INFINITY && bound < INFINITY) ||
-                                        qn - 2.f * tail - bound > dk);
+                                        near - 1.1f * gamma * near > dk);
         if (!settled && lane == 0) redo[atomicAdd(nredo, 1)] = q;
         __syncwarp();
       }

@@ -1,0 +1,32 @@
+// sgt_knn_rules.h -- what the tensor-core kNN filter (sgt_knn.cu) decides by
+// arithmetic alone: the error bound of its keys and the rounding of the
+// distances it returns.  Plain C++, so that a CPU model can run the same code.
+#pragma once
+
+#ifdef __CUDACC__
+#define SGT_RULE __host__ __device__ __forceinline__
+#else
+#define SGT_RULE inline
+#endif
+
+// Bound on the error of 2 key = |q|^2 - d^2, relative to A = |q|^2 + max |c|^2.
+//   Accumulation: an MMA adds 16 exact products to its FP32 accumulator.  Taken
+//     as 17 addends cut to 24 bits at the largest one's exponent and a sum cut
+//     to FP32: 18 errors of 2^-23 B, B <= |q||c| + |c|^2/2 <= |q|^2/2 + |c|^2
+//     a bound of every partial sum; twice that of a key, 36 * 2^-23 A an MMA.
+//   Three terms: hi and lo are rounded to 8 bits, so lo.lo and the two
+//     remainders neglected are 2^-18 |q||c| each: 3 * 2^-18 A.
+//   Norms: FP64 sums rounded to FP32 (2^-24 in |c|^2 and in |q|^2), three BF16
+//     terms of -|c|^2/2 (2^-27); and the comparison |q|^2 - 2 key - bound itself
+//     in FP32 (9 * 2^-24 A): under 2^-20 A together.
+inline constexpr float SGT_KNN_EPS_MMA = 36.f / 8388608.f;
+SGT_RULE float sgt_knn_eps(int dim, bool exact) {
+  const float steps = (float)((dim + 3 + 15) / 16);
+  return (exact ? steps : 3.f * steps) * SGT_KNN_EPS_MMA + (exact ? 0.f : 3.f / 262144.f) +
+         1.f / 1048576.f;
+}
+
+// Relative error of a distance as the searches form it: per dimension one
+// rounded difference (twice in its square) and one rounded multiply-add, all
+// terms of one sign: (dim + 2) 2^-24.
+SGT_RULE float sgt_knn_gamma(int dim) { return (float)(dim + 3) * 6.0e-8f; }
