@@ -558,8 +558,10 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
                          ((KNN_TC_M >> 4) << 24);
   const float eps = sgt_knn_eps(dim, !three), gamma = sgt_knn_gamma(dim),
               cmax = __uint_as_float(*nmax);
-  // running counts of tiles and of pipeline steps over all query blocks
-  unsigned tiles = 0, steps = 0, loads = 0, blocks = 0;
+  // places that run on over all query blocks: stage of the copies, stage of the
+  // MMAs, accumulator (of the MMAs or of the scan)
+  SgtRing load, step, acc;
+  unsigned blocks = 0;
   for (int qb = blockIdx.x; qb < nq; qb += gridDim.x, blocks++) {
     const unsigned total = (unsigned)ntile * (unsigned)nch;  // pipeline steps of a query block
     if (warp == 9) {
@@ -572,10 +574,9 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
           for (int p = 0; p < parts; p++)
             bulk_g2s(sm0 + p * res_part, imgA + ((size_t)qb * 2 + p) * res_part, res_part, bar_a);
         }
-        for (unsigned g = 0; g < total; g++, loads++) {
-          const int st = (int)(loads % (unsigned)nst);
-          const unsigned turn = loads / (unsigned)nst;
-          if (turn > 0) ok = mbar_wait_or(bar_free(st), (turn - 1) & 1, &gave_up);
+        for (unsigned g = 0; g < total; g++, load.next(nst)) {
+          const int st = load.at;
+          ok = mbar_wait_or(bar_free(st), load.phase ^ 1u, &gave_up);
           if (!ok) break;
           const int tile = (int)(g / (unsigned)nch), ch = (int)(g % (unsigned)nch);
           const int uc = min(ku, U - ch * ku);
@@ -596,11 +597,10 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
         bool ok = true;
         if (resident) ok = mbar_wait_or(bar_a, blocks & 1, &gave_up);
         for (unsigned g = 0; g < total && ok; g++) {
-          const int st = (int)(steps % (unsigned)nst), ch = (int)(g % (unsigned)nch);
-          const int ab = (int)(tiles & 1u);
-          if (ch == 0 && tiles >= 2)  // the accumulator has been scanned
-            ok = mbar_wait_or(bar_scan(ab), ((tiles >> 1) - 1) & 1, &gave_up);
-          ok = ok && mbar_wait_or(bar_full(st), (steps / (unsigned)nst) & 1, &gave_up);
+          const int st = step.at, ch = (int)(g % (unsigned)nch), ab = acc.at;
+          if (ch == 0)  // the accumulator has been scanned
+            ok = mbar_wait_or(bar_scan(ab), acc.phase ^ 1u, &gave_up);
+          ok = ok && mbar_wait_or(bar_full(st), step.phase, &gave_up);
           if (!ok) break;
           tc_fence_after();
           const unsigned sb = st0 + st * st_bytes;
@@ -619,10 +619,10 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
             }
           }
           umma_commit(bar_free(st));
-          steps++;
+          step.next(nst);
           if (ch == nch - 1) {
             umma_commit(bar_acc(ab));
-            tiles++;
+            acc.next(2);
           }
         }
       }
@@ -636,9 +636,9 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
       bool ok = true;
       s_live[t] = -INFINITY;
       asm volatile("bar.sync 1, %0;" ::"n"(KNN_TC_SCAN) : "memory");  // the scanning warps
-      for (int tile = 0; tile < ntile; tile++, tiles++) {
-        const int ab = (int)(tiles & 1u);
-        ok = __all_sync(0xffffffffu, mbar_wait_or(bar_acc(ab), (tiles >> 1) & 1, &gave_up));
+      for (int tile = 0; tile < ntile; tile++, acc.next(2)) {
+        const int ab = acc.at;
+        ok = __all_sync(0xffffffffu, mbar_wait_or(bar_acc(ab), acc.phase, &gave_up));
         if (!ok) break;
         tc_fence_after();
         // L keys of the other half of the query's columns lie above its
@@ -791,11 +791,10 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
     // let the copies and MMAs in flight finish before the memory is released
     if (t == KNN_TC_SCAN + 32) {
       atomicExch(err, 1);
-      for (unsigned l = loads > (unsigned)nst ? loads - nst : 0; l < loads; l++)
-        mbar_wait(bar_full((int)(l % (unsigned)nst)), (l / (unsigned)nst) & 1);
+      while (load.back(nst)) mbar_wait(bar_full(load.at), load.phase);
     }
-    if (t == KNN_TC_SCAN && steps > 0)
-      mbar_wait(bar_free((int)((steps - 1) % (unsigned)nst)), ((steps - 1) / (unsigned)nst) & 1);
+    // (MMAs complete in order: the last one's commit)
+    if (t == KNN_TC_SCAN && step.back(nst)) mbar_wait(bar_free(step.at), step.phase);
   }
   tc_fence_before();
   __syncthreads();

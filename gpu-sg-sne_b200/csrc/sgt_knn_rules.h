@@ -1,6 +1,7 @@
 // sgt_knn_rules.h -- what the tensor-core kNN filter (sgt_knn.cu) decides by
-// arithmetic alone: the error bound of its keys and the rounding of the
-// distances it returns.  Plain C++, so that a CPU model can run the same code.
+// arithmetic alone: the error bound of its keys, the rounding of the distances
+// it returns, and the places in its pipeline.  Plain C++, so that a CPU model
+// can run the same code.
 #pragma once
 
 #ifdef __CUDACC__
@@ -30,3 +31,32 @@ SGT_RULE float sgt_knn_eps(int dim, bool exact) {
 // rounded difference (twice in its square) and one rounded multiply-add, all
 // terms of one sign: (dim + 2) 2^-24.
 SGT_RULE float sgt_knn_gamma(int dim) { return (float)(dim + 3) * 6.0e-8f; }
+
+// Place in a ring of buffers whose mbarriers complete one phase per use: the
+// buffer and the parity of its present use's phase, carried along.  (Taken from
+// a 32-bit count of all uses, both go wrong when it wraps, unless the ring's
+// length divides 2^32: after 4 billion tiles, a search of 1e8 points.)  A wait
+// for the use before the present one has the parity phase ^ 1, which a fresh
+// mbarrier passes.
+struct SgtRing {
+  int at = 0, flying = 0;  // flying: uses that may not have completed, at most the ring's length
+  unsigned phase = 0;
+  SGT_RULE void next(int n) {
+    if (flying < n) flying++;
+    if (++at == n) {
+      at = 0;
+      phase ^= 1u;
+    }
+  }
+  // to the use before, while there is one that may be flying
+  SGT_RULE bool back(int n) {
+    if (flying == 0) return false;
+    flying--;
+    if (at == 0) {
+      at = n;
+      phase ^= 1u;
+    }
+    at--;
+    return true;
+  }
+};
