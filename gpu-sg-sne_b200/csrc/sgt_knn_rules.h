@@ -11,19 +11,22 @@
 #endif
 
 // Bound on the error of 2 key = |q|^2 - d^2, relative to A = |q|^2 + max |c|^2.
-//   Accumulation: an MMA adds 16 exact products to its FP32 accumulator.  Taken
-//     as 17 addends cut to 24 bits at the largest one's exponent and a sum cut
-//     to FP32: 18 errors of 2^-23 B, B <= |q||c| + |c|^2/2 <= |q|^2/2 + |c|^2
-//     a bound of every partial sum; twice that of a key, 36 * 2^-23 A an MMA.
+//   Accumulation: an MMA adds 16 exact products to its FP32 accumulator. Its
+//     17 addends are cut at 2^-25 of the largest one's power of two and their
+//     sum is cut to FP32, all towards zero (read off single tiles on a B200:
+//     1 + 16 * 2^-25 is right, 1 + 16 * 2^-26 is 1). So an MMA is off by less
+//     than (17 * 2^-25 + 2^-23) times a bound of the partial sums: |q||c| <=
+//     A / 2, and A from the norm's columns on (the last one or two chunks, at
+//     most 8 MMAs a term). Twice that for 2 key; 2 % for the parts' rounding.
 //   Three terms: hi and lo are rounded to 8 bits, so lo.lo and the two
 //     remainders neglected are 2^-18 |q||c| each: 3 * 2^-18 A.
 //   Norms: FP64 sums rounded to FP32 (2^-24 in |c|^2 and in |q|^2), three BF16
 //     terms of -|c|^2/2 (2^-27); and the comparison |q|^2 - 2 key - bound itself
 //     in FP32 (9 * 2^-24 A): under 2^-20 A together.
-inline constexpr float SGT_KNN_EPS_MMA = 36.f / 8388608.f;
+inline constexpr float SGT_KNN_EPS_MMA = 1.02f * 21.f / 33554432.f;
 SGT_RULE float sgt_knn_eps(int dim, bool exact) {
-  const float steps = (float)((dim + 3 + 15) / 16);
-  return (exact ? steps : 3.f * steps) * SGT_KNN_EPS_MMA + (exact ? 0.f : 3.f / 262144.f) +
+  const int terms = exact ? 1 : 3, steps = (dim + 3 + 15) / 16, late = steps < 8 ? steps : 8;
+  return (float)(terms * (steps + late)) * SGT_KNN_EPS_MMA + (exact ? 0.f : 3.f / 262144.f) +
          1.f / 1048576.f;
 }
 

@@ -4,8 +4,8 @@ from that file.
 
 Keys q.c - |c|^2/2 from BF16 parts, in one term (points that are BF16 numbers)
 or three; MMAs of 16 dimensions in the kernel's order, each cutting its 16
-products and the accumulator to 24 bits at the largest one's exponent and its
-sum to FP32; norms summed in FP64.  The L best keys are kept, those within the
+products and the accumulator at 2^-25 of the largest one's power of two and its
+sum to FP32, towards zero; norms summed in FP64.  The L best keys are kept, those within the
 bound of the k-th key re-ranked with the SIMT search's FP32 sums, and a query
 is settled when everything dropped is farther than the k-th distance.
 
@@ -59,8 +59,8 @@ def mma(acc, a, b):
     """acc[q, c] + sum over 16 dimensions of a[q] b[c], as stated above."""
     p = a[:, None, :].astype(np.float64) * b[None].astype(np.float64)
     p = np.concatenate([p, acc[..., None]], -1)
-    e = np.frexp(np.abs(p).max(-1))[1]  # the largest is below 2^e
-    unit = np.ldexp(1.0, e - 24)[..., None]
+    e = np.frexp(np.abs(p).max(-1))[1]  # the largest's power of two is 2^(e - 1)
+    unit = np.ldexp(1.0, e - 26)[..., None]
     return trunc32((np.trunc(p / unit) * unit).sum(-1))
 
 
@@ -163,7 +163,7 @@ def points(kind, dim, rng):
 
 @pytest.mark.parametrize("kind,dim,k,least", [
     ("blobs", 50, 30, 0.95), ("blobs", 3, 10, 0.95), ("blobs", 130, 97, 0.9), ("ints", 60, 30, 0.9),
-    ("ints", 784, 90, 0.9), ("offset", 16, 10, 0.0), ("sums", 784, 15, 0.0), ("sums3", 784, 15, 0.0),
+    ("ints", 784, 90, 0.9), ("blobs", 63, 30, 0.95), ("blobs", 784, 90, 0.0), ("offset", 16, 10, 0.0), ("sums", 784, 15, 0.0), ("sums3", 784, 15, 0.0),
 ])
 def test_settled_queries_are_right(rules, kind, dim, k, least):
     rng = np.random.default_rng(dim + k)
