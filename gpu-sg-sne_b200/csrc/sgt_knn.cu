@@ -791,10 +791,14 @@ k_knn_tc(const unsigned char *__restrict__ imgA, const unsigned char *__restrict
     // let the copies and MMAs in flight finish before the memory is released
     if (t == KNN_TC_SCAN + 32) {
       atomicExch(err, 1);
+      if (resident) mbar_wait(bar_a, blocks & 1);  // (issued as this query block began)
       while (load.back(nst)) mbar_wait(bar_full(load.at), load.phase);
     }
-    // (MMAs complete in order: the last one's commit)
-    if (t == KNN_TC_SCAN && step.back(nst)) mbar_wait(bar_free(step.at), step.phase);
+    // MMAs complete in order: the last step's commit and the last tile's
+    if (t == KNN_TC_SCAN) {
+      if (step.back(nst)) mbar_wait(bar_free(step.at), step.phase);
+      if (acc.back(2)) mbar_wait(bar_acc(acc.at), acc.phase);
+    }
   }
   tc_fence_before();
   __syncthreads();

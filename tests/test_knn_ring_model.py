@@ -9,7 +9,8 @@ places run on over query blocks, which end in a block barrier.  Checked:
 - an MMA reads the stage and the image that its step means, after their copies;
 - a copy goes to a stage whose MMAs are complete, an image likewise;
 - an MMA goes to an accumulator that has been scanned, a scan reads its tile;
-- nobody waits for good.
+- nobody waits for good;
+- a block that gives up ends with no copy and no MMA in flight.
 
 The model starts at any number of steps, as after hours of a search.  The same
 model with places taken from 32-bit counts fails where they wrap.
@@ -84,23 +85,28 @@ class Barrier:
         return parity is None or (self.done & 1) != parity
 
 
-def run(Ring, nst, nch, ntile, nblk, resident, rng, steps0=0, tiles0=0):
-    """Runs the model; raises AssertionError where it goes wrong."""
+def run(Ring, nst, nch, ntile, nblk, resident, rng, steps0=0, tiles0=0, give_up=None,
+        wait_image=True):
+    """Runs the model; raises AssertionError where it goes wrong.  give_up: the
+    number of events after which the block gives up."""
     used = lambda count, n, k: (count + n - 1 - k) // n  # uses of buffer k before `count`
     full = [Barrier(used(steps0, nst, k)) for k in range(nst)]
     free = [Barrier(used(steps0, nst, k)) for k in range(nst)]
     accb = [Barrier(used(tiles0, 2, k)) for k in range(2)]
     scan = [Barrier(used(tiles0, 2, k)) for k in range(2)]
     image = Barrier(0)
-    s = dict(stage={}, reading={}, acc={}, image=None, flying=0)
+    s = dict(stage={}, reading={}, acc={}, image=None)
+    rings = {}
     late, mmas = [], []  # copies in flight; MMAs and commits, in order
 
     def copier():
         load, step = Ring(nst, steps0), steps0
+        rings["load"] = load
         for blk in range(nblk):
             if resident:
                 assert not mmas, "the image is read"
                 s["image"] = None
+                rings["block"] = blk
                 late.append(("image", blk))
             for g in range(ntile * nch):
                 yield free[load.at], load.before
@@ -114,6 +120,7 @@ def run(Ring, nst, nch, ntile, nblk, resident, rng, steps0=0, tiles0=0):
 
     def issuer():
         at, acc, step, tile = Ring(nst, steps0), Ring(2, tiles0), steps0, tiles0
+        rings["step"], rings["acc"] = at, acc
         for blk in range(nblk):
             if resident:
                 yield image, blk & 1
@@ -147,28 +154,8 @@ def run(Ring, nst, nch, ntile, nblk, resident, rng, steps0=0, tiles0=0):
                 acc.next()
             yield "block"
 
-    agents = [copier(), issuer(), scanner()]
-    want = [next(a) for a in agents]
-    while any(a is not None for a in agents):
-        can = [("agent", i) for i, w in enumerate(want) if agents[i] is not None and w != "block" and
-               (w is None or w[0].passes(w[1]))]
-        can += [("copy", i) for i in range(len(late))]
-        if mmas:
-            can.append(("mma", 0))
-        if all(agents[i] is None or want[i] == "block" for i in range(3)) and not mmas:
-            for i in range(3):
-                if agents[i] is not None:
-                    want[i] = next(agents[i], "end")
-                    if want[i] == "end":
-                        agents[i] = None
-            continue
-        assert can, "everyone waits"
-        what, i = rng.choice(can)
-        if what == "agent":
-            want[i] = next(agents[i], "end")
-            if want[i] == "end":
-                agents[i] = None
-        elif what == "copy":
+    def complete(what, i):
+        if what == "copy":
             c = late.pop(i)
             if c[0] == "image":
                 s["image"] = c[1]
@@ -185,6 +172,46 @@ def run(Ring, nst, nch, ntile, nblk, resident, rng, steps0=0, tiles0=0):
             else:
                 s["acc"][k] = ("full", num)
                 accb[k].done += 1
+
+    def flights():
+        return [("copy", i) for i in range(len(late))] + [("mma", 0)] * bool(mmas)
+
+    agents = [copier(), issuer(), scanner()]
+    want = [next(a) for a in agents]
+    events = 0
+    while any(a is not None for a in agents):
+        if events == give_up:
+            waits = [(image, rings["block"] & 1)] if resident and wait_image else []
+            while rings["load"].back():
+                waits.append((full[rings["load"].at], rings["load"].phase))
+            if rings["step"].back():
+                waits.append((free[rings["step"].at], rings["step"].phase))
+            if rings["acc"].back():
+                waits.append((accb[rings["acc"].at], rings["acc"].phase))
+            while not all(bar.passes(parity) for bar, parity in waits):
+                assert flights(), "the end waits for good"
+                complete(*rng.choice(flights()))
+            assert not late, "a copy in flight at the end"
+            assert not mmas, "an MMA in flight at the end"
+            return
+        events += 1
+        can = [("agent", i) for i, w in enumerate(want) if agents[i] is not None and w != "block" and
+               (w is None or w[0].passes(w[1]))] + flights()
+        if all(agents[i] is None or want[i] == "block" for i in range(3)) and not mmas:
+            can = [("agent", i) for i in range(3) if agents[i] is not None]
+            for _, i in can:
+                want[i] = next(agents[i], "end")
+                if want[i] == "end":
+                    agents[i] = None
+            continue
+        assert can, "everyone waits"
+        what, i = rng.choice(can)
+        if what == "agent":
+            want[i] = next(agents[i], "end")
+            if want[i] == "end":
+                agents[i] = None
+        else:
+            complete(what, i)
 
 
 @pytest.mark.parametrize("nst,nch,resident", [(5, 1, True), (5, 2, True), (3, 3, False),
@@ -216,3 +243,17 @@ def test_back_goes_over_the_uses_in_flight(ring):
             while r.back():
                 got.append((r.at, r.phase))
             assert got == places[::-1][:n]
+
+
+@pytest.mark.parametrize("nst,nch,resident", [(5, 1, True), (5, 2, True), (3, 3, False)])
+def test_nothing_is_in_flight_after_giving_up(ring, nst, nch, resident):
+    rng = random.Random(nst)
+    for events in range(120):
+        run(ring, nst, nch, 7, 3, resident, rng, give_up=events)
+
+
+def test_the_query_image_is_one_of_the_copies_to_wait_for(ring):
+    rng = random.Random(2)
+    with pytest.raises(AssertionError, match="a copy in flight"):
+        for events in range(40):
+            run(ring, 5, 1, 7, 3, True, rng, give_up=events, wait_image=False)
