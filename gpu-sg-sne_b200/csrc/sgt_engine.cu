@@ -526,7 +526,18 @@ static sgt_status job_alloc(sgt_job *J) {
   CK(cudaEventCreateWithFlags(&J->ev_fft, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&J->ev_fft_done, cudaEventDisableTiming));
   CK(cudaMemsetAsync(J->tile_count, 0, sizeof(int) * SGT_HIST_MAX, ctx->stream));
-  CK(cudaMemsetAsync(J->st, 0, sizeof(SgtState), ctx->stream));
+  // Until coordinates are set the job has the smallest grid, one cell wide a
+  // unit: iterations queued before then skip the points outside it. (With an
+  // all-zero state the FFT passes took length 0 for the longest one, beyond a
+  // 3-D job's planes.)
+  SgtState &st0 = *J->st_host;
+  st0.N = 16;
+  st0.M = 32;
+  st0.direct = st0.N <= J->jp.conv_max ? 1 : 0;
+  st0.copies = 1;
+  st0.maxy = st0.scale = (float)(st0.N - 3);
+  st0.inv_hi = st0.h_eff = 1.0f;
+  CK(cudaMemcpyAsync(J->st, J->st_host, sizeof(SgtState), cudaMemcpyHostToDevice, ctx->stream));
   return SGT_OK;
 }
 
