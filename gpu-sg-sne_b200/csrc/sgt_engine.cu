@@ -517,7 +517,7 @@ static sgt_status job_alloc(sgt_job *J) {
   J->jp.conv_max = std::min(J->nmax, SGT_SPEC_MAX(D));
   // the sort of the cell mode, for the jobs that can take it (a shard decides
   // by the points of the whole embedding); job_shapes sets its block count
-  J->jp.cell_blocks = std::max(J->n, J->n_gather) >= SGT_CELL_MIN_N ? 1 : 0;
+  J->jp.cell_blocks = std::max(J->n, J->n_gather) >= sgt_cell_min_n(D) ? 1 : 0;
   if (J->jp.cell_blocks > 0) CKS(jalloc(J, &J->sorted, (size_t)J->n));
   CKS(jalloc(J, &J->st, 1));
   J->st_host = new SgtState();
@@ -2242,7 +2242,7 @@ size_t sgt_job_footprint(const sgt_params *p, int n, long nnz) {
   const int D = p->d, S = D == 3 ? 4 : D;
   const size_t np = (size_t)n * S;
   size_t b = 5 * np * 4;  // Y, Ynext, uY, gains, Frep
-  if (n >= SGT_CELL_MIN_N) b += (size_t)n * 16;  // sorted
+  if (n >= sgt_cell_min_n(D)) b += (size_t)n * 16;  // sorted
   int max_grid = p->max_grid > 0 ? p->max_grid : (D <= 2 ? 512 : 128);
   max_grid = std::min(D == 3 ? 256 : 512, std::max(16, max_grid));
   size_t M = 1;
@@ -2959,7 +2959,8 @@ constexpr int SGT_NA_MMAX_2D = 256;
 constexpr int SGT_NA_MMAX_1D = 1024;
 constexpr int SGT_NA_PARTS = 4096;        // per-block partials of the reductions
 constexpr int SGT_NA_COPY_NODES = 1 << 16;  // grid copies of the scatter mode
-static_assert(SGT_NA_MAX_N < SGT_CELL_MIN_N, "the no-alloc scratch has no cell mode");
+static_assert(SGT_NA_MAX_N < sgt_cell_min_n(1) && SGT_NA_MAX_N < sgt_cell_min_n(2),
+              "the no-alloc scratch has no cell mode");
 constexpr size_t na_al(size_t b) { return (b + 255) & ~(size_t)255; }
 // byte offsets of every buffer inside the array
 constexpr size_t NA_Y = 0;

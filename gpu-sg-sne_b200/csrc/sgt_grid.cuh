@@ -21,8 +21,8 @@
 // graph-capturable with fixed launch shapes.
 #pragma once
 #include "sgt_common.cuh"
+#include "sgt_grid_rules.h"
 
-#define SGT_HIST_MAX 4096  // cells held in shared memory by the binning kernels
 // Scatter mode: lanes that share a point.  The 4 nodes of a stencil row are
 // 64 contiguous bytes (32 in 1-D), so 4 lanes per point make one row one
 // request; 3-D spreads its 16 rows over 16 lanes.  100k points on 64^2 nodes:
@@ -36,9 +36,6 @@
 // instead of 76, 100k on 117^2 10.3 instead of 20.7.  k_spec_rows reads the copies
 // back, so a grid takes them only as it has adds per node.
 #define SGT_COPIES 32
-// Points from which a dense grid is sorted by cell.  Below, scatter mode is
-// faster even with every point in a few hundred cells.
-#define SGT_CELL_MIN_N 300000
 // Points a thread loads before it uses the first of them in the point loops
 // of the binning, S2G (cell mode) and G2S kernels: these kernels are bound by
 // load latency, not bandwidth, at a few warps per SM.
@@ -115,11 +112,7 @@ __device__ void sgt_finalize_grid(SgtState *st, const SgtJobParams &jp,
   long ncell = cells;
   if (D >= 2) ncell *= cells;
   if (D >= 3) ncell *= cells;
-  // cell mode: a large job whose cells fit the cell arrays and hold enough
-  // points each that one block reduction per chunk of a cell is cheaper than
-  // a reduction in L2 per point and node
-  const bool cell_mode = jp.n >= SGT_CELL_MIN_N && jp.cell_blocks > 0 && ncell <= SGT_HIST_MAX &&
-                         (long)jp.n >= 64L * ncell;
+  const bool cell_mode = jp.cell_blocks > 0 && sgt_cell_mode(jp.n, ncell);
   st->T = cell_mode ? 1 : 0;
   st->tiles_dim = cell_mode ? cells : 0;
   st->ntiles = cell_mode ? (int)ncell : 0;
