@@ -87,6 +87,9 @@ struct SgtJobParams {
   float eta;
   int mmax;           // largest FFT length per axis allocated
   long vc_nodes;      // nodes held by the grid copies of the scatter mode
+  int cell_dense;     // points per cell from which a grid is sorted by cell
+  int copy_adds;      // scatter mode: adds of an average node per copy
+  int copies_max;     // scatter mode: most copies
   int chunk_cap;      // max chunks held by the chunk array
   int chunk_min;      // cell mode: fewest points per chunk (0: 1024, 256 in 3-D)
   int conv_max;       // largest N that k_spec_* convolve

@@ -83,6 +83,7 @@ struct sgt_job {
   int2 *pairs_alt = nullptr;
   float *gains_alt = nullptr;
   long host_iter = 0;  // iterations since the last set_y
+  bool full_batch = false;  // st's grid was decided by the rules of a full fused launch
   int relayouts = 0;
   float *Y = nullptr, *Ynext = nullptr, *uY = nullptr, *gains = nullptr,
         *Frep = nullptr, *Fattr = nullptr;
@@ -451,11 +452,9 @@ static sgt_status job_shapes(sgt_job *J) {
   // so one block per SM (each with more points) finishes sooner than four.
   // 1.3M points (67M nonzeros): 337 against 351 us per iteration; 400k
   // (20M): 114 against 119.
-  if (J->jp.cell_blocks > 0) {
-    J->jp.cell_blocks = J->nnz >= SGT_CHAIN_NARROW_NNZ ? nsm : J->nb_pts;
-    J->nb_s2gc = std::min(J->nb_s2gc, J->jp.cell_blocks);
-    J->nb_g2s = J->jp.cell_blocks;
-  }
+  J->nb_g2s = J->nnz >= SGT_CHAIN_NARROW_NNZ ? nsm : J->nb_pts;
+  J->nb_s2gc = std::min(J->nb_s2gc, J->nb_g2s);
+  if (J->jp.cell_blocks > 0) J->jp.cell_blocks = J->nb_g2s;
   // scatter mode: a group of SGT_LPP lanes per point, up to 2048 threads an SM
   const long groups = ((long)J->n * SGT_LPP(D) + SGT_THREADS - 1) / SGT_THREADS;
   const long ggroups = ((long)J->n * SGT_GLPP + SGT_THREADS - 1) / SGT_THREADS;
@@ -518,7 +517,8 @@ static sgt_status job_alloc(sgt_job *J) {
   // the sort of the cell mode, for the jobs that can take it (a shard decides
   // by the points of the whole embedding); job_shapes sets its block count
   J->jp.cell_blocks = std::max(J->n, J->n_gather) >= sgt_cell_min_n(D) ? 1 : 0;
-  if (J->jp.cell_blocks > 0) CKS(jalloc(J, &J->sorted, (size_t)J->n));
+  if (J->jp.cell_blocks > 0 || J->n >= SGT_BATCH_CELL_MIN_N)
+    CKS(jalloc(J, &J->sorted, (size_t)J->n));
   CKS(jalloc(J, &J->st, 1));
   J->st_host = new SgtState();
   CK(cudaEventCreateWithFlags(&J->ev_fork, cudaEventDisableTiming));
@@ -563,6 +563,9 @@ static void fill_jp(sgt_job *J) {
   J->jp.early_iter = p.early_iter;
   J->jp.mom_switch = 250;
   J->jp.eta = 200.0f;
+  J->jp.cell_dense = SGT_CELL_DENSE;
+  J->jp.copy_adds = SGT_COPY_ADDS;
+  J->jp.copies_max = SGT_COPIES;
 }
 
 // empty scratch job for operator calls (no P)
@@ -1364,10 +1367,27 @@ sgt_status sgt_job_set_y(sgt_job *J, const float *y, int layout, int mem_is_devi
   CK(cudaMemsetAsync(J->tile_count, 0, sizeof(int) * SGT_HIST_MAX, s));
   CKS(init_stats(J, s, 1));
   J->host_iter = 0;
+  J->full_batch = false;
   if (staging) {
     CK(cudaStreamSynchronize(s));
     CK(cudaFreeAsync(staging, s));
   }
+  return SGT_OK;
+}
+
+// Before launches that follow the job's own rules, on their stream: the grid
+// decision by those, if a full fused launch took the last one (it may have
+// chosen to sort by cell, which the job's own launches may not be able to).
+static sgt_status own_grid(sgt_job *J, cudaStream_t s) {
+  sgt_ctx *ctx = J->ctx;
+  if (!J->full_batch) return SGT_OK;
+  switch (J->d) {
+    case 1: k_regrid<1><<<1, 1, 0, s>>>(J->st, J->jp); break;
+    case 2: k_regrid<2><<<1, 1, 0, s>>>(J->st, J->jp); break;
+    default: k_regrid<3><<<1, 1, 0, s>>>(J->st, J->jp); break;
+  }
+  CK(cudaGetLastError());
+  J->full_batch = false;
   return SGT_OK;
 }
 
@@ -1484,6 +1504,7 @@ sgt_status sgt_job_run(sgt_job *J, int iters) {
   if (!J || iters < 0) return SGT_ERR_INVALID_ARG;
   sgt_ctx *ctx = J->ctx;
   CK(cudaSetDevice(ctx->device));
+  CKS(own_grid(J, ctx->stream));
   const int every = J->p.relayout_every, kl_every = J->p.kl_every;
   // runs of iterations between the points where host work happens (a
   // relayout before every `every`-th iteration, a KL after every
@@ -1539,7 +1560,7 @@ struct sgt_batch {
   std::vector<sgt_job *> jobs;
   int R = 1;
   cudaGraphExec_t exec_r = nullptr, exec_1 = nullptr;
-  bool fused = false;
+  bool fused = false, full = false;
   std::vector<BatchGroup> groups;
   void *dmem = nullptr;  // the groups' view and prefix tables
 };
@@ -1571,9 +1592,10 @@ static sgt_status batch_build(sgt_batch *b, const std::vector<cudaGraph_t> &iter
 
 }  // extern "C"
 
-static void stage_blocks(const sgt_job *J, int *b);
+static void stage_blocks(const sgt_job *J, int cell_blocks, int *b);
 
-static SgtJobView job_view(const sgt_job *J) {
+// full: the fused launch fills the GPU (SGT_BATCH_FULL)
+static SgtJobView job_view(const sgt_job *J, bool full) {
   SgtJobView v;
   memset(&v, 0, sizeof(v));
   v.Ynext_c = J->Ynext;
@@ -1600,8 +1622,14 @@ static SgtJobView job_view(const sgt_job *J) {
   v.pairs = J->pairs;
   v.jp = J->jp;
   v.n = J->n;
+  if (full) {
+    v.jp.copy_adds = SGT_BATCH_COPY_ADDS;
+    v.jp.copies_max = SGT_BATCH_COPIES;
+    v.jp.cell_dense = SGT_BATCH_CELL_DENSE;
+    if (J->n >= SGT_BATCH_CELL_MIN_N) v.jp.cell_blocks = J->nb_g2s;
+  }
   int bl[FS_STAGES];
-  stage_blocks(J, bl);
+  stage_blocks(J, v.jp.cell_blocks, bl);
   v.nb_s2g = std::max(1, bl[FS_S2G_CELL]);  // the binning sizes chunks for the fused S2G grid
   // short chunks: a chunk is one block's serial work in S2G, and in a fused
   // launch the slowest block of the smallest jobs sets the stage's length
@@ -1618,16 +1646,16 @@ static SgtJobView job_view(const sgt_job *J) {
 // G2S, per 2048 points in the other point passes, up to the job's own grid,
 // and the FFT passes a block per 8 lines of a 64-point grid (they loop over
 // larger ones).
-static void stage_blocks(const sgt_job *J, int *b) {
+static void stage_blocks(const sgt_job *J, int cell_blocks, int *b) {
   for (int k = 0; k < FS_STAGES; k++) b[k] = 0;
   const int work = std::max(1, (J->n + 2047) / 2048);
   const int fine = (J->d == 3 ? 16 : 8) * work;
   b[FS_SCATTER] = std::min(J->nb_scat, fine);
   b[FS_SPEC] = std::min(J->nb_spec, J->d == 3 ? 128 : (J->d == 2 ? 48 : 1));
-  if (J->jp.cell_blocks > 0) {
-    b[FS_BIN_COUNT] = std::min(J->jp.cell_blocks, work);
-    b[FS_G2S] = std::min(J->nb_g2s, 2 * work);
-    b[FS_BIN_SCATTER] = std::min(J->jp.cell_blocks, work);
+  if (cell_blocks > 0) {
+    b[FS_BIN_COUNT] = std::min(cell_blocks, work);
+    b[FS_G2S] = std::min(cell_blocks, 2 * work);
+    b[FS_BIN_SCATTER] = std::min(cell_blocks, work);
     b[FS_S2G_CELL] = std::min(J->nb_s2gc, 2 * work);
   }
   const int rows64 = J->d == 3 ? (2 * 64 * 64 + 128 * 128) / 8 : (2 * 64 + 128) / 8;
@@ -1657,10 +1685,14 @@ struct FusedImage {
     std::vector<std::pair<size_t, size_t>> spmv;  // (views, prefix) per G
   };
   std::vector<Off> offs;
+  bool full = false;  // SGT_BATCH_FULL points or more
   size_t bytes() const { return sizeof(SgtJobView) * views.size() + sizeof(int) * ints.size(); }
 };
 
 static void build_fused_image(const std::vector<sgt_job *> &jobs, FusedImage &im) {
+  long points = 0;
+  for (sgt_job *J : jobs) points += J->n;
+  im.full = points >= SGT_BATCH_FULL;
   for (int D = 1; D <= 3; D++) {
     std::vector<sgt_job *> js;
     for (sgt_job *J : jobs)
@@ -1672,16 +1704,16 @@ static void build_fused_image(const std::vector<sgt_job *> &jobs, FusedImage &im
     FusedImage::Off o;
     o.views = im.views.size();
     for (sgt_job *J : js) {
-      im.views.push_back(job_view(J));
+      im.views.push_back(job_view(J, im.full));
       g.smem_fft = std::max(g.smem_fft, J->smem_fft2);
     }
     for (int k = 0; k < FS_STAGES; k++) {
       o.prefix[k] = im.ints.size();
       int acc = 0;
       im.ints.push_back(0);
-      for (sgt_job *J : js) {
+      for (size_t q = 0; q < js.size(); q++) {
         int bl[FS_STAGES];
-        stage_blocks(J, bl);
+        stage_blocks(js[q], im.views[o.views + q].jp.cell_blocks, bl);
         acc += bl[k];
         im.ints.push_back(acc);
       }
@@ -1699,7 +1731,7 @@ static void build_fused_image(const std::vector<sgt_job *> &jobs, FusedImage &im
       int acc = 0;
       im.ints.push_back(0);
       for (sgt_job *J : gj) {
-        im.views.push_back(job_view(J));
+        im.views.push_back(job_view(J, im.full));
         acc += (int)(((long)J->n * G + SGT_THREADS - 1) / SGT_THREADS);
         im.ints.push_back(acc);
       }
@@ -1741,6 +1773,7 @@ static sgt_status batch_fused_tables(sgt_batch *b) {
   CKS(bind_fused_image(ctx, im, b->dmem, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));  // the host image goes out of scope
   b->groups = im.groups;
+  b->full = im.full;
   for (BatchGroup &g : b->groups) {
     CK(cudaStreamCreateWithFlags(&g.chain, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&g.side, cudaStreamNonBlocking));
@@ -1896,6 +1929,8 @@ sgt_status sgt_batch_step(sgt_ctx *ctx, int njobs, sgt_job *const *jobs, int ite
       default: CKS(fused_attributes<3>(ctx, g)); break;
     }
   }
+  if (!im.full)
+    for (sgt_job *J : js) CKS(own_grid(J, s));
   sgt_status st = SGT_OK;
   for (int it = 0; it < iters && st == SGT_OK; it++) {
     for (BatchGroup &g : im.groups) {
@@ -1912,7 +1947,10 @@ sgt_status sgt_batch_step(sgt_ctx *ctx, int njobs, sgt_job *const *jobs, int ite
   // the groups' views live in ctx->step_tables; their host image goes out
   // of scope here (the uploads were staged at the call)
   if (st == SGT_OK)
-    for (sgt_job *J : js) J->host_iter += iters;
+    for (sgt_job *J : js) {
+      J->host_iter += iters;
+      J->full_batch = im.full;
+    }
   return st;
 }
 
@@ -1978,10 +2016,15 @@ sgt_status sgt_batch_run(sgt_batch *b, int iters) {
   sgt_ctx *ctx = b->ctx;
   CK(cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;
+  if (!b->full)
+    for (sgt_job *J : b->jobs) CKS(own_grid(J, s));
   int left = iters;
   for (; left >= b->R; left -= b->R) CK(cudaGraphLaunch(b->exec_r, s));
   for (; left > 0; left--) CK(cudaGraphLaunch(b->R > 1 ? b->exec_1 : b->exec_r, s));
-  for (sgt_job *J : b->jobs) J->host_iter += iters;
+  for (sgt_job *J : b->jobs) {
+    J->host_iter += iters;
+    J->full_batch = b->full;
+  }
   return SGT_OK;
 }
 
@@ -2242,7 +2285,7 @@ size_t sgt_job_footprint(const sgt_params *p, int n, long nnz) {
   const int D = p->d, S = D == 3 ? 4 : D;
   const size_t np = (size_t)n * S;
   size_t b = 5 * np * 4;  // Y, Ynext, uY, gains, Frep
-  if (n >= sgt_cell_min_n(D)) b += (size_t)n * 16;  // sorted
+  if (n >= std::min(sgt_cell_min_n(D), SGT_BATCH_CELL_MIN_N)) b += (size_t)n * 16;  // sorted
   int max_grid = p->max_grid > 0 ? p->max_grid : (D <= 2 ? 512 : 128);
   max_grid = std::min(D == 3 ? 256 : 512, std::max(16, max_grid));
   size_t M = 1;
@@ -2389,7 +2432,7 @@ extern "C" sgt_status sgt_job_run_timed(sgt_job *J, int iters, double *time_info
   CK(cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;
   cudaEvent_t ev[7] = {};
-  sgt_status st = SGT_OK;
+  sgt_status st = own_grid(J, s);
   for (int i = 0; i < 7 && st == SGT_OK; i++)
     if (cudaEventCreate(&ev[i]) != cudaSuccess) st = fail(ctx, SGT_ERR_CUDA, "event create");
   const int every = J->p.relayout_every, kl_every = J->p.kl_every;
@@ -2437,6 +2480,7 @@ extern "C" sgt_status sgt_job_profile(sgt_job *J, int iters, double *stage_ms) {
   cudaStream_t s = ctx->stream;
   cudaEvent_t ev[7];
   for (int i = 0; i < 7; i++) CK(cudaEventCreate(&ev[i]));
+  CKS(own_grid(J, s));
   for (int it = 0; it < iters; it++) {
     // the kernels of an iteration, one stage after another on one stream
     // (the captured iteration runs the SpMV beside the repulsion instead)

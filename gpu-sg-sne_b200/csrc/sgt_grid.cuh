@@ -31,11 +31,11 @@
 // Lanes per point of the gather: 4 in 3-D too.  Loads of 16 rows fly in one
 // lane as well as in 16, and the stencil is worked out 4 times instead of 16.
 #define SGT_GLPP 4
-// Scatter mode: most copies of the grid.  L2 serialises the reductions that
-// meet on one node; with 32 copies 60k points on 16^2 nodes take 10.5 us
-// instead of 76, 100k on 117^2 10.3 instead of 20.7.  k_spec_rows reads the copies
-// back, so a grid takes them only as it has adds per node.
+// Scatter mode: most copies of the grid, and adds per node and copy, of a job
+// launched alone. With 32 copies 60k points on 16^2 nodes take 10.5 us instead
+// of 76, 100k on 117^2 10.3 instead of 20.7.
 #define SGT_COPIES 32
+#define SGT_COPY_ADDS 16
 // Points a thread loads before it uses the first of them in the point loops
 // of the binning, S2G (cell mode) and G2S kernels: these kernels are bound by
 // load latency, not bandwidth, at a few warps per SM.
@@ -112,20 +112,15 @@ __device__ void sgt_finalize_grid(SgtState *st, const SgtJobParams &jp,
   long ncell = cells;
   if (D >= 2) ncell *= cells;
   if (D >= 3) ncell *= cells;
-  const bool cell_mode = jp.cell_blocks > 0 && sgt_cell_mode(jp.n, ncell);
+  const bool cell_mode = jp.cell_blocks > 0 && sgt_cell_mode(jp.n, ncell, jp.cell_dense);
   st->T = cell_mode ? 1 : 0;
   st->tiles_dim = cell_mode ? cells : 0;
   st->ntiles = cell_mode ? (int)ncell : 0;
-  // scatter mode: a copy per 16 adds that an average node receives, a power
-  // of two that fits the buffer
   long nodes = N;
   if (D >= 2) nodes *= N;
   if (D >= 3) nodes *= N;
-  const long adds = ((long)jp.n << (2 * D)) / nodes;
-  int copies = 1;
-  while (copies < SGT_COPIES && 16L * copies < adds && 2L * copies * nodes <= jp.vc_nodes)
-    copies *= 2;
-  st->copies = copies;
+  st->copies =
+      sgt_copies(((long)jp.n << (2 * D)) / nodes, nodes, jp.vc_nodes, jp.copy_adds, jp.copies_max);
 }
 
 // Scaled coordinate exactly as CU/nuconv.cu:9-36: (y - miny)/maxy, clamp to
@@ -275,6 +270,13 @@ k_init_stats(const typename Vec<D>::T *__restrict__ Y, int n, SgtState *st,
   }
   block_finish_stats<D>(blockIdx.x, gridDim.x, st, jp, &st->done_init, centre != 0, mn, mx, sm,
                         part_min, part_max, part_sum);
+}
+
+// The grid decision again, from the same statistics, by other parameters: a job
+// that leaves a batch may stand in a mode that its own launches do not run.
+template <int D>
+__global__ void k_regrid(SgtState *st, SgtJobParams jp) {
+  sgt_finalize_grid<D>(st, jp, st->minv, st->maxv, st->sum, true);
 }
 
 // ---------------------------------------------------------------------------

@@ -27,6 +27,32 @@ constexpr int SGT_CELL_DENSE = 64;
 // Whether n points on ncell cells are sorted, for a job that can (its cells fit
 // the cell arrays, and one block reduction per chunk of a cell is cheaper than
 // a reduction in L2 per point and node).
-SGT_RULE bool sgt_cell_mode(long n, long ncell) {
-  return ncell <= SGT_HIST_MAX && n >= (long)SGT_CELL_DENSE * ncell;
+SGT_RULE bool sgt_cell_mode(long n, long ncell, int dense) {
+  return ncell <= SGT_HIST_MAX && n >= (long)dense * ncell;
 }
+
+// Copies of the grid in scatter mode: one per copy_adds adds that an average
+// node receives, a power of two up to copies_max that fits vc_nodes. L2
+// serialises the reductions that meet on one node, so copies pay while a job has
+// the GPU to itself; k_spec_rows reads and clears them all.
+SGT_RULE int sgt_copies(long adds, long nodes, long vc_nodes, int copy_adds, int copies_max) {
+  int copies = 1;
+  while (copies < copies_max && (long)copy_adds * copies < adds && 2L * copies * nodes <= vc_nodes)
+    copies *= 2;
+  return copies;
+}
+
+// A fused launch whose jobs hold SGT_BATCH_FULL points together fills the GPU:
+// what counts is the work of all jobs, not the length of one job's chain. There
+// fewer copies pay (their fold is memory traffic) and large jobs sort from fewer
+// points on. 64 jobs of 2,000 to 200,000 points, half 3-D, 1000 iterations: 20.4
+// embeddings/s by the rules above, 22.6 with SGT_BATCH_COPY_ADDS, 21.6 with the
+// sort, 25.8 with both; sorting from 10,000 to 100,000 points on, or dense from
+// 16, within 1 %. us per iteration by the rules above / by these: 24 jobs of 2,000
+// to 40,000 points 346 / 322 (16 points per axis), 661 / 628 (32 in 3-D); 16 of
+// 100,000 to 200,000 1410 / 1078, 1857 / 1609. Below SGT_BATCH_FULL they lose: 2
+// jobs of 20,000 and 50,000 99 / 118, 170 / 198.
+constexpr long SGT_BATCH_FULL = 150000;
+constexpr int SGT_BATCH_COPY_ADDS = 64, SGT_BATCH_COPIES = 8;
+constexpr long SGT_BATCH_CELL_MIN_N = 75000;
+constexpr int SGT_BATCH_CELL_DENSE = 32;

@@ -31,7 +31,7 @@ def rules(tmp_path_factory):
     src = d / "r.cpp"
     src.write_text('#include "sgt_grid_rules.h"\n'
                    'extern "C" int cell(int d, long n, long ncell) {\n'
-                   '  return n >= sgt_cell_min_n(d) && sgt_cell_mode(n, ncell);\n'
+                   '  return n >= sgt_cell_min_n(d) && sgt_cell_mode(n, ncell, SGT_CELL_DENSE);\n'
                    '}\n')
     so = d / "r.so"
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, str(src), "-o",
