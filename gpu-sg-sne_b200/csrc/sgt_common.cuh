@@ -93,6 +93,7 @@ struct SgtJobParams {
   int chunk_cap;      // max chunks held by the chunk array
   int chunk_min;      // cell mode: fewest points per chunk (0: 1024, 256 in 3-D)
   int conv_max;       // largest N that k_spec_* convolve
+  int conv_work;      // 3-D: they convolve grids of 4 N^4 / M^3 below this
   int cell_blocks;    // blocks that work in cell mode (0: no cell mode)
 };
 

@@ -427,6 +427,7 @@ static sgt_status job_shapes(sgt_job *J) {
   // (few blocks beside a long SpMV: even a block with nothing to do waits for
   // a slot there)
   const bool beside = J->nnz >= SGT_LONG_SPMV_NNZ;
+  J->jp.conv_work = beside ? SGT_CONV_WORK_LONG : SGT_CONV_WORK;
   J->nb_spec = D == 1 ? 2 : (D == 3 ? std::min(4 * nsm, cm * cm) : (beside ? 64 : cm));
   J->nb_spec_y = 2 * nsm;
   J->nb_conv = D == 1 ? (cm + 7) / 8 : (D == 3 ? std::min(3 * nsm, cm * ct) : std::min(ct, beside ? 64 : cm));
@@ -533,7 +534,7 @@ static sgt_status job_alloc(sgt_job *J) {
   SgtState &st0 = *J->st_host;
   st0.N = 16;
   st0.M = 32;
-  st0.direct = st0.N <= J->jp.conv_max ? 1 : 0;
+  st0.direct = sgt_plain_conv(D, st0.N, st0.M, J->jp.conv_max, SGT_CONV_WORK) ? 1 : 0;
   st0.copies = 1;
   st0.maxy = st0.scale = (float)(st0.N - 3);
   st0.inv_hi = st0.h_eff = 1.0f;
@@ -720,7 +721,7 @@ static sgt_status enqueue_gather_part(sgt_job *J, cudaStream_t s, cudaEvent_t *e
   if (J->Ygather)  // a shard: the grid has been summed over the ranks meanwhile
     CK(launch_chain(false, k_spec_rows<D>, J->nb_spec, SGT_THREADS, 0, s, (const SgtState *)J->st,
                     (NT *)J->Vc, (NT *)J->V, J->W, SGT_SPEC_TRANSFORM));
-  const bool fft = J->nmax > J->jp.conv_max;  // some grid of this job takes the FFT passes
+  const bool fft = sgt_needs_fft(D, J->nmax, J->jp.conv_max);
   if (fft && !ev && J->ev_fft && J->nnz < SGT_LONG_SPMV_NNZ) {
     // The two convolutions, each with its G2S, on branches of their own: the
     // kernels of the one that this grid does not take return at once, and
@@ -1626,6 +1627,7 @@ static SgtJobView job_view(const sgt_job *J, bool full) {
     v.jp.copy_adds = SGT_BATCH_COPY_ADDS;
     v.jp.copies_max = SGT_BATCH_COPIES;
     v.jp.cell_dense = SGT_BATCH_CELL_DENSE;
+    v.jp.conv_work = SGT_CONV_WORK_BATCH;
     if (J->n >= SGT_BATCH_CELL_MIN_N) v.jp.cell_blocks = J->nb_g2s;
   }
   int bl[FS_STAGES];
@@ -1661,7 +1663,7 @@ static void stage_blocks(const sgt_job *J, int cell_blocks, int *b) {
   const int rows64 = J->d == 3 ? (2 * 64 * 64 + 128 * 128) / 8 : (2 * 64 + 128) / 8;
   b[FS_CONV] = std::min(J->nb_conv, J->d == 3 ? 100 : 48);
   if (J->d == 3) b[FS_SPEC_Y] = std::min(J->nb_spec_y, 64);
-  const bool fft = J->d >= 2 && J->nmax > J->jp.conv_max;
+  const bool fft = J->d >= 2 && sgt_needs_fft(J->d, J->nmax, J->jp.conv_max);
   if (fft) b[FS_FFT_X] = std::min(J->nb_fft_rows, rows64);
   if (fft && J->d == 3) b[FS_FFT_MID_FWD] = b[FS_FFT_MID_INV] = std::min(J->nb_fft, 128);
   if (fft) {

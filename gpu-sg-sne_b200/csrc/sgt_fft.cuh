@@ -9,8 +9,8 @@
 // offsets |x - x'| <= N-1 <= M/2, so K_c[r] = K(min(r, M-r)) reproduces it.
 // Two real charge channels ride in one complex plane (K_c is real and even,
 // so its transform is real and the channels separate after the inverse).
-// Grids up to SgtJobParams::conv_max points per axis take plain transforms of
-// length 2N instead (the k_spec kernels at the end of this file).
+// Grids that sgt_plain_conv picks take plain transforms of length 2N instead (the
+// k_spec kernels further down).
 //
 // FFTs are register-resident: one warp owns one line of M <= 1024 points, a
 // lane holds the E = M/32 points lane + 32 e; butterflies whose span holds
@@ -26,6 +26,7 @@
 // decision, so the chain replays inside a CUDA graph as N changes.
 #pragma once
 #include "sgt_common.cuh"
+#include "sgt_grid_rules.h"
 
 #define SGT_FFT_COLS 8  // columns per CTA in column passes (one per warp)
 #define SGT_FFT_PAD 1   // float2 padding per staged column
@@ -218,11 +219,8 @@ __device__ __forceinline__ float2 node_plane(const typename Node<D>::T &v, int p
 // shared memory in 2-D, for which a block waits until a whole SM has drained
 // of the concurrent SpMV.  The plain transforms cost more operations than FFTs
 // and still only a few microseconds, with 256 threads and 15 KB a block.
-// 3-D grids above 80 points per axis take the FFT passes: the plain transforms
-// grow with N^4 (whole iterations of 8,000 points, plain transforms against
-// FFTs: 52 points per axis 170 / 250 us, 75 560 / 744, 98 1589 / 1369).
+// In 3-D the plain transforms grow with N^4; sgt_plain_conv draws the line.
 // ---------------------------------------------------------------------------
-#define SGT_SPEC_MAX(D) ((D) == 1 ? 512 : ((D) == 2 ? 128 : 80))
 // k_spec_rows in one go, or its halves (the charge grid of a row-split
 // embedding is summed over the ranks between them)
 #define SGT_SPEC_BOTH 0

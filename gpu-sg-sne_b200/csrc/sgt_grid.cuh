@@ -106,7 +106,7 @@ __device__ void sgt_finalize_grid(SgtState *st, const SgtJobParams &jp,
   const double inv = (double)(N - 3) / (double)maxy;
   st->inv_hi = (float)inv;
   st->inv_lo = (float)(inv - (double)st->inv_hi);
-  st->direct = N <= jp.conv_max ? 1 : 0;
+  st->direct = sgt_plain_conv(D, N, M, jp.conv_max, jp.conv_work) ? 1 : 0;
   st->h_eff = __fdiv_rn(maxy, (float)(n1 - 1) - 1.1920928955078125e-7f);
   const int cells = n1 - 1;  // floor bins lie in [0, n1-2]
   long ncell = cells;

@@ -56,3 +56,28 @@ constexpr long SGT_BATCH_FULL = 150000;
 constexpr int SGT_BATCH_COPY_ADDS = 64, SGT_BATCH_COPIES = 8;
 constexpr long SGT_BATCH_CELL_MIN_N = 75000;
 constexpr int SGT_BATCH_CELL_DENSE = 32;
+
+// Largest grids, in points per axis, that the plain transforms (k_spec_*) hold;
+// beyond, and for 3-D grids that sgt_plain_conv leaves to them, the FFT passes.
+#define SGT_SPEC_MAX(D) ((D) == 1 ? 512 : ((D) == 2 ? 128 : 80))
+
+// 3-D: the plain transforms cost N^4, the FFT passes M^3 with M = 64, 96, 128,
+// 192 for N up to 32, 48, 64, 96. The plain ones have the shorter chain, which
+// counts while the chain is alone; beside a long SpMV their work counts too. us
+// per iteration, plain / FFT, at N points per axis: 2,000 points 25: 46 / 54, 39:
+// 86 / 104, 48: 152 / 113, 54: 180 / 165, 63: 282 / 184, 72: 489 / 640; 30,000
+// points (1.5M nonzeros) 40: 123 / 130, 48: 173 / 135, 64: 348 / 201, 72: 561 /
+// 640; 100,000 (5M) 25: 122 / 121, 32: 146 / 123, 40: 181 / 176, 48: 248 / 180, 56:
+// 309 / 235, 66: 517 / 644, 72: 694 / 679, 78: 755 / 715; 299,000 (15M) 40: 287 /
+// 300, 48: 358 / 294, 64: 593 / 384.
+// In a full batch (64 jobs, grids of 20 to 48 points at the end) limits of 24,
+// 32, 40, 48 and 80 points take 3220, 3191, 3097, 3090, 3076 ms.
+constexpr int SGT_CONV_WORK = 16, SGT_CONV_WORK_LONG = 11, SGT_CONV_WORK_BATCH = 24;  // of 4 N^4 / M^3
+SGT_RULE bool sgt_plain_conv(int d, int N, int M, int conv_max, int conv_work) {
+  if (N > conv_max) return false;
+  return d < 3 || 4L * N * N * N * N < (long)conv_work * M * M * M;
+}
+// whether some grid of up to nmax points per axis takes the FFT passes
+SGT_RULE bool sgt_needs_fft(int d, int nmax, int conv_max) {
+  return nmax > conv_max || (d == 3 && nmax > 28);
+}

@@ -25,6 +25,20 @@ CELL = [
 ]
 
 
+# 3-D: (nonzeros of P in millions, points per axis, FFT length, plain transforms,
+# FFT passes)
+CONV = [
+    (0.1, 25, 64, 46, 54), (0.1, 28, 64, 62, 55), (0.1, 39, 96, 86, 104), (0.1, 48, 96, 152, 113),
+    (0.1, 63, 128, 282, 184), (0.1, 72, 192, 489, 640), (1.5, 20, 64, 65, 76),
+    (1.5, 32, 64, 99, 81), (1.5, 40, 96, 121, 128), (1.5, 48, 96, 173, 135),
+    (1.5, 56, 128, 238, 192), (1.5, 64, 128, 348, 201), (1.5, 66, 192, 438, 623),
+    (5, 32, 64, 143, 125), (5, 40, 96, 178, 172), (5, 48, 96, 248, 180), (5, 50, 128, 256, 226),
+    (5, 56, 128, 309, 235), (5, 66, 192, 517, 644), (5, 78, 192, 760, 715),
+    (15, 40, 96, 287, 300), (15, 48, 96, 358, 294), (15, 64, 128, 593, 384),
+    (15, 66, 192, 713, 795), (15, 78, 192, 1007, 872),
+]
+
+
 @pytest.fixture(scope="module")
 def rules(tmp_path_factory):
     d = tmp_path_factory.mktemp("rules")
@@ -32,6 +46,13 @@ def rules(tmp_path_factory):
     src.write_text('#include "sgt_grid_rules.h"\n'
                    'extern "C" int cell(int d, long n, long ncell) {\n'
                    '  return n >= sgt_cell_min_n(d) && sgt_cell_mode(n, ncell, SGT_CELL_DENSE);\n'
+                   '}\n'
+                   'extern "C" int plain(int d, int N, int M, int work) {\n'
+                   '  return sgt_plain_conv(d, N, M, SGT_SPEC_MAX(d),\n'
+                   '                        work ? SGT_CONV_WORK_LONG : SGT_CONV_WORK);\n'
+                   '}\n'
+                   'extern "C" int fft(int d, int nmax) {\n'
+                   '  return sgt_needs_fft(d, nmax, nmax < SGT_SPEC_MAX(d) ? nmax : SGT_SPEC_MAX(d));\n'
                    '}\n')
     so = d / "r.so"
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, str(src), "-o",
@@ -45,3 +66,21 @@ def rules(tmp_path_factory):
 def test_cell_mode(rules, d, n, N, by_cell, scattered):
     picked = bool(rules.cell(d, n, (N - 3) ** d))
     assert (by_cell if picked else scattered) < 1.1 * min(by_cell, scattered)
+
+
+@pytest.mark.parametrize("nnz,N,M,plain,fft", CONV)
+def test_convolution_of_3d_grids(rules, nnz, N, M, plain, fft):
+    picked = bool(rules.plain(3, N, M, int(nnz >= 3)))
+    # (28 points of a light job: 62 / 55, within two of 25's 46 / 54)
+    assert (plain if picked else fft) < 1.13 * min(plain, fft)
+
+
+def test_a_job_whose_grids_can_take_the_passes_has_them(rules):
+    sizes = [8, 9, 10, 11, 12, 13, 14, 15, 16, 20, 25, 26, 28, 32, 33, 35, 36, 39, 40, 42, 44, 45,
+             48, 49, 50, 52, 54, 55, 56, 60, 63, 64, 65, 66, 70, 72, 75, 77, 78, 80, 84, 88, 128]
+    lengths = [32, 64, 96, 128, 192, 256]
+    for d in (2, 3):
+        for nmax in sizes:
+            takes = any(not rules.plain(d, N, next(m for m in lengths if m >= 2 * N - 1), long)
+                        for N in sizes if N <= nmax for long in (0, 1))
+            assert rules.fft(d, nmax) >= takes
