@@ -565,7 +565,7 @@ static void fill_jp(sgt_job *J) {
   J->jp.mom_switch = 250;
   J->jp.eta = 200.0f;
   J->jp.cell_dense = SGT_CELL_DENSE;
-  J->jp.copy_adds = SGT_COPY_ADDS;
+  J->jp.copy_adds = sgt_copy_adds(J->d);
   J->jp.copies_max = SGT_COPIES;
 }
 

@@ -31,11 +31,6 @@
 // Lanes per point of the gather: 4 in 3-D too.  Loads of 16 rows fly in one
 // lane as well as in 16, and the stencil is worked out 4 times instead of 16.
 #define SGT_GLPP 4
-// Scatter mode: most copies of the grid, and adds per node and copy, of a job
-// launched alone. With 32 copies 60k points on 16^2 nodes take 10.5 us instead
-// of 76, 100k on 117^2 10.3 instead of 20.7.
-#define SGT_COPIES 32
-#define SGT_COPY_ADDS 16
 // Points a thread loads before it uses the first of them in the point loops
 // of the binning, S2G (cell mode) and G2S kernels: these kernels are bound by
 // load latency, not bandwidth, at a few warps per SM.

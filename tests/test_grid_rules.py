@@ -51,6 +51,11 @@ def rules(tmp_path_factory):
                    '  return sgt_plain_conv(d, N, M, SGT_SPEC_MAX(d),\n'
                    '                        work ? SGT_CONV_WORK_LONG : SGT_CONV_WORK);\n'
                    '}\n'
+                   'extern "C" int copies(int d, long n, int N) {\n'
+                   '  const long nodes = d == 2 ? (long)N * N : (long)N * N * N;\n'
+                   '  return sgt_copies((n << (2 * d)) / nodes, nodes, d == 2 ? 1l << 18 : 1l << 21,\n'
+                   '                    sgt_copy_adds(d), SGT_COPIES);\n'
+                   '}\n'
                    'extern "C" int fft(int d, int nmax) {\n'
                    '  return sgt_needs_fft(d, nmax, nmax < SGT_SPEC_MAX(d) ? nmax : SGT_SPEC_MAX(d));\n'
                    '}\n')
@@ -59,6 +64,7 @@ def rules(tmp_path_factory):
                     str(so)], check=True)
     lib = ctypes.CDLL(str(so))
     lib.cell.argtypes = [ctypes.c_int, ctypes.c_long, ctypes.c_long]
+    lib.copies.argtypes = [ctypes.c_int, ctypes.c_long, ctypes.c_int]
     return lib
 
 
@@ -84,3 +90,24 @@ def test_a_job_whose_grids_can_take_the_passes_has_them(rules):
             takes = any(not rules.plain(d, N, next(m for m in lengths if m >= 2 * N - 1), long)
                         for N in sizes if N <= nmax for long in (0, 1))
             assert rules.fft(d, nmax) >= takes
+
+
+# (d, points, points per axis, {adds per copy: us per iteration})
+@pytest.mark.parametrize("d,n,N,us", [
+    (3, 100000, 25, {16: 131, 32: 122, 64: 121, 128: 129}),
+    (3, 299000, 40, {16: 328, 32: 287, 64: 294, 128: 305}),
+    (3, 299000, 48, {16: 321, 32: 294, 64: 287, 128: 302}),
+    (3, 299000, 64, {16: 425, 32: 384, 64: 386, 128: 414}),
+    (2, 100000, 40, {16: 56, 32: 55, 64: 60, 128: 62}),
+    (2, 299000, 200, {16: 137, 32: 136, 64: 148, 128: 148}),
+])
+def test_grid_copies(rules, d, n, N, us):
+    adds, fit = (n << (2 * d)) // N ** d, (1 << (18 if d == 2 else 21)) // N ** d
+
+    def copies(per):
+        c = 1
+        while c < 32 and per * c < adds and 2 * c <= fit:
+            c *= 2
+        return c
+    picked = [t for per, t in us.items() if copies(per) == rules.copies(d, n, N)]
+    assert picked and min(picked) <= 1.06 * min(us.values())
