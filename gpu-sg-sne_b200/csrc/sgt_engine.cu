@@ -705,7 +705,8 @@ static sgt_status enqueue_scatter_part(sgt_job *J, cudaStream_t s, cudaEvent_t *
                     J->st, (const int4 *)J->chunks, (NT *)J->V));
   }
   CK(launch_chain(pdl, k_spec_rows<D>, J->nb_spec, SGT_THREADS, 0, s, (const SgtState *)J->st,
-                  (NT *)J->Vc, (NT *)J->V, J->W, J->Ygather ? SGT_SPEC_FOLD : SGT_SPEC_BOTH));
+                  (NT *)J->Vc, (NT *)J->V, J->W,
+                  J->Ygather || ev ? SGT_SPEC_FOLD : SGT_SPEC_BOTH));
   if (ev) CK(cudaEventRecord(ev[2], s));
   CK(cudaGetLastError());
   return SGT_OK;
@@ -718,7 +719,9 @@ static sgt_status enqueue_gather_part(sgt_job *J, cudaStream_t s, cudaEvent_t *e
   sgt_ctx *ctx = J->ctx;
   typedef typename Node<D>::T NT;
   const bool pdl = ev == nullptr;
-  if (J->Ygather)  // a shard: the grid has been summed over the ranks meanwhile
+  // a shard: the grid has been summed over the ranks meanwhile; stage times: the
+  // transforms along x are part of the convolution
+  if (J->Ygather || ev)
     CK(launch_chain(false, k_spec_rows<D>, J->nb_spec, SGT_THREADS, 0, s, (const SgtState *)J->st,
                     (NT *)J->Vc, (NT *)J->V, J->W, SGT_SPEC_TRANSFORM));
   const bool fft = sgt_needs_fft(D, J->nmax, J->jp.conv_max);

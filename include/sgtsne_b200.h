@@ -160,8 +160,8 @@ sgt_status sgt_job_run(sgt_job *job, int iters);
    (kl_minimization, CU/gradient_descend.cu:53-101, 208-247; CU/Frep.cu:
    81-125; CU/nuconv.cu:37-112): j = 0 attractive term, 1 S2G, 2 G2G, 3 G2S,
    4 forces and update, 5 S2G to G2S, 6 centring, grid decision and binning.
-   Without a sort the scatter of the charges is part of slot 6 and slot 1 is
-   empty.
+   Without a sort the scatter of the charges is part of slot 6 and slot 1 sums
+   the copies of the charge grid.
    Synchronises once per iteration; time_info may be NULL. */
 sgt_status sgt_job_run_timed(sgt_job *job, int iters, double *time_info);
 /* Capture and instantiate the iteration graphs sgt_job_run launches (one
