@@ -2142,8 +2142,12 @@ sgt_status sgt_shard_create(sgt_ctx *ctx, const sgt_params *params, int n_all, i
     return fail(ctx, SGT_ERR_UNSUPPORTED, "sgt_shard_create: shards take P in CSR format");
   if (params->relayout_every > 0 || params->kl_every > 0)
     return fail(ctx, SGT_ERR_UNSUPPORTED, "sgt_shard_create: no relayout or in-loop KL");
+  // the rows keep the caller's order: the coordinates are the caller's array (one
+  // rank's shard of every row would otherwise be put in locality order)
+  sgt_params sp = *params;
+  sp.locality_order = 0;
   sgt_job *J = nullptr;
-  CKS(job_create_impl(ctx, params, nrows, n_all, rowptr, col, val, mem_is_device, &J));
+  CKS(job_create_impl(ctx, &sp, nrows, n_all, rowptr, col, val, mem_is_device, &J));
   const size_t need = (size_t)J->nmax * (J->d >= 2 ? J->nmax : 1) * (J->d >= 3 ? J->nmax : 1) *
                       (J->d == 1 ? 2 : 4);
   if (grid_floats < need) {
