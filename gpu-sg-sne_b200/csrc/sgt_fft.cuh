@@ -218,7 +218,7 @@ __device__ __forceinline__ float2 node_plane(const typename Node<D>::T &v, int p
 // power of two or three times one, and their column pass needs 100 KB of
 // shared memory in 2-D, for which a block waits until a whole SM has drained
 // of the concurrent SpMV.  The plain transforms cost more operations than FFTs
-// and still only a few microseconds, with 256 threads and 15 KB a block.
+// and still only a few microseconds, with 256 threads and 13 to 22 KB a block.
 // In 3-D the plain transforms grow with N^4; sgt_plain_conv draws the line.
 // ---------------------------------------------------------------------------
 // k_spec_rows in one go, or its halves (the charge grid of a row-split
@@ -465,8 +465,8 @@ __device__ __forceinline__ void k_spec_y_body(int vb_, int vg_, const SgtState *
     sgt_pdl_wait();
     return;
   }
-  __shared__ float2 tw[2 * 128];
-  __shared__ float4 in[128 * FS * 2];
+  __shared__ float2 tw[2 * SGT_SPEC_MAX(3)];
+  __shared__ float4 in[SGT_SPEC_MAX(3) * FS * 2];
   const SpecBuf<3> B(W, N);
   spec_twiddles(tw, M);
   const int t = threadIdx.x;

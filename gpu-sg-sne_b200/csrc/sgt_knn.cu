@@ -295,8 +295,9 @@ __global__ void k_knn_norms(const float *__restrict__ X, int n, int dim, float *
 // hi/lo images of the points in blocks of `rows` ([block][part][unit][row],
 // 8 dimensions of 2 bytes), as queries (ones in columns dim .. dim + 2 of the
 // hi part) or candidates (-|c|^2/2 in three BF16 terms there).  Unused columns
-// and rows past n are zero, but candidate rows past n have the key -inf, which
-// no threshold admits.
+// and rows past n are zero, but candidate rows past n have -inf in column dim of
+// the hi part: their key is -inf in one term, and NaN in three (the lo part of a
+// query is 0 there). No threshold admits either: keys are taken by v > threshold.
 __global__ void k_knn_split(const float *__restrict__ X, const float *__restrict__ nrm, int n,
                             int dim, int U, int rows, int nblk, int candidates,
                             uint4 *__restrict__ img) {

@@ -39,7 +39,8 @@ def get(S, job, n, d):
 CASES = [
     (2, [(80000, 12.0), (75000, 46.0), (74999, 12.0), (3000, 30.0), (1500, 140.0)]),
     (2, [(80000, 60.0), (90000, 12.0)]),
-    (3, [(80000, 12.0), (76000, 30.0), (2500, 12.0), (2000, 46.0), (1500, 90.0)]),
+    (3, [(80000, 12.0), (76000, 30.0), (2500, 12.0), (2000, 46.0), (1500, 77.0),
+         (1500, 90.0)]),
     (1, [(100000, 12.0), (80000, 300.0), (2000, 40.0)]),
 ]
 
