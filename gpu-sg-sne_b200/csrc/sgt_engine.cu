@@ -644,12 +644,12 @@ static sgt_status enqueue_g2g_fft(sgt_job *J, cudaStream_t s, bool first_pdl, bo
                     (const SgtState *)J->st, (const NT *)J->V, J->W));
     if constexpr (D == 3)
       CK(launch_chain(pdl, k_fft_cols<D, MODE_MID_FWD>, J->nb_fft, SGT_THREADS, J->smem_fft2, s,
-                      (const SgtState *)J->st, J->W, (const NT *)J->V, (NT *)J->Phi));
+                      (const SgtState *)J->st, J->W));
     CK(launch_chain(pdl, k_fft_cols<D, MODE_LAST>, J->nb_fft, SGT_THREADS, J->smem_fft2, s,
-                    (const SgtState *)J->st, J->W, (const NT *)J->V, (NT *)J->Phi));
+                    (const SgtState *)J->st, J->W));
     if constexpr (D == 3)
       CK(launch_chain(pdl, k_fft_cols<D, MODE_MID_INV>, J->nb_fft, SGT_THREADS, J->smem_fft2, s,
-                      (const SgtState *)J->st, J->W, (const NT *)J->V, (NT *)J->Phi));
+                      (const SgtState *)J->st, J->W));
     CK(launch_chain(pdl, k_fft_final_x<D>, J->nb_fft_rows, SGT_THREADS, 0, s,
                     (const SgtState *)J->st, (const float2 *)J->W, (NT *)J->Phi));
   }

@@ -933,9 +933,8 @@ __device__ void cols_body(int vb_, int vg_, const SgtState *st, float2 *__restri
 }
 
 template <int D, int MODE>
-__device__ __forceinline__ void k_fft_cols_body(int vb_, int vg_, const SgtState *st, float2 *__restrict__ W,
-                                                const typename Node<D>::T *__restrict__ V,
-                                                typename Node<D>::T *__restrict__ Phi) {
+__device__ __forceinline__ void k_fft_cols_body(int vb_, int vg_, const SgtState *st,
+                                                float2 *__restrict__ W) {
   sgt_pdl_wait();
   extern __shared__ float2 sm[];
   if (st->direct) return;
@@ -950,9 +949,8 @@ __device__ __forceinline__ void k_fft_cols_body(int vb_, int vg_, const SgtState
 }
 template <int D, int MODE>
 __global__ void __launch_bounds__(SGT_THREADS)
-k_fft_cols(const SgtState *st, float2 *__restrict__ W, const typename Node<D>::T *__restrict__ V,
-           typename Node<D>::T *__restrict__ Phi) {
-  k_fft_cols_body<D, MODE>(blockIdx.x, gridDim.x, st, W, V, Phi);
+k_fft_cols(const SgtState *st, float2 *__restrict__ W) {
+  k_fft_cols_body<D, MODE>(blockIdx.x, gridDim.x, st, W);
 }
 
 // ---------------------------------------------------------------------------

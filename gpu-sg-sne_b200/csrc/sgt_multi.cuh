@@ -121,8 +121,7 @@ template <int D, int MODE>
 __global__ void __launch_bounds__(SGT_THREADS)
 km_fft_cols(const SgtJobView *__restrict__ views, const int *__restrict__ prefix, int njobs) {
   SGT_MULTI_JOB
-  k_fft_cols_body<D, MODE>(vb, vg, v.st, v.W, (const typename Node<D>::T *)v.V,
-                           (typename Node<D>::T *)v.Phi);
+  k_fft_cols_body<D, MODE>(vb, vg, v.st, v.W);
 }
 
 template <int D>
