@@ -919,14 +919,7 @@ extern "C" sgt_status sgt_knn_ex(sgt_ctx *ctx, int n, int dim, const float *X, i
     return sgti_fail(ctx, SGT_ERR_CUDA, "sgt_knn: set device");
   if (n_redo) *n_redo = 0;
   sgt_status st;
-  // The automatic choice takes the filter for any width and k where its
-  // set-up of 50 us and the re-ranking of whole blocks of 128 queries are less
-  // than the SIMT search's serial list updates (filter against SIMT search,
-  // us): 256 points 10-D k = 15 175 / 267, 50-D k = 30 204 / 1912, 784-D
-  // k = 90 952 / 6537; 1024 points 3-D k = 4 274 / 256, 50-D k = 30
-  // 301 / 5745; 128 points 10-D k = 15 158 / 154.
-  const int n_min = k >= 10 ? 256 : 1024;
-  if (method == SGT_KNN_TENSOR || (method == SGT_KNN_AUTO && n >= n_min && n <= (1 << 28))) {
+  if (method == SGT_KNN_TENSOR || (method == SGT_KNN_AUTO && n >= sgt_knn_min_n(dim, k) && n <= (1 << 28))) {
     st = knn_tc(ctx, n, dim, X, k, idx, d2, n_redo);
     // the filter's operand images (about 8 bytes per point and dimension)
     // did not fit: the automatic choice falls back to the SIMT search

@@ -1,13 +1,15 @@
 // sgt_knn_rules.h -- what the tensor-core kNN filter (sgt_knn.cu) decides by
 // arithmetic alone: the error bound of its keys, the rounding of the distances
-// it returns, and the places in its pipeline.  Plain C++, so that a CPU model
-// can run the same code.
+// it returns, the points it is chosen from, and the places in its pipeline.
+// Plain C++, so that a CPU model can run the same code.
 #pragma once
 
+#ifndef SGT_RULE
 #ifdef __CUDACC__
 #define SGT_RULE __host__ __device__ __forceinline__
 #else
 #define SGT_RULE inline
+#endif
 #endif
 
 // Bound on the error of 2 key = |q|^2 - d^2, relative to A = |q|^2 + max |c|^2.
@@ -34,6 +36,17 @@ SGT_RULE float sgt_knn_eps(int dim, bool exact) {
 // rounded difference (twice in its square) and one rounded multiply-add, all
 // terms of one sign: (dim + 2) 2^-24.
 SGT_RULE float sgt_knn_gamma(int dim) { return (float)(dim + 3) * 6.0e-8f; }
+
+// Points from which the automatic choice takes the filter, for any width and k:
+// where its set-up of 50 us and the re-ranking of whole blocks of 128 queries are
+// less than the SIMT search's serial list updates. us, filter / SIMT search: 256
+// points 10-D k = 15 175 / 267, 50-D k = 30 204 / 1912, 784-D k = 90 952 / 6537; 128
+// points 10-D k = 15 158 / 154. Short lists of few dimensions update little: 1024
+// points 2-D k = 1 276 / 192, k = 4 274 / 262, k = 9 273 / 430; 1500 k = 1 288 / 273,
+// k = 4 297 / 347; 2048 k = 1 334 / 360; 1024 points 50-D k = 1 309 / 337.
+SGT_RULE int sgt_knn_min_n(int dim, int k) {
+  return k >= 10 ? 256 : 1024 + (dim < 32 && k < 5 ? 150 * (5 - k) : 0);
+}
 
 // Place in a ring of buffers whose mbarriers complete one phase per use: the
 // buffer and the parity of its present use's phase, carried along.  (Taken from

@@ -463,9 +463,9 @@ sgt_status sgt_knn(sgt_ctx *ctx, int n, int dim, const float *X, int k, int *idx
      query, re-ranked with the SIMT arithmetic; queries whose list could miss
      a neighbour under the filter's error bound are redone by the SIMT search.
    SGT_KNN_AUTO: the tensor-core filter, for any dim and k, from n = 256
-     (1024 for k < 10); the SIMT search below, or when the filter's operand
-     images (about 8 bytes per point and dimension) do not fit in device
-     memory. */
+     (1024 for k < 10, up to 1624 for k < 5 and dim < 32); the SIMT search
+     below, or when the filter's operand images (about 8 bytes per point and
+     dimension) do not fit in device memory. */
 enum { SGT_KNN_AUTO = 0, SGT_KNN_SIMT = 1, SGT_KNN_TENSOR = 2 };
 
 /* sgt_knn with a method; *n_redo (may be NULL) receives the number of

@@ -1,5 +1,6 @@
-"""The rules by which a grid's size picks the form of the repulsion
-(gpu-sg-sne_b200/csrc/sgt_grid_rules.h, compiled from that file) against
+"""The rules by which a grid's size picks the form of the repulsion and the
+points' number that of the kNN search (gpu-sg-sne_b200/csrc/sgt_grid_rules.h and
+sgt_knn_rules.h, compiled from those files) against
 measurements: where one form took a tenth longer than the other on a B200, the
 rule must not pick it.  Times are us per iteration of CSR jobs with k = 30.
 """
@@ -43,7 +44,8 @@ CONV = [
 def rules(tmp_path_factory):
     d = tmp_path_factory.mktemp("rules")
     src = d / "r.cpp"
-    src.write_text('#include "sgt_grid_rules.h"\n'
+    src.write_text('#include "sgt_grid_rules.h"\n#include "sgt_knn_rules.h"\n'
+                   'extern "C" int knn_min_n(int dim, int k) { return sgt_knn_min_n(dim, k); }\n'
                    'extern "C" int cell(int d, long n, long ncell) {\n'
                    '  return n >= sgt_cell_min_n(d) && sgt_cell_mode(n, ncell, SGT_CELL_DENSE);\n'
                    '}\n'
@@ -111,3 +113,15 @@ def test_grid_copies(rules, d, n, N, us):
         return c
     picked = [t for per, t in us.items() if copies(per) == rules.copies(d, n, N)]
     assert picked and min(picked) <= 1.06 * min(us.values())
+
+
+# (dim, k, points, us of the filter, us of the SIMT search)
+@pytest.mark.parametrize("dim,k,n,tensor,simt", [
+    (2, 1, 1024, 276, 192), (2, 1, 1500, 288, 273), (2, 1, 2048, 334, 360), (2, 4, 1024, 274, 262),
+    (2, 4, 1500, 297, 347), (2, 9, 1024, 273, 430), (2, 10, 256, 175, 183), (10, 1, 1024, 285, 216),
+    (10, 1, 2048, 346, 407), (10, 4, 1500, 308, 394), (10, 15, 256, 178, 281),
+    (50, 1, 1024, 309, 337), (50, 4, 1024, 311, 438), (50, 10, 256, 202, 237),
+    (784, 10, 256, 483, 959),
+])
+def test_choice_of_the_knn_search(rules, dim, k, n, tensor, simt):
+    assert (tensor if n >= rules.knn_min_n(dim, k) else simt) <= 1.05 * min(tensor, simt)

@@ -16,11 +16,22 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("kind,dim,k", [("sums", 784, 15), ("sums3", 784, 15), ("sums", 1100, 20),
                                         ("offset", 16, 10), ("offset", 300, 40)])
 def test_auto_equals_simt_where_norms_are_large(kind, dim, k):
+    both_searches(model.points(kind, dim, np.random.default_rng(799)), k)
+
+
+@pytest.mark.parametrize("n,dim,k", [(1623, 2, 1), (1624, 2, 1), (1474, 31, 2), (1174, 3, 4),
+                                     (1024, 32, 1), (1024, 4, 5)])
+def test_auto_equals_simt_at_its_least_points(n, dim, k):
+    rng = np.random.default_rng(n + dim)
+    X = (rng.standard_normal((8, dim)) * 4)[rng.integers(0, 8, n)] + rng.standard_normal((n, dim))
+    both_searches(np.ascontiguousarray(X, np.float32), k)
+
+
+def both_searches(X, k):
     import torch
 
     import sgtsne_b200 as S
-    X = model.points(kind, dim, np.random.default_rng(799))
-    n = len(X)
+    n, dim = X.shape
     Xd = torch.from_numpy(X).cuda()
     ctx = S.Context(0)
     out = []
